@@ -821,13 +821,6 @@ __global__ void k_frontier_init(i64 n, const C* A, const C* totals, int k, const
         block_append(static_cast<int>(v), boundary, f.rows, f.count);
     }
 }
-// Repair donors that are not in the frontier must read as non-proposers
-// (target -1) in the next LP round, as after a proposal pass over all rows.
-__global__ void k_reset_targets(i64 count, const u32* donors, int* targets) {
-    const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < count) targets[donors[i]] = -1;
-}
-
 // Heavy candidates: partial corrections per chunk, then the decision
 // (incremental_heavy_priority / incremental_finish_heavy_priority,
 // incremental.cuh:395-438).
@@ -1050,14 +1043,13 @@ __global__ void k_compact_movers(LpParams q, u32* state, u64* entries) {
 
 // incremental_commit (incremental.cuh:532-547) with per-block aggregation of
 // the part-load changes.
-// Also keeps rlabels (the labels in repair order, rposition[v] the place of
-// v) current and clears each mover's flag.  The last block to finish (a
+// Also clears each mover's flag.  The last block to finish (a
 // counter that every block increments once after its load changes; that
 // block resets it for the next launch) writes the largest part load to
 // *max_load, so no separate launch reads the loads back.
 __global__ void k_commit(i64 count, const int* movers, const u64* live_count, int* labels, const int* targets,
-                         const u32* vw, int k, u64* loads, unsigned char* locks, int* flags, const u32* rposition,
-                         int* rlabels, u32* state, u64* max_load, unsigned int* blocks_done) {
+                         const u32* vw, int k, u64* loads, unsigned char* locks, int* flags, u32* state,
+                         u64* max_load, unsigned int* blocks_done) {
     extern __shared__ long long diff[];
     __shared__ bool last;
     if (live_count) count = static_cast<i64>(*live_count);
@@ -1070,7 +1062,6 @@ __global__ void k_commit(i64 count, const int* movers, const u64* live_count, in
         atomicAdd(reinterpret_cast<u64*>(diff + s), static_cast<u64>(-w));
         atomicAdd(reinterpret_cast<u64*>(diff + t), static_cast<u64>(w));
         labels[v] = t;
-        rlabels[rposition[v]] = t;
         if (state) state[v] = static_cast<u32>(t);
         if (locks) locks[v] = 1;
         flags[v] = 0;
@@ -1126,8 +1117,10 @@ __device__ int gain_bucket(u64 best, u64 current, u64 relief) {
 // initialize_receiver_slack (rebalance_select.cuh:79-104) by one thread.
 // One thread per part; the CDF is a saturating prefix sum over the parts.
 __device__ __forceinline__ u64 saturating_add(u64 a, u64 b) { return ~0ULL - a < b ? ~0ULL : a + b; }
+// Also clears the iteration's three counts (placed donors, donors, listed
+// donors).
 __global__ void __launch_bounds__(kMaxParts) k_slack(int k, const u64* loads, u64 capacity, u64* slack, u64* requests,
-                                                     u64* cdf) {
+                                                     u64* cdf, u64* counts) {
     __shared__ u64 warp_total[kMaxParts / 32], warp_min[kMaxParts / 32];
     const int p = threadIdx.x, lane = p & 31, warp = p >> 5;
     const u64 room = p < k ? (loads[p] < capacity ? capacity - loads[p] : 0) : 0;
@@ -1149,6 +1142,7 @@ __global__ void __launch_bounds__(kMaxParts) k_slack(int k, const u64* loads, u6
         requests[p] = 0;
         cdf[p] = saturating_add(before, inc);
     }
+    if (p < 3) counts[p] = 0;
     if (p == 0) {
         u64 m = ~0ULL;
         for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) m = warp_min[w] < m ? warp_min[w] : m;
@@ -1156,28 +1150,18 @@ __global__ void __launch_bounds__(kMaxParts) k_slack(int k, const u64* loads, u6
     }
 }
 
-// Position i of the repair order is a donor when its vertex's part is
-// overloaded; rlabels holds the labels in repair order, so this reads
-// sequentially.
-struct IsDonor {
-    const int* rlabels;
-    const u64* loads;
-    u64 capacity;
-    __device__ bool operator()(i64 i) const { return loads[rlabels[i]] > capacity; }
-};
-// Labels in repair order, and each vertex's position in that order.
-__global__ void k_repair_positions(i64 n, const u32* order, const int* labels, u32* position, int* rlabels) {
-    const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const u32 v = order[i];
-    position[v] = static_cast<u32>(i);
-    rlabels[i] = labels[v];
+// A donor's plan of one repair iteration, one word per vertex: its order
+// class (gain bucket * 16 + section, below kBalanceWidth) in the low half,
+// its destination in the high half; kNoPlan without a destination.
+constexpr u32 kNoPlan = 0xffffffffU;
+__device__ __forceinline__ int plan_class(u32 plan) { return static_cast<int>(plan & 0xffffu); }
+__device__ __forceinline__ int plan_part(u32 plan) { return plan == kNoPlan ? -1 : static_cast<int>(plan >> 16); }
+__device__ __forceinline__ u32 make_plan(int v, int part, u64 conn, u64 current, u64 weight, u64 excess) {
+    if (part < 0) return kNoPlan;
+    const u64 relief = weight < excess ? weight : excess;
+    return static_cast<u32>(gain_bucket(conn, current, relief) * 16) + mix32(static_cast<u32>(v)) % 16 +
+           (static_cast<u32>(part) << 16);
 }
-struct WriteOrdered {
-    const u32* order;
-    u32* out;
-    __device__ void operator()(u32 slot, i64 i) const { out[slot] = order[i]; }
-};
 
 // Loads N consecutive affinities of a row (one 16-byte load when N > 1).
 template <class C, int N>
@@ -1193,98 +1177,121 @@ __device__ __forceinline__ void load_affinities(const C* p, C (&val)[N]) {
 
 // enumerate_repair_destination (rebalance_select.cuh:9-75), dense layout, plus
 // the bucket of incremental_rebalance_proposals (incremental.cuh:559-622).
-// W lanes per donor; the parts' free room is staged per block.  A part p is a
-// feasible destination for weight w when w <= room[p] (room = C - load for
-// parts under capacity, else 0; vertex weights are positive).
+// A warp takes 32 consecutive vertices, its lanes find the donors among them
+// (vertices of overloaded parts) and W lanes scan each donor's row; the parts'
+// free room is staged per block.  A part p is a feasible destination for
+// weight w when w <= room[p] (room = C - load for parts under capacity, else
+// 0; vertex weights are positive).  Every donor's weight is added to its
+// class of its part in `hist` (kBalanceWidth per part), from which
+// k_repair_bounds finds how far down the classes the part gives vertices up.
+//
+// Donors are met in vertex order, not in repair order: a level's parts are
+// mostly runs of nearby vertices, so labels, weights and rows are read nearly
+// in sequence, and no array in repair order has to exist.  On the 256^3 mesh
+// at k = 128 (100 M donors over 32 iterations at the finest level) reading the
+// destinations in hashed order took 37 ms and ordering the donors by class
+// with a radix sort about 20 ms more; a partition went from 202 to 189 ms, one
+// of a 256x256 grid at k = 8 from 20.1 to 16.0 ms.
 template <class C, int W, bool Vectorized>
-__global__ void __launch_bounds__(kThreads) k_repair_dest(i64 count, const u32* donors, const C* A, const C* totals,
-                                                          const int* labels, const u32* vw, int k, const u64* loads,
-                                                          u64 capacity, const u64* cdf, int* targets, u64* bucket_keys) {
+__global__ void __launch_bounds__(kThreads) k_repair_dest(i64 n, const C* A, const C* totals, const int* labels,
+                                                          const u32* vw, int k, const u64* loads, u64 capacity,
+                                                          const u64* cdf, u32* plan, u64* hist, u64* donor_count) {
     constexpr int N = Vectorized ? AffinityVec<C>::N : 1;
     constexpr int G = 32 / W;
-    __shared__ u64 s_room[kMaxParts];
-    for (int p = threadIdx.x; p < k; p += blockDim.x) s_room[p] = loads[p] < capacity ? capacity - loads[p] : 0;
+    __shared__ u64 s_room[kMaxParts], s_excess[kMaxParts];
+    for (int p = threadIdx.x; p < k; p += blockDim.x) {
+        s_room[p] = loads[p] < capacity ? capacity - loads[p] : 0;
+        s_excess[p] = loads[p] > capacity ? loads[p] - capacity : 0;
+    }
     __syncthreads();
     const int lane = threadIdx.x & 31, gid = lane / W, sub = lane % W;
-    const i64 warps = (static_cast<i64>(gridDim.x) * blockDim.x) >> 5;
     const int span = (k + W - 1) / W;  // contiguous parts per lane for the fallback ticket
-    for (i64 i0 = ((static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * G; i0 < count; i0 += warps * G) {
-        const i64 i = i0 + gid;
-        const bool valid = i < count;
-        const int v = valid ? static_cast<int>(donors[i]) : 0;
-        const int src = valid ? labels[v] : 0;
-        const u64 w = valid ? vw[v] : 0;
-        const u64 current = valid ? static_cast<u64>(A[static_cast<i64>(v) * k + src]) : 0;
-        const bool scan = valid && current != static_cast<u64>(totals[v]);
-        int part = -1;
-        u64 conn = 0, best_room = 0;
-        if (scan) {
-            const C* row = A + static_cast<i64>(v) * k;
-            for (int p0 = sub * N; p0 < k; p0 += W * N) {
-                C val[N];
-                load_affinities<C, N>(row + p0, val);
+    u64 donors = 0;
+    for (i64 base = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) & ~31LL; base < n;
+         base += static_cast<i64>(gridDim.x) * blockDim.x) {
+        const int own = base + lane < n ? labels[base + lane] : -1;
+        unsigned pending = __ballot_sync(0xffffffffu, own >= 0 && s_excess[own < 0 ? 0 : own] != 0);
+        if (lane == 0) donors += __popc(pending);
+        while (pending) {
+            unsigned mine = pending;
+            for (int q = 0; q < gid; ++q) mine &= mine - 1;
+            for (int q = 0; q < G; ++q) pending &= pending - 1;
+            const bool valid = mine != 0;
+            const int owner = valid ? __ffs(mine) - 1 : 0;
+            const int v = static_cast<int>(base) + owner;
+            const int src = __shfl_sync(0xffffffffu, own, owner);
+            const u64 w = valid ? vw[v] : 0;
+            const u64 current = valid ? static_cast<u64>(A[static_cast<i64>(v) * k + src]) : 0;
+            const bool scan = valid && current != static_cast<u64>(totals[v]);
+            int part = -1;
+            u64 conn = 0, best_room = 0;
+            if (scan) {
+                const C* row = A + static_cast<i64>(v) * k;
+                for (int p0 = sub * N; p0 < k; p0 += W * N) {
+                    C val[N];
+                    load_affinities<C, N>(row + p0, val);
 #pragma unroll
-                for (int e = 0; e < N; ++e) {
-                    const int p = p0 + e;
-                    const u64 room = s_room[p];
-                    if (p == src || w > room) continue;
-                    const u64 value = val[e];
-                    if (part < 0 || value > conn || (value == conn && room > best_room)) { part = p; conn = value; best_room = room; }
+                    for (int e = 0; e < N; ++e) {
+                        const int p = p0 + e;
+                        const u64 room = s_room[p];
+                        if (p == src || w > room) continue;
+                        const u64 value = val[e];
+                        if (part < 0 || value > conn || (value == conn && room > best_room)) { part = p; conn = value; best_room = room; }
+                    }
                 }
             }
-        }
 #pragma unroll
-        for (int d = W / 2; d; d >>= 1) {
-            const int op = __shfl_xor_sync(0xffffffffu, part, d, W);
-            const u64 oc = __shfl_xor_sync(0xffffffffu, conn, d, W);
-            const u64 orm = __shfl_xor_sync(0xffffffffu, best_room, d, W);
-            if (op >= 0 && (part < 0 || oc > conn || (oc == conn && (orm > best_room || (orm == best_room && op < part))))) {
-                part = op; conn = oc; best_room = orm;
+            for (int d = W / 2; d; d >>= 1) {
+                const int op = __shfl_xor_sync(0xffffffffu, part, d, W);
+                const u64 oc = __shfl_xor_sync(0xffffffffu, conn, d, W);
+                const u64 orm = __shfl_xor_sync(0xffffffffu, best_room, d, W);
+                if (op >= 0 && (part < 0 || oc > conn || (oc == conn && (orm > best_room || (orm == best_room && op < part))))) {
+                    part = op; conn = oc; best_room = orm;
+                }
             }
-        }
-        if (!conn) part = -1;
-        // Fallback ticket over the parts' room when no connected destination
-        // fits: from the slack CDF when the source is at capacity, else over
-        // the parts that fit w, in part order (saturating sums).
-        const bool ticket = valid && part < 0 && !(loads[src] >= capacity && w <= cdf[k]);
-        const u32 hash = mix32(static_cast<u32>(v));
-        if (__any_sync(0xffffffffu, ticket)) {
-            const int lo = sub * span, hi = min(k, lo + span);
-            u64 mine = 0;
-            if (ticket)
-                for (int p = lo; p < hi; ++p)
-                    if (p != src && w <= s_room[p]) mine = ~0ULL - mine < s_room[p] ? ~0ULL : mine + s_room[p];
-            u64 upto = mine;  // inclusive scan over the group, saturating
-#pragma unroll
-            for (int d = 1; d < W; d <<= 1) {
-                const u64 o = __shfl_up_sync(0xffffffffu, upto, d, W);
-                if (sub >= d) upto = ~0ULL - upto < o ? ~0ULL : upto + o;
-            }
-            const u64 total = __shfl_sync(0xffffffffu, upto, W - 1, W);
-            // Exclusive prefix, saturated: exact for the lane holding the
-            // ticket (ticket < total), above the ticket for every later lane.
-            const u64 prev = __shfl_up_sync(0xffffffffu, upto, 1, W);
-            const u64 before = sub == 0 ? 0 : prev;
-            int found = -1;
-            if (ticket && total) {
-                u64 t = static_cast<u64>(hash) % total;
-                if (t >= before && (t - before) < mine) {
-                    t -= before;
+            if (!conn) part = -1;
+            // Fallback ticket over the parts' room when no connected destination
+            // fits: from the slack CDF when the source is at capacity, else over
+            // the parts that fit w, in part order (saturating sums).
+            // (A donor's part is over capacity.)
+            const bool ticket = valid && part < 0 && w > cdf[k];
+            const u32 hash = mix32(static_cast<u32>(v));
+            if (__any_sync(0xffffffffu, ticket)) {
+                const int lo = sub * span, hi = min(k, lo + span);
+                u64 mine = 0;
+                if (ticket)
                     for (int p = lo; p < hi; ++p)
-                        if (p != src && w <= s_room[p]) {
-                            if (t < s_room[p]) { found = p; break; }
-                            t -= s_room[p];
-                        }
-                }
-            }
+                        if (p != src && w <= s_room[p]) mine = ~0ULL - mine < s_room[p] ? ~0ULL : mine + s_room[p];
+                u64 upto = mine;  // inclusive scan over the group, saturating
 #pragma unroll
-            for (int d = W / 2; d; d >>= 1) found = max(found, __shfl_xor_sync(0xffffffffu, found, d, W));
-            if (ticket) part = found;
-        }
-        if (valid && sub == 0) {
-            if (part < 0 && !ticket) {
-                conn = 0;
-                if (loads[src] >= capacity && w <= cdf[k]) {
+                for (int d = 1; d < W; d <<= 1) {
+                    const u64 o = __shfl_up_sync(0xffffffffu, upto, d, W);
+                    if (sub >= d) upto = ~0ULL - upto < o ? ~0ULL : upto + o;
+                }
+                const u64 total = __shfl_sync(0xffffffffu, upto, W - 1, W);
+                // Exclusive prefix, saturated: exact for the lane holding the
+                // ticket (ticket < total), above the ticket for every later lane.
+                const u64 prev = __shfl_up_sync(0xffffffffu, upto, 1, W);
+                const u64 before = sub == 0 ? 0 : prev;
+                int found = -1;
+                if (ticket && total) {
+                    u64 t = static_cast<u64>(hash) % total;
+                    if (t >= before && (t - before) < mine) {
+                        t -= before;
+                        for (int p = lo; p < hi; ++p)
+                            if (p != src && w <= s_room[p]) {
+                                if (t < s_room[p]) { found = p; break; }
+                                t -= s_room[p];
+                            }
+                    }
+                }
+#pragma unroll
+                for (int d = W / 2; d; d >>= 1) found = max(found, __shfl_xor_sync(0xffffffffu, found, d, W));
+                if (ticket) part = found;
+            }
+            if (valid && sub == 0) {
+                if (part < 0 && !ticket) {
+                    conn = 0;
                     const u64 sum = cdf[k - 1];
                     if (sum) {
                         const u64 t = static_cast<u64>(hash) % sum;
@@ -1293,35 +1300,36 @@ __global__ void __launch_bounds__(kThreads) k_repair_dest(i64 count, const u32* 
                         part = lo;
                     }
                 }
+                if (ticket) conn = 0;
+                const u32 word = make_plan(v, part, conn, current, w, s_excess[src]);
+                plan[v] = word;
+                if (part >= 0) atomicAdd(hist + src * kBalanceWidth + plan_class(word), w);
             }
-            if (ticket) conn = 0;
-            targets[v] = part;
-            u64 key = ~0ULL;
-            if (part >= 0) {
-                const u64 excess = loads[src] - capacity;
-                const u64 relief = w < excess ? w : excess;
-                key = static_cast<u64>(src) * kBalanceWidth + gain_bucket(conn, current, relief) * 16 +
-                      mix32(static_cast<u32>(v)) % 16;
-            }
-            bucket_keys[i] = key;
         }
     }
+    block_atomic_add(donor_count, donors);
 }
 
-// k_repair_dest with on-demand affinities, one thread per donor: the best
+// k_repair_dest with on-demand affinities, one thread per vertex: the best
 // connected destination with room (largest affinity, then room, then lowest
 // part), else the same fallback tickets.
 template <int D>
-__global__ void __launch_bounds__(kThreads) k_repair_dest_od(i64 count, const u32* donors, const int* off,
-                                                             const int* nbr, const u32* ew, const int* labels,
-                                                             const u32* vw, int k, const u64* loads, u64 capacity,
-                                                             const u64* cdf, int* targets, u64* bucket_keys) {
-    __shared__ u64 s_room[kMaxParts];
-    for (int p = threadIdx.x; p < k; p += blockDim.x) s_room[p] = loads[p] < capacity ? capacity - loads[p] : 0;
+__global__ void __launch_bounds__(kThreads) k_repair_dest_od(i64 n, const int* off, const int* nbr, const u32* ew,
+                                                             const int* labels, const u32* vw, int k, const u64* loads,
+                                                             u64 capacity, const u64* cdf, u32* plan, u64* hist,
+                                                             u64* donor_count) {
+    __shared__ u64 s_room[kMaxParts], s_excess[kMaxParts];
+    for (int p = threadIdx.x; p < k; p += blockDim.x) {
+        s_room[p] = loads[p] < capacity ? capacity - loads[p] : 0;
+        s_excess[p] = loads[p] > capacity ? loads[p] - capacity : 0;
+    }
     __syncthreads();
-    for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += static_cast<i64>(gridDim.x) * blockDim.x) {
-        const int v = static_cast<int>(donors[i]);
+    u64 donors = 0;
+    for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += static_cast<i64>(gridDim.x) * blockDim.x) {
+        const int v = static_cast<int>(i);
         const int src = labels[v];
+        if (!s_excess[src]) continue;
+        ++donors;
         const u64 w = vw[v];
         RowRegs<D> r;
         r.load(v, off, nbr, ew, labels);
@@ -1344,7 +1352,7 @@ __global__ void __launch_bounds__(kThreads) k_repair_dest_od(i64 count, const u3
         if (part < 0) {
             conn = 0;
             const u32 hash = mix32(static_cast<u32>(v));
-            if (loads[src] >= capacity && w <= cdf[k]) {
+            if (w <= cdf[k]) {  // a donor's part is over capacity
                 const u64 sum = cdf[k - 1];
                 if (sum) {
                     const u64 t = static_cast<u64>(hash) % sum;
@@ -1366,15 +1374,11 @@ __global__ void __launch_bounds__(kThreads) k_repair_dest_od(i64 count, const u3
                 }
             }
         }
-        targets[v] = part;
-        u64 key = ~0ULL;
-        if (part >= 0) {
-            const u64 excess = loads[src] - capacity;
-            const u64 relief = w < excess ? w : excess;
-            key = static_cast<u64>(src) * kBalanceWidth + gain_bucket(conn, current, relief) * 16 + mix32(static_cast<u32>(v)) % 16;
-        }
-        bucket_keys[i] = key;
+        const u32 word = make_plan(v, part, conn, current, w, s_excess[src]);
+        plan[v] = word;
+        if (part >= 0) atomicAdd(hist + src * kBalanceWidth + plan_class(word), w);
     }
+    block_atomic_add(donor_count, donors);
 }
 
 // Receiver choice of one donor with on-demand affinities (k_choose, attempt
@@ -1402,7 +1406,7 @@ __device__ __forceinline__ int choose_od(int v, const int* off, const int* nbr, 
 template <int D>
 __global__ void __launch_bounds__(kThreads) k_choose_od(i64 count, const u32* active, int attempt, const int* off,
                                                         const int* nbr, const u32* ew, const int* labels,
-                                                        const u32* vw, int k, const int* proposal, const u64* slack,
+                                                        const u32* vw, int k, const u32* plan, const u64* slack,
                                                         const u64* requests, const u64* tried, unsigned char* state,
                                                         int* want, u64* requesters) {
     __shared__ u64 s_avail[kMaxParts];
@@ -1415,7 +1419,7 @@ __global__ void __launch_bounds__(kThreads) k_choose_od(i64 count, const u32* ac
             continue;
         }
         const int v = static_cast<int>(active[i]);
-        const int target = attempt == 0 ? proposal[v]
+        const int target = attempt == 0 ? plan_part(plan[v])
                                         : choose_od<D>(v, off, nbr, ew, labels, k, vw[v], tried[2 * i], tried[2 * i + 1], s_avail);
         want[i] = target;
         if (target < 0) state[i] = 2;
@@ -1424,46 +1428,82 @@ __global__ void __launch_bounds__(kThreads) k_choose_od(i64 count, const u32* ac
     block_atomic_add(requesters, asked);
 }
 
-constexpr u64 kNoBucket = 0xffffffULL;  // donors without a destination sort last
-
-__global__ void k_clamp_keys(i64 count, u64* keys) {
-    const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < count && keys[i] > kNoBucket) keys[i] = kNoBucket;
+// A part gives up donors in the order (class, repair hash, id) until the
+// weight given up reaches its excess (reserve_receiver_prefixes' donor test,
+// rebalance_graph.cuh:104-107: a donor is active while the weight of the
+// donors before it is below the excess).  A block per part scans its class
+// weights for the last class that starts below the excess (bound[p], the
+// weight of the classes before it in start[p]; -1 for a part that is not
+// overloaded): classes before it are active whole, classes after it not at
+// all, and only within it the order of the donors matters.  So the donors are
+// never sorted by class; what k_repair_list collects, the active classes and
+// the bounding one, is all that is put in order.  Leaves the weights it read
+// zero for the next iteration.
+__global__ void __launch_bounds__(kScanThreads) k_repair_bounds(const u64* loads, u64 capacity, u64* hist, int* bound,
+                                                                u64* start) {
+    constexpr int kPer = 4;
+    static_assert(kScanThreads * kPer >= kBalanceWidth, "one pass over a part's classes");
+    __shared__ u64 smem[9];
+    const int p = blockIdx.x;
+    if (loads[p] <= capacity) {
+        if (threadIdx.x == 0) bound[p] = -1;
+        return;
+    }
+    const u64 excess = loads[p] - capacity;
+    u64* row = hist + static_cast<i64>(p) * kBalanceWidth;
+    u64 w[kPer], local = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const int c = threadIdx.x * kPer + j;
+        w[j] = c < kBalanceWidth ? row[c] : 0;
+        if (c < kBalanceWidth) row[c] = 0;
+        local += w[j];
+    }
+    u64 total;
+    u64 before = block_exclusive_scan<u64>(local, total, smem);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const int c = threadIdx.x * kPer + j;
+        if (c < kBalanceWidth && before < excess && (c == kBalanceWidth - 1 || before + w[j] >= excess)) {
+            bound[p] = c;
+            start[p] = before;
+        }
+        before += w[j];
+    }
 }
-__global__ void k_repair_keys(i64 n, u64* keys, u32* order) {
-    const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (v >= n) return;
-    keys[v] = repair_hash(static_cast<int>(v));
-    order[v] = static_cast<u32>(v);
+
+// The donors up to their part's bounding class, unordered: repair hash in the
+// high half, vertex in the low half.  The hash is a bijection of the vertex
+// id, so ordering the words is the repair order (ascending hash, then id).
+__global__ void __launch_bounds__(kThreads) k_repair_list(i64 n, int k, const int* labels, const u32* plan,
+                                                          const int* bound, u64* list, u64* count) {
+    __shared__ int s_bound[kMaxParts];
+    for (int p = threadIdx.x; p < k; p += blockDim.x) s_bound[p] = bound[p];
+    __syncthreads();
+    for (i64 base = static_cast<i64>(blockIdx.x) * blockDim.x; base < n; base += static_cast<i64>(gridDim.x) * blockDim.x) {
+        const i64 v = base + threadIdx.x;
+        const int last = v < n ? s_bound[labels[v]] : -1;
+        const u32 word = last >= 0 ? plan[v] : kNoPlan;
+        const bool take = word != kNoPlan && plan_class(word) <= last;
+        if (!__syncthreads_or(take)) continue;
+        block_append((static_cast<u64>(repair_hash(static_cast<int>(v))) << 32) | static_cast<u64>(v), take, list, count);
+    }
 }
 
-struct SortedWeight {
-    const u32* items;
-    const u32* vw;
-    __device__ u64 operator()(i64 i) const { return vw[items[i]]; }
-};
-
-// Segment base per source part over the bucket-sorted donors.
-__global__ void k_part_heads(i64 count, const u64* keys, const u64* prefix, u64* part_base) {
-    const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= count || keys[i] == kNoBucket) return;
-    const u64 part = keys[i] / kBalanceWidth;
-    if (i == 0 || keys[i - 1] / kBalanceWidth != part) part_base[part] = prefix[i];
-}
-// reserve_receiver_prefixes' donor test (rebalance_graph.cuh:104-107).
-__global__ void k_donor_test(i64 count, const u64* keys, const u32* items, const u64* prefix, const u64* part_base,
-                             const u64* loads, u64 capacity, unsigned char* active) {
+// A long list, sorted: vertex and, for the donors of a bounding class, the
+// part whose weight their order counts (-1 for the others).
+__global__ void k_repair_unpack(i64 count, const u64* list, const int* labels, const u32* plan, const int* bound,
+                                u32* items, int* want) {
     const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    const int v = static_cast<int>(items[i]);
-    if (keys[i] == kNoBucket) { active[v] = 0; return; }
-    const u64 part = keys[i] / kBalanceWidth;
-    active[v] = prefix[i] - part_base[part] < loads[part] - capacity;
+    const int v = static_cast<int>(list[i] & 0xffffffffULL);
+    const int src = labels[v];
+    items[i] = static_cast<u32>(v);
+    want[i] = plan_class(plan[v]) == bound[src] ? src : -1;
 }
 struct IsActive {
-    const u32* donors;
     const unsigned char* active;
-    __device__ bool operator()(i64 i) const { return active[donors[i]] != 0; }
+    __device__ bool operator()(i64 i) const { return active[i] != 0; }
 };
 struct WriteFrom {
     const u32* src;
@@ -1477,7 +1517,7 @@ struct WriteFrom {
 // the parts' remaining room is staged per block.
 template <class C, int W, bool Vectorized>
 __global__ void __launch_bounds__(kThreads) k_choose(i64 count, const u32* active, int attempt, const C* A,
-                                                     const int* labels, const u32* vw, int k, const int* proposal,
+                                                     const int* labels, const u32* vw, int k, const u32* plan,
                                                      const u64* slack, const u64* requests, u64* tried,
                                                      unsigned char* state, int* want, u64* requesters) {
     constexpr int N = Vectorized ? AffinityVec<C>::N : 1;
@@ -1496,7 +1536,7 @@ __global__ void __launch_bounds__(kThreads) k_choose(i64 count, const u32* activ
         const int v = open ? static_cast<int>(active[i]) : 0;
         int target = -1;
         if (attempt == 0) {
-            if (open) target = proposal[v];
+            if (open) target = plan_part(plan[v]);
         } else {
             u64 best = 0, room = 0;
             if (open) {
@@ -1634,6 +1674,37 @@ __global__ void k_admit_tiles(i64 count, const int* want, const u32* active, con
     }
     if (threadIdx.x == 0) *blocks_done = 0;
 }
+// The donor test over a long list in repair order, tile by tile as
+// k_admit_tiles orders requests: want[i] is the part whose bounding class
+// donor i is in, offsets the scan of k_part_requests' sums of their weights.
+__global__ void k_repair_active(i64 count, const int* want, const u32* items, const u32* vw, const u64* offsets,
+                                int tiles, const u64* loads, u64 capacity, const u64* start, int k,
+                                unsigned char* active) {
+    constexpr int kWarps = kAdmitTile / 32;
+    __shared__ u64 s_warp[kMaxParts][kWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int x = threadIdx.x; x < k * kWarps; x += blockDim.x) s_warp[x / kWarps][x % kWarps] = 0;
+    __syncthreads();
+    const i64 i = static_cast<i64>(blockIdx.x) * kAdmitTile + threadIdx.x;
+    const int t = i < count ? want[i] : -1;
+    const u64 w = t >= 0 ? vw[items[i]] : 0;
+    const unsigned peers = __match_any_sync(0xffffffffu, t);
+    u64 before = 0, sum = 0;
+    for (unsigned rest = peers; rest; rest &= rest - 1) {
+        const int l = __ffs(rest) - 1;
+        const u64 o = __shfl_sync(peers, w, l);
+        sum += o;
+        if (l < lane) before += o;
+    }
+    if (t >= 0 && lane == __ffs(peers) - 1) s_warp[t][warp] = sum;
+    __syncthreads();
+    if (t >= 0) {
+        for (int q = 0; q < warp; ++q) before += s_warp[t][q];
+        before += start[t] + offsets[static_cast<i64>(t) * tiles + blockIdx.x] - offsets[static_cast<i64>(t) * tiles];
+    }
+    if (i < count) active[i] = t < 0 || before < loads[t] - capacity;
+}
+
 // The remaining attempts of a receiver reservation by one block, for a small
 // set of open donors: the choice of k_choose and the ticket rule of k_admit,
 // attempt after attempt, without a round trip to the host.  open[j] (j <
@@ -1666,46 +1737,96 @@ constexpr size_t attempt_smem(int count) {
     return static_cast<size_t>(count) * (2 * sizeof(u64) + (kShortlist + 1) * sizeof(C) + 2 * sizeof(u32) +
                                          4 + kShortlist);
 }
-template <class C, int D>
-__global__ void __launch_bounds__(kAttemptThreads) k_attempts(const u32* open, const u32* count_ptr, int first_attempt,
-                                                              const u32* active, const C* A, const int* off,
-                                                              const int* nbr, const u32* ew, const int* labels,
-                                                              const u32* vw, int k, const int* proposal,
-                                                              const u64* slack, u64* requests, u64* tried,
-                                                              unsigned char* state, int* targets, int* flags) {
-    constexpr int kWarps = kAttemptThreads / 32;
-    __shared__ u64 s_slack[kMaxParts], s_requests[kMaxParts], s_base[kMaxParts], s_avail[kMaxParts];
-    __shared__ u64 s_warp[kMaxParts][kWarps];  // per part, the weight each warp requests
-    __shared__ int s_want[kAttemptCap];
-    __shared__ unsigned char s_order[kMaxParts];  // parts by (room desc, part asc), per attempt
-    __shared__ int s_any;
-    extern __shared__ __align__(16) unsigned char attempt_smem_raw[];
-    const int count = static_cast<int>(*count_ptr);
-    // Per-donor arrays (j < count), widest first.
-    u64* d_tried = reinterpret_cast<u64*>(attempt_smem_raw);          // 2 per donor
-    C* d_list_c = reinterpret_cast<C*>(d_tried + 2 * count);           // kShortlist per donor
-    C* d_bound = d_list_c + kShortlist * count;                         // largest unlisted affinity
-    u32* d_v = reinterpret_cast<u32*>(d_bound + count);
-    u32* d_w = d_v + count;
-    unsigned char* d_src = reinterpret_cast<unsigned char*>(d_w + count);
-    unsigned char* d_state = d_src + count;
-    unsigned char* d_list_n = d_state + count;  // listed parts; kNoPart: no shortlist yet
-    unsigned char* d_bounded = d_list_n + count;  // 1 when some eligible part is unlisted
-    unsigned char* d_list_p = d_bounded + count;  // kShortlist per donor
+// Per-donor arrays (j < count) in dynamic shared memory, widest first.
+template <class C>
+struct AttemptDonors {
+    u64* tried;   // 2 per donor
+    C* list_c;    // kShortlist per donor
+    C* bound;     // largest unlisted affinity
+    u32* v;
+    u32* w;
+    unsigned char* src;
+    unsigned char* state;
+    unsigned char* list_n;   // listed parts; kNoPart: no shortlist yet
+    unsigned char* bounded;  // 1 when some eligible part is unlisted
+    unsigned char* list_p;   // kShortlist per donor
+    __device__ AttemptDonors(unsigned char* raw, int count) {
+        tried = reinterpret_cast<u64*>(raw);
+        list_c = reinterpret_cast<C*>(tried + 2 * count);
+        bound = list_c + kShortlist * count;
+        v = reinterpret_cast<u32*>(bound + count);
+        w = v + count;
+        src = reinterpret_cast<unsigned char*>(w + count);
+        state = src + count;
+        list_n = state + count;
+        bounded = list_n + count;
+        list_p = bounded + count;
+    }
+};
+struct AttemptParts {
+    static constexpr int kWarps = kAttemptThreads / 32;
+    u64 slack[kMaxParts], requests[kMaxParts], base[kMaxParts], avail[kMaxParts];
+    u64 warp[kMaxParts][kWarps];  // per part, the weight each warp requests
+    int want[kAttemptCap];
+    unsigned char order[kMaxParts];  // parts by (room desc, part asc), per attempt
+    int any;
+};
+// For one chunk of the donors (one per thread, in order): turns sm.warp, the
+// weight each warp asks per part, into the weight asked before each warp on
+// top of sm.base, and moves sm.base on.  before: the thread's own start.
+__device__ __forceinline__ u64 order_chunk(AttemptParts& sm, int k, int t, u64 w) {
+    constexpr int kWarps = AttemptParts::kWarps;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int p = threadIdx.x; p < k; p += blockDim.x) { s_slack[p] = slack[p]; s_requests[p] = requests[p]; }
-    for (int j = threadIdx.x; j < count; j += blockDim.x) {
-        const u32 i = open[j];
-        const u32 v = active[i];
-        d_v[j] = v;
-        d_w[j] = vw[v];
-        d_src[j] = static_cast<unsigned char>(labels[v]);
-        d_state[j] = state[i];
-        d_tried[2 * j] = tried[2 * i];
-        d_tried[2 * j + 1] = tried[2 * i + 1];
-        d_list_n[j] = kNoPart;
+    for (int x = threadIdx.x; x < kWarps * k; x += blockDim.x) sm.warp[x / kWarps][x % kWarps] = 0;
+    __syncthreads();
+    const unsigned peers = __match_any_sync(0xffffffffu, t);
+    u64 before = 0, sum = 0;
+    for (unsigned rest = peers; rest; rest &= rest - 1) {
+        const int l = __ffs(rest) - 1;
+        const u64 o = __shfl_sync(peers, w, l);
+        sum += o;
+        if (l < lane) before += o;
+    }
+    if (t >= 0 && lane == __ffs(peers) - 1) sm.warp[t][warp] = sum;
+    __syncthreads();
+    // Warp `warp` scans the parts warp, warp + 32, ... across its lanes (lane
+    // l holds warp l's sum).
+    static_assert(kWarps == 32, "one lane per warp of the block");
+    for (int p = warp; p < k; p += kWarps) {
+        const u64 x = sm.warp[p][lane], base = sm.base[p];
+        u64 inc = x;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const u64 o = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += o;
+        }
+        sm.warp[p][lane] = base + inc - x;
+        __syncwarp();
+        if (lane == 31) sm.base[p] = base + inc;
     }
     __syncthreads();
+    return t >= 0 ? sm.warp[t][warp] + before : 0;
+}
+// The attempts from first_attempt on, until no donor asks: leaves the donors'
+// states and tried parts in `donor` and the requests in sm.requests.
+template <class C, int D>
+__device__ void run_attempts(AttemptParts& sm, const AttemptDonors<C>& donor, int count, int first_attempt, const C* A,
+                             const int* off, const int* nbr, const u32* ew, const int* labels, int k, const u32* plan,
+                             int* targets, int* flags) {
+    u64* d_tried = donor.tried;
+    C* d_list_c = donor.list_c;
+    C* d_bound = donor.bound;
+    u32* d_v = donor.v;
+    u32* d_w = donor.w;
+    unsigned char* d_src = donor.src;
+    unsigned char* d_state = donor.state;
+    unsigned char* d_list_n = donor.list_n;
+    unsigned char* d_bounded = donor.bounded;
+    unsigned char* d_list_p = donor.list_p;
+    u64 *s_slack = sm.slack, *s_requests = sm.requests, *s_avail = sm.avail;
+    unsigned char* s_order = sm.order;
+    int* s_want = sm.want;
+    int& s_any = sm.any;
     for (int attempt = first_attempt; attempt < k; ++attempt) {
         if (threadIdx.x == 0) s_any = 0;
         for (int p = threadIdx.x; p < k; p += blockDim.x)
@@ -1736,7 +1857,7 @@ __global__ void __launch_bounds__(kAttemptThreads) k_attempts(const u32* open, c
                     return !(((p < 64 ? t0 : t1) >> (p & 63)) & 1) && s_avail[p] >= w;
                 };
                 if (attempt == 0) {
-                    target = proposal[v];
+                    target = plan_part(plan[v]);
                 } else if (!A) {  // on-demand affinities
                     target = choose_od<D>(v, off, nbr, ew, labels, k, w, t0, t1, s_avail);
                 } else {
@@ -1849,43 +1970,13 @@ __global__ void __launch_bounds__(kAttemptThreads) k_attempts(const u32* open, c
         // Admission in chunks of one request per thread, in j order: each
         // request starts after the weight requested for its part by earlier
         // requests (earlier chunks, earlier warps, earlier lanes).
-        for (int p = threadIdx.x; p < k; p += blockDim.x) s_base[p] = s_requests[p];
+        for (int p = threadIdx.x; p < k; p += blockDim.x) sm.base[p] = s_requests[p];
         for (int chunk = 0; chunk < count; chunk += blockDim.x) {
-            for (int x = threadIdx.x; x < kWarps * k; x += blockDim.x) s_warp[x / kWarps][x % kWarps] = 0;
-            __syncthreads();
             const int j = chunk + threadIdx.x;
             const int t = j < count ? s_want[j] : -1;
             const u64 w = t >= 0 ? d_w[j] : 0;
-            const unsigned peers = __match_any_sync(0xffffffffu, t);
-            u64 before = 0, sum = 0;
-            for (unsigned rest = peers; rest; rest &= rest - 1) {
-                const int l = __ffs(rest) - 1;
-                const u64 o = __shfl_sync(peers, w, l);
-                sum += o;
-                if (l < lane) before += o;
-            }
-            if (t >= 0 && lane == __ffs(peers) - 1) s_warp[t][warp] = sum;
-            __syncthreads();
-            // Per part, the weight requested before each warp (from the
-            // running base), and the base for the next chunk: warp `warp`
-            // scans the parts warp, warp + 32, ... across its lanes (lane l
-            // holds warp l's sum).
-            static_assert(kWarps == 32, "one lane per warp of the block");
-            for (int p = warp; p < k; p += kWarps) {
-                const u64 x = s_warp[p][lane], base = s_base[p];
-                u64 inc = x;
-#pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const u64 o = __shfl_up_sync(0xffffffffu, inc, d);
-                    if (lane >= d) inc += o;
-                }
-                s_warp[p][lane] = base + inc - x;
-                __syncwarp();
-                if (lane == 31) s_base[p] = base + inc;
-            }
-            __syncthreads();
+            const u64 begin = order_chunk(sm, k, t, w);
             if (t >= 0) {
-                const u64 begin = s_warp[t][warp] + before;
                 d_tried[2 * j + (t >> 6)] |= 1ULL << (t & 63);
                 if (begin <= s_slack[t] && w <= s_slack[t] - begin) {
                     targets[d_v[j]] = t;
@@ -1895,16 +1986,118 @@ __global__ void __launch_bounds__(kAttemptThreads) k_attempts(const u32* open, c
             }
             __syncthreads();
         }
-        for (int p = threadIdx.x; p < k; p += blockDim.x) s_requests[p] = s_base[p];
+        for (int p = threadIdx.x; p < k; p += blockDim.x) s_requests[p] = sm.base[p];
         __syncthreads();
     }
-    for (int p = threadIdx.x; p < k; p += blockDim.x) requests[p] = s_requests[p];
+}
+// The open donors of a long list once few are left.
+template <class C, int D>
+__global__ void __launch_bounds__(kAttemptThreads) k_attempts(const u32* open, const u32* count_ptr, int first_attempt,
+                                                              const u32* active, const C* A, const int* off,
+                                                              const int* nbr, const u32* ew, const int* labels,
+                                                              const u32* vw, int k, const u32* plan,
+                                                              const u64* slack, u64* requests, u64* tried,
+                                                              unsigned char* state, int* targets, int* flags) {
+    __shared__ AttemptParts sm;
+    extern __shared__ __align__(16) unsigned char attempt_smem_raw[];
+    const int count = static_cast<int>(*count_ptr);
+    const AttemptDonors<C> donor(attempt_smem_raw, count);
+    for (int p = threadIdx.x; p < k; p += blockDim.x) { sm.slack[p] = slack[p]; sm.requests[p] = requests[p]; }
     for (int j = threadIdx.x; j < count; j += blockDim.x) {
         const u32 i = open[j];
-        state[i] = d_state[j];
-        tried[2 * i] = d_tried[2 * j];
-        tried[2 * i + 1] = d_tried[2 * j + 1];
+        const u32 v = active[i];
+        donor.v[j] = v;
+        donor.w[j] = vw[v];
+        donor.src[j] = static_cast<unsigned char>(labels[v]);
+        donor.state[j] = state[i];
+        donor.tried[2 * j] = tried[2 * i];
+        donor.tried[2 * j + 1] = tried[2 * i + 1];
+        donor.list_n[j] = kNoPart;
     }
+    __syncthreads();
+    run_attempts<C, D>(sm, donor, count, first_attempt, A, off, nbr, ew, labels, k, plan, targets, flags);
+    for (int p = threadIdx.x; p < k; p += blockDim.x) requests[p] = sm.requests[p];
+    for (int j = threadIdx.x; j < count; j += blockDim.x) {
+        const u32 i = open[j];
+        state[i] = donor.state[j];
+        tried[2 * i] = donor.tried[2 * j];
+        tried[2 * i + 1] = donor.tried[2 * j + 1];
+    }
+}
+// A short list (at most kAttemptCap donors) from the collected words to the
+// movers, by one block: the repair order (a bitonic network over the words),
+// the donor test, and all attempts.  One launch in place of two selections, a
+// sort, a scan and the attempts, and nothing for the host to read in between.
+// With a longer list it does nothing and places nobody; the host sees the
+// count with the batch's counters and takes the device-wide path.
+template <class C>
+constexpr size_t repair_block_smem() { return attempt_smem<C>(kAttemptCap) + kAttemptCap * sizeof(u64); }
+template <class C, int D>
+__global__ void __launch_bounds__(kAttemptThreads) k_repair_block(const u64* list, const u64* list_count, const C* A,
+                                                                  const int* off, const int* nbr, const u32* ew,
+                                                                  const int* labels, const u32* vw, int k,
+                                                                  const u32* plan, const int* bound, const u64* start,
+                                                                  const u64* loads, u64 capacity, const u64* slack,
+                                                                  int* targets, int* flags, int* movers, u64* placed) {
+    __shared__ AttemptParts sm;
+    __shared__ u32 s_scan[33];
+    __shared__ u32 s_placed;
+    extern __shared__ __align__(16) unsigned char attempt_smem_raw[];
+    if (*list_count > kAttemptCap) return;
+    const int listed = static_cast<int>(*list_count);
+    u64* word = reinterpret_cast<u64*>(attempt_smem_raw);
+    const AttemptDonors<C> donor(attempt_smem_raw + kAttemptCap * sizeof(u64), kAttemptCap);
+    int size = 32;
+    while (size < listed) size <<= 1;
+    for (int j = threadIdx.x; j < size; j += blockDim.x) word[j] = j < listed ? list[j] : ~0ULL;
+    for (int p = threadIdx.x; p < k; p += blockDim.x) {
+        sm.slack[p] = slack[p];
+        sm.requests[p] = 0;
+        sm.base[p] = bound[p] >= 0 ? start[p] : 0;
+    }
+    if (threadIdx.x == 0) s_placed = 0;
+    __syncthreads();
+    for (int kk = 2; kk <= size; kk <<= 1)
+        for (int jj = kk >> 1; jj; jj >>= 1) {
+            for (int q = threadIdx.x; q < size / 2; q += blockDim.x) {
+                const int i = (q / jj) * 2 * jj + q % jj;
+                const u64 a = word[i], b = word[i + jj];
+                if ((a > b) == ((i & kk) == 0)) {
+                    word[i] = b;
+                    word[i + jj] = a;
+                }
+            }
+            __syncthreads();
+        }
+    // The donor test, and the active donors in repair order.
+    int count = 0;
+    for (int chunk = 0; chunk < listed; chunk += blockDim.x) {
+        const int j = chunk + threadIdx.x;
+        const int v = j < listed ? static_cast<int>(word[j] & 0xffffffffULL) : 0;
+        const int src = j < listed ? labels[v] : 0;
+        const u64 w = j < listed ? vw[v] : 0;
+        const int t = j < listed && plan_class(plan[v]) == bound[src] ? src : -1;
+        const u64 before = order_chunk(sm, k, t, t >= 0 ? w : 0);
+        const bool active = j < listed && (t < 0 || before < loads[src] - capacity);
+        u32 total;
+        const u32 slot = block_exclusive_scan_wide<u32>(active ? 1u : 0u, total, s_scan) + static_cast<u32>(count);
+        if (active) {
+            donor.v[slot] = static_cast<u32>(v);
+            donor.w[slot] = static_cast<u32>(w);
+            donor.src[slot] = static_cast<unsigned char>(src);
+            donor.state[slot] = 0;
+            donor.tried[2 * slot] = donor.tried[2 * slot + 1] = 0;
+            donor.list_n[slot] = kNoPart;
+        }
+        count += static_cast<int>(total);
+        __syncthreads();
+    }
+    run_attempts<C, D>(sm, donor, count, 0, A, off, nbr, ew, labels, k, plan, targets, flags);
+    __syncthreads();
+    for (int j = threadIdx.x; j < count; j += blockDim.x)
+        if (donor.state[j] == 1) movers[atomicAdd(&s_placed, 1u)] = static_cast<int>(donor.v[j]);
+    __syncthreads();
+    if (threadIdx.x == 0) *placed = s_placed;
 }
 struct IsOpen {
     const unsigned char* state;
@@ -2642,9 +2835,7 @@ private:
     int* movers = nullptr;
     double* prices = nullptr;
     Sample* samples = nullptr;
-    u32* rorder = nullptr;
-    u32* rposition = nullptr;  // place of each vertex in the repair order
-    int* rlabels = nullptr;    // labels in repair order
+    u64* class_weights = nullptr;  // repair: donor weight per part and class (zero between iterations)
     u32* state = nullptr;      // packed label / target / batch bit per vertex (dense-cache levels)
     int* chunk_work = nullptr;      // chunks of the heavy rows taking part in a batch (k_heavy_chunk_list)
     u64* chunk_work_count = nullptr;
@@ -2653,6 +2844,7 @@ private:
     u64 cut = 0, revision = 0;
     u64 rebuild_entries = ~0ULL;  // mover entries above which apply() rebuilds the cache
     i64 repair_iterations = 0, repair_donors = 0;  // for the per-level log line
+    i64 last_listed = 0;  // donors the last repair iteration listed
     bool on_demand = false;  // no dense cache: affinities recomputed from the rows
     Frontier frontier{};         // levels above 65,536 vertices: the rows the LP proposals visit
     bool frontier_on = false;
@@ -2760,7 +2952,7 @@ private:
         launch(k_commit, std::min(grid_for(host_count, kThreads), 148 * 4), kThreads, sizeof(long long) * k, s(),
                host_count, list, live,
                labels, targets, g.vw, k, loads, lp ? locks : static_cast<unsigned char*>(nullptr), flags,
-               static_cast<const u32*>(rposition), rlabels, state, counters + 3,
+               state, counters + 3,
                reinterpret_cast<unsigned int*>(counters + 8));
         if (frontier_on) {
             launch(k_touch_rows, grid_for(host_count * 32, kThreads), kThreads, 0, s(), host_count, list, live, g.off,
@@ -2846,6 +3038,10 @@ private:
     void enqueue_lp_round(double filter);
     i64 lp_round(double filter);
     bool repair();
+    void offer_list(const u64* list_count, u64* placed_count, const u32* plan, const u64* list, const int* bound,
+                    const u64* start, const u64* slack);
+    void reserve_long(i64 listed, u64* list, const u32* plan, const int* bound, const u64* start, const u64* slack,
+                      u64* requests);
     void exchange(u64& best);
 };
 
@@ -2904,168 +3100,211 @@ bool LevelRefiner<T>::repair() {
     u64* slack = A_.alloc<u64>(k);
     u64* requests = A_.alloc<u64>(k);
     u64* cdf = A_.alloc<u64>(k + 1);
-    u64* part_base = A_.alloc<u64>(k);
-    u32* donors = A_.alloc<u32>(n);
-    u32* donor_count = reinterpret_cast<u32*>(counters + 4);
-    unsigned char* active_flag = A_.alloc<unsigned char>(n);
+    int* bound = A_.alloc<int>(k);
+    u64* start = A_.alloc<u64>(k);
+    u32* plan = A_.alloc<u32>(n);
+    u64* list = A_.alloc<u64>(n);
+    // counters[9]: placed donors, [10]: donors, [11]: listed donors.
+    u64 *placed_count = counters + 9, *donor_count = counters + 10, *list_count = counters + 11;
     int iterations = 0;
     while (true) {
         ArenaScope it(A_);
-        launch(k_slack, 1, kMaxParts, 0, s(), k, loads, C, slack, requests, cdf);
-        select_if(A_, s(), n, IsDonor{rlabels, loads, C}, WriteOrdered{rorder, donors}, donor_count);
-        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 4, sizeof(u64), cudaMemcpyDeviceToHost, s()));
-        GP_CUDA(cudaStreamSynchronize(s()));
-        const i64 dcount = static_cast<i64>(ctx.host_scalars[0] & 0xffffffffULL);
-        ++repair_iterations;
-        repair_donors += dcount;
-        i64 placed = 0;
-        long long delta = 0;
-        if (dcount > 0) {
-            u64* keys = A_.alloc<u64>(dcount);
-            u64* keys_alt = A_.alloc<u64>(dcount);
-            u32* items = A_.alloc<u32>(dcount);
-            u32* items_alt = A_.alloc<u32>(dcount);
-            if (on_demand)
-                with_row_size([&](auto d) {
-                    launch(k_repair_dest_od<decltype(d)::value>, grid_for(dcount, kThreads), kThreads, 0, s(), dcount,
-                           static_cast<const u32*>(donors), static_cast<const int*>(g.off), static_cast<const int*>(g.nbr),
-                           static_cast<const u32*>(g.ew), static_cast<const int*>(labels), static_cast<const u32*>(g.vw),
-                           k, static_cast<const u64*>(loads), C, static_cast<const u64*>(cdf), targets, keys);
-                });
-            else
-                with_groups([&](auto width, auto vec) {
-                    constexpr int W = decltype(width)::value;
-                    launch(k_repair_dest<T, W, decltype(vec)::value>, grid_for(dcount * W, kThreads), kThreads, 0, s(),
-                           dcount, donors, static_cast<const T*>(A), static_cast<const T*>(totals), labels, g.vw, k, loads,
-                           C, cdf, targets, keys);
-                });
-            GP_CUDA(cudaMemcpyAsync(items, donors, sizeof(u32) * dcount, cudaMemcpyDeviceToDevice, s()));
-            // Stable sort by bucket keeps the repair order inside a bucket;
-            // bucket keys are below k*800 < 2^17, the sentinel sorts last.
-            launch(k_clamp_keys, blocks_for(dcount, kThreads), kThreads, 0, s(), dcount, keys);
-            radix_sort_pairs(A_, s(), dcount, keys, items, keys_alt, items_alt, 0, 24);
-            u64* prefix = A_.alloc<u64>(dcount);
-            exclusive_scan<u64>(A_, s(), dcount, SortedWeight{items, g.vw}, prefix, static_cast<u64*>(nullptr));
-            launch(k_part_heads, blocks_for(dcount, kThreads), kThreads, 0, s(), dcount, keys, prefix, part_base);
-            launch(k_donor_test, blocks_for(dcount, kThreads), kThreads, 0, s(), dcount, keys, items, prefix, part_base,
-                   loads, C, active_flag);
-            // Active donors, back in repair order.
-            u32* active = A_.alloc<u32>(dcount);
-            select_if(A_, s(), dcount, IsActive{donors, active_flag}, WriteFrom{donors, active}, donor_count);
-            GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 4, sizeof(u64), cudaMemcpyDeviceToHost, s()));
+        launch(k_slack, 1, kMaxParts, 0, s(), k, loads, C, slack, requests, cdf, counters + 9);
+        if (on_demand)
+            with_row_size([&](auto d) {
+                launch(k_repair_dest_od<decltype(d)::value>, grid_for(n, kThreads), kThreads, 0, s(), n,
+                       static_cast<const int*>(g.off), static_cast<const int*>(g.nbr), static_cast<const u32*>(g.ew),
+                       static_cast<const int*>(labels), static_cast<const u32*>(g.vw), k,
+                       static_cast<const u64*>(loads), C, static_cast<const u64*>(cdf), plan, class_weights,
+                       donor_count);
+            });
+        else
+            with_groups([&](auto width, auto vec) {
+                constexpr int W = decltype(width)::value;
+                launch(k_repair_dest<T, W, decltype(vec)::value>, grid_for(n, kThreads), kThreads, 0, s(), n,
+                       static_cast<const T*>(A), static_cast<const T*>(totals), static_cast<const int*>(labels),
+                       static_cast<const u32*>(g.vw), k, static_cast<const u64*>(loads), C,
+                       static_cast<const u64*>(cdf), plan, class_weights, donor_count);
+            });
+        launch(k_repair_bounds, k, kScanThreads, 0, s(), static_cast<const u64*>(loads), C, class_weights, bound,
+               start);
+        launch(k_repair_list, grid_for(n, kThreads), kThreads, 0, s(), n, k, static_cast<const int*>(labels),
+               static_cast<const u32*>(plan), static_cast<const int*>(bound), list, list_count);
+        // The next list is mostly about as long as the last one: after a long
+        // one, its length is read first instead of offering it to one block.
+        const bool offered = last_listed <= kAttemptCap;
+        if (offered) offer_list(list_count, placed_count, plan, list, bound, start, slack);
+        auto read_batch = [&]() {
+            GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 2, 10 * sizeof(u64), cudaMemcpyDeviceToHost, s()));
             GP_CUDA(cudaStreamSynchronize(s()));
-            const i64 acount = static_cast<i64>(ctx.host_scalars[0] & 0xffffffffULL);
-            if (acount > 0) {
-                u64* tried = A_.alloc<u64>(2 * acount);
-                unsigned char* state = A_.alloc<unsigned char>(acount);
-                int* want = A_.alloc<int>(acount);
-                GP_CUDA(cudaMemsetAsync(tried, 0, sizeof(u64) * 2 * acount, s()));
-                GP_CUDA(cudaMemsetAsync(state, 0, acount, s()));
-                const int tiles = blocks_for(acount, kAdmitTile);
-                u64* tile_sums = A_.alloc<u64>(static_cast<size_t>(k) * tiles);
-                u64* tile_offsets = A_.alloc<u64>(static_cast<size_t>(k) * tiles);
-                u64* tile_total = A_.alloc<u64>(1);
-                u32* open = A_.alloc<u32>(acount);
-                u32* open_count = reinterpret_cast<u32*>(counters + 5);
-                // Small sets of open donors finish all their attempts in one block.
-                auto finish_in_block = [&](int first_attempt) {
-                    auto go = [&](auto d) {
-                        // Sized for kAttemptCap donors (the count is on the
-                        // device); the limit is set on every call, as it
-                        // belongs to the kernel on whichever device is current.
-                        constexpr size_t smem = attempt_smem<T>(kAttemptCap);
-                        GP_CUDA(cudaFuncSetAttribute(k_attempts<T, decltype(d)::value>,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     static_cast<int>(smem)));
-                        launch(k_attempts<T, decltype(d)::value>, 1, kAttemptThreads, smem, s(), static_cast<const u32*>(open),
-                               static_cast<const u32*>(open_count), first_attempt, static_cast<const u32*>(active),
-                               static_cast<const T*>(A), static_cast<const int*>(g.off), static_cast<const int*>(g.nbr),
-                               static_cast<const u32*>(g.ew), static_cast<const int*>(labels), g.vw, k,
-                               static_cast<const int*>(targets), static_cast<const u64*>(slack), requests, tried, state,
-                               targets, flags);
-                    };
-                    // The row size matters only for on-demand affinities; a
-                    // dense level takes the smallest instantiation (fewest
-                    // registers: one block of 1024 threads has 64 each).
-                    if (on_demand) with_row_size(go);
-                    else go(std::integral_constant<int, 8>{});
-                };
-                if (acount <= kAttemptCap) {
-                    select_if(A_, s(), acount, IsOpen{state}, WriteIdx{open}, open_count);
-                    finish_in_block(0);
-                }
-                for (int attempt = 0; attempt < k && acount > kAttemptCap; ++attempt) {
-                    GP_CUDA(cudaMemsetAsync(counters + 5, 0, sizeof(u64), s()));
-                    if (on_demand)
-                        with_row_size([&](auto d) {
-                            launch(k_choose_od<decltype(d)::value>, grid_for(acount, kThreads), kThreads, 0, s(), acount,
-                                   static_cast<const u32*>(active), attempt, static_cast<const int*>(g.off),
-                                   static_cast<const int*>(g.nbr), static_cast<const u32*>(g.ew),
-                                   static_cast<const int*>(labels), static_cast<const u32*>(g.vw), k,
-                                   static_cast<const int*>(targets), static_cast<const u64*>(slack),
-                                   static_cast<const u64*>(requests), static_cast<const u64*>(tried), state, want,
-                                   counters + 5);
-                        });
-                    else
-                        with_groups([&](auto width, auto vec) {
-                            constexpr int W = decltype(width)::value;
-                            launch(k_choose<T, W, decltype(vec)::value>, grid_for(acount * W, kThreads), kThreads, 0, s(),
-                                   acount, active, attempt, static_cast<const T*>(A), labels, g.vw, k, targets, slack,
-                                   requests, tried, state, want, counters + 5);
-                        });
-                    // Admission of this attempt's requests (a no-op when none
-                    // asked), then one read-back of the number that asked.
-                    launch(k_part_requests, tiles, kAdmitTile, 0, s(), acount, static_cast<const int*>(want),
-                           static_cast<const u32*>(active), static_cast<const u32*>(g.vw), k, tiles, tile_sums);
-                    exclusive_scan<u64>(A_, s(), static_cast<i64>(k) * tiles, LoadOf<u64>{tile_sums}, tile_offsets,
-                                        tile_total);
-                    launch(k_admit_tiles, tiles, kAdmitTile, 0, s(), acount, static_cast<const int*>(want),
-                           static_cast<const u32*>(active), static_cast<const u32*>(g.vw),
-                           static_cast<const u64*>(tile_offsets), static_cast<const u64*>(tile_total), tiles,
-                           static_cast<const u64*>(slack), requests, tried, state, targets, flags, k,
-                           reinterpret_cast<unsigned int*>(counters + 8));
-                    GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 5, sizeof(u64), cudaMemcpyDeviceToHost, s()));
-                    GP_CUDA(cudaStreamSynchronize(s()));
-                    const i64 rcount = static_cast<i64>(ctx.host_scalars[0]);
-                    if (!rcount) break;
-                    // At most rcount donors remain open.
-                    if (rcount <= kAttemptCap && attempt + 1 < k) {
-                        select_if(A_, s(), acount, IsOpen{state}, WriteIdx{open}, open_count);
-                        finish_in_block(attempt + 1);
-                        break;
-                    }
-                }
-                // Movers = placed donors, in repair order, applied with their
-                // count left on the device (counters[9], whose upper half
-                // stays zero): one read-back brings the count and the
-                // batch's counters together.  An empty batch changes nothing
-                // on the device.
-                select_if(A_, s(), acount, IsPlaced{state}, WriteActiveVertex{active, movers},
-                          reinterpret_cast<u32*>(counters + 9));
-                apply(movers, counters + 9, acount, false, samples != nullptr);
-                GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 2, 8 * sizeof(u64), cudaMemcpyDeviceToHost, s()));
-                GP_CUDA(cudaStreamSynchronize(s()));
-                placed = static_cast<i64>(ctx.host_scalars[7] & 0xffffffffULL);
-                if (placed) {
-                    delta = settled_delta(ctx.host_scalars);
-                    max_load_host = ctx.host_scalars[1];
-                    stats.accepted += static_cast<u64>(placed);
-                    if (delta >= 0) stats.rebalance_gain += static_cast<u64>(delta);
-                    else stats.rebalance_loss += static_cast<u64>(-delta);
-                    account(delta);
-                    ++revision;
-                    check_state("GPU rebalance cut mismatch");
-                }
-            }
+        };
+        read_batch();
+        const i64 listed = static_cast<i64>(ctx.host_scalars[9]);
+        last_listed = listed;
+        ++repair_iterations;
+        repair_donors += static_cast<i64>(ctx.host_scalars[8]);
+        if (listed > kAttemptCap || !offered) {
+            reserve_long(listed, list, plan, bound, start, slack, requests);
+            read_batch();
         }
-        if (frontier_on && dcount > 0)
-            launch(k_reset_targets, blocks_for(dcount, kThreads), kThreads, 0, s(), dcount,
-                   static_cast<const u32*>(donors), targets);
+        const i64 placed = static_cast<i64>(ctx.host_scalars[7] & 0xffffffffULL);
+        if (placed) {
+            const long long delta = settled_delta(ctx.host_scalars);
+            max_load_host = ctx.host_scalars[1];
+            stats.accepted += static_cast<u64>(placed);
+            if (delta >= 0) stats.rebalance_gain += static_cast<u64>(delta);
+            else stats.rebalance_loss += static_cast<u64>(-delta);
+            account(delta);
+            ++revision;
+            check_state("GPU rebalance cut mismatch");
+        }
         ++iterations;
         ++stats.admission_iterations;
         const bool feasible = max_load_host <= C;
         if (feasible || placed == 0 || iterations >= 2 * k + 4) return feasible;
     }
+}
+
+// Offers the listed donors to one block (k_repair_block) and applies those it
+// placed, their count on the device: one read-back then brings the counts and
+// the batch's counters together.  An empty batch changes nothing.
+template <class T>
+void LevelRefiner<T>::offer_list(const u64* list_count, u64* placed_count, const u32* plan, const u64* list,
+                                 const int* bound, const u64* start, const u64* slack) {
+    auto go = [&](auto d) {
+        // Sized for kAttemptCap donors (the count is on the device); the limit
+        // is set on every call, as it belongs to the kernel on whichever
+        // device is current.
+        constexpr size_t smem = repair_block_smem<T>();
+        GP_CUDA(cudaFuncSetAttribute(k_repair_block<T, decltype(d)::value>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        launch(k_repair_block<T, decltype(d)::value>, 1, kAttemptThreads, smem, s(), static_cast<const u64*>(list),
+               list_count, static_cast<const T*>(A), static_cast<const int*>(g.off), static_cast<const int*>(g.nbr),
+               static_cast<const u32*>(g.ew), static_cast<const int*>(labels), static_cast<const u32*>(g.vw), k,
+               static_cast<const u32*>(plan), static_cast<const int*>(bound), static_cast<const u64*>(start),
+               static_cast<const u64*>(loads), C, static_cast<const u64*>(slack), targets, flags, movers,
+               placed_count);
+    };
+    // The row size matters only for on-demand affinities; a dense level takes
+    // the smallest instantiation (fewest registers: one block of 1024 threads
+    // has 64 each).
+    if (on_demand) with_row_size(go);
+    else go(std::integral_constant<int, 8>{});
+    apply(movers, placed_count, std::min<i64>(n, kAttemptCap), false, samples != nullptr);
+}
+
+// The receiver reservation of more listed donors than one block takes: the
+// list sorted into repair order, the donor test by tiles, and device-wide
+// attempts until few donors are left.  Applies the placed donors.
+template <class T>
+void LevelRefiner<T>::reserve_long(i64 listed, u64* list, const u32* plan, const int* bound, const u64* start,
+                                   const u64* slack, u64* requests) {
+    Arena& A_ = ctx.scratch;
+    u32* donor_count = reinterpret_cast<u32*>(counters + 4);
+    if (listed == 0) return;
+    GP_CUDA(cudaMemsetAsync(counters + 4, 0, sizeof(u64), s()));
+    {
+        u64* list_alt = A_.alloc<u64>(listed);
+        u32 *none = nullptr, *none_alt = nullptr;
+        radix_sort_pairs(A_, s(), listed, list, none, list_alt, none_alt, 32, 64);
+    }
+    u32* items = A_.alloc<u32>(listed);
+    int* want = A_.alloc<int>(listed);
+    u32* active = A_.alloc<u32>(listed);
+    i64 acount = 0;
+    {
+        ArenaScope test(A_);
+        unsigned char* active_flag = A_.alloc<unsigned char>(listed);
+        const int tiles = blocks_for(listed, kAdmitTile);
+        u64* tile_sums = A_.alloc<u64>(static_cast<size_t>(k) * tiles);
+        u64* tile_offsets = A_.alloc<u64>(static_cast<size_t>(k) * tiles);
+        launch(k_repair_unpack, blocks_for(listed, kThreads), kThreads, 0, s(), listed, static_cast<const u64*>(list),
+               static_cast<const int*>(labels), plan, bound, items, want);
+        launch(k_part_requests, tiles, kAdmitTile, 0, s(), listed, static_cast<const int*>(want),
+               static_cast<const u32*>(items), static_cast<const u32*>(g.vw), k, tiles, tile_sums);
+        exclusive_scan<u64>(A_, s(), static_cast<i64>(k) * tiles, LoadOf<u64>{tile_sums}, tile_offsets,
+                            static_cast<u64*>(nullptr));
+        launch(k_repair_active, tiles, kAdmitTile, 0, s(), listed, static_cast<const int*>(want),
+               static_cast<const u32*>(items), static_cast<const u32*>(g.vw), static_cast<const u64*>(tile_offsets),
+               tiles, static_cast<const u64*>(loads), C, start, k, active_flag);
+        // Active donors, in repair order.
+        select_if(A_, s(), listed, IsActive{active_flag}, WriteFrom{items, active}, donor_count);
+        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 4, sizeof(u64), cudaMemcpyDeviceToHost, s()));
+        GP_CUDA(cudaStreamSynchronize(s()));
+        acount = static_cast<i64>(ctx.host_scalars[0] & 0xffffffffULL);
+    }
+    if (acount == 0) return;
+    u64* tried = A_.alloc<u64>(2 * acount);
+    unsigned char* state = A_.alloc<unsigned char>(acount);
+    GP_CUDA(cudaMemsetAsync(tried, 0, sizeof(u64) * 2 * acount, s()));
+    GP_CUDA(cudaMemsetAsync(state, 0, acount, s()));
+    const int tiles = blocks_for(acount, kAdmitTile);
+    u64* tile_sums = A_.alloc<u64>(static_cast<size_t>(k) * tiles);
+    u64* tile_offsets = A_.alloc<u64>(static_cast<size_t>(k) * tiles);
+    u64* tile_total = A_.alloc<u64>(1);
+    u32* open = A_.alloc<u32>(acount);
+    u32* open_count = reinterpret_cast<u32*>(counters + 5);
+    // Small sets of open donors finish all their attempts in one block.
+    auto finish_in_block = [&](int first_attempt) {
+        auto go = [&](auto d) {
+            constexpr size_t smem = attempt_smem<T>(kAttemptCap);
+            GP_CUDA(cudaFuncSetAttribute(k_attempts<T, decltype(d)::value>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+            launch(k_attempts<T, decltype(d)::value>, 1, kAttemptThreads, smem, s(), static_cast<const u32*>(open),
+                   static_cast<const u32*>(open_count), first_attempt, static_cast<const u32*>(active),
+                   static_cast<const T*>(A), static_cast<const int*>(g.off), static_cast<const int*>(g.nbr),
+                   static_cast<const u32*>(g.ew), static_cast<const int*>(labels), static_cast<const u32*>(g.vw), k,
+                   plan, slack, requests, tried, state, targets, flags);
+        };
+        if (on_demand) with_row_size(go);
+        else go(std::integral_constant<int, 8>{});
+    };
+    if (acount <= kAttemptCap) {
+        select_if(A_, s(), acount, IsOpen{state}, WriteIdx{open}, open_count);
+        finish_in_block(0);
+    }
+    for (int attempt = 0; attempt < k && acount > kAttemptCap; ++attempt) {
+        GP_CUDA(cudaMemsetAsync(counters + 5, 0, sizeof(u64), s()));
+        if (on_demand)
+            with_row_size([&](auto d) {
+                launch(k_choose_od<decltype(d)::value>, grid_for(acount, kThreads), kThreads, 0, s(), acount,
+                       static_cast<const u32*>(active), attempt, static_cast<const int*>(g.off),
+                       static_cast<const int*>(g.nbr), static_cast<const u32*>(g.ew),
+                       static_cast<const int*>(labels), static_cast<const u32*>(g.vw), k, plan, slack,
+                       static_cast<const u64*>(requests), static_cast<const u64*>(tried), state, want, counters + 5);
+            });
+        else
+            with_groups([&](auto width, auto vec) {
+                constexpr int W = decltype(width)::value;
+                launch(k_choose<T, W, decltype(vec)::value>, grid_for(acount * W, kThreads), kThreads, 0, s(), acount,
+                       active, attempt, static_cast<const T*>(A), labels, g.vw, k, plan, slack, requests, tried, state,
+                       want, counters + 5);
+            });
+        // Admission of this attempt's requests (a no-op when none asked),
+        // then one read-back of the number that asked.
+        launch(k_part_requests, tiles, kAdmitTile, 0, s(), acount, static_cast<const int*>(want),
+               static_cast<const u32*>(active), static_cast<const u32*>(g.vw), k, tiles, tile_sums);
+        exclusive_scan<u64>(A_, s(), static_cast<i64>(k) * tiles, LoadOf<u64>{tile_sums}, tile_offsets, tile_total);
+        launch(k_admit_tiles, tiles, kAdmitTile, 0, s(), acount, static_cast<const int*>(want),
+               static_cast<const u32*>(active), static_cast<const u32*>(g.vw),
+               static_cast<const u64*>(tile_offsets), static_cast<const u64*>(tile_total), tiles, slack, requests,
+               tried, state, targets, flags, k, reinterpret_cast<unsigned int*>(counters + 8));
+        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 5, sizeof(u64), cudaMemcpyDeviceToHost, s()));
+        GP_CUDA(cudaStreamSynchronize(s()));
+        const i64 rcount = static_cast<i64>(ctx.host_scalars[0]);
+        if (!rcount) break;
+        // At most rcount donors remain open.
+        if (rcount <= kAttemptCap && attempt + 1 < k) {
+            select_if(A_, s(), acount, IsOpen{state}, WriteIdx{open}, open_count);
+            finish_in_block(attempt + 1);
+            break;
+        }
+    }
+    // Movers = placed donors, their count left on the device (a 32-bit count
+    // in a zeroed word).
+    select_if(A_, s(), acount, IsPlaced{state}, WriteActiveVertex{active, movers},
+              reinterpret_cast<u32*>(counters + 9));
+    apply(movers, counters + 9, acount, false, samples != nullptr);
 }
 
 template <class T>
@@ -3260,9 +3499,10 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known) {
     cand = A_.alloc<int>(n);
     movers = A_.alloc<int>(n);
     // [8]: k_commit's finished-block count, zero between launches; [9]: the
-    // repair's placed-donor count (a 32-bit count in a zeroed word).
-    counters = A_.alloc<u64>(10);
-    GP_CUDA(cudaMemsetAsync(counters + 8, 0, 2 * sizeof(u64), s()));
+    // movers of a repair or exchange (a 32-bit count in a zeroed word); [10],
+    // [11]: the repair's donors and listed donors.
+    counters = A_.alloc<u64>(12);
+    GP_CUDA(cudaMemsetAsync(counters + 8, 0, 4 * sizeof(u64), s()));
     corr_acc = A_.alloc<long long>(g.heavy_count + 1);
     if (g.chunks) {
         chunk_work = A_.alloc<int>(g.chunks);
@@ -3279,18 +3519,8 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known) {
         GP_CUDA(cudaMemsetAsync(prices, 0, sizeof(double) * k, s()));
         GP_CUDA(cudaMemsetAsync(samples, 0, sizeof(Sample) * k, s()));
     }
-    {  // repair order: ascending (repair hash, id)
-        rorder = A_.alloc<u32>(n);
-        u32* rorder_alt = A_.alloc<u32>(n);
-        u64* keys = A_.alloc<u64>(n);
-        u64* keys_alt = A_.alloc<u64>(n);
-        launch(k_repair_keys, blocks_for(n, kThreads), kThreads, 0, s(), n, keys, rorder);
-        radix_sort_pairs(A_, s(), n, keys, rorder, keys_alt, rorder_alt, 0, 32);
-        rposition = A_.alloc<u32>(n);
-        rlabels = A_.alloc<int>(n);
-        launch(k_repair_positions, blocks_for(n, kThreads), kThreads, 0, s(), n, static_cast<const u32*>(rorder),
-               static_cast<const int*>(labels), rposition, rlabels);
-    }
+    class_weights = A_.alloc<u64>(static_cast<size_t>(k) * kBalanceWidth);
+    GP_CUDA(cudaMemsetAsync(class_weights, 0, sizeof(u64) * k * kBalanceWidth, s()));
     // An entry-by-entry update touches two random cache counters per entry
     // (about 128 bytes of DRAM traffic); a rebuild writes the whole cache and
     // reads the CSR once.
@@ -3382,8 +3612,6 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known) {
         GP_CUDA(cudaMemcpyAsync(labels, saved_labels, sizeof(int) * n, cudaMemcpyDeviceToDevice, s()));
         if (state)
             launch(k_state_init, grid_for(n, kThreads), kThreads, 0, s(), n, static_cast<const int*>(labels), state);
-        launch(k_repair_positions, blocks_for(n, kThreads), kThreads, 0, s(), n, static_cast<const u32*>(rorder),
-               static_cast<const int*>(labels), rposition, rlabels);
         GP_CUDA(cudaMemcpyAsync(loads, saved_loads, sizeof(u64) * k, cudaMemcpyDeviceToDevice, s()));
         launch(k_max_load, 1, 32, 0, s(), k, loads, counters + 3);
         GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 3, sizeof(u64), cudaMemcpyDeviceToHost, s()));
