@@ -954,13 +954,15 @@ __global__ void k_scatter_chunks(DGraph g, const int* map, const int* base, int*
     }
 }
 
-// Row classes by raw size: 0 <= 128 entries, 1 <= 512, 2 <= 1024, 3 <= 2048,
-// 4 <= 4096, 5 <= 8192, 6 larger; sc[kRowClasses] counts the records of class 6.
-constexpr int kRowClasses = 7;
+// Row classes by raw size: 7 <= 16 entries, 0 <= 128, 1 <= 512, 2 <= 1024,
+// 3 <= 2048, 4 <= 4096, 5 <= 8192, 6 larger; sc[kRowClasses] counts the
+// records of class 6.
+constexpr int kRowClasses = 8, kLargeClass = 6, kShortClass = 7, kShortRow = 16;
 __global__ void k_row_classes(i64 nc, const int* raw, int* lists, i64 stride, u64* sc) {
     const i64 c = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int r = c < nc ? raw[c] : 0;
     const int cls = c >= nc                  ? -1
+                    : r <= kShortRow         ? kShortClass
                     : r <= 128               ? 0
                     : r <= 512               ? 1
                     : r <= 1024              ? 2
@@ -970,7 +972,7 @@ __global__ void k_row_classes(i64 nc, const int* raw, int* lists, i64 stride, u6
                                              : 6;
 #pragma unroll
     for (int k = 0; k < kRowClasses; ++k) block_append(static_cast<int>(c), cls == k, lists + k * stride, sc + k);
-    block_atomic_add(sc + kRowClasses, cls == kRowClasses - 1 ? static_cast<u64>(r) : 0ULL);
+    block_atomic_add(sc + kRowClasses, cls == kLargeClass ? static_cast<u64>(r) : 0ULL);
 }
 
 // contraction_warp_sort / contraction_sort_row (contraction_rows.cuh:40-116):
@@ -1118,6 +1120,49 @@ __device__ void warp_radix_row(int begin, int degree, int* keys_io, u32* w_io, i
     for (int j = 0; j < Items; ++j)
         if (k[j] == nc) k[j] = INT_MAX;
     warp_emit_row<Items>(k, v, begin, keys_io, w_io, lane, count_out);
+}
+
+// Rows of up to kShortRow raw entries, one entry per lane of a group of that
+// many, two rows to a warp: the same network and run reduction as the warp's,
+// ten steps instead of fifteen and no idle half.  Mesh levels consist of such
+// rows: sorted by a warp each they took 10.1 ms of the 189 ms partition of the
+// 256^3 mesh at k = 128; with this and the matching's lanes it takes 172-181.
+__global__ void __launch_bounds__(256) k_sort_rows_short(i64 count, const int* rows, const int* raw_off, int* raw_t,
+                                                         u32* raw_w, int* ucount) {
+    constexpr int W = kShortRow;
+    const i64 index = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) / W;
+    const int lane = threadIdx.x & 31, sub = lane % W;
+    const int c = index < count ? rows[index] : -1;
+    const int begin = c >= 0 ? raw_off[c] : 0, degree = c >= 0 ? raw_off[c + 1] - begin : 0;
+    int key = sub < degree ? raw_t[begin + sub] : INT_MAX;
+    u32 sum = sub < degree ? raw_w[begin + sub] : 0u;
+#pragma unroll
+    for (int size = 2; size <= W; size <<= 1)
+#pragma unroll
+        for (int dist = size >> 1; dist; dist >>= 1) {
+            const int ok = __shfl_xor_sync(0xffffffffu, key, dist);
+            const u32 ov = __shfl_xor_sync(0xffffffffu, sum, dist);
+            const bool lower = ((sub & dist) == 0) == ((sub & size) == 0);
+            if (lower ? ok < key : ok > key) {
+                key = ok;
+                sum = ov;
+            }
+        }
+#pragma unroll
+    for (int d = 1; d < W; d <<= 1) {
+        const int ok = __shfl_up_sync(0xffffffffu, key, d, W);
+        const u32 os = __shfl_up_sync(0xffffffffu, sum, d, W);
+        if (sub >= d && key == ok) sum += os;
+    }
+    const int next = __shfl_down_sync(0xffffffffu, key, 1, W);
+    const bool emit = key != INT_MAX && (sub == W - 1 || key != next);
+    const unsigned heads = (__ballot_sync(0xffffffffu, emit) >> (lane & ~(W - 1))) & ((1u << W) - 1u);
+    if (emit) {
+        const int out = begin + __popc(heads & ((1u << sub) - 1u));
+        raw_t[out] = key;
+        raw_w[out] = sum;
+    }
+    if (c >= 0 && sub == 0) ucount[c] = __popc(heads);
 }
 
 template <bool Long>
@@ -1607,8 +1652,14 @@ AggregateOut Aggregator::run() {
     if (matching) {  // src/coarsen.cu:505-535
         int* choice = proposals;
         const u32 salt = seed ^ (static_cast<u32>(level) * 0x9e3779b9U);
+        // Lanes per row by the average row (matching levels have at most
+        // o.heavy_limit entries a row): one thread below 8 entries, 8 lanes
+        // up to 32, a warp above (a warp for the 10-13 entries of a 256^3
+        // mesh's coarse levels took 5.9 ms of a partition, mostly idle lanes).
         if (g.m / n < 8)
             launch(k_match_choose<1>, vb, kThreads, 0, s, n, g.off, g.nbr, g.ew, g.vw, C, salt, choice);
+        else if (g.m / n < 32)
+            launch(k_match_choose<8>, blocks_for(n * 8, kThreads), kThreads, 0, s, n, g.off, g.nbr, g.ew, g.vw, C, salt, choice);
         else
             launch(k_match_choose<32>, blocks_for(n * 32, kThreads), kThreads, 0, s, n, g.off, g.nbr, g.ew, g.vw, C, salt, choice);
         launch(k_match_roots, vb, kThreads, 0, s, n, choice, clusters);
@@ -1837,6 +1888,9 @@ DGraph contract(Context& ctx, const DGraph& fine, AggregateOut& agg, Workspace& 
     for (int c = 0; c < kRowClasses; ++c) count[c] = static_cast<i64>(cls[c]);
     const i64 large_records = static_cast<i64>(cls[kRowClasses]);
     int* ucount = raw;  // raw sizes are no longer needed once the classes exist
+    if (count[kShortClass])
+        launch(k_sort_rows_short, blocks_for(count[kShortClass] * kShortRow, kThreads), kThreads, 0, s,
+               count[kShortClass], lists + kShortClass * nc, raw_off, raw_t, raw_w, ucount);
     if (count[0])
         launch(k_sort_rows_warp<false>, blocks_for(count[0] * 32, kThreads), kThreads, 0, s, count[0], lists, raw_off,
                raw_t, raw_w, ucount, static_cast<int>(nc), bit_length(static_cast<u64>(nc)));
