@@ -91,6 +91,31 @@ inline void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem
     if (timed) g_profiler->after(stream);
 }
 
+// One thread-block cluster of `blocks` blocks (more than 8 need the kernel's
+// non-portable attribute).
+template <class... Params, class... Args>
+inline void launch_cluster(void (*kernel)(Params...), int blocks, int threads, size_t smem, cudaStream_t stream,
+                           Args&&... args) {
+    ++g_launches;
+    const bool timed = g_profiler && g_profiler->matches(reinterpret_cast<const void*>(kernel));
+    if (g_profiler) g_profiler->last_timed = timed;
+    if (timed) g_profiler->before(stream);
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(static_cast<unsigned>(blocks));
+    config.blockDim = dim3(static_cast<unsigned>(threads));
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute shape{};
+    shape.id = cudaLaunchAttributeClusterDimension;
+    shape.val.clusterDim.x = static_cast<unsigned>(blocks);
+    shape.val.clusterDim.y = 1;
+    shape.val.clusterDim.z = 1;
+    config.attrs = &shape;
+    config.numAttrs = 1;
+    GP_CUDA(cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...));
+    if (timed) g_profiler->after(stream);
+}
+
 inline int blocks_for(i64 items, int per_block) {
     const i64 b = (items + per_block - 1) / per_block;
     return static_cast<int>(b < 1 ? 1 : b);

@@ -1763,8 +1763,9 @@ struct AttemptDonors {
         list_p = bounded + count;
     }
 };
+template <int Threads>
 struct AttemptParts {
-    static constexpr int kWarps = kAttemptThreads / 32;
+    static constexpr int kWarps = Threads / 32;
     u64 slack[kMaxParts], requests[kMaxParts], base[kMaxParts], avail[kMaxParts];
     u64 warp[kMaxParts][kWarps];  // per part, the weight each warp requests
     int want[kAttemptCap];
@@ -1774,10 +1775,11 @@ struct AttemptParts {
 // For one chunk of the donors (one per thread, in order): turns sm.warp, the
 // weight each warp asks per part, into the weight asked before each warp on
 // top of sm.base, and moves sm.base on.  before: the thread's own start.
-__device__ __forceinline__ u64 order_chunk(AttemptParts& sm, int k, int t, u64 w) {
-    constexpr int kWarps = AttemptParts::kWarps;
+template <int Threads>
+__device__ __forceinline__ u64 order_chunk(AttemptParts<Threads>& sm, int k, int t, u64 w) {
+    constexpr int kWarps = Threads / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int x = threadIdx.x; x < kWarps * k; x += blockDim.x) sm.warp[x / kWarps][x % kWarps] = 0;
+    for (int x = threadIdx.x; x < kWarps * k; x += Threads) sm.warp[x / kWarps][x % kWarps] = 0;
     __syncthreads();
     const unsigned peers = __match_any_sync(0xffffffffu, t);
     u64 before = 0, sum = 0;
@@ -1791,16 +1793,16 @@ __device__ __forceinline__ u64 order_chunk(AttemptParts& sm, int k, int t, u64 w
     __syncthreads();
     // Warp `warp` scans the parts warp, warp + 32, ... across its lanes (lane
     // l holds warp l's sum).
-    static_assert(kWarps == 32, "one lane per warp of the block");
+    static_assert(kWarps <= 32, "one lane per warp of the block");
     for (int p = warp; p < k; p += kWarps) {
-        const u64 x = sm.warp[p][lane], base = sm.base[p];
+        const u64 x = lane < kWarps ? sm.warp[p][lane] : 0, base = sm.base[p];
         u64 inc = x;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const u64 o = __shfl_up_sync(0xffffffffu, inc, d);
             if (lane >= d) inc += o;
         }
-        sm.warp[p][lane] = base + inc - x;
+        if (lane < kWarps) sm.warp[p][lane] = base + inc - x;
         __syncwarp();
         if (lane == 31) sm.base[p] = base + inc;
     }
@@ -1809,8 +1811,8 @@ __device__ __forceinline__ u64 order_chunk(AttemptParts& sm, int k, int t, u64 w
 }
 // The attempts from first_attempt on, until no donor asks: leaves the donors'
 // states and tried parts in `donor` and the requests in sm.requests.
-template <class C, int D>
-__device__ void run_attempts(AttemptParts& sm, const AttemptDonors<C>& donor, int count, int first_attempt, const C* A,
+template <class C, int D, int Threads>
+__device__ void run_attempts(AttemptParts<Threads>& sm, const AttemptDonors<C>& donor, int count, int first_attempt, const C* A,
                              const int* off, const int* nbr, const u32* ew, const int* labels, int k, const u32* plan,
                              int* targets, int* flags) {
     u64* d_tried = donor.tried;
@@ -1834,16 +1836,18 @@ __device__ void run_attempts(AttemptParts& sm, const AttemptDonors<C>& donor, in
         __syncthreads();
         if (attempt > 0 && A) {
             // Rank of part p: the parts before it, counted by 8 lanes.
-            const int p = threadIdx.x >> 3, sub = threadIdx.x & 7;
-            int rank = 0;
-            if (p < k) {
-                const u64 a = s_avail[p];
-                for (int q = sub; q < k; q += 8) rank += s_avail[q] > a || (s_avail[q] == a && q < p);
+            for (int first = 0; first < k; first += Threads / 8) {
+                const int p = first + (threadIdx.x >> 3), sub = threadIdx.x & 7;
+                int rank = 0;
+                if (p < k) {
+                    const u64 a = s_avail[p];
+                    for (int q = sub; q < k; q += 8) rank += s_avail[q] > a || (s_avail[q] == a && q < p);
+                }
+                rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+                rank += __shfl_xor_sync(0xffffffffu, rank, 2);
+                rank += __shfl_xor_sync(0xffffffffu, rank, 4);
+                if (p < k && sub == 0) s_order[rank] = static_cast<unsigned char>(p);
             }
-            rank += __shfl_xor_sync(0xffffffffu, rank, 1);
-            rank += __shfl_xor_sync(0xffffffffu, rank, 2);
-            rank += __shfl_xor_sync(0xffffffffu, rank, 4);
-            if (p < k && sub == 0) s_order[rank] = static_cast<unsigned char>(p);
             __syncthreads();
         }
         // Choice (k_choose).
@@ -1998,7 +2002,7 @@ __global__ void __launch_bounds__(kAttemptThreads) k_attempts(const u32* open, c
                                                               const u32* vw, int k, const u32* plan,
                                                               const u64* slack, u64* requests, u64* tried,
                                                               unsigned char* state, int* targets, int* flags) {
-    __shared__ AttemptParts sm;
+    __shared__ AttemptParts<kAttemptThreads> sm;
     extern __shared__ __align__(16) unsigned char attempt_smem_raw[];
     const int count = static_cast<int>(*count_ptr);
     const AttemptDonors<C> donor(attempt_smem_raw, count);
@@ -2015,7 +2019,7 @@ __global__ void __launch_bounds__(kAttemptThreads) k_attempts(const u32* open, c
         donor.list_n[j] = kNoPart;
     }
     __syncthreads();
-    run_attempts<C, D>(sm, donor, count, first_attempt, A, off, nbr, ew, labels, k, plan, targets, flags);
+    run_attempts<C, D, kAttemptThreads>(sm, donor, count, first_attempt, A, off, nbr, ew, labels, k, plan, targets, flags);
     for (int p = threadIdx.x; p < k; p += blockDim.x) requests[p] = sm.requests[p];
     for (int j = threadIdx.x; j < count; j += blockDim.x) {
         const u32 i = open[j];
@@ -2024,43 +2028,22 @@ __global__ void __launch_bounds__(kAttemptThreads) k_attempts(const u32* open, c
         tried[2 * i + 1] = donor.tried[2 * j + 1];
     }
 }
-// A short list (at most kAttemptCap donors) from the collected words to the
-// movers, by one block: the repair order (a bitonic network over the words),
-// the donor test, and all attempts.  One launch in place of two selections, a
-// sort, a scan and the attempts, and nothing for the host to read in between.
-// With a longer list it does nothing and places nobody; the host sees the
-// count with the batch's counters and takes the device-wide path.
-template <class C>
-constexpr size_t repair_block_smem() { return attempt_smem<C>(kAttemptCap) + kAttemptCap * sizeof(u64); }
-template <class C, int D>
-__global__ void __launch_bounds__(kAttemptThreads) k_repair_block(const u64* list, const u64* list_count, const C* A,
-                                                                  const int* off, const int* nbr, const u32* ew,
-                                                                  const int* labels, const u32* vw, int k,
-                                                                  const u32* plan, const int* bound, const u64* start,
-                                                                  const u64* loads, u64 capacity, const u64* slack,
-                                                                  int* targets, int* flags, int* movers, u64* placed) {
-    __shared__ AttemptParts sm;
-    __shared__ u32 s_scan[33];
-    __shared__ u32 s_placed;
-    extern __shared__ __align__(16) unsigned char attempt_smem_raw[];
-    if (*list_count > kAttemptCap) return;
-    const int listed = static_cast<int>(*list_count);
-    u64* word = reinterpret_cast<u64*>(attempt_smem_raw);
-    const AttemptDonors<C> donor(attempt_smem_raw + kAttemptCap * sizeof(u64), kAttemptCap);
+// A short list (at most kAttemptCap donors) put into repair order (a bitonic
+// network over the words) and through the donor test; the active donors are
+// left in `donor`, their number returned.  sm.slack, sm.requests and, as each
+// part's weight before its bounding class, sm.base are set by the caller.
+template <class C, int Threads>
+__device__ int order_donors(AttemptParts<Threads>& sm, const AttemptDonors<C>& donor, u64* word, const u64* list,
+                            int listed, const int* labels, const u32* vw, int k, const u32* plan, const int* bound,
+                            const u64* loads, u64 capacity, u32* scan) {
     int size = 32;
     while (size < listed) size <<= 1;
-    for (int j = threadIdx.x; j < size; j += blockDim.x) word[j] = j < listed ? list[j] : ~0ULL;
-    for (int p = threadIdx.x; p < k; p += blockDim.x) {
-        sm.slack[p] = slack[p];
-        sm.requests[p] = 0;
-        sm.base[p] = bound[p] >= 0 ? start[p] : 0;
-    }
-    if (threadIdx.x == 0) s_placed = 0;
+    for (int j = threadIdx.x; j < size; j += Threads) word[j] = j < listed ? list[j] : ~0ULL;
     __syncthreads();
     for (int kk = 2; kk <= size; kk <<= 1)
         for (int jj = kk >> 1; jj; jj >>= 1) {
-            for (int q = threadIdx.x; q < size / 2; q += blockDim.x) {
-                const int i = (q / jj) * 2 * jj + q % jj;
+            for (int q = threadIdx.x; q < size / 2; q += Threads) {
+                const int i = 2 * q - (q & (jj - 1));  // jj is a power of two
                 const u64 a = word[i], b = word[i + jj];
                 if ((a > b) == ((i & kk) == 0)) {
                     word[i] = b;
@@ -2069,9 +2052,8 @@ __global__ void __launch_bounds__(kAttemptThreads) k_repair_block(const u64* lis
             }
             __syncthreads();
         }
-    // The donor test, and the active donors in repair order.
     int count = 0;
-    for (int chunk = 0; chunk < listed; chunk += blockDim.x) {
+    for (int chunk = 0; chunk < listed; chunk += Threads) {
         const int j = chunk + threadIdx.x;
         const int v = j < listed ? static_cast<int>(word[j] & 0xffffffffULL) : 0;
         const int src = j < listed ? labels[v] : 0;
@@ -2080,7 +2062,7 @@ __global__ void __launch_bounds__(kAttemptThreads) k_repair_block(const u64* lis
         const u64 before = order_chunk(sm, k, t, t >= 0 ? w : 0);
         const bool active = j < listed && (t < 0 || before < loads[src] - capacity);
         u32 total;
-        const u32 slot = block_exclusive_scan_wide<u32>(active ? 1u : 0u, total, s_scan) + static_cast<u32>(count);
+        const u32 slot = block_exclusive_scan_wide<u32>(active ? 1u : 0u, total, scan) + static_cast<u32>(count);
         if (active) {
             donor.v[slot] = static_cast<u32>(v);
             donor.w[slot] = static_cast<u32>(w);
@@ -2092,7 +2074,38 @@ __global__ void __launch_bounds__(kAttemptThreads) k_repair_block(const u64* lis
         count += static_cast<int>(total);
         __syncthreads();
     }
-    run_attempts<C, D>(sm, donor, count, 0, A, off, nbr, ew, labels, k, plan, targets, flags);
+    return count;
+}
+// The listed donors' reservation by one block: repair order, donor test and
+// all attempts.  One launch in place of two selections, a sort, a scan and the
+// attempts, and nothing for the host to read in between.  With more than
+// kAttemptCap listed it does nothing and places nobody; the host sees the
+// count with the batch's counters and takes the device-wide path.
+template <class C>
+constexpr size_t repair_block_smem() { return attempt_smem<C>(kAttemptCap) + kAttemptCap * sizeof(u64); }
+template <class C, int D>
+__global__ void __launch_bounds__(kAttemptThreads) k_repair_block(const u64* list, const u64* list_count, const C* A,
+                                                                  const int* off, const int* nbr, const u32* ew,
+                                                                  const int* labels, const u32* vw, int k,
+                                                                  const u32* plan, const int* bound, const u64* start,
+                                                                  const u64* loads, u64 capacity, const u64* slack,
+                                                                  int* targets, int* flags, int* movers, u64* placed) {
+    __shared__ AttemptParts<kAttemptThreads> sm;
+    __shared__ u32 s_scan[33];
+    __shared__ u32 s_placed;
+    extern __shared__ __align__(16) unsigned char attempt_smem_raw[];
+    if (*list_count > kAttemptCap) return;
+    const AttemptDonors<C> donor(attempt_smem_raw + kAttemptCap * sizeof(u64), kAttemptCap);
+    for (int p = threadIdx.x; p < k; p += blockDim.x) {
+        sm.slack[p] = slack[p];
+        sm.requests[p] = 0;
+        sm.base[p] = bound[p] >= 0 ? start[p] : 0;
+    }
+    if (threadIdx.x == 0) s_placed = 0;
+    const int count = order_donors<C, kAttemptThreads>(sm, donor, reinterpret_cast<u64*>(attempt_smem_raw), list,
+                                                       static_cast<int>(*list_count), labels, vw, k, plan, bound, loads,
+                                                       capacity, s_scan);
+    run_attempts<C, D, kAttemptThreads>(sm, donor, count, 0, A, off, nbr, ew, labels, k, plan, targets, flags);
     __syncthreads();
     for (int j = threadIdx.x; j < count; j += blockDim.x)
         if (donor.state[j] == 1) movers[atomicAdd(&s_placed, 1u)] = static_cast<int>(donor.v[j]);
@@ -2788,8 +2801,25 @@ struct Flagged {
     __device__ bool operator()(i64 v) const { return flags[v] != 0; }
 };
 
+}  // namespace
+}  // namespace gp
+
+#include "gp_refine_cluster.cuh"
+
+namespace gp {
+namespace {
+
 // ---------------------------------------------------------------- host side
 
+// Levels that k_refine_cluster refines: small ones of short rows, which one
+// GPC's worth of SMs handles faster than launches can follow each other.
+// Measured per level against the launch-by-launch path (ms): 256x256 grid,
+// k = 8: 0.68 against 0.88 at 1731 vertices, 1.04 against 1.29 at 20,087, equal
+// at 65,536 (cells 2^19); 256^3 mesh, k = 128: 2.02 against 2.35 at 3852
+// vertices (493 k cells), 3.10 against 2.97 at 12,552 (1.6 M), 7.6 against 4.6
+// at 41,881; skewed graphs, whose coarse rows are long: 1.77 against 1.37 at
+// 1894 vertices of 98 entries, 6.5 against 2.1 at 2315 of 510.
+constexpr i64 kClusterVertices = 65536, kClusterCells = 1 << 19, kClusterEntries = 1 << 18, kClusterRow = 16;
 
 struct LevelResult {
     u64 cut = 0;
@@ -2835,13 +2865,23 @@ private:
     int* movers = nullptr;
     double* prices = nullptr;
     Sample* samples = nullptr;
-    u64* class_weights = nullptr;  // repair: donor weight per part and class (zero between iterations)
+    // Repair: donor weight per part and class (zero between iterations), each
+    // part's bounding class and the weight before it, free room, requests,
+    // prefix sums of the room, and the donors' plans and list.
+    u64* class_weights = nullptr;
+    int* bound = nullptr;
+    u64 *start = nullptr, *slack = nullptr, *requests = nullptr, *cdf = nullptr, *list = nullptr;
+    u32* plan = nullptr;
+    bool in_cluster = false;  // the rounds run in one launch (k_refine_cluster)
+    int* saved_labels = nullptr;
+    u64* saved_loads = nullptr;
     u32* state = nullptr;      // packed label / target / batch bit per vertex (dense-cache levels)
     int* chunk_work = nullptr;      // chunks of the heavy rows taking part in a batch (k_heavy_chunk_list)
     u64* chunk_work_count = nullptr;
     u64* counters = nullptr;  // device: 0 cand, 1 movers, 2 delta, 3 max load, 4.. scratch
     long long* corr_acc = nullptr;  // per heavy row: priority-filter correction
     u64 cut = 0, revision = 0;
+    u64 feasible_start = 0;  // cut once the parts first fit
     u64 rebuild_entries = ~0ULL;  // mover entries above which apply() rebuilds the cache
     i64 repair_iterations = 0, repair_donors = 0;  // for the per-level log line
     i64 last_listed = 0;  // donors the last repair iteration listed
@@ -3037,9 +3077,11 @@ private:
     }
     void enqueue_lp_round(double filter);
     i64 lp_round(double filter);
-    bool repair();
-    void offer_list(const u64* list_count, u64* placed_count, const u32* plan, const u64* list, const int* bound,
-                    const u64* start, const u64* slack);
+    bool repair(i64 interrupted = 0, int iterations = 0);
+    void restore_best(bool moved);
+    u64 propagate(double filter, int& rounds, bool& restored);
+    void refine_in_cluster(double filter, LevelResult& res, int& rounds, bool& restored);
+    void offer_list(const u64* list_count, u64* placed_count);
     void reserve_long(i64 listed, u64* list, const u32* plan, const int* bound, const u64* start, const u64* slack,
                       u64* requests);
     void exchange(u64& best);
@@ -3092,58 +3134,59 @@ i64 LevelRefiner<T>::lp_round(double filter) {
 
 // One capacity repair (RebalanceGraph, rebalance_graph.cuh:160-280) in the
 // deterministic order.  Returns feasibility.
+// `interrupted`: the donors already listed by k_refine_cluster, in its
+// iteration number `iterations`, that one block could not take.
 template <class T>
-bool LevelRefiner<T>::repair() {
+bool LevelRefiner<T>::repair(i64 interrupted, int iterations) {
     if (max_load_host <= C) return true;
     Arena& A_ = ctx.scratch;
-    ArenaScope scope(A_);
-    u64* slack = A_.alloc<u64>(k);
-    u64* requests = A_.alloc<u64>(k);
-    u64* cdf = A_.alloc<u64>(k + 1);
-    int* bound = A_.alloc<int>(k);
-    u64* start = A_.alloc<u64>(k);
-    u32* plan = A_.alloc<u32>(n);
-    u64* list = A_.alloc<u64>(n);
     // counters[9]: placed donors, [10]: donors, [11]: listed donors.
     u64 *placed_count = counters + 9, *donor_count = counters + 10, *list_count = counters + 11;
-    int iterations = 0;
+    auto read_batch = [&]() {
+        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 2, 10 * sizeof(u64), cudaMemcpyDeviceToHost, s()));
+        GP_CUDA(cudaStreamSynchronize(s()));
+    };
     while (true) {
         ArenaScope it(A_);
-        launch(k_slack, 1, kMaxParts, 0, s(), k, loads, C, slack, requests, cdf, counters + 9);
-        if (on_demand)
-            with_row_size([&](auto d) {
-                launch(k_repair_dest_od<decltype(d)::value>, grid_for(n, kThreads), kThreads, 0, s(), n,
-                       static_cast<const int*>(g.off), static_cast<const int*>(g.nbr), static_cast<const u32*>(g.ew),
-                       static_cast<const int*>(labels), static_cast<const u32*>(g.vw), k,
-                       static_cast<const u64*>(loads), C, static_cast<const u64*>(cdf), plan, class_weights,
-                       donor_count);
-            });
-        else
-            with_groups([&](auto width, auto vec) {
-                constexpr int W = decltype(width)::value;
-                launch(k_repair_dest<T, W, decltype(vec)::value>, grid_for(n, kThreads), kThreads, 0, s(), n,
-                       static_cast<const T*>(A), static_cast<const T*>(totals), static_cast<const int*>(labels),
-                       static_cast<const u32*>(g.vw), k, static_cast<const u64*>(loads), C,
-                       static_cast<const u64*>(cdf), plan, class_weights, donor_count);
-            });
-        launch(k_repair_bounds, k, kScanThreads, 0, s(), static_cast<const u64*>(loads), C, class_weights, bound,
-               start);
-        launch(k_repair_list, grid_for(n, kThreads), kThreads, 0, s(), n, k, static_cast<const int*>(labels),
-               static_cast<const u32*>(plan), static_cast<const int*>(bound), list, list_count);
-        // The next list is mostly about as long as the last one: after a long
-        // one, its length is read first instead of offering it to one block.
-        const bool offered = last_listed <= kAttemptCap;
-        if (offered) offer_list(list_count, placed_count, plan, list, bound, start, slack);
-        auto read_batch = [&]() {
-            GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 2, 10 * sizeof(u64), cudaMemcpyDeviceToHost, s()));
-            GP_CUDA(cudaStreamSynchronize(s()));
-        };
-        read_batch();
-        const i64 listed = static_cast<i64>(ctx.host_scalars[9]);
-        last_listed = listed;
+        i64 listed = interrupted;
+        bool offered = false;
+        interrupted = 0;
+        if (listed) {
+            GP_CUDA(cudaMemsetAsync(counters + 2, 0, 10 * sizeof(u64), s()));
+        } else {
+            launch(k_slack, 1, kMaxParts, 0, s(), k, loads, C, slack, requests, cdf, counters + 9);
+            if (on_demand)
+                with_row_size([&](auto d) {
+                    launch(k_repair_dest_od<decltype(d)::value>, grid_for(n, kThreads), kThreads, 0, s(), n,
+                           static_cast<const int*>(g.off), static_cast<const int*>(g.nbr), static_cast<const u32*>(g.ew),
+                           static_cast<const int*>(labels), static_cast<const u32*>(g.vw), k,
+                           static_cast<const u64*>(loads), C, static_cast<const u64*>(cdf), plan, class_weights,
+                           donor_count);
+                });
+            else
+                with_groups([&](auto width, auto vec) {
+                    constexpr int W = decltype(width)::value;
+                    launch(k_repair_dest<T, W, decltype(vec)::value>, grid_for(n, kThreads), kThreads, 0, s(), n,
+                           static_cast<const T*>(A), static_cast<const T*>(totals), static_cast<const int*>(labels),
+                           static_cast<const u32*>(g.vw), k, static_cast<const u64*>(loads), C,
+                           static_cast<const u64*>(cdf), plan, class_weights, donor_count);
+                });
+            launch(k_repair_bounds, k, kScanThreads, 0, s(), static_cast<const u64*>(loads), C, class_weights, bound,
+                   start);
+            launch(k_repair_list, grid_for(n, kThreads), kThreads, 0, s(), n, k, static_cast<const int*>(labels),
+                   static_cast<const u32*>(plan), static_cast<const int*>(bound), list, list_count);
+            // The next list is mostly about as long as the last one: after a
+            // long one, its length is read first instead of offering it to
+            // one block.
+            offered = last_listed <= kAttemptCap;
+            if (offered) offer_list(list_count, placed_count);
+            read_batch();
+            listed = static_cast<i64>(ctx.host_scalars[9]);
+            last_listed = listed;
+            repair_donors += static_cast<i64>(ctx.host_scalars[8]);
+        }
         ++repair_iterations;
-        repair_donors += static_cast<i64>(ctx.host_scalars[8]);
-        if (listed > kAttemptCap || !offered) {
+        if (!offered || listed > kAttemptCap) {
             reserve_long(listed, list, plan, bound, start, slack, requests);
             read_batch();
         }
@@ -3169,8 +3212,7 @@ bool LevelRefiner<T>::repair() {
 // placed, their count on the device: one read-back then brings the counts and
 // the batch's counters together.  An empty batch changes nothing.
 template <class T>
-void LevelRefiner<T>::offer_list(const u64* list_count, u64* placed_count, const u32* plan, const u64* list,
-                                 const int* bound, const u64* start, const u64* slack) {
+void LevelRefiner<T>::offer_list(const u64* list_count, u64* placed_count) {
     auto go = [&](auto d) {
         // Sized for kAttemptCap donors (the count is on the device); the limit
         // is set on every call, as it belongs to the kernel on whichever
@@ -3305,6 +3347,128 @@ void LevelRefiner<T>::reserve_long(i64 listed, u64* list, const u32* plan, const
     select_if(A_, s(), acount, IsPlaced{state}, WriteActiveVertex{active, movers},
               reinterpret_cast<u32*>(counters + 9));
     apply(movers, counters + 9, acount, false, samples != nullptr);
+}
+
+// The initial repair and the label-propagation rounds by k_refine_cluster.
+// The host only steps in where a repair lists more donors than one block
+// orders, and starts the kernel again after it.
+template <class T>
+void LevelRefiner<T>::refine_in_cluster(double filter, LevelResult& res, int& rounds, bool& restored) {
+    if constexpr (std::is_same_v<T, u32>) {
+        Arena& A_ = ctx.scratch;
+        ArenaScope scope(A_);
+        // Each block's share of the vertices, in passes of kClusterThreads.
+        const int passes = blocks_for(n, kClusterThreads * kClusterBlocks);
+        const int region = passes * kClusterThreads;
+        ClusterLevel<T> L{};
+        L.n = n;
+        L.k = k;
+        L.max_rounds = budget.rounds;
+        L.heavy_min = mapping.refine_heavy_small;
+        L.region = region;
+        L.capacity = C;
+        L.filter = filter;
+        L.off = g.off;
+        L.nbr = g.nbr;
+        L.ew = g.ew;
+        L.vw = g.vw;
+        L.labels = labels;
+        L.loads = loads;
+        L.A = A;
+        L.totals = totals;
+        L.gains = gains;
+        L.proposal = proposal;
+        L.locks = locks;
+        L.flags = flags;
+        L.targets = targets;
+        L.state = state;
+        L.samples = samples;
+        L.prices = prices;
+        L.cand = A_.alloc<int>(static_cast<size_t>(region) * kClusterBlocks);
+        L.movers = A_.alloc<int>(std::max<size_t>(static_cast<size_t>(region) * kClusterBlocks, kAttemptCap));
+        L.plan = plan;
+        L.class_weights = class_weights;
+        L.bound = bound;
+        L.start = start;
+        L.list = list;
+        L.slack = slack;
+        L.requests = requests;
+        L.saved_labels = saved_labels;
+        L.saved_loads = saved_loads;
+        L.ctl = A_.alloc<u64>(4 * kCtlWords);
+        L.io = A_.alloc<ClusterState>(1);
+        static_assert(sizeof(ClusterState) <= sizeof(u64) * kScalars, "staged in the context's scalars");
+        GP_CUDA(cudaMemsetAsync(L.ctl, 0, sizeof(u64) * 4 * kCtlWords, s()));
+        constexpr size_t smem = cluster_smem<T>();
+        GP_CUDA(cudaFuncSetAttribute(k_refine_cluster<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        GP_CUDA(cudaFuncSetAttribute(k_refine_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     static_cast<int>(smem)));
+        ClusterState st{};
+        st.loop.cut = cut;
+        st.loop.start = kStartLevel;
+        while (true) {
+            auto* staged = reinterpret_cast<ClusterState*>(ctx.host_scalars);
+            *staged = st;
+            GP_CUDA(cudaMemcpyAsync(L.io, staged, sizeof(ClusterState), cudaMemcpyHostToDevice, s()));
+            launch_cluster(k_refine_cluster<T>, kClusterBlocks, kClusterThreads, smem, s(), L);
+            GP_CUDA(cudaMemcpyAsync(staged, L.io, sizeof(ClusterState), cudaMemcpyDeviceToHost, s()));
+            GP_CUDA(cudaStreamSynchronize(s()));
+            st = *staged;
+            max_load_host = st.max_load;
+            cut = st.loop.cut;
+            const int status = st.loop.status;
+            if (status == kClusterCutUnderflow) fail(GP_INTERNAL, "incremental cut underflow");
+            if (status != kClusterHostInitialRepair && status != kClusterHostRoundRepair) break;
+            // A long repair, completed step by step.  Its statistics go to
+            // `stats`, the kernel's own are added at the end.
+            const i64 listed = static_cast<i64>(st.listed);
+            const u64 before = revision;
+            const bool feasible = repair(listed, static_cast<int>(st.iterations));
+            st.loop.cut = cut;
+            st.loop.status = kClusterDone;
+            if (revision != before) st.loop.moved = 1;
+            if (!feasible && status == kClusterHostInitialRepair) {
+                st.loop.status = kClusterInitialRepairFailed;
+                break;
+            }
+            if (!feasible) {  // the rounds end here
+                restore_best(st.loop.moved != 0);
+                break;
+            }
+            st.loop.start = status == kClusterHostInitialRepair ? kStartAfterInitialRepair : kStartAfterRoundRepair;
+        }
+        stats.proposals += st.totals.proposals;
+        stats.accepted += st.totals.accepted;
+        stats.lp_gain += st.totals.lp_gain;
+        stats.lp_loss += st.totals.lp_loss;
+        stats.rebalance_gain += st.totals.rebalance_gain;
+        stats.rebalance_loss += st.totals.rebalance_loss;
+        stats.admission_iterations += static_cast<int>(st.totals.admission_iterations);
+        stats.checkpoint_updates += static_cast<int>(st.totals.checkpoint_updates);
+        repair_iterations += static_cast<i64>(st.totals.admission_iterations);
+        repair_donors += static_cast<i64>(st.totals.repair_donors);
+        rounds = st.loop.rounds;
+        restored = st.loop.moved != 0;
+        res.repair_failed = st.loop.status == kClusterInitialRepairFailed;
+        if (!res.repair_failed) {
+            cut = st.loop.best;
+            feasible_start = st.loop.feasible_start;
+        }
+    }
+}
+
+// Back to the best labels and loads of the rounds (the cache is not).
+template <class T>
+void LevelRefiner<T>::restore_best(bool moved) {
+    if (!moved) return;
+    GP_CUDA(cudaMemcpyAsync(labels, saved_labels, sizeof(int) * n, cudaMemcpyDeviceToDevice, s()));
+    if (state)
+        launch(k_state_init, grid_for(n, kThreads), kThreads, 0, s(), n, static_cast<const int*>(labels), state);
+    GP_CUDA(cudaMemcpyAsync(loads, saved_loads, sizeof(u64) * k, cudaMemcpyDeviceToDevice, s()));
+    launch(k_max_load, 1, 32, 0, s(), k, loads, counters + 3);
+    GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 3, sizeof(u64), cudaMemcpyDeviceToHost, s()));
+    GP_CUDA(cudaStreamSynchronize(s()));
+    max_load_host = ctx.host_scalars[0];
 }
 
 template <class T>
@@ -3454,6 +3618,60 @@ void LevelRefiner<T>::exchange(u64& best_cut) {
     }
 }
 
+// The label-propagation rounds of a level whose parts fit, launch by launch;
+// leaves the best labels in place and returns their cut.
+template <class T>
+u64 LevelRefiner<T>::propagate(double filter, int& rounds, bool& restored) {
+    Arena& A_ = ctx.scratch;
+    // Levels above 65,536 vertices (no exchange step): the LP proposals visit
+    // a conservative frontier when it starts with at most a quarter of the
+    // rows (the reference's rule, incremental.cuh:783-797).
+    if (n > 65536) {
+        frontier.members = A_.alloc<int>(n);
+        frontier.rows = A_.alloc<int>(n);
+        frontier.count = A_.alloc<u64>(1);
+        GP_CUDA(cudaMemsetAsync(frontier.count, 0, sizeof(u64), s()));
+        if (on_demand)
+            with_row_size([&](auto d) {
+                launch(k_frontier_init_od<decltype(d)::value>, grid_for(n, kThreads), kThreads, 0, s(), n,
+                       static_cast<const int*>(g.off), static_cast<const int*>(g.nbr), static_cast<const u32*>(g.ew),
+                       static_cast<const int*>(labels), targets, frontier);
+            });
+        else
+            launch(k_frontier_init<T>, grid_for(n, kThreads), kThreads, 0, s(), n, static_cast<const T*>(A),
+                   static_cast<const T*>(totals), k, static_cast<const int*>(labels), targets, frontier);
+        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, frontier.count, sizeof(u64), cudaMemcpyDeviceToHost, s()));
+        GP_CUDA(cudaStreamSynchronize(s()));
+        frontier_on = ctx.host_scalars[0] <= static_cast<u64>(n) / 4;
+    }
+    u64 best = cut;
+    GP_CUDA(cudaMemcpyAsync(saved_labels, labels, sizeof(int) * n, cudaMemcpyDeviceToDevice, s()));
+    GP_CUDA(cudaMemcpyAsync(saved_loads, loads, sizeof(u64) * k, cudaMemcpyDeviceToDevice, s()));
+    u64 best_revision = revision;
+    int stale = 0, empty = 0;
+    for (int phase = 0; phase < budget.rounds && stale < 3; ++phase) {
+        ++rounds;
+        if (samples) GP_CUDA(cudaMemsetAsync(samples, 0, sizeof(Sample) * k, s()));
+        const i64 count = lp_round(filter);
+        if (!count) { if (++empty >= 2) break; ++stale; continue; }
+        empty = 0;
+        if (!repair()) break;
+        if (prices) launch(k_prices, 1, 128, 0, s(), k, static_cast<const Sample*>(samples), prices);
+        ++stale;
+        if (cut < best) {
+            if (best - cut > best / 1000) stale = 0;
+            best = cut;
+            GP_CUDA(cudaMemcpyAsync(saved_labels, labels, sizeof(int) * n, cudaMemcpyDeviceToDevice, s()));
+            GP_CUDA(cudaMemcpyAsync(saved_loads, loads, sizeof(u64) * k, cudaMemcpyDeviceToDevice, s()));
+            best_revision = revision;
+            ++stats.checkpoint_updates;
+        }
+    }
+    restored = revision != best_revision;
+    restore_best(restored);
+    return best;
+}
+
 // run_incremental_refinement_typed (incremental.cuh:660-1051).
 template <class T>
 LevelResult LevelRefiner<T>::run(bool has_known, u64 known) {
@@ -3463,9 +3681,12 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known) {
     // Smaller levels: rows above a lower threshold (coarse hubs) go through
     // the block-per-chunk kernels instead of one warp each, which otherwise
     // set the time of every row-parallel pass of the level.
+    // (No level this small goes without a cache.)
+    in_cluster = std::is_same_v<T, u32> && !verify && n <= kClusterVertices && n * k <= kClusterCells &&
+                 g.m <= kClusterEntries && g.m <= kClusterRow * n;
     const int heavy_min = n <= 65536 ? mapping.refine_heavy_small
                           : n <= (1 << 20) ? mapping.refine_heavy_mid : mapping.refine_heavy_large;
-    if (heavy_min != g.heavy_min && (g.maximum_degree > static_cast<u64>(std::min(heavy_min, g.heavy_min)) || g.heavy_count))
+    if (!in_cluster && heavy_min != g.heavy_min && (g.maximum_degree > static_cast<u64>(std::min(heavy_min, g.heavy_min)) || g.heavy_count))
         build_chunks(ctx, g, heavy_min, &A_);
     uint64_t cap = 0;
     if (gp_status st = capacity_of(total, k, eps, &cap); st != GP_OK) fail(st, last_error());
@@ -3508,8 +3729,8 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known) {
         chunk_work = A_.alloc<int>(g.chunks);
         chunk_work_count = A_.alloc<u64>(1);
     }
-    int* saved_labels = A_.alloc<int>(n);
-    u64* saved_loads = A_.alloc<u64>(k);
+    saved_labels = A_.alloc<int>(n);
+    saved_loads = A_.alloc<u64>(k);
     GP_CUDA(cudaMemsetAsync(locks, 0, n, s()));
     GP_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * n, s()));
     fill<int>(s(), targets, n, -1);
@@ -3519,6 +3740,13 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known) {
         GP_CUDA(cudaMemsetAsync(prices, 0, sizeof(double) * k, s()));
         GP_CUDA(cudaMemsetAsync(samples, 0, sizeof(Sample) * k, s()));
     }
+    slack = A_.alloc<u64>(k);
+    requests = A_.alloc<u64>(k);
+    cdf = A_.alloc<u64>(k + 1);
+    bound = A_.alloc<int>(k);
+    start = A_.alloc<u64>(k);
+    plan = A_.alloc<u32>(n);
+    list = A_.alloc<u64>(n);
     class_weights = A_.alloc<u64>(static_cast<size_t>(k) * kBalanceWidth);
     GP_CUDA(cudaMemsetAsync(class_weights, 0, sizeof(u64) * k * kBalanceWidth, s()));
     // An entry-by-entry update touches two random cache counters per entry
@@ -3532,10 +3760,12 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known) {
         launch(k_state_init, grid_for(n, kThreads), kThreads, 0, s(), n, static_cast<const int*>(labels), state);
     }
     build(has_known ? nullptr : counters + 7);
-    launch(k_max_load, 1, 32, 0, s(), k, loads, counters + 3);
-    GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 3, 5 * sizeof(u64), cudaMemcpyDeviceToHost, s()));
-    GP_CUDA(cudaStreamSynchronize(s()));
-    max_load_host = ctx.host_scalars[0];
+    if (!in_cluster || !has_known) {  // the cluster kernel reads the loads itself
+        launch(k_max_load, 1, 32, 0, s(), k, loads, counters + 3);
+        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 3, 5 * sizeof(u64), cudaMemcpyDeviceToHost, s()));
+        GP_CUDA(cudaStreamSynchronize(s()));
+        max_load_host = ctx.host_scalars[0];
+    }
     if (has_known) {
         cut = known;
     } else if (on_demand) {
@@ -3546,77 +3776,27 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known) {
     }
     LevelResult res;
     stats.initial_cut = cut;
-    if (max_load_host > C) {
-        if (!repair()) {
-            res.cut = cut;
-            res.repair_failed = true;
-            stats.repair_failed = true;
-            stats.final_cut = cut;
-            stats.final_max_load = max_load_host;
-            return res;
-        }
-    }
-    // Levels above 65,536 vertices (no exchange step): the LP proposals visit
-    // a conservative frontier when it starts with at most a quarter of the
-    // rows (the reference's rule, incremental.cuh:783-797).
-    if (n > 65536) {
-        frontier.members = A_.alloc<int>(n);
-        frontier.rows = A_.alloc<int>(n);
-        frontier.count = A_.alloc<u64>(1);
-        GP_CUDA(cudaMemsetAsync(frontier.count, 0, sizeof(u64), s()));
-        if (on_demand)
-            with_row_size([&](auto d) {
-                launch(k_frontier_init_od<decltype(d)::value>, grid_for(n, kThreads), kThreads, 0, s(), n,
-                       static_cast<const int*>(g.off), static_cast<const int*>(g.nbr), static_cast<const u32*>(g.ew),
-                       static_cast<const int*>(labels), targets, frontier);
-            });
-        else
-            launch(k_frontier_init<T>, grid_for(n, kThreads), kThreads, 0, s(), n, static_cast<const T*>(A),
-                   static_cast<const T*>(totals), k, static_cast<const int*>(labels), targets, frontier);
-        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, frontier.count, sizeof(u64), cudaMemcpyDeviceToHost, s()));
-        GP_CUDA(cudaStreamSynchronize(s()));
-        frontier_on = ctx.host_scalars[0] <= static_cast<u64>(n) / 4;
-    }
-    const u64 feasible_start = cut;
-    u64 best = cut;
-    GP_CUDA(cudaMemcpyAsync(saved_labels, labels, sizeof(int) * n, cudaMemcpyDeviceToDevice, s()));
-    GP_CUDA(cudaMemcpyAsync(saved_loads, loads, sizeof(u64) * k, cudaMemcpyDeviceToDevice, s()));
-    u64 best_revision = revision;
     double filter = 0.25;
     if (g.ew) {
         ctx.clear_scalars(1);
         launch(k_max_edge, std::min(blocks_for(g.m, kThreads), 148 * 8), kThreads, 0, s(), g.m, g.ew, ctx.dev_scalars);
         filter = ctx.read_scalars(1)[0] <= 1 ? 0.25 : 0.75;
     }
-    int stale = 0, empty = 0, rounds = 0;
-    for (int phase = 0; phase < budget.rounds && stale < 3; ++phase) {
-        ++rounds;
-        if (samples) GP_CUDA(cudaMemsetAsync(samples, 0, sizeof(Sample) * k, s()));
-        const i64 count = lp_round(filter);
-        if (!count) { if (++empty >= 2) break; ++stale; continue; }
-        empty = 0;
-        if (!repair()) break;
-        if (prices) launch(k_prices, 1, 128, 0, s(), k, static_cast<const Sample*>(samples), prices);
-        ++stale;
-        if (cut < best) {
-            if (best - cut > best / 1000) stale = 0;
-            best = cut;
-            GP_CUDA(cudaMemcpyAsync(saved_labels, labels, sizeof(int) * n, cudaMemcpyDeviceToDevice, s()));
-            GP_CUDA(cudaMemcpyAsync(saved_loads, loads, sizeof(u64) * k, cudaMemcpyDeviceToDevice, s()));
-            best_revision = revision;
-            ++stats.checkpoint_updates;
-        }
+    int rounds = 0;
+    bool restored = false;
+    if (in_cluster) refine_in_cluster(filter, res, rounds, restored);
+    else if (max_load_host > C) res.repair_failed = !repair();
+    if (res.repair_failed) {
+        res.cut = cut;
+        stats.repair_failed = true;
+        stats.final_cut = cut;
+        stats.final_max_load = max_load_host;
+        return res;
     }
-    const bool restored = revision != best_revision;
-    if (restored) {
-        GP_CUDA(cudaMemcpyAsync(labels, saved_labels, sizeof(int) * n, cudaMemcpyDeviceToDevice, s()));
-        if (state)
-            launch(k_state_init, grid_for(n, kThreads), kThreads, 0, s(), n, static_cast<const int*>(labels), state);
-        GP_CUDA(cudaMemcpyAsync(loads, saved_loads, sizeof(u64) * k, cudaMemcpyDeviceToDevice, s()));
-        launch(k_max_load, 1, 32, 0, s(), k, loads, counters + 3);
-        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 3, sizeof(u64), cudaMemcpyDeviceToHost, s()));
-        GP_CUDA(cudaStreamSynchronize(s()));
-        max_load_host = ctx.host_scalars[0];
+    u64 best = cut;
+    if (!in_cluster) {
+        feasible_start = cut;
+        best = propagate(filter, rounds, restored);
     }
     cut = best;
     if (budget.rounds > 0 && budget.exchange_rounds > 0 && n <= 65536) {
