@@ -38,14 +38,15 @@ constexpr int kMediumWarps = 4;
 // record_bound_kernel (src/coarsen.cu:51-99) plus the weight invariants of
 // aggregate_typed (:483-493).  Scalars: 0 max row bound, 1 unsorted,
 // 2 zero weight, 3 non-unit weight, 4 max raw degree, 5 total vertex
-// weight, 6 max vertex weight.
+// weight, 6 max vertex weight, 7 directed edge-weight sum (the packed-weight
+// decision, src/coarsen.cu:1839-1848).
 template <int W>
 __global__ void __launch_bounds__(256) k_level0_meta(i64 n, const int* off, const int* nbr, const u32* ew,
                                                      const u32* vw, u64* bounds, u64* sc) {
     const int lane = threadIdx.x & (W - 1);
     constexpr int kGroups = 32 / W;  // rows per warp and pass
     const i64 warps = (static_cast<i64>(gridDim.x) * blockDim.x) >> 5;
-    u64 d_max = 0, raw_max = 0, total = 0, v_max = 0;
+    u64 d_max = 0, raw_max = 0, total = 0, v_max = 0, directed = 0;
     u32 flags = 0;
     // Warp-uniform pass count, so the group shuffles see the whole warp.
     for (i64 base = ((static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kGroups; base < n;
@@ -69,6 +70,7 @@ __global__ void __launch_bounds__(256) k_level0_meta(i64 n, const int* off, cons
         }
         if (valid && lane == 0) {
             bounds[v] = d;
+            directed += d;
             d_max = d > d_max ? d : d_max;
             raw_max = static_cast<u64>(end - begin) > raw_max ? static_cast<u64>(end - begin) : raw_max;
             total += vw[v];
@@ -82,6 +84,7 @@ __global__ void __launch_bounds__(256) k_level0_meta(i64 n, const int* off, cons
     block_atomic_max(sc + 4, raw_max);
     block_atomic_add(sc + 5, total);
     block_atomic_max(sc + 6, v_max);
+    block_atomic_add(sc + 7, directed);
 }
 
 // Heavy rows of record_bound_kernel, one block per chunk.
@@ -100,7 +103,10 @@ __global__ void k_level0_meta_chunks(DGraph g, u64* bounds, u64* sc) {
     d = warp_sum(d);
     flags = __reduce_or_sync(0xffffffffu, flags);
     if ((threadIdx.x & 31) == 0) {
-        if (d) atomicAdd(bounds + v, d);
+        if (d) {
+            atomicAdd(bounds + v, d);
+            atomicAdd(sc + 7, d);
+        }
         if (flags & 1u) atomicOr(sc + 1, 1ULL);
         if (flags & 2u) atomicOr(sc + 2, 1ULL);
         if (flags & 4u) atomicOr(sc + 3, 1ULL);
@@ -109,15 +115,6 @@ __global__ void k_level0_meta_chunks(DGraph g, u64* bounds, u64* sc) {
 __global__ void k_heavy_bound_max(i64 count, const int* heavy, const u64* bounds, u64* sc) {
     const i64 h = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (h < count) atomicMax(sc + 0, bounds[heavy[h]]);
-}
-
-// Directed edge-weight sum (packed-weight decision, src/coarsen.cu:1839-1848).
-__global__ void k_weight_sum(i64 m, const u32* ew, u64* out) {
-    u64 s = 0;
-    for (i64 e = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += static_cast<i64>(gridDim.x) * blockDim.x)
-        s += ew[e];
-    s = warp_sum(s);
-    if ((threadIdx.x & 31) == 0 && s) atomicAdd(out, s);
 }
 
 // Degree classes (sclp_compact_degree_classes, aggregation.cuh:5-71): exact
@@ -203,23 +200,22 @@ __global__ void k_match_choose(i64 n, const int* off, const int* nbr, const u32*
 }
 
 // matching_commit + matching_roots + residual_seed_weights.
-__global__ void k_match_roots(i64 n, const int* choice, int* clusters) {
-    const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (v >= n) return;
-    const int u = choice[v];
-    int root = static_cast<int>(v);
-    if (u >= 0 && choice[u] == v) root = min(static_cast<int>(v), u);
-    clusters[v] = root;
+// *merged counts the pairs.
+__global__ void k_match_roots(i64 n, const int* choice, int* clusters, u64* merged) {
+    u64 pairs = 0;
+    for (i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += static_cast<i64>(gridDim.x) * blockDim.x) {
+        const int u = choice[v];
+        int root = static_cast<int>(v);
+        if (u >= 0 && choice[u] == v) root = min(static_cast<int>(v), u);
+        clusters[v] = root;
+        pairs += root != v;
+    }
+    block_atomic_add(merged, pairs);
 }
 
 __global__ void k_cluster_weights(i64 n, const int* clusters, const u32* vw, u64* cw) {
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (v < n) atomicAdd(cw + clusters[v], static_cast<u64>(vw[v]));
-}
-
-__global__ void k_count_nonzero(i64 n, const u64* values, u64* out) {
-    const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    block_atomic_add(out, i < n && values[i] != 0 ? 1ULL : 0ULL);
 }
 
 // ---------------------------------------------------------------- rounds
@@ -241,14 +237,16 @@ struct RoundParams {
     u64* gains;
     u64* regret;
     u32* ties;
+    u64* demand;  // per cluster, the weight proposed to it (nullptr: not needed)
 };
 
-// residual_freeze_roles (singleton_growth.cuh:27-40); also resets proposals.
+// residual_freeze_roles (singleton_growth.cuh:27-40); also resets proposals
+// and, with `demand`, the weight proposed to each cluster.
 // Also writes recv[v], the cluster weight with the role folded in (all ones
 // for a mover, which no capacity admits), so that considering a neighbour
 // cluster is one gather instead of the role and weight gathers.
 __global__ void k_roles(i64 n, const int* clusters, const u32* vw, const u64* cw, u32 salt, u32 threshold,
-                        bool all_singletons, unsigned char* roles, u64* recv, int* proposals) {
+                        bool all_singletons, unsigned char* roles, u64* recv, int* proposals, u64* demand) {
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (v >= n) return;
     const u64 weight = cw[v];
@@ -257,6 +255,7 @@ __global__ void k_roles(i64 n, const int* clusters, const u32* vw, const u64* cw
     roles[v] = role;
     recv[v] = role ? ~0ULL : weight;
     proposals[v] = kInvalid;
+    if (demand) demand[v] = 0;
 }
 
 // Candidate summary of one row: best (value, tie) with the reference's
@@ -331,6 +330,7 @@ __device__ __forceinline__ void decode(const RoundParams& p, int v, int src, con
     const int target = static_cast<int>(0xffffffffULL - (s.tie & 0xffffffffULL));
     if (target < 0 || target == src) return;
     p.proposals[v] = target;
+    if (p.demand) atomicAdd(p.demand + target, static_cast<u64>(p.vw[v]));
     p.gains[v] = gain;
     if (p.second_on) p.regret[v] = s.best - s.second;
     p.ties[v] = static_cast<u32>(s.tie >> 32);
@@ -643,14 +643,10 @@ __global__ void k_emit_segments(i64 count, const int* heavy, const int* off, con
     }
 }
 
-// Admission (src/coarsen.cu:1015-1075).  Total demand per target first;
-// requests to a target whose whole demand fits are accepted without any
-// ordering, the rest are ordered by (target, regret desc, tie desc, vertex).
-__global__ void k_requests(i64 n, const int* proposals, const u32* vw, u64* demand) {
-    const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (v < n && proposals[v] != kInvalid) atomicAdd(demand + proposals[v], static_cast<u64>(vw[v]));
-}
-
+// Admission (src/coarsen.cu:1015-1075).  Total demand per target first
+// (summed by decode()); requests to a target whose whole demand fits are
+// accepted without any ordering, the rest are ordered by (target, regret
+// desc, tie desc, vertex).
 // accept: 0 reject, 1 accept, 2 needs the ordered prefix test.
 __global__ void k_classify(i64 n, const int* proposals, const u64* cw, const u64* demand, u64 capacity,
                            unsigned char* accept) {
@@ -685,13 +681,26 @@ __global__ void k_key_target(i64 count, const u32* items, const int* targets, u6
     if (i < count) keys[i] = static_cast<u64>(targets[items[i]]);
 }
 
-// order_by_target for at most one sort tile of items, in one block: each of
-// the three stable stages builds its keys from the current order and sorts
-// them in shared memory, the same passes the separate launches make.
-__global__ void __launch_bounds__(kSortThreads) k_order_small(int count, u32* items, const u32* ties,
+// The ordered part of an admission (or, with Pairs, of the two-hop pairing)
+// for at most one sort tile of items, in one block: the three stable stages of
+// order_by_target, each building its keys from the current order, then the
+// weight prefix (or rank) within each item's target group, found by a binary
+// search over the ordered targets.  The item count is on the device; with more
+// items than a tile it does nothing, and the host, which reads the count with
+// the round's results, takes the device-wide path.  Small levels spend their
+// time between launches and on read-backs, not in the kernels: this replaces
+// five launches and one read-back per round.
+template <bool Pairs>
+__global__ void __launch_bounds__(kSortThreads) k_order_block(const u32* count_ptr, const u32* items, const u32* ties,
                                                              const u64* key_values, u64 mask, int key_bits,
-                                                             const int* targets, int target_bits) {
+                                                             const int* targets, int target_bits, const u32* vw,
+                                                             u64* cw, u64 capacity, unsigned char* accept, u64 budget,
+                                                             int* clusters, u64* merged) {
     __shared__ SortTileSmem sm;
+    __shared__ u64 scan64[33];
+    __shared__ u32 scan32[33];
+    if (*count_ptr > kSortTile) return;
+    const int count = static_cast<int>(*count_ptr);
     u64 k[kSortItems];
     u32 v[kSortItems];
     bool valid[kSortItems];
@@ -712,9 +721,83 @@ __global__ void __launch_bounds__(kSortThreads) k_order_small(int count, u32* it
 #pragma unroll
     for (int j = 0; j < kSortItems; ++j) k[j] = valid[j] ? static_cast<u64>(targets[v[j]]) : 0;
     tile_sort_passes<true>(sm, k, v, valid, 0, target_bits);
+    // Order in shared memory, then eight consecutive items per thread.
+    __shared__ int s_target[kSortTile];
 #pragma unroll
     for (int j = 0; j < kSortItems; ++j)
-        if (valid[j]) items[sort_index(0, j)] = v[j];
+        if (valid[j]) {
+            const i64 i = sort_index(0, j);
+            sm.vals[i] = v[j];
+            s_target[i] = targets[v[j]];
+        }
+    __syncthreads();
+    const int first = static_cast<int>(threadIdx.x) * kSortItems;
+    auto head = [&](int i) {  // first item of i's target
+        const int t = s_target[i];
+        int lo = 0, hi = i;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (s_target[mid] < t) lo = mid + 1;
+            else hi = mid;
+        }
+        return lo;
+    };
+    if constexpr (!Pairs) {
+        // sclp_commit_kernel's test (aggregation.cuh:641): base <= C and the
+        // inclusive weight prefix within the target fits in C - base.
+        u64 w[kSortItems], local = 0;
+#pragma unroll
+        for (int j = 0; j < kSortItems; ++j) {
+            w[j] = first + j < count ? vw[sm.vals[first + j]] : 0;
+            local += w[j];
+        }
+        u64 total;
+        u64 run = block_exclusive_scan_wide<u64>(local, total, scan64);
+#pragma unroll
+        for (int j = 0; j < kSortItems; ++j) {
+            sm.keys[first + j] = run;  // exclusive prefix
+            run += w[j];
+        }
+        __syncthreads();
+        for (int j = 0; j < kSortItems; ++j) {
+            const int i = first + j;
+            if (i >= count) break;
+            const u64 base = cw[s_target[i]];
+            const u64 inclusive = sm.keys[i] + w[j] - sm.keys[head(i)];
+            accept[sm.vals[i]] = base <= capacity && inclusive <= capacity - base;
+        }
+    } else {
+        // k_pair_flags, the scan of the flags and k_pair_commit.
+        u32 flag[kSortItems], local = 0;
+#pragma unroll
+        for (int j = 0; j < kSortItems; ++j) {
+            const int i = first + j;
+            flag[j] = 0;
+            if (i < count && i > 0)
+                flag[j] = ((i - head(i) + 1) & 1) == 0 &&
+                          static_cast<u64>(vw[sm.vals[i - 1]]) <= capacity - vw[sm.vals[i]];
+            local += flag[j];
+        }
+        u32 total;
+        u32 run = block_exclusive_scan_wide<u32>(local, total, scan32);
+        u64 pairs = 0;
+        for (int j = 0; j < kSortItems; ++j) {
+            const int i = first + j;
+            if (flag[j] && run < budget) {
+                const u32 x = sm.vals[i];
+                const int s = clusters[x], t = clusters[sm.vals[i - 1]];
+                if (s != t) {
+                    const u64 w = vw[x];
+                    atomicAdd(cw + s, 0ULL - w);
+                    atomicAdd(cw + t, w);
+                    clusters[x] = t;
+                    ++pairs;
+                }
+            }
+            run += flag[j];
+        }
+        block_atomic_add(merged, pairs);
+    }
 }
 
 // Segment heads of an ordered list grouped by target.
@@ -748,16 +831,24 @@ __global__ void k_ordered_accept(i64 count, const u32* items, const int* targets
     accept[v] = base <= capacity && inclusive <= capacity - base;
 }
 
+// A mover is a cluster of its own that nobody joins (receivers are not
+// movers), so every move empties one cluster: *merged counts them.  With
+// `items` set, does nothing when more were to be ordered than k_order_block
+// takes.
 __global__ void k_commit(i64 n, const int* proposals, const unsigned char* accept, const u32* vw, int* clusters,
-                         u64* cw) {
-    const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (v >= n) return;
-    const int t = proposals[v];
-    if (t == kInvalid || (accept && accept[v] != 1)) return;
-    const u64 w = vw[v];
-    atomicAdd(cw + clusters[v], 0ULL - w);
-    atomicAdd(cw + t, w);
-    clusters[v] = t;
+                         u64* cw, const u32* items, u64* merged) {
+    if (items && *items > kSortTile) return;
+    u64 moved = 0;
+    for (i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += static_cast<i64>(gridDim.x) * blockDim.x) {
+        const int t = proposals[v];
+        if (t == kInvalid || (accept && accept[v] != 1)) continue;
+        const u64 w = vw[v];
+        atomicAdd(cw + clusters[v], 0ULL - w);
+        atomicAdd(cw + t, w);
+        clusters[v] = t;
+        ++moved;
+    }
+    block_atomic_add(merged, moved);
 }
 
 // ---------------------------------------------------------------- isolated, two-hop
@@ -783,18 +874,21 @@ __global__ void k_isolated_rep(i64 count, const int* list, const u64* prefix, co
     if (fb == lb) atomicMin(reps + fb, v);
 }
 __global__ void k_isolated_commit(i64 count, const int* list, const u64* prefix, const u32* vw, u64 capacity,
-                                  const int* reps, int* clusters, u64* cw) {
-    const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const int v = list[i];
-    const u64 incl = prefix[i] + vw[v];
-    const u64 fb = prefix[i] / capacity, lb = (incl - 1) / capacity;
-    if (fb != lb) return;
-    const int t = reps[fb];
-    if (t == v) return;
-    clusters[v] = t;
-    cw[v] = 0;
-    atomicAdd(cw + t, static_cast<u64>(vw[v]));
+                                  const int* reps, int* clusters, u64* cw, u64* merged) {
+    u64 moved = 0;
+    for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += static_cast<i64>(gridDim.x) * blockDim.x) {
+        const int v = list[i];
+        const u64 incl = prefix[i] + vw[v];
+        const u64 fb = prefix[i] / capacity, lb = (incl - 1) / capacity;
+        if (fb != lb) continue;
+        const int t = reps[fb];
+        if (t == v) continue;
+        clusters[v] = t;
+        cw[v] = 0;
+        atomicAdd(cw + t, static_cast<u64>(vw[v]));
+        ++moved;
+    }
+    block_atomic_add(merged, moved);
 }
 
 // sclp_singleton_favorite_kernel (aggregation.cuh:654-664).
@@ -818,17 +912,22 @@ struct LoadU32 {
     __device__ u32 operator()(i64 i) const { return p[i]; }
 };
 // sclp_two_hop_pair_commit_kernel (aggregation.cuh:678-696).
+// Both are clusters of one vertex, so every pair empties one: *merged counts.
 __global__ void k_pair_commit(i64 count, const u32* items, const u32* flags, const u32* positions, u64 budget,
-                              const u32* vw, int* clusters, u64* cw) {
-    const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= count || !flags[i] || positions[i] >= budget) return;
-    const int v = static_cast<int>(items[i]);
-    const int s = clusters[v], t = clusters[items[i - 1]];
-    if (s == t) return;
-    const u64 w = vw[v];
-    atomicAdd(cw + s, 0ULL - w);
-    atomicAdd(cw + t, w);
-    clusters[v] = t;
+                              const u32* vw, int* clusters, u64* cw, u64* merged) {
+    u64 moved = 0;
+    for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += static_cast<i64>(gridDim.x) * blockDim.x) {
+        if (!flags[i] || positions[i] >= budget) continue;
+        const int v = static_cast<int>(items[i]);
+        const int s = clusters[v], t = clusters[items[i - 1]];
+        if (s == t) continue;
+        const u64 w = vw[v];
+        atomicAdd(cw + s, 0ULL - w);
+        atomicAdd(cw + t, w);
+        clusters[v] = t;
+        ++moved;
+    }
+    block_atomic_add(merged, moved);
 }
 
 // ---------------------------------------------------------------- compaction
@@ -847,16 +946,18 @@ __global__ void k_count_isolated(i64 n, const int* off, u64* out) {
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     block_atomic_add(out, v < n && off[v] == off[v + 1] ? 1ULL : 0ULL);
 }
-__global__ void k_map(i64 n, const int* clusters, const int* ids, const u32* vw, int* map, u32* cvw) {
+// The map, and each coarse vertex's weight: its cluster's.
+__global__ void k_map(i64 n, const int* clusters, const int* ids, const u64* cw, int* map, u32* cvw) {
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (v >= n) return;
-    const int c = ids[clusters[v]];
-    map[v] = c;
-    atomicAdd(cvw + c, vw[v]);
+    map[v] = ids[clusters[v]];
+    if (cw[v]) cvw[ids[v]] = static_cast<u32>(cw[v]);
 }
-__global__ void k_max_u32(i64 n, const u32* values, u64* out) {
-    const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
-    block_atomic_max(out, i < n ? static_cast<u64>(values[i]) : 0ULL);
+__global__ void k_max_weight(i64 n, const u64* cw, u64* out) {
+    u64 m = 0;
+    for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += static_cast<i64>(gridDim.x) * blockDim.x)
+        m = max(m, cw[i] & 0xffffffffULL);
+    block_atomic_max(out, m);
 }
 
 // ---------------------------------------------------------------- contraction
@@ -1485,6 +1586,33 @@ __global__ void k_emit_chunks(i64 count, const int* heavy, const int* off, const
 
 // ---------------------------------------------------------------- host orchestration
 
+// Heavy rows, chunks and entries in heavy rows of g, into scalars 0-2 (zero).
+void count_heavy(Context& ctx, const DGraph& g, int heavy_min) {
+    launch(k_heavy_counts, blocks_for(g.n, 256), 256, 0, ctx.stream, g.n, g.off, heavy_min, ctx.dev_scalars);
+}
+// The lists of those counts (host copies).
+void list_chunks(Context& ctx, DGraph& g, int heavy_min, const u64* counts, Arena& out) {
+    cudaStream_t s = ctx.stream;
+    g.heavy_min = heavy_min;
+    g.heavy = nullptr;
+    g.heavy_chunk0 = nullptr;
+    g.heavy_count = static_cast<i64>(counts[0]);
+    g.chunks = static_cast<i64>(counts[1]);
+    g.heavy_entries = static_cast<i64>(counts[2]);
+    if (!g.heavy_count) return;
+    g.heavy = out.alloc<int>(g.heavy_count);
+    g.chunk_row = out.alloc<int>(g.chunks);
+    g.chunk_hidx = out.alloc<int>(g.chunks);
+    g.chunk_begin = out.alloc<int>(g.chunks);
+    g.heavy_chunk0 = out.alloc<int>(g.heavy_count);
+    int* chunk_off = g.heavy_chunk0;
+    ArenaScope scope(ctx.scratch);
+    select_if(ctx.scratch, s, g.n, IsHeavyRow{g.off, heavy_min}, WriteIndex{g.heavy}, static_cast<u32*>(nullptr));
+    exclusive_scan<int>(ctx.scratch, s, g.heavy_count, ChunkCount{g.heavy, g.off}, chunk_off, static_cast<int*>(nullptr));
+    launch(k_emit_chunks, blocks_for(g.heavy_count, 256), 256, 0, s, g.heavy_count, g.heavy, g.off,
+           static_cast<const int*>(chunk_off), g.chunk_row, g.chunk_hidx, g.chunk_begin);
+}
+
 struct Workspace {  // SclpWorkspace::Impl state (src/coarsen.cu:299-396)
     bool positive = false, unit = false, sorted_unique = false, invariants_known = false;
     bool packed_weights = false;
@@ -1504,16 +1632,9 @@ struct AggregateOut {
 constexpr int kThreads = 256;
 
 // Orders `items` (vertex ids, `count` of them, ascending on entry) by
-// (target asc, key desc, tie desc): three stable LSD stages (one block for at
-// most one sort tile).
+// (target asc, key desc, tie desc): three stable LSD stages.
 void order_by_target(Context& ctx, i64 count, u32*& items, u32*& items_alt, const int* targets, const u64* key_values,
                      int key_bits, const u32* ties, int target_bits) {
-    if (count <= kSortTile) {
-        const u64 mask = key_bits >= 64 ? ~0ULL : ((1ULL << key_bits) - 1);
-        launch(k_order_small, 1, kSortThreads, 0, ctx.stream, static_cast<int>(count), items, ties, key_values, mask,
-               key_bits, targets, target_bits);
-        return;
-    }
     Arena& A = ctx.scratch;
     ArenaScope scope(A);
     u64* keys = A.alloc<u64>(static_cast<size_t>(count));
@@ -1574,13 +1695,24 @@ private:
     Summary* partial = nullptr;
     i64 segments = 0;
     int gain_bits = 64, target_bits = 32;
+    i64 last_ordered = 0;  // requests the last round had to order
 
-    u64 count_clusters() {
-        ctx.clear_scalars(1);
-        launch(k_count_nonzero, blocks_for(g.n, kThreads), kThreads, 0, ctx.stream, g.n, cw, ctx.dev_scalars);
-        return ctx.read_scalars(1)[0];
+    template <bool Pairs>
+    void order_in_block(const u32* items, const int* targets, const u64* key_values, unsigned char* accept, u64 capacity,
+                        u64 budget) {
+        const u64 mask = gain_bits >= 64 ? ~0ULL : ((1ULL << gain_bits) - 1);
+        launch(k_order_block<Pairs>, 1, kSortThreads, 0, ctx.stream, static_cast<const u32*>(ordered()), items, ties,
+               key_values, mask, gain_bits, targets, target_bits, g.vw, cw, capacity, accept, budget, clusters, merged());
     }
-    void form_proposals(u64 capacity, int round, bool filter_roles, u32 threshold, bool need_regret);
+    // Device scalars read together: the degree classes in [0, 9), then
+    static constexpr int kMerged = 16, kOrdered = 17, kCoarse = 18, kMaxWeight = 19, kRead = 20;
+    u64* merged() const { return ctx.dev_scalars + kMerged; }
+    u32* ordered() const { return reinterpret_cast<u32*>(ctx.dev_scalars + kOrdered); }
+    void clear_counts() { GP_CUDA(cudaMemsetAsync(ctx.dev_scalars + kMerged, 0, 2 * sizeof(u64), ctx.stream)); }
+    // Clusters that the work since clear_counts() emptied.
+    i64 read_merged() { return static_cast<i64>(ctx.read_scalars(kRead)[kMerged]); }
+    int grid() const { return static_cast<int>(std::min<i64>(blocks_for(g.n, kThreads), 148 * 16)); }
+    void form_proposals(u64 capacity, int round, bool filter_roles, u32 threshold, bool need_regret, u64* demand);
     // Table-based classes: medium, large (two table sizes) and heavy rows.
     template <class Table>
     void launch_tables(const RoundParams& p) {
@@ -1611,14 +1743,15 @@ private:
     }
 };
 
-void Aggregator::form_proposals(u64 capacity, int round, bool filter_roles, u32 threshold, bool need_regret) {
+void Aggregator::form_proposals(u64 capacity, int round, bool filter_roles, u32 threshold, bool need_regret,
+                                u64* demand) {
     const u32 role_salt = seed ^ (static_cast<u32>(level) * 0x9e3779b9U) ^ (static_cast<u32>(round) * 0x85ebca6bU) ^ 0x27d4eb2dU;
     const u32 tie_salt = seed ^ (static_cast<u32>(level) * 0xc2b2ae35U) ^ (static_cast<u32>(round) * 0x165667b1U) ^ 0xd3a2646cU;
     const i64 n = g.n;
     launch(k_roles, blocks_for(n, kThreads), kThreads, 0, ctx.stream, n, clusters, g.vw, cw, role_salt, threshold,
-           !filter_roles, roles, recv, proposals);
+           !filter_roles, roles, recv, proposals, demand);
     RoundParams p{g.off, g.nbr, g.ew, g.vw, clusters, cw, roles, recv, capacity, tie_salt, filter_roles,
-                  filter_roles && need_regret, proposals, gains, regret, ties};
+                  filter_roles && need_regret, proposals, gains, regret, ties, demand};
     if (list_size[0])
         launch(k_affinity_low, blocks_for(list_size[0] * 8, kThreads), kThreads, 0, ctx.stream, list_size[0], lists[0], p);
     if (packed) launch_tables<PackedTable>(p);
@@ -1649,6 +1782,7 @@ AggregateOut Aggregator::run() {
     regret = A.alloc<u64>(n);
     ties = A.alloc<u32>(n);
     i64 cluster_count = n;
+    ctx.clear_scalars(kRead);
     if (matching) {  // src/coarsen.cu:505-535
         int* choice = proposals;
         const u32 salt = seed ^ (static_cast<u32>(level) * 0x9e3779b9U);
@@ -1662,10 +1796,9 @@ AggregateOut Aggregator::run() {
             launch(k_match_choose<8>, blocks_for(n * 8, kThreads), kThreads, 0, s, n, g.off, g.nbr, g.ew, g.vw, C, salt, choice);
         else
             launch(k_match_choose<32>, blocks_for(n * 32, kThreads), kThreads, 0, s, n, g.off, g.nbr, g.ew, g.vw, C, salt, choice);
-        launch(k_match_roots, vb, kThreads, 0, s, n, choice, clusters);
+        launch(k_match_roots, grid(), kThreads, 0, s, n, choice, clusters, merged());
         GP_CUDA(cudaMemsetAsync(cw, 0, sizeof(u64) * n, s));
         launch(k_cluster_weights, vb, kThreads, 0, s, n, clusters, g.vw, cw);
-        cluster_count = static_cast<i64>(count_clusters());
     } else {
         launch(k_iota_clusters, vb, kThreads, 0, s, n, g.vw, clusters, cw);
     }
@@ -1680,17 +1813,18 @@ AggregateOut Aggregator::run() {
             out.stats_heavy = false;
             list_size[0] = n;
             list_size[1] = list_size[2] = list_size[3] = list_size[4] = 0;
-            ctx.clear_scalars(1);
             launch(k_count_isolated, vb, kThreads, 0, s, n, g.off, ctx.dev_scalars);
-            isolated = static_cast<i64>(ctx.read_scalars(1)[0]);
+            const u64* sc = ctx.read_scalars(kRead);
+            isolated = static_cast<i64>(sc[0]);
+            cluster_count -= static_cast<i64>(sc[kMerged]);
         } else {
             int* storage = A.alloc<int>(static_cast<size_t>(n) * 5);
             for (int c = 0; c < 5; ++c) lists[c] = storage + static_cast<size_t>(n) * c;
-            ctx.clear_scalars(9);
             launch(k_degree_classes, static_cast<int>(std::min<i64>(vb, 148 * 8)), kThreads, 0, s, n, g.off, lists[0],
                    lists[1], lists[2], lists[3], lists[4], std::min(o.mapping.medium_degree, kMediumDegree),
                    std::min(o.mapping.large_narrow, kLargeDegree), ctx.dev_scalars);
-            const u64* sc = ctx.read_scalars(9);
+            const u64* sc = ctx.read_scalars(kRead);
+            cluster_count -= static_cast<i64>(sc[kMerged]);
             out.stats_max_degree = sc[0];
             out.stats_heavy = sc[1] != 0;
             for (int c = 0; c < 4; ++c) list_size[c] = static_cast<i64>(sc[2 + c]);
@@ -1740,31 +1874,46 @@ AggregateOut Aggregator::run() {
         const u64 degree = out.stats_max_degree;
         const bool all_fit = o.fast_path && (degree == 0 || bound <= room / maxv / degree);
         const u64 next_bound = all_fit ? bound + bound * degree * maxv : C;
-        form_proposals(C, round, true, threshold, !all_fit);
+        form_proposals(C, round, true, threshold, !all_fit, all_fit ? nullptr : demand);
+        clear_counts();
+        i64 moved = 0;
         if (all_fit) {
-            launch(k_commit, vb, kThreads, 0, s, n, proposals, static_cast<const unsigned char*>(nullptr), g.vw, clusters, cw);
+            launch(k_commit, grid(), kThreads, 0, s, n, proposals, static_cast<const unsigned char*>(nullptr), g.vw,
+                   clusters, cw, static_cast<const u32*>(nullptr), merged());
+            moved = read_merged();
         } else {
-            GP_CUDA(cudaMemsetAsync(demand, 0, sizeof(u64) * n, s));
-            launch(k_requests, vb, kThreads, 0, s, n, proposals, g.vw, demand);
             launch(k_classify, vb, kThreads, 0, s, n, proposals, cw, demand, C, accept);
             ArenaScope rs(A);
             u32* items = A.alloc<u32>(n);
-            u32* count_dev = reinterpret_cast<u32*>(ctx.dev_scalars);
-            select_if(A, s, n, NeedsOrder{accept}, WriteU32Index{items}, count_dev);
-            const i64 count = static_cast<i64>(static_cast<u32>(ctx.read_scalars(1)[0] & 0xffffffffULL));
-            if (count > 0) {
-                u32* items_alt = A.alloc<u32>(count);
-                order_by_target(ctx, count, items, items_alt, proposals, regret, gain_bits, ties, target_bits);
-                u64* prefix = A.alloc<u64>(count);
-                exclusive_scan<u64>(A, s, count, OrderedWeight{items, g.vw}, prefix, static_cast<u64*>(nullptr));
-                const int cb = blocks_for(count, kThreads);
-                launch(k_segment_heads, cb, kThreads, 0, s, count, items, proposals, prefix, demand, static_cast<int*>(nullptr));
-                launch(k_ordered_accept, cb, kThreads, 0, s, count, items, proposals, g.vw, prefix, demand, cw, C, accept);
+            select_if(A, s, n, NeedsOrder{accept}, WriteU32Index{items}, ordered());
+            // One block orders few requests and the commit follows at once;
+            // after a round with many, the count is read first.
+            const bool offered = last_ordered <= kSortTile;
+            if (offered) {
+                order_in_block<false>(items, proposals, regret, accept, C, 0);
+                launch(k_commit, grid(), kThreads, 0, s, n, proposals, accept, g.vw, clusters, cw,
+                       static_cast<const u32*>(ordered()), merged());
             }
-            launch(k_commit, vb, kThreads, 0, s, n, proposals, accept, g.vw, clusters, cw);
+            const u64* sc = ctx.read_scalars(kRead);
+            const i64 count = last_ordered = static_cast<i64>(static_cast<u32>(sc[kOrdered] & 0xffffffffULL));
+            moved = static_cast<i64>(sc[kMerged]);
+            if (!offered || count > kSortTile) {
+                if (count > 0) {
+                    u32* items_alt = A.alloc<u32>(count);
+                    order_by_target(ctx, count, items, items_alt, proposals, regret, gain_bits, ties, target_bits);
+                    u64* prefix = A.alloc<u64>(count);
+                    exclusive_scan<u64>(A, s, count, OrderedWeight{items, g.vw}, prefix, static_cast<u64*>(nullptr));
+                    const int cb = blocks_for(count, kThreads);
+                    launch(k_segment_heads, cb, kThreads, 0, s, count, items, proposals, prefix, demand, static_cast<int*>(nullptr));
+                    launch(k_ordered_accept, cb, kThreads, 0, s, count, items, proposals, g.vw, prefix, demand, cw, C, accept);
+                }
+                launch(k_commit, grid(), kThreads, 0, s, n, proposals, accept, g.vw, clusters, cw,
+                       static_cast<const u32*>(nullptr), merged());
+                moved = read_merged();
+            }
         }
         const i64 before = cluster_count;
-        cluster_count = static_cast<i64>(count_clusters());
+        cluster_count -= moved;
         if (cluster_count > before) fail(GP_INTERNAL, "residual singleton merge accounting failed");
         bound = next_bound;
         if (o.log)
@@ -1777,26 +1926,31 @@ AggregateOut Aggregator::run() {
         int* list = A.alloc<int>(isolated);
         u64* prefix = A.alloc<u64>(isolated);
         select_if(A, s, n, IsIsolated{g.off}, WriteIndex{list}, static_cast<u32*>(nullptr));
-        u64* total_dev = ctx.dev_scalars;
-        exclusive_scan<u64>(A, s, isolated, IsolatedWeight{list, g.vw}, prefix, total_dev);
-        const u64 iso_total = ctx.read_scalars(1)[0];
-        const i64 bins = static_cast<i64>(iso_total / C + (iso_total % C != 0));
-        int* reps = A.alloc<int>(bins);
-        fill<int>(s, reps, bins, INT_MAX);
+        exclusive_scan<u64>(A, s, isolated, IsolatedWeight{list, g.vw}, prefix, static_cast<u64*>(nullptr));
+        // Bins of weight C: no more than vertices, each of which fits one.
+        int* reps = A.alloc<int>(isolated);
+        fill<int>(s, reps, isolated, INT_MAX);
         const int ib = blocks_for(isolated, kThreads);
+        clear_counts();
         launch(k_isolated_rep, ib, kThreads, 0, s, isolated, list, prefix, g.vw, C, reps);
-        launch(k_isolated_commit, ib, kThreads, 0, s, isolated, list, prefix, g.vw, C, reps, clusters, cw);
-        cluster_count = static_cast<i64>(count_clusters());
+        launch(k_isolated_commit, std::min(ib, 148 * 16), kThreads, 0, s, isolated, list, prefix, g.vw, C, reps, clusters,
+               cw, merged());
+        cluster_count -= read_merged();
     }
     if (static_cast<double>(cluster_count) > 0.60 * n) {  // two-hop, src/coarsen.cu:1166-1259
-        form_proposals(C, 4, false, 0, false);
+        form_proposals(C, 4, false, 0, false, nullptr);
         launch(k_favorites, vb, kThreads, 0, s, n, g.vw, cw, clusters, proposals);
         ArenaScope ts(A);
         u32* items = A.alloc<u32>(n);
-        select_if(A, s, n, HasValue{proposals}, WriteU32Index{items}, reinterpret_cast<u32*>(ctx.dev_scalars));
-        const i64 count = static_cast<i64>(static_cast<u32>(ctx.read_scalars(1)[0] & 0xffffffffULL));
+        clear_counts();
+        select_if(A, s, n, HasValue{proposals}, WriteU32Index{items}, ordered());
         const u64 budget = static_cast<u64>(std::max<i64>(0, cluster_count - desired));
-        if (count > 0 && budget > 0) {
+        const bool offered = n <= 16 * kSortTile;  // larger levels have more than a tile of favourites
+        if (offered) order_in_block<true>(items, proposals, gains, nullptr, C, budget);
+        const u64* sc = ctx.read_scalars(kRead);
+        const i64 count = static_cast<i64>(static_cast<u32>(sc[kOrdered] & 0xffffffffULL));
+        i64 moved = static_cast<i64>(sc[kMerged]);
+        if ((!offered || count > kSortTile) && count > 0 && budget > 0) {
             u32* items_alt = A.alloc<u32>(count);
             order_by_target(ctx, count, items, items_alt, proposals, gains, gain_bits, ties, target_bits);
             int* first = A.alloc<int>(n);  // first position of every favourite's group
@@ -1807,25 +1961,26 @@ AggregateOut Aggregator::run() {
             u32* positions = A.alloc<u32>(count);
             launch(k_pair_flags, cb, kThreads, 0, s, count, items, proposals, first, g.vw, C, flags);
             exclusive_scan<u32>(A, s, count, LoadU32{flags}, positions, static_cast<u32*>(nullptr));
-            launch(k_pair_commit, cb, kThreads, 0, s, count, items, flags, positions, budget, g.vw, clusters, cw);
+            launch(k_pair_commit, std::min(cb, 148 * 16), kThreads, 0, s, count, items, flags, positions, budget, g.vw,
+                   clusters, cw, merged());
+            moved = read_merged();
         }
-        cluster_count = static_cast<i64>(count_clusters());
+        cluster_count -= moved;
     }
     // Compaction (src/coarsen.cu:1261-1298).
     {
         ArenaScope cs(A);
         int* ids = A.alloc<int>(n);
-        u64* nc_dev = ctx.dev_scalars;
-        GP_CUDA(cudaMemsetAsync(nc_dev, 0, sizeof(u64), s));
-        exclusive_scan<int>(A, s, n, NonEmptyInt{cw}, ids, reinterpret_cast<int*>(nc_dev));
-        out.nc = static_cast<i64>(static_cast<int>(ctx.read_scalars(1)[0] & 0xffffffffULL));
+        GP_CUDA(cudaMemsetAsync(ctx.dev_scalars + kCoarse, 0, 2 * sizeof(u64), s));
+        exclusive_scan<int>(A, s, n, NonEmptyInt{cw}, ids, reinterpret_cast<int*>(ctx.dev_scalars + kCoarse));
+        launch(k_max_weight, grid(), kThreads, 0, s, n, static_cast<const u64*>(cw), ctx.dev_scalars + kMaxWeight);
+        const u64* sc = ctx.read_scalars(kRead);
+        out.nc = static_cast<i64>(static_cast<int>(sc[kCoarse] & 0xffffffffULL));
+        out.max_w = sc[kMaxWeight];
         out.map = ctx.persist.alloc<int>(n);
         out.cvw = ctx.persist.alloc<u32>(out.nc);
-        GP_CUDA(cudaMemsetAsync(out.cvw, 0, sizeof(u32) * out.nc, s));
-        launch(k_map, vb, kThreads, 0, s, n, clusters, ids, g.vw, out.map, out.cvw);
-        ctx.clear_scalars(1);
-        launch(k_max_u32, blocks_for(out.nc, kThreads), kThreads, 0, s, out.nc, out.cvw, ctx.dev_scalars);
-        out.max_w = ctx.read_scalars(1)[0];
+        launch(k_map, vb, kThreads, 0, s, n, clusters, static_cast<const int*>(ids), static_cast<const u64*>(cw), out.map,
+               out.cvw);
     }
     ws.max_vw = out.max_w;
     if (out.max_w > C) fail(GP_INTERNAL, "SCLP coarsening exceeded cluster capacity");
@@ -1847,14 +2002,11 @@ DGraph contract(Context& ctx, const DGraph& fine, AggregateOut& agg, Workspace& 
     GP_CUDA(cudaMemsetAsync(raw, 0, sizeof(int) * (nc + 1), s));
     const bool bounded = n > 0 && ws.maximum_row_weight <= ~0ULL / static_cast<u64>(n);
     launch(k_contract_bounds, vb, kThreads, 0, s, n, agg.map, fine.off, ws.row_bounds, next_bounds, raw, bounded);
-    ctx.clear_scalars(2);
-    launch(k_max_pair, blocks_for(nc, kThreads), kThreads, 0, s, nc, next_bounds, raw, ctx.dev_scalars);
-    const u64* sc = ctx.read_scalars(2);
-    const u64 row_bound = sc[0], raw_max = sc[1];
-    const bool count_raw = ws.positive && n >= 65536 && fine.maximum_degree <= 512;
-    const u64 raw_bound = count_raw ? raw_max : ~0ULL;
-    const u64 degree_bound = count_raw && fine.maximum_degree <= 128 ? raw_bound : row_bound;
-    const bool short_rows = count_raw && raw_bound <= 512;
+    // Scalars: the row classes in [0, kRowClasses], then the largest row
+    // bound and raw size, read together.
+    constexpr int kBounds = kRowClasses + 1;
+    ctx.clear_scalars(kBounds + 2);
+    launch(k_max_pair, blocks_for(nc, kThreads), kThreads, 0, s, nc, next_bounds, raw, ctx.dev_scalars + kBounds);
 
     // Raw segments of every coarse row, filled by one scatter of the fine CSR.
     int* raw_off = A.alloc<int>(nc + 1);
@@ -1881,9 +2033,13 @@ DGraph contract(Context& ctx, const DGraph& fine, AggregateOut& agg, Workspace& 
     }
     // Row classes by raw size.
     int* lists = A.alloc<int>(static_cast<size_t>(nc) * kRowClasses);
-    ctx.clear_scalars(kRowClasses + 1);
     launch(k_row_classes, blocks_for(nc, kThreads), kThreads, 0, s, nc, raw, lists, nc, ctx.dev_scalars);
-    const u64* cls = ctx.read_scalars(kRowClasses + 1);
+    const u64* cls = ctx.read_scalars(kBounds + 2);
+    const u64 row_bound = cls[kBounds], raw_max = cls[kBounds + 1];
+    const bool count_raw = ws.positive && n >= 65536 && fine.maximum_degree <= 512;
+    const u64 raw_bound = count_raw ? raw_max : ~0ULL;
+    const u64 degree_bound = count_raw && fine.maximum_degree <= 128 ? raw_bound : row_bound;
+    const bool short_rows = count_raw && raw_bound <= 512;
     i64 count[kRowClasses];
     for (int c = 0; c < kRowClasses; ++c) count[c] = static_cast<i64>(cls[c]);
     const i64 large_records = static_cast<i64>(cls[kRowClasses]);
@@ -1949,15 +2105,17 @@ DGraph contract(Context& ctx, const DGraph& fine, AggregateOut& agg, Workspace& 
     DGraph coarse;
     coarse.n = nc;
     coarse.off = ctx.persist.alloc<int>(nc + 1);
-    u64* m_dev = ctx.dev_scalars + 8;
-    GP_CUDA(cudaMemsetAsync(m_dev, 0, sizeof(u64), s));
-    exclusive_scan<int>(A, s, nc + 1, UniqueCount{ucount, nc}, coarse.off, static_cast<int*>(nullptr));
-    GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, coarse.off + nc, sizeof(int), cudaMemcpyDeviceToHost, s));
-    GP_CUDA(cudaStreamSynchronize(s));
-    coarse.m = *reinterpret_cast<const int*>(ctx.host_scalars);
+    // The entry count and the heavy rows' counts are read together.
+    constexpr int kEntries = 3;
+    ctx.clear_scalars(kEntries + 1);
+    exclusive_scan<int>(A, s, nc + 1, UniqueCount{ucount, nc}, coarse.off,
+                        reinterpret_cast<int*>(ctx.dev_scalars + kEntries));
+    count_heavy(ctx, coarse, kHeavyRow);
+    const u64* counts = ctx.read_scalars(kEntries + 1);
+    coarse.m = static_cast<i64>(static_cast<int>(counts[kEntries] & 0xffffffffULL));
     coarse.nbr = ctx.persist.alloc<int>(coarse.m);
     coarse.ew = ctx.persist.alloc<u32>(coarse.m);
-    build_chunks(ctx, coarse);
+    list_chunks(ctx, coarse, kHeavyRow, counts, ctx.persist);
     if (coarse.m - coarse.heavy_entries > 64 * (nc - coarse.heavy_count))
         launch(k_copy_rows<32>, blocks_for(nc * 32, kThreads), kThreads, 0, s, nc, raw_off, raw_t, raw_w, coarse.off,
                coarse.nbr, coarse.ew);
@@ -1983,33 +2141,10 @@ DGraph contract(Context& ctx, const DGraph& fine, AggregateOut& agg, Workspace& 
 
 // Heavy-row list and chunk list of a level, in the hierarchy's storage.
 void build_chunks(Context& ctx, DGraph& g, int heavy_min, Arena* storage) {
-    cudaStream_t s = ctx.stream;
-    Arena& out = storage ? *storage : ctx.persist;
-    g.heavy_min = heavy_min;
-    g.heavy = nullptr;
-    g.heavy_chunk0 = nullptr;
-    g.heavy_count = 0;
-    g.chunks = 0;
-    g.heavy_entries = 0;
     if (g.n <= 0) return;
     ctx.clear_scalars(3);
-    launch(k_heavy_counts, blocks_for(g.n, kThreads), kThreads, 0, s, g.n, g.off, heavy_min, ctx.dev_scalars);
-    const u64* sc = ctx.read_scalars(3);
-    g.heavy_count = static_cast<i64>(sc[0]);
-    g.chunks = static_cast<i64>(sc[1]);
-    g.heavy_entries = static_cast<i64>(sc[2]);
-    if (!g.heavy_count) return;
-    g.heavy = out.alloc<int>(g.heavy_count);
-    g.chunk_row = out.alloc<int>(g.chunks);
-    g.chunk_hidx = out.alloc<int>(g.chunks);
-    g.chunk_begin = out.alloc<int>(g.chunks);
-    g.heavy_chunk0 = out.alloc<int>(g.heavy_count);
-    int* chunk_off = g.heavy_chunk0;
-    ArenaScope scope(ctx.scratch);
-    select_if(ctx.scratch, s, g.n, IsHeavyRow{g.off, heavy_min}, WriteIndex{g.heavy}, static_cast<u32*>(nullptr));
-    exclusive_scan<int>(ctx.scratch, s, g.heavy_count, ChunkCount{g.heavy, g.off}, chunk_off, static_cast<int*>(nullptr));
-    launch(k_emit_chunks, blocks_for(g.heavy_count, kThreads), kThreads, 0, s, g.heavy_count, g.heavy, g.off,
-           static_cast<const int*>(chunk_off), g.chunk_row, g.chunk_hidx, g.chunk_begin);
+    count_heavy(ctx, g, heavy_min);
+    list_chunks(ctx, g, heavy_min, ctx.read_scalars(3), storage ? *storage : ctx.persist);
 }
 
 // coarsen_impl (src/coarsen.cu:1762-2060).
@@ -2021,7 +2156,7 @@ Hierarchy coarsen(Context& ctx, const DGraph& input, const CoarsenOptions& o) {
     if (current.n > 0) {
         build_chunks(ctx, current);
         ws.row_bounds = ctx.persist.alloc<u64>(current.n);
-        ctx.clear_scalars(7);
+        ctx.clear_scalars(8);
         const int meta_grid = static_cast<int>(std::min<i64>(blocks_for(current.n * 8, kThreads), 148 * 16));
         // 8 lanes per row unless the light rows (the heavier ones go by
         // chunks) average more than 64 entries.
@@ -2038,7 +2173,7 @@ Hierarchy coarsen(Context& ctx, const DGraph& input, const CoarsenOptions& o) {
             launch(k_heavy_bound_max, blocks_for(current.heavy_count, kThreads), kThreads, 0, s, current.heavy_count,
                    static_cast<const int*>(current.heavy), static_cast<const u64*>(ws.row_bounds), ctx.dev_scalars);
         }
-        const u64* sc = ctx.read_scalars(7);
+        const u64* sc = ctx.read_scalars(8);
         ws.original_vertices = current.n;
         ws.maximum_row_weight = sc[0];
         current.incident_bound = sc[0];
@@ -2050,14 +2185,7 @@ Hierarchy coarsen(Context& ctx, const DGraph& input, const CoarsenOptions& o) {
         ws.total_vw = sc[5];
         ws.max_vw = sc[6];
         ws.invariants_known = true;
-        if (ws.unit) {
-            ws.packed_weights = static_cast<u64>(current.m) <= 0xffffffffULL;
-        } else {
-            ctx.clear_scalars(1);
-            launch(k_weight_sum, std::min(blocks_for(current.m, kThreads), 148 * 8), kThreads, 0, s, 
-                current.m, current.ew, ctx.dev_scalars);
-            ws.packed_weights = ctx.read_scalars(1)[0] <= 0xffffffffULL;
-        }
+        ws.packed_weights = (ws.unit ? static_cast<u64>(current.m) : sc[7]) <= 0xffffffffULL;
     }
     const i64 cutoff = std::max<i64>(32, static_cast<i64>(o.cluster_size_factor) * o.parts);
     for (int level = 0; level < o.max_levels && current.n > cutoff; ++level) {
