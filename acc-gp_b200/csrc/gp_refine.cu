@@ -2223,6 +2223,15 @@ struct MoveOrder {  // JointOrder (exchange.cuh:29-36)
         return r;
     }
 };
+// Device counts of one exchange pass.  k_match_parts clears them; the lists
+// grow by atomic appends (their order does not matter: the sorts' comparators
+// end with the move's unique id).
+struct JointCounts {
+    u64 fragments;  // appended by k_grow
+    u64 moves;      // appended by k_grow and k_combine
+    u32 unique;     // distinct fragments
+    u32 active;     // ordered moves; 0 when a list is longer than one block sorts
+};
 template <class Cmp>
 __global__ void k_move_keys(int count, const JointMove* moves, MoveKey* keys) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2307,15 +2316,11 @@ __global__ void __launch_bounds__(1024) k_bitonic_local(int size, int count, con
 }
 // A whole sort of up to kBitonicSegment moves in one block: the full network
 // over indices in shared memory (the same compare-exchange steps as
-// k_bitonic_local over one segment) and the gather of the sorted moves.
-// The keys stay in place, indexed by move, so an exchange writes two
-// indices and no keys.
+// k_bitonic_local over one segment).  The keys stay in place, indexed by move,
+// so an exchange writes two indices and no keys.  Leaves the order in s_idx.
 template <class Cmp>
-__global__ void __launch_bounds__(1024) k_sort_moves_block(int size, int count, const JointMove* in, JointMove* out,
-                                                          Cmp cmp) {
-    extern __shared__ __align__(16) unsigned char bitonic_smem[];
-    MoveKey* s_key = reinterpret_cast<MoveKey*>(bitonic_smem);  // by move
-    int* s_idx = reinterpret_cast<int*>(s_key + size);
+__device__ __forceinline__ void sort_moves_smem(int size, int count, const JointMove* in, MoveKey* s_key, int* s_idx,
+                                                Cmp cmp) {
     for (int i = threadIdx.x; i < size; i += blockDim.x) {
         s_idx[i] = i;
         if (i < count) s_key[i] = Cmp::key(in[i]);
@@ -2324,7 +2329,7 @@ __global__ void __launch_bounds__(1024) k_sort_moves_block(int size, int count, 
     for (int kk = 2; kk <= size; kk <<= 1)
         for (int jj = kk >> 1; jj; jj >>= 1) {
             for (int p = threadIdx.x; p < size / 2; p += blockDim.x) {
-                const int i = (p / jj) * 2 * jj + p % jj;
+                const int i = 2 * p - (p & (jj - 1));
                 const int x = i + jj;
                 const int a = s_idx[i], b = s_idx[x];
                 bool greater;
@@ -2338,7 +2343,28 @@ __global__ void __launch_bounds__(1024) k_sort_moves_block(int size, int count, 
             }
             __syncthreads();
         }
-    for (int i = threadIdx.x; i < count; i += blockDim.x) out[i] = in[s_idx[i]];
+}
+// The fragments sorted and without duplicates, when one block takes them.
+__global__ void __launch_bounds__(1024) k_sort_fragments(const JointMove* in, JointMove* out, JointCounts* counts) {
+    extern __shared__ __align__(16) unsigned char bitonic_smem[];
+    __shared__ u32 s_scan[33];
+    if (counts->fragments > kBitonicSegment) return;
+    const int count = static_cast<int>(counts->fragments);
+    int size = 1;
+    while (size < count) size <<= 1;
+    MoveKey* s_key = reinterpret_cast<MoveKey*>(bitonic_smem);
+    int* s_idx = reinterpret_cast<int*>(s_key + size);
+    sort_moves_smem(size, count, in, s_key, s_idx, NetOrder{});
+    u32 kept = 0;
+    for (int base = 0; base < count; base += blockDim.x) {
+        const int i = base + static_cast<int>(threadIdx.x);
+        const bool head = i < count && (i == 0 || !joint_same(in[s_idx[i - 1]], in[s_idx[i]]));
+        u32 total;
+        const u32 slot = kept + block_exclusive_scan_wide<u32>(head ? 1u : 0u, total, s_scan);
+        if (head) out[slot] = in[s_idx[i]];
+        kept += total;
+    }
+    if (threadIdx.x == 0) counts->unique = kept;
 }
 __global__ void k_iota(int n, int* idx) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2366,7 +2392,15 @@ __global__ void k_quotient(i64 n, const int* labels, const C* A, int k, u64* quo
 // takes part in later rounds); each round a warp per part picks its best
 // unmatched partner, the highest score and on ties the lowest part.
 constexpr int kMatchThreads = 1024;
-__global__ void __launch_bounds__(kMatchThreads) k_match_parts(int k, const u64* quotient, int* partner, int* visits) {
+// Also clears the pass's seeds and counts.
+__global__ void __launch_bounds__(kMatchThreads) k_match_parts(int k, const u64* quotient, int* partner, int* visits,
+                                                               u64* seeds, int seed_count, JointCounts* counts,
+                                                               u64* movers) {
+    for (int x = threadIdx.x; x < seed_count; x += blockDim.x) seeds[x] = ~0ULL;
+    if (threadIdx.x == 0) {
+        *counts = JointCounts{0, 0, 0, 0};
+        *movers = 0;
+    }
     extern __shared__ double s_score[];  // k * k, pair (a, b) with a < b at a * k + b; -1 = no edge
     __shared__ int s_partner[kMaxParts], s_choice[kMaxParts], s_progress;
     for (int x = threadIdx.x; x < k * k; x += blockDim.x) {
@@ -2419,10 +2453,12 @@ __global__ void __launch_bounds__(kMatchThreads) k_match_parts(int k, const u64*
     }
     for (int p = threadIdx.x; p < k; p += blockDim.x) partner[p] = s_partner[p];
 }
-// joint_seeds (exchange.cuh:83-93).
+// joint_seeds (exchange.cuh:83-93).  Also frees every vertex of an owner.
 template <class C>
-__global__ void k_seeds(i64 n, const int* labels, const C* A, int k, const int* partner, u64* seeds, int sw, int pass) {
+__global__ void k_seeds(i64 n, const int* labels, const C* A, int k, const int* partner, u64* seeds, int sw, int pass,
+                        int* owners) {
     for (i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += static_cast<i64>(gridDim.x) * blockDim.x) {
+        owners[v] = INT_MAX;
         const int p = labels[v], q = partner[p];
         if (q < 0 || !A[v * k + q]) continue;
         const u32 h = mix32(static_cast<u32>(v) ^ mix32(static_cast<u32>(pass + 17)));
@@ -2430,21 +2466,18 @@ __global__ void k_seeds(i64 n, const int* labels, const C* A, int k, const int* 
     }
 }
 
-// joint_grow (exchange.cuh:95-204): one warp per (seed, policy) slot.
+// joint_grow (exchange.cuh:95-204): one warp per (seed, policy) slot.  Its
+// partial moves are appended to the fragments, its best one to the moves.
 template <class C>
 __global__ void k_grow(int slots, int sw, const u64* seeds, const int* partner, const int* off, const int* nbr,
                        const u32* ew, const u32* masses, const int* labels, const C* A, int k, const u64* loads,
-                       u64 capacity, JointMove* moves, JointMove* archive) {
+                       u64 capacity, JointMove* moves, JointMove* fragments, JointCounts* joint) {
     const int lane = threadIdx.x & 31;
     const int slot = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (slot >= slots) return;
     const int policy = slot % 2;
     JointMove best = empty_move();
     best.id = slot;
-    if (!lane) {
-        moves[slot] = best;
-        for (int j = 0; j < kJointArchive; ++j) archive[slot * kJointArchive + j] = empty_move();
-    }
     const u64 enc = seeds[slot / 2];
     if (enc == ~0ULL) return;
     const int root = static_cast<int>(static_cast<u32>(enc)), source = labels[root], target = partner[source];
@@ -2466,7 +2499,7 @@ __global__ void k_grow(int slots, int sw, const u64* seeds, const int* partner, 
                 while (pos && st.vertices[pos - 1] > members[j]) { st.vertices[pos] = st.vertices[pos - 1]; --pos; }
                 st.vertices[pos] = members[j];
             }
-            archive[slot * kJointArchive + step] = st;
+            fragments[atomicAdd(&joint->fragments, 1ULL)] = st;
         }
         if (gain > best.gain && !joint_gap(net, lo, hi)) {
             best.size = size; best.a = min(source, target); best.b = max(source, target);
@@ -2532,13 +2565,9 @@ __global__ void k_grow(int slots, int sw, const u64* seeds, const int* partner, 
         gain += cgain;
         net += side ? -static_cast<long long>(masses[chosen]) : static_cast<long long>(masses[chosen]);
     }
-    if (!lane) moves[slot] = best;
+    if (!lane && best.size) moves[atomicAdd(&joint->moves, 1ULL)] = best;
 }
 
-struct NonEmptyMove {
-    const JointMove* moves;
-    __device__ bool operator()(i64 i) const { return moves[i].size != 0; }
-};
 struct CopyMove {
     const JointMove* in;
     JointMove* out;
@@ -2549,20 +2578,20 @@ struct UniqueHead {
     __device__ bool operator()(i64 i) const { return i == 0 || !joint_same(moves[i - 1], moves[i]); }
 };
 
-// joint_combine (complementary_moves.cuh:31-75): one warp per fragment.
-__global__ void k_combine(int count, const JointMove* archive, const int* off, const int* nbr, const u32* ew,
+// joint_combine (complementary_moves.cuh:31-75): one warp per fragment of the
+// distinct sorted ones; appends to the moves.
+__global__ void k_combine(JointCounts* counts, const JointMove* archive, const int* off, const int* nbr, const u32* ew,
                           const int* labels, const u64* loads, u64 capacity, int id_base, JointMove* out) {
     const int lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int count = static_cast<int>(counts->unique);
     if (i >= count) return;
     const JointMove x = archive[i];
     const long long lo = static_cast<long long>(loads[x.a]) - static_cast<long long>(capacity);
     const long long hi = static_cast<long long>(capacity) - static_cast<long long>(loads[x.b]);
-    if (!lane) {
+    if (!lane && !joint_gap(x.net, lo, hi)) {
         JointMove y = x;
         y.id = id_base + i;
-        if (joint_gap(x.net, lo, hi)) y.size = 0;
-        out[i] = y;
-        out[count + i] = empty_move();
+        out[atomicAdd(&counts->moves, 1ULL)] = y;
     }
     // First position whose move does not come before (x.a, net) (after it,
     // with upper).  The warp probes 32 evenly spaced positions at once, so
@@ -2657,7 +2686,7 @@ __global__ void k_combine(int count, const JointMove* archive, const int* off, c
         r.gain = best_gain;
         r.net += y.net;
         r.id = id_base + count + i;
-        out[count + i] = r;
+        out[atomicAdd(&counts->moves, 1ULL)] = r;
     }
 }
 __global__ void k_claim(int count, const JointMove* moves, int* owners) {
@@ -2697,12 +2726,86 @@ struct EventChunks {
         return static_cast<u32>((off[v + 1] - off[v] + kEventChunk - 1) / kEventChunk);
     }
 };
-__global__ void k_events(int count, const JointMove* moves, const u32* chunk_off, const u32* total_chunks,
+// The moves sorted, their claims settled (k_claim, k_resolve, k_mark) and the
+// chunks of their rows counted, by one block when neither list of the pass is
+// longer than it sorts; otherwise leaves no active move.
+__global__ void __launch_bounds__(1024) k_rank_moves(const JointMove* in, JointMove* out, JointCounts* counts,
+                                                     const int* off, const int* labels, int* owners, int* targets,
+                                                     u64* events, u32* chunk_off, u32* total_chunks) {
+    extern __shared__ __align__(16) unsigned char bitonic_smem[];
+    __shared__ u32 s_scan[33];
+    constexpr int kPer = kBitonicSegment / 1024;  // consecutive moves per thread
+    if (counts->fragments > kBitonicSegment || counts->moves > kBitonicSegment) return;
+    const int count = static_cast<int>(counts->moves);
+    int size = 1;
+    while (size < count) size <<= 1;
+    MoveKey* s_key = reinterpret_cast<MoveKey*>(bitonic_smem);
+    int* s_idx = reinterpret_cast<int*>(s_key + size);
+    sort_moves_smem(size, count, in, s_key, s_idx, MoveOrder{});
+    // Every vertex goes to the first move that wants it; a move keeps its
+    // vertices only if it gets them all.
+    const int first = static_cast<int>(threadIdx.x) * kPer;
+    for (int i = first; i < first + kPer && i < count; ++i) {
+        const JointMove& m = in[s_idx[i]];
+        for (int j = 0; j < m.size; ++j) atomicMin(owners + m.vertices[j], i);
+    }
+    __syncthreads();
+    unsigned wins = 0;
+    for (int i = first; i < first + kPer && i < count; ++i) {
+        const JointMove& m = in[s_idx[i]];
+        bool all = true;
+        for (int j = 0; j < m.size; ++j) all &= __ldcg(owners + m.vertices[j]) == i;
+        wins |= all ? 1u << (i - first) : 0u;
+    }
+    __syncthreads();
+    for (int i = first; i < first + kPer && i < count; ++i) {
+        const JointMove& m = in[s_idx[i]];
+        for (int j = 0; j < m.size; ++j) owners[m.vertices[j]] = INT_MAX;
+    }
+    __syncthreads();
+    u32 chunks[kPer][2 * kJointSide], local = 0;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q)
+#pragma unroll
+        for (int j = 0; j < 2 * kJointSide; ++j) chunks[q][j] = 0;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const int i = first + q;
+        if (i >= count) continue;
+        JointMove m = in[s_idx[i]];
+        if (!(wins & (1u << q))) m.size = 0;
+#pragma unroll
+        for (int j = 0; j < 2 * kJointSide; ++j)
+            if (j < m.size) {
+                const int v = m.vertices[j];
+                owners[v] = i;
+                targets[v] = labels[v] == m.a ? m.b : m.a;
+                chunks[q][j] = static_cast<u32>((off[v + 1] - off[v] + kEventChunk - 1) / kEventChunk);
+                local += chunks[q][j];
+            }
+        out[i] = m;
+        events[i] = 0;
+    }
+    u32 total;
+    u32 run = block_exclusive_scan_wide<u32>(local, total, s_scan);
+#pragma unroll
+    for (int q = 0; q < kPer; ++q)
+#pragma unroll
+        for (int j = 0; j < 2 * kJointSide; ++j) {
+            if (first + q < count) chunk_off[(first + q) * 2 * kJointSide + j] = run;
+            run += chunks[q][j];
+        }
+    if (threadIdx.x == 0) {
+        *total_chunks = total;
+        counts->active = static_cast<u32>(count);
+    }
+}
+__global__ void k_events(const u32* count_ptr, const JointMove* moves, const u32* chunk_off, const u32* total_chunks,
                          const int* owners, const int* targets, const int* labels, const int* off, const int* nbr,
                          const u32* ew, u64* events) {
     const int lane = threadIdx.x & 31;
-    const u32 total = *total_chunks;
-    const int items = count * 8;
+    const int items = static_cast<int>(*count_ptr) * 8;
+    const u32 total = items ? *total_chunks : 0;
     for (u32 w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < total; w += (gridDim.x * blockDim.x) >> 5) {
         int lo = 0, hi = items - 1;  // the last item whose chunks start at or before w
         while (lo < hi) {
@@ -2739,9 +2842,12 @@ __global__ void k_events(int count, const JointMove* moves, const u32* chunk_off
 // and net of a's moves (in order, empty moves adding nothing) are block
 // scans, and the stop is the first feasible move whose running gain is the
 // largest one above zero, the move at which the serial scan last improved.
+// Then appends the vertices of the moves up to it to the movers.
 constexpr int kPrefixThreads = kScanThreads;
-__global__ void __launch_bounds__(kPrefixThreads) k_prefix(int count, int k, const JointMove* moves, const u64* events,
-                                                           const u64* loads, u64 capacity, int* stops) {
+__global__ void __launch_bounds__(kPrefixThreads) k_prefix(const u32* count_ptr, const JointMove* moves,
+                                                           const u64* events, const u64* loads, u64 capacity,
+                                                           int* movers, u64* mover_count) {
+    const int count = static_cast<int>(*count_ptr);
     __shared__ long long s_scan[9];
     __shared__ int s_range[2];
     __shared__ long long s_best_gain[kPrefixThreads / 32];
@@ -2788,18 +2894,17 @@ __global__ void __launch_bounds__(kPrefixThreads) k_prefix(int count, int k, con
                 best = s_best_gain[w];
                 stop = s_best_index[w];
             }
-        stops[a] = stop;
+        s_best_index[0] = stop;
+    }
+    __syncthreads();
+    stop = s_best_index[0];
+    for (int i = first + static_cast<int>(threadIdx.x); i <= stop; i += kPrefixThreads) {
+        const JointMove& m = moves[i];
+        if (!m.size) continue;
+        const u64 at = atomicAdd(mover_count, static_cast<u64>(m.size));
+        for (int j = 0; j < m.size; ++j) movers[at + j] = m.vertices[j];
     }
 }
-__global__ void k_accept(int count, const JointMove* moves, const int* stops, int* flags) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count && moves[i].size && i <= stops[moves[i].a])
-        for (int j = 0; j < moves[i].size; ++j) flags[moves[i].vertices[j]] = 1;
-}
-struct Flagged {
-    const int* flags;
-    __device__ bool operator()(i64 v) const { return flags[v] != 0; }
-};
 
 }  // namespace
 }  // namespace gp
@@ -3471,6 +3576,9 @@ void LevelRefiner<T>::restore_best(bool moved) {
     max_load_host = ctx.host_scalars[0];
 }
 
+// The exchange passes.  A pass runs on device counts from the matching to the
+// applied batch, so the host reads back once per pass; only when it finds a
+// list longer than one block sorts does it finish the pass step by step.
 template <class T>
 void LevelRefiner<T>::exchange(u64& best_cut) {
     Arena& A_ = ctx.scratch;
@@ -3481,98 +3589,94 @@ void LevelRefiner<T>::exchange(u64& best_cut) {
     int* visits = A_.alloc<int>(static_cast<size_t>(k) * k);
     int* partner = A_.alloc<int>(k);
     u64* seeds = A_.alloc<u64>(static_cast<size_t>(k) * sw);
-    JointMove* moves = A_.alloc<JointMove>(slots);
-    JointMove* archive = A_.alloc<JointMove>(static_cast<size_t>(slots) * kJointArchive);
-    JointMove* frag = A_.alloc<JointMove>(static_cast<size_t>(slots) * kJointArchive);
-    JointMove* frag_sorted = A_.alloc<JointMove>(static_cast<size_t>(slots) * kJointArchive);
-    const size_t pool_cap = static_cast<size_t>(slots) + 2 * static_cast<size_t>(slots) * kJointArchive;
-    JointMove* pool = A_.alloc<JointMove>(pool_cap);
-    JointMove* act = A_.alloc<JointMove>(pool_cap);
-    JointMove* act_sorted = A_.alloc<JointMove>(pool_cap);
-    int* idx = A_.alloc<int>(2 * pool_cap);
-    MoveKey* move_keys = A_.alloc<MoveKey>(pool_cap);
+    const size_t frag_cap = static_cast<size_t>(slots) * kJointArchive;
+    const size_t move_cap = static_cast<size_t>(slots) + 2 * frag_cap;
+    JointMove* frag = A_.alloc<JointMove>(frag_cap);
+    JointMove* frag_sorted = A_.alloc<JointMove>(frag_cap);
+    JointMove* act = A_.alloc<JointMove>(move_cap);
+    JointMove* act_sorted = A_.alloc<JointMove>(move_cap);
     int* owners = A_.alloc<int>(n);
-    u64* events = A_.alloc<u64>(pool_cap);
-    int* stops = A_.alloc<int>(k);
-    u32* cnt = reinterpret_cast<u32*>(counters + 4);
+    u64* events = A_.alloc<u64>(move_cap);
+    u32* chunk_off = A_.alloc<u32>(move_cap * 8);
+    u32* total_chunks = A_.alloc<u32>(1);
+    JointCounts* counts = A_.alloc<JointCounts>(1);
+    u64* mover_count = counters + 9;
     GP_CUDA(cudaMemsetAsync(quotient, 0, sizeof(u64) * k * k, s()));
     GP_CUDA(cudaMemsetAsync(visits, 0, sizeof(int) * k * k, s()));
     launch(k_quotient<T>, grid_for(n, kThreads), kThreads, 0, s(), n, labels, static_cast<const T*>(A), k, quotient);
-    auto read_count = [&]() -> i64 {
-        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 4, sizeof(u64), cudaMemcpyDeviceToHost, s()));
+    auto read_counts = [&]() {
+        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars + 16, counts, sizeof(JointCounts), cudaMemcpyDeviceToHost, s()));
+        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 2, 8 * sizeof(u64), cudaMemcpyDeviceToHost, s()));
         GP_CUDA(cudaStreamSynchronize(s()));
-        return static_cast<i64>(ctx.host_scalars[0] & 0xffffffffULL);
+        return *reinterpret_cast<const JointCounts*>(ctx.host_scalars + 16);
     };
-    auto sort_moves = [&](JointMove* in, JointMove* out, int count, auto cmp) {
+    // (Shared-memory limits are set to one value for every size, on every
+    // call: the limit belongs to the kernel for the whole process, on
+    // whichever device is current, and concurrent worker contexts must not
+    // lower it under each other's launches.)
+    auto allow = [](auto kernel, size_t smem) {
+        GP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    };
+    constexpr size_t sort_smem = kBitonicEntryBytes * kBitonicSegment;
+    // Events, prefixes and the batch of the ordered moves.
+    auto settle = [&]() {
+        launch(k_events, 148 * 8, kThreads, 0, s(), static_cast<const u32*>(&counts->active),
+               static_cast<const JointMove*>(act_sorted), static_cast<const u32*>(chunk_off),
+               static_cast<const u32*>(total_chunks), static_cast<const int*>(owners), static_cast<const int*>(targets),
+               static_cast<const int*>(labels), g.off, g.nbr, g.ew, events);
+        launch(k_prefix, k, kPrefixThreads, 0, s(), static_cast<const u32*>(&counts->active),
+               static_cast<const JointMove*>(act_sorted), static_cast<const u64*>(events),
+               static_cast<const u64*>(loads), C, movers, mover_count);
+        apply(movers, mover_count, n, false, false);
+    };
+    auto sort_long = [&](JointMove* in, JointMove* out, int count, auto cmp) {
         using Cmp = decltype(cmp);
-        int size = 1;
+        ArenaScope ss(A_);
+        int size = kBitonicSegment;
         while (size < count) size <<= 1;
-        // (Shared-memory limits are set to one value for every size, on every
-        // call that needs more than the default: the limit belongs to the
-        // kernel for the whole process, on whichever device is current, and
-        // concurrent worker contexts must not lower it under each other's
-        // launches.)
-        if (size <= kBitonicSegment) {
-            const size_t smem = kBitonicEntryBytes * size;
-            if (smem > 48 * 1024)
-                GP_CUDA(cudaFuncSetAttribute(k_sort_moves_block<Cmp>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(kBitonicEntryBytes * kBitonicSegment)));
-            launch(k_sort_moves_block<Cmp>, 1, 1024, smem, s(), size, count, static_cast<const JointMove*>(in), out,
-                   cmp);
-            return;
-        }
+        int* idx = A_.alloc<int>(size);
+        MoveKey* move_keys = A_.alloc<MoveKey>(count);
         launch(k_iota, blocks_for(size, kThreads), kThreads, 0, s(), size, idx);
         launch(k_move_keys<Cmp>, blocks_for(count, kThreads), kThreads, 0, s(), count,
                static_cast<const JointMove*>(in), move_keys);
         // Stages whose partner distance stays inside a segment run in shared
         // memory, the rest one launch per stage.
-        const size_t smem = kBitonicEntryBytes * kBitonicSegment;
-        GP_CUDA(cudaFuncSetAttribute(k_bitonic_local<Cmp>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(smem)));
+        allow(k_bitonic_local<Cmp>, sort_smem);
         const int segments = size / kBitonicSegment;
         const JointMove* m = in;
         const MoveKey* mk = move_keys;
-        launch(k_bitonic_local<Cmp>, segments, 1024, smem, s(), size, count, m, mk, idx, 2, kBitonicSegment, 1, cmp);
+        launch(k_bitonic_local<Cmp>, segments, 1024, sort_smem, s(), size, count, m, mk, idx, 2, kBitonicSegment, 1, cmp);
         for (int kk = 2 * kBitonicSegment; kk <= size; kk <<= 1) {
             for (int jj = kk >> 1; jj >= kBitonicSegment; jj >>= 1)
                 launch(k_bitonic<Cmp>, blocks_for(size, kThreads), kThreads, 0, s(), size, count, m, mk, idx, kk, jj,
                        cmp);
-            launch(k_bitonic_local<Cmp>, segments, 1024, smem, s(), size, count, m, mk, idx, kk, kk,
+            launch(k_bitonic_local<Cmp>, segments, 1024, sort_smem, s(), size, count, m, mk, idx, kk, kk,
                    kBitonicSegment / 2, cmp);
         }
         launch(k_gather_moves, blocks_for(count, kThreads), kThreads, 0, s(), count, static_cast<const int*>(idx),
                static_cast<const JointMove*>(in), out);
     };
-    int empty = 0;
-    for (int pass = 0; pass < budget.exchange_rounds; ++pass) {
-        const size_t match_smem = sizeof(double) * k * k;
-        // One value for every k: the limit belongs to the kernel for the whole
-        // process, and concurrent worker contexts must not lower it under
-        // each other's launches.
-        GP_CUDA(cudaFuncSetAttribute(k_match_parts, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(sizeof(double) * kMaxParts * kMaxParts)));
-        launch(k_match_parts, 1, kMatchThreads, match_smem, s(), k, quotient, partner, visits);
-        GP_CUDA(cudaMemsetAsync(seeds, 0xff, sizeof(u64) * k * sw, s()));
-        launch(k_seeds<T>, grid_for(n, kThreads), kThreads, 0, s(), n, labels, static_cast<const T*>(A), k, partner,
-               seeds, sw, pass);
-        launch(k_grow<T>, blocks_for(slots, 8), kThreads, 0, s(), slots, sw, seeds, partner, g.off, g.nbr, g.ew, g.vw,
-               labels, static_cast<const T*>(A), k, loads, C, moves, archive);
-        select_if(A_, s(), static_cast<i64>(slots) * kJointArchive, NonEmptyMove{archive}, CopyMove{archive, frag}, cnt);
-        int fragments = static_cast<int>(read_count());
-        if (fragments) {
-            sort_moves(frag, frag_sorted, fragments, NetOrder{});
-            select_if(A_, s(), fragments, UniqueHead{frag_sorted}, CopyMove{frag_sorted, frag}, cnt);
-            fragments = static_cast<int>(read_count());
+    auto combine = [&](int most) {
+        launch(k_combine, blocks_for(most, 8), kThreads, 0, s(), counts, static_cast<const JointMove*>(frag_sorted),
+               g.off, g.nbr, g.ew, labels, loads, C, slots, act);
+    };
+    // A pass with a long list, from the lists on the device.
+    auto finish_long = [&](JointCounts found) {
+        if (found.fragments > kBitonicSegment) {  // no fragment was combined yet
+            const int fragments = static_cast<int>(found.fragments);
+            ArenaScope fs(A_);
+            JointMove* ordered = A_.alloc<JointMove>(fragments);
+            sort_long(frag, ordered, fragments, NetOrder{});
+            select_if(A_, s(), fragments, UniqueHead{ordered}, CopyMove{ordered, frag_sorted}, &counts->unique);
+            combine(fragments);
+            found = read_counts();
         }
-        const int pool_size = slots + 2 * fragments;
-        GP_CUDA(cudaMemcpyAsync(pool, moves, sizeof(JointMove) * slots, cudaMemcpyDeviceToDevice, s()));
-        if (fragments)
-            launch(k_combine, blocks_for(fragments, 8), kThreads, 0, s(), fragments, static_cast<const JointMove*>(frag),
-                   g.off, g.nbr, g.ew, labels, loads, C, slots, pool + slots);
-        select_if(A_, s(), pool_size, NonEmptyMove{pool}, CopyMove{pool, act}, cnt);
-        const int active = static_cast<int>(read_count());
-        if (!active) { if (++empty >= 2) break; continue; }
-        sort_moves(act, act_sorted, active, MoveOrder{});
+        const int active = static_cast<int>(found.moves);
+        if (!active) return;
+        sort_long(act, act_sorted, active, MoveOrder{});
+        const u32 length = static_cast<u32>(active);
+        ctx.host_scalars[24] = length;
+        GP_CUDA(cudaMemcpyAsync(&counts->active, ctx.host_scalars + 24, sizeof(u32), cudaMemcpyHostToDevice, s()));
         fill<int>(s(), owners, n, INT_MAX);
         launch(k_claim, blocks_for(active, kThreads), kThreads, 0, s(), active, static_cast<const JointMove*>(act_sorted), owners);
         launch(k_resolve, blocks_for(active, kThreads), kThreads, 0, s(), active, act_sorted, static_cast<const int*>(owners));
@@ -3580,28 +3684,30 @@ void LevelRefiner<T>::exchange(u64& best_cut) {
         launch(k_mark, blocks_for(active, kThreads), kThreads, 0, s(), active, static_cast<const JointMove*>(act_sorted),
                static_cast<const int*>(labels), owners, targets);
         GP_CUDA(cudaMemsetAsync(events, 0, sizeof(u64) * active, s()));
-        {
-            ArenaScope es(A_);
-            u32* chunk_off = A_.alloc<u32>(static_cast<size_t>(active) * 8);
-            u32* total_chunks = A_.alloc<u32>(1);
-            exclusive_scan<u32>(A_, s(), static_cast<i64>(active) * 8,
-                                EventChunks{static_cast<const JointMove*>(act_sorted), g.off}, chunk_off, total_chunks);
-            launch(k_events, 148 * 8, kThreads, 0, s(), active, static_cast<const JointMove*>(act_sorted),
-                   static_cast<const u32*>(chunk_off), static_cast<const u32*>(total_chunks),
-                   static_cast<const int*>(owners), static_cast<const int*>(targets), static_cast<const int*>(labels),
-                   g.off, g.nbr, g.ew, events);
-        }
-        launch(k_prefix, k, kPrefixThreads, 0, s(), active, k, static_cast<const JointMove*>(act_sorted),
-               static_cast<const u64*>(events), static_cast<const u64*>(loads), C, stops);
-        launch(k_accept, blocks_for(active, kThreads), kThreads, 0, s(), active, static_cast<const JointMove*>(act_sorted),
-               static_cast<const int*>(stops), flags);
-        // The accepted moves applied with their count left on the device
-        // (as the repair does): one read-back for the count and the
-        // batch's counters; an empty batch changes nothing.
-        select_if(A_, s(), n, Flagged{flags}, WriteIndex{movers}, reinterpret_cast<u32*>(counters + 9));
-        apply(movers, counters + 9, n, false, false);
-        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 2, 8 * sizeof(u64), cudaMemcpyDeviceToHost, s()));
-        GP_CUDA(cudaStreamSynchronize(s()));
+        exclusive_scan<u32>(A_, s(), static_cast<i64>(active) * 8,
+                            EventChunks{static_cast<const JointMove*>(act_sorted), g.off}, chunk_off, total_chunks);
+        settle();
+        read_counts();
+    };
+    int empty = 0;
+    for (int pass = 0; pass < budget.exchange_rounds; ++pass) {
+        // One value for every k (see `allow`).
+        allow(k_match_parts, sizeof(double) * kMaxParts * kMaxParts);
+        launch(k_match_parts, 1, kMatchThreads, sizeof(double) * k * k, s(), k, quotient, partner, visits, seeds, k * sw,
+               counts, mover_count);
+        launch(k_seeds<T>, grid_for(n, kThreads), kThreads, 0, s(), n, labels, static_cast<const T*>(A), k, partner,
+               seeds, sw, pass, owners);
+        launch(k_grow<T>, blocks_for(slots, 8), kThreads, 0, s(), slots, sw, seeds, partner, g.off, g.nbr, g.ew, g.vw,
+               labels, static_cast<const T*>(A), k, loads, C, act, frag, counts);
+        allow(k_sort_fragments, sort_smem);
+        launch(k_sort_fragments, 1, 1024, sort_smem, s(), static_cast<const JointMove*>(frag), frag_sorted, counts);
+        combine(kBitonicSegment);
+        allow(k_rank_moves, sort_smem);
+        launch(k_rank_moves, 1, 1024, sort_smem, s(), static_cast<const JointMove*>(act), act_sorted, counts, g.off,
+               static_cast<const int*>(labels), owners, targets, events, chunk_off, total_chunks);
+        settle();
+        const JointCounts found = read_counts();
+        if (found.fragments > kBitonicSegment || found.moves > kBitonicSegment) finish_long(found);
         const i64 count = static_cast<i64>(ctx.host_scalars[7] & 0xffffffffULL);
         if (!count) { if (++empty >= 2) break; continue; }
         empty = 0;
