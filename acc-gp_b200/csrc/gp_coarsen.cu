@@ -43,6 +43,7 @@ constexpr int kMediumWarps = 4;
 template <int W>
 __global__ void __launch_bounds__(256) k_level0_meta(i64 n, const int* off, const int* nbr, const u32* ew,
                                                      const u32* vw, u64* bounds, u64* sc) {
+    after_previous();
     const int lane = threadIdx.x & (W - 1);
     constexpr int kGroups = 32 / W;  // rows per warp and pass
     const i64 warps = (static_cast<i64>(gridDim.x) * blockDim.x) >> 5;
@@ -89,6 +90,7 @@ __global__ void __launch_bounds__(256) k_level0_meta(i64 n, const int* off, cons
 
 // Heavy rows of record_bound_kernel, one block per chunk.
 __global__ void k_level0_meta_chunks(DGraph g, u64* bounds, u64* sc) {
+    after_previous();
     const int c = blockIdx.x, v = g.chunk_row[c];
     const int begin = g.off[v];
     u64 d = 0;
@@ -113,6 +115,7 @@ __global__ void k_level0_meta_chunks(DGraph g, u64* bounds, u64* sc) {
     }
 }
 __global__ void k_heavy_bound_max(i64 count, const int* heavy, const u64* bounds, u64* sc) {
+    after_previous();
     const i64 h = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (h < count) atomicMax(sc + 0, bounds[heavy[h]]);
 }
@@ -127,6 +130,7 @@ __global__ void k_heavy_bound_max(i64 count, const int* heavy, const u64* bounds
 __global__ void __launch_bounds__(256) k_degree_classes(i64 n, const int* off, int* low, int* medium, int* large,
                                                         int* heavy, int* large_wide, int medium_degree,
                                                         int large_narrow, u64* sc) {
+    after_previous();
     u64 d_max = 0, isolated = 0;
     int big = 0;
     // Block-uniform passes: the appends synchronise the block.
@@ -173,6 +177,7 @@ struct HeavySlots {
 template <int W>
 __global__ void k_match_choose(i64 n, const int* off, const int* nbr, const u32* ew, const u32* vw, u64 capacity,
                                u32 salt, int* choice) {
+    after_previous();
     const i64 v = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) / W;
     const int lane = threadIdx.x & (W - 1);
     const bool valid = v < n;
@@ -202,6 +207,7 @@ __global__ void k_match_choose(i64 n, const int* off, const int* nbr, const u32*
 // matching_commit + matching_roots + residual_seed_weights.
 // *merged counts the pairs.
 __global__ void k_match_roots(i64 n, const int* choice, int* clusters, u64* merged) {
+    after_previous();
     u64 pairs = 0;
     for (i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += static_cast<i64>(gridDim.x) * blockDim.x) {
         const int u = choice[v];
@@ -214,6 +220,7 @@ __global__ void k_match_roots(i64 n, const int* choice, int* clusters, u64* merg
 }
 
 __global__ void k_cluster_weights(i64 n, const int* clusters, const u32* vw, u64* cw) {
+    after_previous();
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (v < n) atomicAdd(cw + clusters[v], static_cast<u64>(vw[v]));
 }
@@ -247,6 +254,7 @@ struct RoundParams {
 // cluster is one gather instead of the role and weight gathers.
 __global__ void k_roles(i64 n, const int* clusters, const u32* vw, const u64* cw, u32 salt, u32 threshold,
                         bool all_singletons, unsigned char* roles, u64* recv, int* proposals, u64* demand) {
+    after_previous();
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (v >= n) return;
     const u64 weight = cw[v];
@@ -446,6 +454,7 @@ __device__ __forceinline__ void consider_slots(const RoundParams& p, Summary& s,
 // Rows of degree <= 8: one 8-lane group per row; equal clusters are grouped
 // with match_any (sclp_affinity_low_match_kernel, aggregation.cuh:268-341).
 __global__ void k_affinity_low(i64 count, const int* rows, RoundParams p) {
+    after_previous();
     const int lane = threadIdx.x & 31, sub = lane & 7;
     const i64 index = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 3;
     int v = -1, src = -1;
@@ -482,6 +491,7 @@ __global__ void k_affinity_low(i64 count, const int* rows, RoundParams p) {
 // (sclp_affinity_medium_hash_kernel, aggregation.cuh:343-422).
 template <class Table>
 __global__ void __launch_bounds__(kMediumWarps * 32) k_affinity_medium(i64 count, const int* rows, RoundParams p) {
+    after_previous();
     __shared__ __align__(16) unsigned char raw[kMediumWarps * kMediumHash * Table::kSlotBytes];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     u64* vals = reinterpret_cast<u64*>(raw);
@@ -531,6 +541,7 @@ __global__ void __launch_bounds__(kMediumWarps * 32) k_affinity_medium(i64 count
 // entries (values first, then keys).
 template <class Table>
 __global__ void __launch_bounds__(256, 5) k_affinity_large(i64 count, const int* rows, RoundParams p) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ Summary warp_sum_s[8];
     const int v = rows[blockIdx.x];
@@ -563,6 +574,7 @@ __global__ void __launch_bounds__(256, 5) k_affinity_large(i64 count, const int*
 template <class Table>
 __global__ void __launch_bounds__(256) k_affinity_heavy_insert(DGraph g, const u64* table_off, int* keys, u64* vals,
                                                                 RoundParams p) {
+    after_previous();
     const int c = blockIdx.x, v = g.chunk_row[c];
     int src;
     if (!is_mover(p, v, src)) return;
@@ -578,6 +590,7 @@ template <class Table>
 __global__ void __launch_bounds__(256) k_affinity_heavy_summary(const int* heavy, const int* seg_hidx,
                                                                  const int* seg_index, const u64* table_off, int* keys,
                                                                  u64* vals, RoundParams p, Summary* partial) {
+    after_previous();
     constexpr int kPerThread = kSegment / 256;
     __shared__ Summary warp_part[8];
     const int sg = blockIdx.x, h = seg_hidx[sg], v = heavy[h];
@@ -613,6 +626,7 @@ __global__ void __launch_bounds__(256) k_affinity_heavy_summary(const int* heavy
 }
 __global__ void k_affinity_heavy_finish(i64 count, const int* heavy, const int* seg_off, const Summary* partial,
                                         RoundParams p) {
+    after_previous();
     const int lane = threadIdx.x & 31;
     const i64 h = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     if (h >= count) return;
@@ -634,6 +648,7 @@ struct HeavySegments {
 };
 __global__ void k_emit_segments(i64 count, const int* heavy, const int* off, const int* seg_off, int* seg_hidx,
                                 int* seg_index) {
+    after_previous();
     const i64 h = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (h >= count) return;
     const int segs = static_cast<int>(heavy_slots(off[heavy[h] + 1] - off[heavy[h]]) / kSegment);
@@ -650,6 +665,7 @@ __global__ void k_emit_segments(i64 count, const int* heavy, const int* off, con
 // accept: 0 reject, 1 accept, 2 needs the ordered prefix test.
 __global__ void k_classify(i64 n, const int* proposals, const u64* cw, const u64* demand, u64 capacity,
                            unsigned char* accept) {
+    after_previous();
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (v >= n) return;
     const int t = proposals[v];
@@ -669,14 +685,17 @@ struct HasValue {
 
 // Keys for the LSD passes over an ordered list of vertices.
 __global__ void k_key_tie(i64 count, const u32* items, const u32* ties, u64* keys) {
+    after_previous();
     const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < count) keys[i] = static_cast<u64>(~ties[items[i]]);
 }
 __global__ void k_key_gain(i64 count, const u32* items, const u64* gains, u64 mask, u64* keys) {
+    after_previous();
     const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < count) keys[i] = mask - (gains[items[i]] & mask);
 }
 __global__ void k_key_target(i64 count, const u32* items, const int* targets, u64* keys) {
+    after_previous();
     const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < count) keys[i] = static_cast<u64>(targets[items[i]]);
 }
@@ -696,6 +715,7 @@ __global__ void __launch_bounds__(kSortThreads) k_order_block(const u32* count_p
                                                              const int* targets, int target_bits, const u32* vw,
                                                              u64* cw, u64 capacity, unsigned char* accept, u64 budget,
                                                              int* clusters, u64* merged) {
+    after_previous();
     __shared__ SortTileSmem sm;
     __shared__ u64 scan64[33];
     __shared__ u32 scan32[33];
@@ -803,6 +823,7 @@ __global__ void __launch_bounds__(kSortThreads) k_order_block(const u32* count_p
 // Segment heads of an ordered list grouped by target.
 __global__ void k_segment_heads(i64 count, const u32* items, const int* targets, const u64* prefix, u64* segment_base,
                                 int* segment_first) {
+    after_previous();
     const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const int t = targets[items[i]];
@@ -822,6 +843,7 @@ struct OrderedWeight {
 // inclusive weight prefix within the target fits in C - base.
 __global__ void k_ordered_accept(i64 count, const u32* items, const int* targets, const u32* vw, const u64* prefix,
                                  const u64* segment_base, const u64* cw, u64 capacity, unsigned char* accept) {
+    after_previous();
     const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const int v = static_cast<int>(items[i]);
@@ -837,6 +859,7 @@ __global__ void k_ordered_accept(i64 count, const u32* items, const int* targets
 // takes.
 __global__ void k_commit(i64 n, const int* proposals, const unsigned char* accept, const u32* vw, int* clusters,
                          u64* cw, const u32* items, u64* merged) {
+    after_previous();
     if (items && *items > kSortTile) return;
     u64 moved = 0;
     for (i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += static_cast<i64>(gridDim.x) * blockDim.x) {
@@ -866,6 +889,7 @@ struct IsIsolated {
 // isolated_representative_kernel / isolated_commit_kernel (aggregation.cuh:713-745);
 // `prefix` is exclusive here.
 __global__ void k_isolated_rep(i64 count, const int* list, const u64* prefix, const u32* vw, u64 capacity, int* reps) {
+    after_previous();
     const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const int v = list[i];
@@ -875,6 +899,7 @@ __global__ void k_isolated_rep(i64 count, const int* list, const u64* prefix, co
 }
 __global__ void k_isolated_commit(i64 count, const int* list, const u64* prefix, const u32* vw, u64 capacity,
                                   const int* reps, int* clusters, u64* cw, u64* merged) {
+    after_previous();
     u64 moved = 0;
     for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += static_cast<i64>(gridDim.x) * blockDim.x) {
         const int v = list[i];
@@ -893,6 +918,7 @@ __global__ void k_isolated_commit(i64 count, const int* list, const u64* prefix,
 
 // sclp_singleton_favorite_kernel (aggregation.cuh:654-664).
 __global__ void k_favorites(i64 n, const u32* vw, const u64* cw, const int* clusters, int* proposals) {
+    after_previous();
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (v < n && cw[clusters[v]] != static_cast<u64>(vw[v])) proposals[v] = kInvalid;
 }
@@ -901,6 +927,7 @@ __global__ void k_favorites(i64 n, const u32* vw, const u64* cw, const int* clus
 // a favourite's group pair with their predecessor when both fit.
 __global__ void k_pair_flags(i64 count, const u32* items, const int* favorites, const int* segment_first,
                              const u32* vw, u64 capacity, u32* flags) {
+    after_previous();
     const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const int v = static_cast<int>(items[i]);
@@ -915,6 +942,7 @@ struct LoadU32 {
 // Both are clusters of one vertex, so every pair empties one: *merged counts.
 __global__ void k_pair_commit(i64 count, const u32* items, const u32* flags, const u32* positions, u64 budget,
                               const u32* vw, int* clusters, u64* cw, u64* merged) {
+    after_previous();
     u64 moved = 0;
     for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += static_cast<i64>(gridDim.x) * blockDim.x) {
         if (!flags[i] || positions[i] >= budget) continue;
@@ -937,23 +965,27 @@ struct NonEmptyInt {
     __device__ int operator()(i64 i) const { return cw[i] > 0 ? 1 : 0; }
 };
 __global__ void k_iota_clusters(i64 n, const u32* vw, int* clusters, u64* cw) {
+    after_previous();
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (v >= n) return;
     clusters[v] = static_cast<int>(v);
     cw[v] = vw[v];
 }
 __global__ void k_count_isolated(i64 n, const int* off, u64* out) {
+    after_previous();
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     block_atomic_add(out, v < n && off[v] == off[v + 1] ? 1ULL : 0ULL);
 }
 // The map, and each coarse vertex's weight: its cluster's.
 __global__ void k_map(i64 n, const int* clusters, const int* ids, const u64* cw, int* map, u32* cvw) {
+    after_previous();
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (v >= n) return;
     map[v] = ids[clusters[v]];
     if (cw[v]) cvw[ids[v]] = static_cast<u32>(cw[v]);
 }
 __global__ void k_max_weight(i64 n, const u64* cw, u64* out) {
+    after_previous();
     u64 m = 0;
     for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += static_cast<i64>(gridDim.x) * blockDim.x)
         m = max(m, cw[i] & 0xffffffffULL);
@@ -966,6 +998,7 @@ __global__ void k_max_weight(i64 n, const u64* cw, u64* out) {
 // member counts.
 __global__ void k_contract_bounds(i64 n, const int* map, const int* off, const u64* fine_bounds, u64* coarse_bounds,
                                   int* raw, bool bounded) {
+    after_previous();
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (v >= n) return;
     const int c = map[v];
@@ -981,6 +1014,7 @@ __global__ void k_contract_bounds(i64 n, const int* map, const int* off, const u
     }
 }
 __global__ void k_max_pair(i64 n, const u64* a, const int* b, u64* out) {
+    after_previous();
     const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     block_atomic_max(out, i < n ? a[i] : 0ULL);
     block_atomic_max(out + 1, i < n ? static_cast<u64>(b[i]) : 0ULL);
@@ -996,6 +1030,7 @@ struct LoadInt {
 // The row's slot in the segment is reserved first (one atomic per row), then
 // light rows are copied by 8 lanes and heavy rows chunk-parallel.
 __global__ void k_row_base(i64 n, const int* off, const int* map, int* cursor, int* base) {
+    after_previous();
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (v < n) base[v] = atomicAdd(cursor + map[v], off[v + 1] - off[v]);
 }
@@ -1005,6 +1040,7 @@ __global__ void k_row_base(i64 n, const int* off, const int* map, int* cursor, i
 template <int W>
 __global__ void k_scatter(i64 n, const int* off, const int* nbr, const u32* ew, const int* map, const int* base,
                           int* raw_t, u32* raw_w) {
+    after_previous();
     constexpr int U = 4;
     const i64 v = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) / W;
     const int lane = threadIdx.x % W;
@@ -1035,6 +1071,7 @@ __global__ void k_scatter(i64 n, const int* off, const int* nbr, const u32* ew, 
 // A block per chunk; every thread's entries (kChunk / blockDim of them) have
 // their neighbour and map gathers in flight together.
 __global__ void k_scatter_chunks(DGraph g, const int* map, const int* base, int* raw_t, u32* raw_w) {
+    after_previous();
     constexpr int U = 8;
     const int ch = blockIdx.x, v = g.chunk_row[ch];
     const int c = map[v];
@@ -1060,6 +1097,7 @@ __global__ void k_scatter_chunks(DGraph g, const int* map, const int* base, int*
 // records of class 6.
 constexpr int kRowClasses = 8, kLargeClass = 6, kShortClass = 7, kShortRow = 16;
 __global__ void k_row_classes(i64 nc, const int* raw, int* lists, i64 stride, u64* sc) {
+    after_previous();
     const i64 c = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int r = c < nc ? raw[c] : 0;
     const int cls = c >= nc                  ? -1
@@ -1230,6 +1268,7 @@ __device__ void warp_radix_row(int begin, int degree, int* keys_io, u32* w_io, i
 // 256^3 mesh at k = 128; with this and the matching's lanes it takes 172-181.
 __global__ void __launch_bounds__(256) k_sort_rows_short(i64 count, const int* rows, const int* raw_off, int* raw_t,
                                                          u32* raw_w, int* ucount) {
+    after_previous();
     constexpr int W = kShortRow;
     const i64 index = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) / W;
     const int lane = threadIdx.x & 31, sub = lane % W;
@@ -1269,6 +1308,7 @@ __global__ void __launch_bounds__(256) k_sort_rows_short(i64 count, const int* r
 template <bool Long>
 __global__ void __launch_bounds__(256) k_sort_rows_warp(i64 count, const int* rows, const int* raw_off, int* raw_t,
                                                         u32* raw_w, int* ucount, int nc, int bits) {
+    after_previous();
     __shared__ int skeys[Long ? 8 : 1][512];
     __shared__ u32 svals[Long ? 8 : 1][512];
     __shared__ u32 counts[Long ? 8 : 1][kRadix];
@@ -1336,6 +1376,7 @@ __device__ __forceinline__ void sort_row_in_smem(int* keys, u32* vals, u32 (*war
 template <int Items>
 __global__ void __launch_bounds__(256) k_sort_rows_block(const int* rows, const int* raw_off, int* raw_t, u32* raw_w,
                                                          int* ucount, int nc, int bits) {
+    after_previous();
     static_assert(Items * 256 <= 2048, "row class of the 256-thread block sort");
     __shared__ int keys[Items * 256];
     __shared__ u32 vals[Items * 256];
@@ -1382,6 +1423,7 @@ template <int Threads>
 __global__ void __launch_bounds__(Threads, 1024 / Threads) k_sort_rows_big(const int* rows, const int* raw_off,
                                                                           int* raw_t, u32* raw_w, int* ucount, int nc,
                                                                           int bits) {
+    after_previous();
     constexpr int kRow = Threads * 8;
     extern __shared__ __align__(16) unsigned char big_smem[];
     int* keys = reinterpret_cast<int*>(big_smem);
@@ -1424,6 +1466,7 @@ __global__ void __launch_bounds__(Threads, 1024 / Threads) k_sort_rows_big(const
 // one boundary.
 __global__ void k_large_records(i64 records, i64 count, const int* rows, const int* raw_off, const int* rec_off,
                                 const int* raw_t, const u32* raw_w, int tbits, u64* keys, u32* vals) {
+    after_previous();
     __shared__ int s_row;
     const u64 sentinel = (1ULL << tbits) - 1;
     for (i64 base = static_cast<i64>(blockIdx.x) * blockDim.x; base < records;
@@ -1474,6 +1517,7 @@ struct RecordHead {
 };
 __global__ void k_large_write(i64 records, const u64* keys, const u32* vals, int shift, const u32* hpos, int tbits,
                               const int* rows, const int* rec_off, const int* raw_off, int* raw_t, u32* raw_w) {
+    after_previous();
     const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= records) return;
     const u64 k = keys[i] >> shift;
@@ -1490,6 +1534,7 @@ __global__ void k_large_write(i64 records, const u64* keys, const u32* vals, int
 }
 __global__ void k_large_counts(i64 count, const int* rows, const int* rec_off, const u32* hpos, const u32* total,
                                i64 records, int* ucount) {
+    after_previous();
     const i64 j = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (j >= count) return;
     const u32 first = hpos[rec_off[j]];
@@ -1502,6 +1547,7 @@ __global__ void k_large_counts(i64 count, const int* rows, const int* rec_off, c
 template <int W>
 __global__ void k_copy_rows(i64 nc, const int* raw_off, const int* raw_t, const u32* raw_w, const int* off, int* nbr,
                             u32* ew) {
+    after_previous();
     constexpr int U = 4;
     const i64 c = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) / W;
     const int lane = threadIdx.x % W;
@@ -1526,6 +1572,7 @@ __global__ void k_copy_rows(i64 nc, const int* raw_off, const int* raw_t, const 
     }
 }
 __global__ void k_copy_chunks(DGraph g, const int* raw_off, const int* raw_t, const u32* raw_w) {
+    after_previous();
     constexpr int U = 8;
     const int ch = blockIdx.x, c = g.chunk_row[ch];
     const int shift = raw_off[c] - g.off[c];
@@ -1551,6 +1598,7 @@ __global__ void k_copy_chunks(DGraph g, const int* raw_off, const int* raw_t, co
 // ---------------------------------------------------------------- chunk lists
 
 __global__ void k_heavy_counts(i64 n, const int* off, int heavy_min, u64* sc) {
+    after_previous();
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     u64 rows = 0, chunks = 0, entries = 0;
     if (v < n) {
@@ -1573,6 +1621,7 @@ struct ChunkCount {
 };
 __global__ void k_emit_chunks(i64 count, const int* heavy, const int* off, const int* chunk_off, int* chunk_row,
                               int* chunk_hidx, int* chunk_begin) {
+    after_previous();
     const i64 h = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (h >= count) return;
     const int v = heavy[h], d = off[v + 1] - off[v];

@@ -73,6 +73,18 @@ inline unsigned long long* work_counter(K kernel) {
                ? g_profiler->device_bytes : nullptr;
 }
 
+// Waits until the kernel before this one in the stream is complete and its
+// writes are visible.  The first statement of every kernel that launch()
+// starts: launch() lets a kernel's blocks be set up while the previous kernel
+// drains, and this is what still orders the two.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Starts a kernel as the programmatic dependent of the one before it in the
+// stream.  A dependent chain of short kernels, which most of a V-cycle is,
+// takes 2.3 us a kernel instead of 2.9-3.5 (148-592 blocks of 256 threads) and
+// 3.1 instead of 4.6 (4096 blocks).  No kernel triggers its dependents early:
+// their waiting blocks would take the place of its own last ones (4.6 us
+// again at 4096 blocks).
 template <class... Params, class... Args>
 inline void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                    Args&&... args) {
@@ -80,11 +92,36 @@ inline void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem
     const bool timed = g_profiler && g_profiler->matches(reinterpret_cast<const void*>(kernel));
     if (g_profiler) g_profiler->last_timed = timed;
     if (timed) g_profiler->before(stream);
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute dependent{};
+    dependent.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    dependent.val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = &dependent;
+    config.numAttrs = 1;
     // A launch that did not start (bad configuration, missing shared-memory
     // opt-in) must fail the call, not leave its results silently unwritten.
     // This library clears the error of every failure it has handled where it
     // handles it (GP_CUDA, the server's own allocations), so what is pending
     // here belongs to this launch or to an unhandled fault.
+    cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+    if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess)
+        ::gp::fail(GP_CUDA_ERROR, std::string("kernel launch: ") + cudaGetErrorString(e));
+    if (timed) g_profiler->after(stream);
+}
+
+// Starts a kernel the ordinary way: on a caller's stream, where what ran
+// before is not ours (and may be under capture).
+template <class... Params, class... Args>
+inline void launch_ordinary(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                            Args&&... args) {
+    ++g_launches;
+    const bool timed = g_profiler && g_profiler->matches(reinterpret_cast<const void*>(kernel));
+    if (g_profiler) g_profiler->last_timed = timed;
+    if (timed) g_profiler->before(stream);
     kernel<<<grid, block, smem, stream>>>(static_cast<Params>(args)...);
     if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess)
         ::gp::fail(GP_CUDA_ERROR, std::string("kernel launch: ") + cudaGetErrorString(e));

@@ -243,9 +243,9 @@ void launch_evaluate(const gp_csr* g, const int32_t* labels, int32_t k, uint64_t
                      u64* partial, u64* invalid, cudaStream_t s) {
     // No more blocks than give every warp one window of entries.
     const int blocks = std::min(blocks_for(g->n + g->m, kEvalWarps * kEvalWindow), kEvalBlocks);
-    launch(k_eval_partials, blocks, kEvalThreads, 0, s, static_cast<i64>(g->n), static_cast<i64>(g->m),
+    launch_ordinary(k_eval_partials, blocks, kEvalThreads, 0, s, static_cast<i64>(g->n), static_cast<i64>(g->m),
            g->offsets, g->neighbors, g->edge_weights, g->vertex_weights, labels, static_cast<int>(k), partial);
-    launch(k_eval_reduce, 1, 1024, 0, s, blocks, static_cast<int>(k), static_cast<const u64*>(partial),
+    launch_ordinary(k_eval_reduce, 1, 1024, 0, s, blocks, static_cast<int>(k), static_cast<const u64*>(partial),
            reinterpret_cast<u64*>(cut_out), reinterpret_cast<u64*>(loads_out), invalid);
 }
 

@@ -102,6 +102,7 @@ namespace {
 // [0, n).
 __global__ void k_narrow(i64 count, const long long* in, int* out, bool neighbors, long long n, long long previous,
                          u64 first_index, u64* bad) {
+    after_previous();
     for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < count;
          i += static_cast<i64>(gridDim.x) * blockDim.x) {
         const long long x = in[i];
@@ -118,6 +119,7 @@ __global__ void k_narrow(i64 count, const long long* in, int* out, bool neighbor
 }
 
 __global__ void k_fill_ones(i64 n, u32* p) {
+    after_previous();
     for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += static_cast<i64>(gridDim.x) * blockDim.x)
         p[i] = 1u;
 }
@@ -127,6 +129,7 @@ __global__ void k_fill_ones(i64 n, u32* p) {
 // do not serialise.  Scalars: 0 bad offsets, 1 bad neighbour, 2 zero vertex
 // weight, 3 total vertex weight, 4 directed edge-weight sum.
 __global__ void k_validate_vertices(i64 n, i64 m, const int* off, const u32* vw, u64* sc) {
+    after_previous();
     u64 total = 0;
     u32 bad = 0, zero = 0;
     for (i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += static_cast<i64>(gridDim.x) * blockDim.x) {
@@ -146,6 +149,7 @@ __global__ void k_validate_vertices(i64 n, i64 m, const int* off, const u32* vw,
     }
 }
 __global__ void k_validate_edges(i64 n, i64 m, const int* nbr, const u32* ew, u64* sc) {
+    after_previous();
     u64 directed = 0;
     u32 bad = 0;
     for (i64 e = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += static_cast<i64>(gridDim.x) * blockDim.x) {

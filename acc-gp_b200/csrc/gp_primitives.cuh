@@ -70,6 +70,7 @@ __device__ __forceinline__ T block_exclusive_scan_wide(T value, T& total, T* sme
 
 template <class T, class In>
 __global__ void k_tile_sums(i64 n, In in, T* sums) {
+    after_previous();
     __shared__ T smem[9];
     const i64 base = static_cast<i64>(blockIdx.x) * kScanTile;
     T local = 0;
@@ -86,6 +87,7 @@ __global__ void k_tile_sums(i64 n, In in, T* sums) {
 // Exclusive scan of `count` values in place, by one block; optional total.
 template <class T>
 __global__ void k_scan_small(i64 count, T* values, T* total) {
+    after_previous();
     __shared__ T smem[9];
     T carry = 0;
     for (i64 base = 0; base < count; base += kScanTile) {
@@ -129,6 +131,7 @@ __device__ __forceinline__ T sum_before(const T* sums, int tiles, T* smem /* >= 
 // Direct: `offsets` holds the tile sums, not their exclusive scan.
 template <class T, class In, bool Direct = false>
 __global__ void k_scan_tiles(i64 n, In in, const T* offsets, T* out, T* total) {
+    after_previous();
     __shared__ T smem[9];
     const i64 base = static_cast<i64>(blockIdx.x) * kScanTile;
     T v[kScanItems];
@@ -187,6 +190,7 @@ void exclusive_scan(Arena& arena, cudaStream_t s, i64 n, In in, T* out, T* total
 
 template <class Pred>
 __global__ void k_select_count(i64 n, Pred pred, u32* counts) {
+    after_previous();
     __shared__ u32 smem[9];
     const i64 base = static_cast<i64>(blockIdx.x) * kScanTile;
     u32 local = 0;
@@ -202,6 +206,7 @@ __global__ void k_select_count(i64 n, Pred pred, u32* counts) {
 
 template <class Pred, class Out, bool Direct = false>
 __global__ void k_select_write(i64 n, Pred pred, const u32* offsets, Out out, u32* count) {
+    after_previous();
     __shared__ u32 smem[9];
     const i64 base = static_cast<i64>(blockIdx.x) * kScanTile;
     bool f[kScanItems];
@@ -270,6 +275,7 @@ __device__ __forceinline__ i64 sort_index(i64 base, int j) {
 }
 
 __global__ void k_radix_upsweep(i64 count, const u64* keys, int shift, u32* hist) {
+    after_previous();
     __shared__ u32 local[kRadix];
     for (int d = threadIdx.x; d < kRadix; d += kSortThreads) local[d] = 0;
     __syncthreads();
@@ -388,6 +394,7 @@ __device__ __forceinline__ void rank_tile(u32 (*warp_count)[kRadix], u32* local_
 template <bool WithValues, bool Direct>
 __global__ void __launch_bounds__(kSortThreads) k_radix_downsweep(i64 count, const u64* keys, const u32* vals, int shift,
                                                                   const u32* offsets, u64* keys_out, u32* vals_out) {
+    after_previous();
     __shared__ SortTileSmem sm;
     const i64 base = static_cast<i64>(blockIdx.x) * kSortTile;
     const int tile_items = static_cast<int>(count - base < kSortTile ? count - base : kSortTile);
@@ -465,6 +472,7 @@ __device__ __forceinline__ void tile_sort_passes(SortTileSmem& sm, u64 (&k)[kSor
 // place.
 template <bool WithValues>
 __global__ void __launch_bounds__(kSortThreads) k_radix_tile_sort(int count, u64* keys, u32* vals, int begin_bit, int end_bit) {
+    after_previous();
     __shared__ SortTileSmem sm;
     u64 k[kSortItems];
     u32 v[kSortItems];
@@ -531,6 +539,7 @@ inline int bit_length(u64 x) {
 
 template <class T>
 __global__ void k_fill(i64 n, T* p, T value) {
+    after_previous();
     for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += static_cast<i64>(gridDim.x) * blockDim.x)
         p[i] = value;
 }

@@ -29,6 +29,7 @@ struct Sample {
 // ---------------------------------------------------------------- small kernels
 
 __global__ void k_cut_chunks(DGraph g, const int* labels, u64* out) {
+    after_previous();
     const int c = blockIdx.x, v = g.chunk_row[c];
     const int p = labels[v];
     u64 local = 0;
@@ -37,6 +38,7 @@ __global__ void k_cut_chunks(DGraph g, const int* labels, u64* out) {
     block_atomic_add(out, local);
 }
 __global__ void k_cut(i64 n, const int* off, const int* nbr, const u32* ew, const int* labels, int heavy_min, u64* out) {
+    after_previous();
     __shared__ WarpSum cut_sum;
     cut_sum.init();
     const int lane = threadIdx.x & 31;
@@ -52,11 +54,13 @@ __global__ void k_cut(i64 n, const int* off, const int* nbr, const u32* ew, cons
 }
 
 __global__ void k_project(i64 n, const int* map, const int* coarse, int* fine) {
+    after_previous();
     const i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (v < n) fine[v] = coarse[map[v]];
 }
 
 __global__ void k_loads(i64 n, int k, const int* labels, const u32* vw, u64* loads) {
+    after_previous();
     extern __shared__ u64 part[];
     for (int p = threadIdx.x; p < k; p += blockDim.x) part[p] = 0;
     __syncthreads();
@@ -68,6 +72,7 @@ __global__ void k_loads(i64 n, int k, const int* labels, const u32* vw, u64* loa
 }
 
 __global__ void k_max_load(int k, const u64* loads, u64* out) {
+    after_previous();
     u64 m = 0;
     for (int p = threadIdx.x; p < k; p += 32) m = max(m, loads[p]);
     m = warp_max(m);
@@ -75,6 +80,7 @@ __global__ void k_max_load(int k, const u64* loads, u64* out) {
 }
 
 __global__ void k_max_edge(i64 m, const u32* ew, u64* out) {
+    after_previous();
     u32 mx = 0;
     for (i64 e = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; e < m; e += static_cast<i64>(gridDim.x) * blockDim.x)
         mx = max(mx, ew[e]);
@@ -83,6 +89,7 @@ __global__ void k_max_edge(i64 m, const u32* ew, u64* out) {
 
 // publish_repair_prices (incremental.cuh:161-164).
 __global__ void k_prices(int k, const Sample* samples, double* prices) {
+    after_previous();
     for (int p = threadIdx.x; p < k; p += blockDim.x)
         if (samples[p].weight)
             prices[p] = samples[p].loss > 0 ? static_cast<double>(samples[p].loss) / static_cast<double>(samples[p].weight) : 0.0;
@@ -139,6 +146,7 @@ __global__ void __launch_bounds__(kThreads) k_build(i64 n, const int* off, const
                                                     const int* labels, int k, C* A, C* totals, u64* directed_cut,
                                                     const u64* gate, u64 threshold, u64* work, u64 work_bytes,
                                                     int short_max, bool long_rows_apart, int heavy_min) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ WarpSum cut_sum;
     if (gate && *gate <= threshold) return;  // incremental update chosen
@@ -212,6 +220,7 @@ __global__ void __launch_bounds__(kThreads) k_build_long(i64 count, const int* r
                                                          const u32* ew, const int* labels, int k, C* A, C* totals,
                                                          u64* directed_cut, const u64* gate, u64 threshold, u64* work,
                                                          u64 work_bytes) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem_long[];
     __shared__ WarpSum cut_sum;
     if (gate && *gate <= threshold) return;
@@ -244,6 +253,7 @@ __global__ void __launch_bounds__(kThreads) k_build_long(i64 count, const int* r
 }
 // Sum of the row lengths of rows[0 .. *count).
 __global__ void k_row_entries(const u32* count, const int* rows, const int* off, u64* out) {
+    after_previous();
     const i64 c = static_cast<i64>(*count);
     u64 sum = 0;
     for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < c; i += static_cast<i64>(gridDim.x) * blockDim.x)
@@ -262,6 +272,7 @@ struct IsLongRow {
 // GP_FLAG_VERIFY: the incremental cache against an independent rebuild.
 template <class C>
 __global__ void k_compare_cache(i64 cells, const C* A, const C* B, i64 n, const C* ta, const C* tb, u64* mismatch) {
+    after_previous();
     u32 bad = 0;
     for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < cells; i += static_cast<i64>(gridDim.x) * blockDim.x)
         bad |= A[i] != B[i];
@@ -274,6 +285,7 @@ __global__ void k_compare_cache(i64 cells, const C* A, const C* B, i64 n, const 
 template <class C>
 __global__ void k_heavy_cut(i64 count, const int* heavy, const int* labels, int k, const C* A, const C* totals,
                             u64* directed_cut, const u64* gate, u64 threshold) {
+    after_previous();
     if (gate && *gate <= threshold) return;
     u64 cut = 0;
     for (i64 h = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; h < count; h += static_cast<i64>(gridDim.x) * blockDim.x) {
@@ -286,6 +298,7 @@ __global__ void k_heavy_cut(i64 count, const int* heavy, const int* labels, int 
 template <class C>
 __global__ void k_build_chunks(DGraph g, const int* labels, int k, C* A, C* totals, const u64* gate, u64 threshold,
                                u64* work, u64 work_bytes) {
+    after_previous();
     extern __shared__ unsigned char smem_build[];
     if (gate && *gate <= threshold) return;
     if (work && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(work, work_bytes);
@@ -361,6 +374,7 @@ __device__ __forceinline__ long long packed_gain(u64 w, const long long* gains, 
 template <class C, int W, bool Vectorized>
 __global__ void __launch_bounds__(kThreads) k_proposals(LpParams q, const C* A, const C* totals, const int* rows,
                                                         const u64* row_count) {
+    after_previous();
     using Vec = AffinityVec<C>;
     constexpr int N = Vectorized ? Vec::N : 1;
     constexpr int G = 32 / W;
@@ -520,6 +534,7 @@ struct RowRegs {
 // level's frontier); every other vertex is interior and would not propose.
 template <int D>
 __global__ void __launch_bounds__(kThreads) k_proposals_od(LpParams q, const int* rows, const u64* row_count) {
+    after_previous();
     __shared__ u64 s_slack[kMaxParts];
     __shared__ double s_price[kMaxParts];
     if (q.prices)
@@ -611,6 +626,7 @@ __device__ __forceinline__ long long filter_entries(const LpParams& q, int v, in
 // whole warp after them.
 constexpr int kFilterShort = 16;
 __global__ void __launch_bounds__(kThreads, 6) k_filter(LpParams q) {
+    after_previous();
     constexpr int W = 8, G = 32 / W;
     const int lane = threadIdx.x & 31, gid = lane / W, sub = lane % W;
     const i64 count = static_cast<i64>(q.counters[0]);
@@ -655,6 +671,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_filter(LpParams q) {
 // on-demand levels: a warp per six-entry row would leave most lanes idle).
 template <int D>
 __global__ void __launch_bounds__(kThreads) k_filter_od(LpParams q) {
+    after_previous();
     const i64 count = static_cast<i64>(q.counters[0]);
     for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += static_cast<i64>(gridDim.x) * blockDim.x) {
         const int v = q.cand[i];
@@ -693,6 +710,7 @@ __global__ void __launch_bounds__(kThreads) k_update_od(i64 count, const int* mo
                                                         const int* off, const int* nbr, const u32* ew, const u32* vw,
                                                         const int* labels, const int* targets, const int* flags,
                                                         long long* delta, Sample* samples) {
+    after_previous();
     __shared__ WarpSum delta_sum;
     delta_sum.init();
     if (live_count) count = static_cast<i64>(*live_count);
@@ -740,6 +758,7 @@ __device__ __forceinline__ void touch(const Frontier& f, int v) {
 // neighbours of heavy movers by k_touch_chunks.
 __global__ void k_touch_rows(i64 count, const int* movers, const u64* live_count, const int* off, const int* nbr,
                              int heavy_min, Frontier f) {
+    after_previous();
     if (live_count) count = static_cast<i64>(*live_count);
     const int lane = threadIdx.x & 31;
     for (i64 i = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; i < count;
@@ -753,6 +772,7 @@ __global__ void k_touch_rows(i64 count, const int* movers, const u64* live_count
 // The chunks of heavy rows of a list (k_heavy_chunk_list) of movers, a block
 // per chunk.
 __global__ void k_touch_chunks(DGraph g, const int* work, const u64* work_count, Frontier f) {
+    after_previous();
     const i64 count = static_cast<i64>(*work_count);
     for (i64 w = blockIdx.x; w < count; w += gridDim.x) {
         const int c = work[w], v = g.chunk_row[c];
@@ -768,6 +788,7 @@ __global__ void k_touch_chunks(DGraph g, const int* work, const u64* work_count,
 // integer contributions.
 __global__ void k_heavy_chunk_list(i64 count, const int* list, const u64* live_count, DGraph g, int* work,
                                    u64* work_count) {
+    after_previous();
     if (live_count) count = static_cast<i64>(*live_count);
     for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += static_cast<i64>(gridDim.x) * blockDim.x) {
         const int v = list[i];
@@ -791,6 +812,7 @@ __global__ void k_heavy_chunk_list(i64 count, const int* list, const u64* live_c
 template <int D>
 __global__ void __launch_bounds__(kThreads) k_frontier_init_od(i64 n, const int* off, const int* nbr, const u32* ew,
                                                                const int* labels, int* targets, Frontier f) {
+    after_previous();
     for (i64 block_base = static_cast<i64>(blockIdx.x) * blockDim.x; block_base < n;
          block_base += static_cast<i64>(gridDim.x) * blockDim.x) {
         const i64 v = block_base + threadIdx.x;
@@ -809,6 +831,7 @@ __global__ void __launch_bounds__(kThreads) k_frontier_init_od(i64 n, const int*
 template <class C>
 __global__ void k_frontier_init(i64 n, const C* A, const C* totals, int k, const int* labels, int* targets,
                                 Frontier f) {
+    after_previous();
     for (i64 block_base = static_cast<i64>(blockIdx.x) * blockDim.x; block_base < n;
          block_base += static_cast<i64>(gridDim.x) * blockDim.x) {
         const i64 v = block_base + threadIdx.x;
@@ -825,6 +848,7 @@ __global__ void k_frontier_init(i64 n, const C* A, const C* totals, int k, const
 // (incremental_heavy_priority / incremental_finish_heavy_priority,
 // incremental.cuh:395-438).
 __global__ void k_filter_chunks(DGraph g, LpParams q, long long* corr_acc, const int* work, const u64* work_count) {
+    after_previous();
     const i64 count = static_cast<i64>(*work_count);
     for (i64 w = blockIdx.x; w < count; w += gridDim.x) {
         const int c = work[w], v = g.chunk_row[c];
@@ -841,6 +865,7 @@ __global__ void k_filter_chunks(DGraph g, LpParams q, long long* corr_acc, const
     }
 }
 __global__ void k_filter_finish(i64 count, const int* heavy, const long long* corr_acc, LpParams q) {
+    after_previous();
     const i64 h = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (h >= count) return;
     const int v = heavy[h];
@@ -870,6 +895,7 @@ __device__ __forceinline__ int state_next(u32 st) {  // the label after this bat
 }
 
 __global__ void k_state_init(i64 n, const int* labels, u32* state) {
+    after_previous();
     for (i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += static_cast<i64>(gridDim.x) * blockDim.x)
         state[v] = static_cast<u32>(labels[v]);
 }
@@ -930,6 +956,7 @@ template <class C>
 __global__ void __launch_bounds__(kThreads, 6) k_update(i64 count, const int* movers, const u64* live_count, const int* off, const int* nbr,
                          const u32* ew, const u32* vw, const u32* state, int k, C* A, long long* delta,
                          Sample* samples, const u64* gate, u64 threshold, int heavy_min, u64* work) {
+    after_previous();
     constexpr int W = 8, G = 32 / W;
     __shared__ WarpSum delta_sum;
     const int lane = threadIdx.x & 31, gid = lane / W, sub = lane % W;
@@ -985,6 +1012,7 @@ __global__ void __launch_bounds__(kThreads, 6) k_update(i64 count, const int* mo
 template <class C>
 __global__ void k_update_chunks(DGraph g, const int* chunk_list, const u64* chunk_count, const u32* state, int k, C* A,
                                 long long* delta, Sample* samples, const u64* gate, u64 threshold, u64* work) {
+    after_previous();
     if (gate && *gate > threshold) return;
     const i64 count = static_cast<i64>(*chunk_count);
     for (i64 w = blockIdx.x; w < count; w += gridDim.x) {
@@ -1011,6 +1039,7 @@ __global__ void k_update_chunks(DGraph g, const int* chunk_list, const u64* chun
 // Also marks the batch in the packed state (target and batch bit).
 __global__ void k_mark_movers(i64 count, const int* movers, const u64* live_count, const int* off, const int* targets,
                               u32* state, u64* out) {
+    after_previous();
     if (live_count) count = static_cast<i64>(*live_count);
     u64 entries = 0;
     for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += static_cast<i64>(gridDim.x) * blockDim.x) {
@@ -1026,6 +1055,7 @@ __global__ void k_mark_movers(i64 count, const int* movers, const u64* live_coun
 // in the packed state and adds its row's entries to *entries (the rebuild
 // gate), so the batch needs no separate marking launch.
 __global__ void k_compact_movers(LpParams q, u32* state, u64* entries) {
+    after_previous();
     const i64 count = static_cast<i64>(q.counters[0]);
     u64 mine = 0;
     for (i64 base = static_cast<i64>(blockIdx.x) * blockDim.x; base < count; base += static_cast<i64>(gridDim.x) * blockDim.x) {
@@ -1050,6 +1080,7 @@ __global__ void k_compact_movers(LpParams q, u32* state, u64* entries) {
 __global__ void k_commit(i64 count, const int* movers, const u64* live_count, int* labels, const int* targets,
                          const u32* vw, int k, u64* loads, unsigned char* locks, int* flags, u32* state,
                          u64* max_load, unsigned int* blocks_done) {
+    after_previous();
     extern __shared__ long long diff[];
     __shared__ bool last;
     if (live_count) count = static_cast<i64>(*live_count);
@@ -1121,6 +1152,7 @@ __device__ __forceinline__ u64 saturating_add(u64 a, u64 b) { return ~0ULL - a <
 // donors).
 __global__ void __launch_bounds__(kMaxParts) k_slack(int k, const u64* loads, u64 capacity, u64* slack, u64* requests,
                                                      u64* cdf, u64* counts) {
+    after_previous();
     __shared__ u64 warp_total[kMaxParts / 32], warp_min[kMaxParts / 32];
     const int p = threadIdx.x, lane = p & 31, warp = p >> 5;
     const u64 room = p < k ? (loads[p] < capacity ? capacity - loads[p] : 0) : 0;
@@ -1196,6 +1228,7 @@ template <class C, int W, bool Vectorized>
 __global__ void __launch_bounds__(kThreads) k_repair_dest(i64 n, const C* A, const C* totals, const int* labels,
                                                           const u32* vw, int k, const u64* loads, u64 capacity,
                                                           const u64* cdf, u32* plan, u64* hist, u64* donor_count) {
+    after_previous();
     constexpr int N = Vectorized ? AffinityVec<C>::N : 1;
     constexpr int G = 32 / W;
     __shared__ u64 s_room[kMaxParts], s_excess[kMaxParts];
@@ -1318,6 +1351,7 @@ __global__ void __launch_bounds__(kThreads) k_repair_dest_od(i64 n, const int* o
                                                              const int* labels, const u32* vw, int k, const u64* loads,
                                                              u64 capacity, const u64* cdf, u32* plan, u64* hist,
                                                              u64* donor_count) {
+    after_previous();
     __shared__ u64 s_room[kMaxParts], s_excess[kMaxParts];
     for (int p = threadIdx.x; p < k; p += blockDim.x) {
         s_room[p] = loads[p] < capacity ? capacity - loads[p] : 0;
@@ -1409,6 +1443,7 @@ __global__ void __launch_bounds__(kThreads) k_choose_od(i64 count, const u32* ac
                                                         const u32* vw, int k, const u32* plan, const u64* slack,
                                                         const u64* requests, const u64* tried, unsigned char* state,
                                                         int* want, u64* requesters) {
+    after_previous();
     __shared__ u64 s_avail[kMaxParts];
     for (int p = threadIdx.x; p < k; p += blockDim.x) s_avail[p] = requests[p] < slack[p] ? slack[p] - requests[p] : 0;
     __syncthreads();
@@ -1441,6 +1476,7 @@ __global__ void __launch_bounds__(kThreads) k_choose_od(i64 count, const u32* ac
 // zero for the next iteration.
 __global__ void __launch_bounds__(kScanThreads) k_repair_bounds(const u64* loads, u64 capacity, u64* hist, int* bound,
                                                                 u64* start) {
+    after_previous();
     constexpr int kPer = 4;
     static_assert(kScanThreads * kPer >= kBalanceWidth, "one pass over a part's classes");
     __shared__ u64 smem[9];
@@ -1477,6 +1513,7 @@ __global__ void __launch_bounds__(kScanThreads) k_repair_bounds(const u64* loads
 // id, so ordering the words is the repair order (ascending hash, then id).
 __global__ void __launch_bounds__(kThreads) k_repair_list(i64 n, int k, const int* labels, const u32* plan,
                                                           const int* bound, u64* list, u64* count) {
+    after_previous();
     __shared__ int s_bound[kMaxParts];
     for (int p = threadIdx.x; p < k; p += blockDim.x) s_bound[p] = bound[p];
     __syncthreads();
@@ -1494,6 +1531,7 @@ __global__ void __launch_bounds__(kThreads) k_repair_list(i64 n, int k, const in
 // part whose weight their order counts (-1 for the others).
 __global__ void k_repair_unpack(i64 count, const u64* list, const int* labels, const u32* plan, const int* bound,
                                 u32* items, int* want) {
+    after_previous();
     const i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= count) return;
     const int v = static_cast<int>(list[i] & 0xffffffffULL);
@@ -1520,6 +1558,7 @@ __global__ void __launch_bounds__(kThreads) k_choose(i64 count, const u32* activ
                                                      const int* labels, const u32* vw, int k, const u32* plan,
                                                      const u64* slack, const u64* requests, u64* tried,
                                                      unsigned char* state, int* want, u64* requesters) {
+    after_previous();
     constexpr int N = Vectorized ? AffinityVec<C>::N : 1;
     constexpr int G = 32 / W;
     __shared__ u64 s_avail[kMaxParts];
@@ -1598,6 +1637,7 @@ struct WriteIdx {
 constexpr int kAdmitTile = kThreads;
 __global__ void k_part_requests(i64 count, const int* want, const u32* active, const u32* vw, int k, int tiles,
                                 u64* tile_sums) {
+    after_previous();
     __shared__ u64 s_sum[kMaxParts];
     for (int p = threadIdx.x; p < k; p += blockDim.x) s_sum[p] = 0;
     __syncthreads();
@@ -1622,6 +1662,7 @@ __global__ void k_part_requests(i64 count, const int* want, const u32* active, c
 __global__ void k_admit_tiles(i64 count, const int* want, const u32* active, const u32* vw, const u64* offsets,
                               const u64* total, int tiles, const u64* slack, u64* requests, u64* tried,
                               unsigned char* state, int* targets, int* flags, int k, unsigned int* blocks_done) {
+    after_previous();
     __shared__ bool last;
     constexpr int kWarps = kAdmitTile / 32;
     __shared__ u64 s_warp[kMaxParts][kWarps];  // per part, the weight each warp asks (then its start)
@@ -1680,6 +1721,7 @@ __global__ void k_admit_tiles(i64 count, const int* want, const u32* active, con
 __global__ void k_repair_active(i64 count, const int* want, const u32* items, const u32* vw, const u64* offsets,
                                 int tiles, const u64* loads, u64 capacity, const u64* start, int k,
                                 unsigned char* active) {
+    after_previous();
     constexpr int kWarps = kAdmitTile / 32;
     __shared__ u64 s_warp[kMaxParts][kWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -2002,6 +2044,7 @@ __global__ void __launch_bounds__(kAttemptThreads) k_attempts(const u32* open, c
                                                               const u32* vw, int k, const u32* plan,
                                                               const u64* slack, u64* requests, u64* tried,
                                                               unsigned char* state, int* targets, int* flags) {
+    after_previous();
     __shared__ AttemptParts<kAttemptThreads> sm;
     extern __shared__ __align__(16) unsigned char attempt_smem_raw[];
     const int count = static_cast<int>(*count_ptr);
@@ -2090,6 +2133,7 @@ __global__ void __launch_bounds__(kAttemptThreads) k_repair_block(const u64* lis
                                                                   const u32* plan, const int* bound, const u64* start,
                                                                   const u64* loads, u64 capacity, const u64* slack,
                                                                   int* targets, int* flags, int* movers, u64* placed) {
+    after_previous();
     __shared__ AttemptParts<kAttemptThreads> sm;
     __shared__ u32 s_scan[33];
     __shared__ u32 s_placed;
@@ -2234,6 +2278,7 @@ struct JointCounts {
 };
 template <class Cmp>
 __global__ void k_move_keys(int count, const JointMove* moves, MoveKey* keys) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < count) keys[i] = Cmp::key(moves[i]);
 }
@@ -2252,6 +2297,7 @@ __device__ __forceinline__ bool move_before(const MoveKey& kb, const MoveKey& ka
 template <class Cmp>
 __global__ void k_bitonic(int size, int count, const JointMove* moves, const MoveKey* keys, int* idx, int kk, int jj,
                           Cmp cmp) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= size) return;
     const int x = i ^ jj;
@@ -2298,6 +2344,7 @@ constexpr size_t kBitonicEntryBytes = sizeof(MoveKey) + sizeof(int);
 template <class Cmp>
 __global__ void __launch_bounds__(1024) k_bitonic_local(int size, int count, const JointMove* moves, const MoveKey* keys,
                                                        int* idx, int kk_first, int kk_last, int jj_first, Cmp cmp) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char bitonic_smem[];
     MoveKey* s_key = reinterpret_cast<MoveKey*>(bitonic_smem);
     int* s_idx = reinterpret_cast<int*>(s_key + kBitonicSegment);
@@ -2346,6 +2393,7 @@ __device__ __forceinline__ void sort_moves_smem(int size, int count, const Joint
 }
 // The fragments sorted and without duplicates, when one block takes them.
 __global__ void __launch_bounds__(1024) k_sort_fragments(const JointMove* in, JointMove* out, JointCounts* counts) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char bitonic_smem[];
     __shared__ u32 s_scan[33];
     if (counts->fragments > kBitonicSegment) return;
@@ -2367,10 +2415,12 @@ __global__ void __launch_bounds__(1024) k_sort_fragments(const JointMove* in, Jo
     if (threadIdx.x == 0) counts->unique = kept;
 }
 __global__ void k_iota(int n, int* idx) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) idx[i] = i;
 }
 __global__ void k_gather_moves(int count, const int* idx, const JointMove* in, JointMove* out) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < count) out[i] = in[idx[i]];
 }
@@ -2378,6 +2428,7 @@ __global__ void k_gather_moves(int count, const int* idx, const JointMove* in, J
 // joint_quotient (exchange.cuh:41-54).
 template <class C>
 __global__ void k_quotient(i64 n, const int* labels, const C* A, int k, u64* quotient) {
+    after_previous();
     for (i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += static_cast<i64>(gridDim.x) * blockDim.x) {
         const int a = labels[v];
         for (int b = a + 1; b < k; ++b) {
@@ -2396,6 +2447,7 @@ constexpr int kMatchThreads = 1024;
 __global__ void __launch_bounds__(kMatchThreads) k_match_parts(int k, const u64* quotient, int* partner, int* visits,
                                                                u64* seeds, int seed_count, JointCounts* counts,
                                                                u64* movers) {
+    after_previous();
     for (int x = threadIdx.x; x < seed_count; x += blockDim.x) seeds[x] = ~0ULL;
     if (threadIdx.x == 0) {
         *counts = JointCounts{0, 0, 0, 0};
@@ -2457,6 +2509,7 @@ __global__ void __launch_bounds__(kMatchThreads) k_match_parts(int k, const u64*
 template <class C>
 __global__ void k_seeds(i64 n, const int* labels, const C* A, int k, const int* partner, u64* seeds, int sw, int pass,
                         int* owners) {
+    after_previous();
     for (i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += static_cast<i64>(gridDim.x) * blockDim.x) {
         owners[v] = INT_MAX;
         const int p = labels[v], q = partner[p];
@@ -2472,6 +2525,7 @@ template <class C>
 __global__ void k_grow(int slots, int sw, const u64* seeds, const int* partner, const int* off, const int* nbr,
                        const u32* ew, const u32* masses, const int* labels, const C* A, int k, const u64* loads,
                        u64 capacity, JointMove* moves, JointMove* fragments, JointCounts* joint) {
+    after_previous();
     const int lane = threadIdx.x & 31;
     const int slot = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (slot >= slots) return;
@@ -2582,6 +2636,7 @@ struct UniqueHead {
 // distinct sorted ones; appends to the moves.
 __global__ void k_combine(JointCounts* counts, const JointMove* archive, const int* off, const int* nbr, const u32* ew,
                           const int* labels, const u64* loads, u64 capacity, int id_base, JointMove* out) {
+    after_previous();
     const int lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5);
     const int count = static_cast<int>(counts->unique);
     if (i >= count) return;
@@ -2690,17 +2745,20 @@ __global__ void k_combine(JointCounts* counts, const JointMove* archive, const i
     }
 }
 __global__ void k_claim(int count, const JointMove* moves, int* owners) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < count && moves[i].size)
         for (int j = 0; j < moves[i].size; ++j) atomicMin(owners + moves[i].vertices[j], i);
 }
 __global__ void k_resolve(int count, JointMove* moves, const int* owners) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     for (int j = 0; j < moves[i].size; ++j)
         if (owners[moves[i].vertices[j]] != i) { moves[i].size = 0; break; }
 }
 __global__ void k_mark(int count, const JointMove* moves, const int* labels, int* owners, int* targets) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < count)
         for (int j = 0; j < moves[i].size; ++j) {
@@ -2732,6 +2790,7 @@ struct EventChunks {
 __global__ void __launch_bounds__(1024) k_rank_moves(const JointMove* in, JointMove* out, JointCounts* counts,
                                                      const int* off, const int* labels, int* owners, int* targets,
                                                      u64* events, u32* chunk_off, u32* total_chunks) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char bitonic_smem[];
     __shared__ u32 s_scan[33];
     constexpr int kPer = kBitonicSegment / 1024;  // consecutive moves per thread
@@ -2803,6 +2862,7 @@ __global__ void __launch_bounds__(1024) k_rank_moves(const JointMove* in, JointM
 __global__ void k_events(const u32* count_ptr, const JointMove* moves, const u32* chunk_off, const u32* total_chunks,
                          const int* owners, const int* targets, const int* labels, const int* off, const int* nbr,
                          const u32* ew, u64* events) {
+    after_previous();
     const int lane = threadIdx.x & 31;
     const int items = static_cast<int>(*count_ptr) * 8;
     const u32 total = items ? *total_chunks : 0;
@@ -2847,6 +2907,7 @@ constexpr int kPrefixThreads = kScanThreads;
 __global__ void __launch_bounds__(kPrefixThreads) k_prefix(const u32* count_ptr, const JointMove* moves,
                                                            const u64* events, const u64* loads, u64 capacity,
                                                            int* movers, u64* mover_count) {
+    after_previous();
     const int count = static_cast<int>(*count_ptr);
     __shared__ long long s_scan[9];
     __shared__ int s_range[2];

@@ -838,6 +838,7 @@ constexpr size_t cluster_smem() { return repair_block_smem<C>(); }
 
 template <class C>
 __global__ void __launch_bounds__(kClusterThreads, 1) k_refine_cluster(const __grid_constant__ ClusterLevel<C> L) {
+    after_previous();
     __shared__ ClusterShared<C> sm;
     extern __shared__ __align__(16) unsigned char cluster_raw[];
     ClusterRefiner<C>(L, sm, cluster_raw).run();

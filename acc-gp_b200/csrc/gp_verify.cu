@@ -14,6 +14,7 @@ constexpr int kThreads = 256;
 
 // Flags: 1 not bidirectional, 2 reverse weights differ, 4 self loop.
 __global__ void k_verify_csr(i64 n, const int* off, const int* nbr, const u32* ew, bool allow_self_loops, u64* flags) {
+    after_previous();
     const int lane = threadIdx.x & 31;
     u64 bad = 0;
     for (i64 v = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; v < n;
@@ -37,10 +38,12 @@ __global__ void k_verify_csr(i64 n, const int* off, const int* nbr, const u32* e
 // Coarse vertex weights against the fine weights they sum, and the cap.
 // Flags: 8 weight mismatch, 16 above the cap.
 __global__ void k_sum_members(i64 n, const int* map, const u32* vw, u64* sums) {
+    after_previous();
     for (i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += static_cast<i64>(gridDim.x) * blockDim.x)
         atomicAdd(sums + map[v], static_cast<u64>(vw[v]));
 }
 __global__ void k_check_weights(i64 nc, const u64* sums, const u32* cvw, u64 cap, u64* flags) {
+    after_previous();
     u64 bad = 0;
     for (i64 c = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; c < nc; c += static_cast<i64>(gridDim.x) * blockDim.x) {
         if (sums[c] != static_cast<u64>(cvw[c])) bad |= 8;
@@ -57,6 +60,7 @@ __device__ __forceinline__ int probe_label(const int* map, int v) {
     return static_cast<int>((x * 2654435761ULL + 17) % 23);
 }
 __global__ void k_probe_cut(i64 n, const int* off, const int* nbr, const u32* ew, const int* map, u64* out) {
+    after_previous();
     const int lane = threadIdx.x & 31;
     u64 cut = 0;
     for (i64 v = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; v < n;
