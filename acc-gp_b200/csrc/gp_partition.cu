@@ -124,6 +124,14 @@ __global__ void k_fill_ones(i64 n, u32* p) {
         p[i] = 1u;
 }
 
+__global__ void k_publish(const u64* from, u64* to, int words, u64* flag, u64 sequence) {
+    after_previous();
+    for (int i = threadIdx.x; i < words; i += blockDim.x) to[i] = from[i];
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) *static_cast<volatile u64*>(flag) = sequence;
+}
+
 // Shape and range checks of a device CSR (validate_weighted_shape,
 // src/graph.cpp:118-155), as two flat grid-stride sweeps so that long rows
 // do not serialise.  Scalars: 0 bad offsets, 1 bad neighbour, 2 zero vertex
@@ -271,6 +279,10 @@ Input prepare_input(Context& ctx, const gp_csr* in, bool device_input) {
 }
 
 }  // namespace
+
+void publish(cudaStream_t stream, const u64* from, u64* to, int words, u64* flag, u64 sequence) {
+    launch(k_publish, 1, 128, 0, stream, from, to, words, flag, sequence);
+}
 
 // Kept hierarchies of resident graphs (see gp_internal.h).  An entry owns the
 // arena its levels live in; entries in use by a call are never dropped.
@@ -631,7 +643,8 @@ gp_status gp_context_create(int device, gp_context** out) {
         try {
             GP_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
             GP_CUDA(cudaMalloc(&c.dev_scalars, sizeof(u64) * kScalars));
-            GP_CUDA(cudaMallocHost(&c.host_scalars, sizeof(u64) * kScalars));
+            GP_CUDA(cudaMallocHost(&c.host_scalars, sizeof(u64) * (kScalars + 1)));
+            c.host_scalars[kScalars] = 0;
             for (auto& e : c.ev) GP_CUDA(cudaEventCreate(&e));
         } catch (...) {
             delete h;

@@ -2988,7 +2988,7 @@ namespace {
 constexpr i64 kClusterVertices = 65536, kClusterCells = 1 << 19, kClusterEntries = 1 << 18, kClusterRow = 16;
 
 struct LevelResult {
-    u64 cut = 0;
+    u64 cut = 0, max_load = 0;
     bool refined = false, repair_failed = false;
 };
 
@@ -3000,7 +3000,7 @@ public:
         : ctx(c), g(g), k(k), eps(eps), labels(labels), loads(loads), total(total), log(log), verify(verify),
           mapping(mapping), budget(budget) {}
 
-    LevelResult run(bool has_known, u64 known);
+    LevelResult run(bool has_known, u64 known, u64 known_load);
     LevelStats stats;
 
 private:
@@ -3281,8 +3281,7 @@ void LevelRefiner<T>::enqueue_lp_round(double filter) {
 template <class T>
 i64 LevelRefiner<T>::lp_round(double filter) {
     enqueue_lp_round(filter);
-    GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters, 8 * sizeof(u64), cudaMemcpyDeviceToHost, s()));
-    GP_CUDA(cudaStreamSynchronize(s()));
+    ctx.fetch(counters, 8);
     const i64 count = static_cast<i64>(ctx.host_scalars[1]);
     const long long delta = settled_delta(ctx.host_scalars + 2);
     max_load_host = ctx.host_scalars[3];
@@ -3309,8 +3308,7 @@ bool LevelRefiner<T>::repair(i64 interrupted, int iterations) {
     // counters[9]: placed donors, [10]: donors, [11]: listed donors.
     u64 *placed_count = counters + 9, *donor_count = counters + 10, *list_count = counters + 11;
     auto read_batch = [&]() {
-        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 2, 10 * sizeof(u64), cudaMemcpyDeviceToHost, s()));
-        GP_CUDA(cudaStreamSynchronize(s()));
+        ctx.fetch(counters + 2, 10);
     };
     while (true) {
         ArenaScope it(A_);
@@ -3437,8 +3435,7 @@ void LevelRefiner<T>::reserve_long(i64 listed, u64* list, const u32* plan, const
                tiles, static_cast<const u64*>(loads), C, start, k, active_flag);
         // Active donors, in repair order.
         select_if(A_, s(), listed, IsActive{active_flag}, WriteFrom{items, active}, donor_count);
-        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 4, sizeof(u64), cudaMemcpyDeviceToHost, s()));
-        GP_CUDA(cudaStreamSynchronize(s()));
+        ctx.fetch(counters + 4, 1);
         acount = static_cast<i64>(ctx.host_scalars[0] & 0xffffffffULL);
     }
     if (acount == 0) return;
@@ -3497,8 +3494,7 @@ void LevelRefiner<T>::reserve_long(i64 listed, u64* list, const u32* plan, const
                static_cast<const u32*>(active), static_cast<const u32*>(g.vw),
                static_cast<const u64*>(tile_offsets), static_cast<const u64*>(tile_total), tiles, slack, requests,
                tried, state, targets, flags, k, reinterpret_cast<unsigned int*>(counters + 8));
-        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 5, sizeof(u64), cudaMemcpyDeviceToHost, s()));
-        GP_CUDA(cudaStreamSynchronize(s()));
+        ctx.fetch(counters + 5, 1);
         const i64 rcount = static_cast<i64>(ctx.host_scalars[0]);
         if (!rcount) break;
         // At most rcount donors remain open.
@@ -3577,8 +3573,8 @@ void LevelRefiner<T>::refine_in_cluster(double filter, LevelResult& res, int& ro
             *staged = st;
             GP_CUDA(cudaMemcpyAsync(L.io, staged, sizeof(ClusterState), cudaMemcpyHostToDevice, s()));
             launch_cluster(k_refine_cluster<T>, kClusterBlocks, kClusterThreads, smem, s(), L);
-            GP_CUDA(cudaMemcpyAsync(staged, L.io, sizeof(ClusterState), cudaMemcpyDeviceToHost, s()));
-            GP_CUDA(cudaStreamSynchronize(s()));
+            static_assert(sizeof(ClusterState) % sizeof(u64) == 0, "fetched by words");
+            ctx.fetch(reinterpret_cast<const u64*>(L.io), sizeof(ClusterState) / sizeof(u64));
             st = *staged;
             max_load_host = st.max_load;
             cut = st.loop.cut;
@@ -3632,8 +3628,7 @@ void LevelRefiner<T>::restore_best(bool moved) {
         launch(k_state_init, grid_for(n, kThreads), kThreads, 0, s(), n, static_cast<const int*>(labels), state);
     GP_CUDA(cudaMemcpyAsync(loads, saved_loads, sizeof(u64) * k, cudaMemcpyDeviceToDevice, s()));
     launch(k_max_load, 1, 32, 0, s(), k, loads, counters + 3);
-    GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 3, sizeof(u64), cudaMemcpyDeviceToHost, s()));
-    GP_CUDA(cudaStreamSynchronize(s()));
+    ctx.fetch(counters + 3, 1);
     max_load_host = ctx.host_scalars[0];
 }
 
@@ -3660,16 +3655,16 @@ void LevelRefiner<T>::exchange(u64& best_cut) {
     u64* events = A_.alloc<u64>(move_cap);
     u32* chunk_off = A_.alloc<u32>(move_cap * 8);
     u32* total_chunks = A_.alloc<u32>(1);
-    JointCounts* counts = A_.alloc<JointCounts>(1);
+    // Behind the batch's counters, so that one fetch brings both.
+    constexpr int kJointWords = sizeof(JointCounts) / sizeof(u64);
+    JointCounts* counts = reinterpret_cast<JointCounts*>(counters + 10);
     u64* mover_count = counters + 9;
     GP_CUDA(cudaMemsetAsync(quotient, 0, sizeof(u64) * k * k, s()));
     GP_CUDA(cudaMemsetAsync(visits, 0, sizeof(int) * k * k, s()));
     launch(k_quotient<T>, grid_for(n, kThreads), kThreads, 0, s(), n, labels, static_cast<const T*>(A), k, quotient);
     auto read_counts = [&]() {
-        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars + 16, counts, sizeof(JointCounts), cudaMemcpyDeviceToHost, s()));
-        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 2, 8 * sizeof(u64), cudaMemcpyDeviceToHost, s()));
-        GP_CUDA(cudaStreamSynchronize(s()));
-        return *reinterpret_cast<const JointCounts*>(ctx.host_scalars + 16);
+        ctx.fetch(counters + 2, 8 + kJointWords);
+        return *reinterpret_cast<const JointCounts*>(ctx.host_scalars + 8);
     };
     // (Shared-memory limits are set to one value for every size, on every
     // call: the limit belongs to the kernel for the whole process, on
@@ -3807,8 +3802,7 @@ u64 LevelRefiner<T>::propagate(double filter, int& rounds, bool& restored) {
         else
             launch(k_frontier_init<T>, grid_for(n, kThreads), kThreads, 0, s(), n, static_cast<const T*>(A),
                    static_cast<const T*>(totals), k, static_cast<const int*>(labels), targets, frontier);
-        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, frontier.count, sizeof(u64), cudaMemcpyDeviceToHost, s()));
-        GP_CUDA(cudaStreamSynchronize(s()));
+        ctx.fetch(frontier.count, 1);
         frontier_on = ctx.host_scalars[0] <= static_cast<u64>(n) / 4;
     }
     u64 best = cut;
@@ -3841,7 +3835,7 @@ u64 LevelRefiner<T>::propagate(double filter, int& rounds, bool& restored) {
 
 // run_incremental_refinement_typed (incremental.cuh:660-1051).
 template <class T>
-LevelResult LevelRefiner<T>::run(bool has_known, u64 known) {
+LevelResult LevelRefiner<T>::run(bool has_known, u64 known, u64 known_load) {
     Arena& A_ = ctx.scratch;
     ArenaScope scope(A_);
     n = g.n;
@@ -3888,9 +3882,10 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known) {
     movers = A_.alloc<int>(n);
     // [8]: k_commit's finished-block count, zero between launches; [9]: the
     // movers of a repair or exchange (a 32-bit count in a zeroed word); [10],
-    // [11]: the repair's donors and listed donors.
-    counters = A_.alloc<u64>(12);
-    GP_CUDA(cudaMemsetAsync(counters + 8, 0, 4 * sizeof(u64), s()));
+    // [11]: the repair's donors and listed donors; [10] to [12]: the exchange's
+    // JointCounts.
+    counters = A_.alloc<u64>(13);
+    GP_CUDA(cudaMemsetAsync(counters + 8, 0, 5 * sizeof(u64), s()));
     corr_acc = A_.alloc<long long>(g.heavy_count + 1);
     if (g.chunks) {
         chunk_work = A_.alloc<int>(g.chunks);
@@ -3927,19 +3922,15 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known) {
         launch(k_state_init, grid_for(n, kThreads), kThreads, 0, s(), n, static_cast<const int*>(labels), state);
     }
     build(has_known ? nullptr : counters + 7);
-    if (!in_cluster || !has_known) {  // the cluster kernel reads the loads itself
-        launch(k_max_load, 1, 32, 0, s(), k, loads, counters + 3);
-        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, counters + 3, 5 * sizeof(u64), cudaMemcpyDeviceToHost, s()));
-        GP_CUDA(cudaStreamSynchronize(s()));
-        max_load_host = ctx.host_scalars[0];
-    }
+    max_load_host = known_load;
+    if (!has_known && !on_demand) ctx.fetch(counters + 7, 1);
     if (has_known) {
         cut = known;
     } else if (on_demand) {
         cut = device_cut(ctx, g, labels);
     } else {
-        if (ctx.host_scalars[4] & 1ULL) fail(GP_INTERNAL, "refinement cut is not symmetric");
-        cut = ctx.host_scalars[4] / 2;
+        if (ctx.host_scalars[0] & 1ULL) fail(GP_INTERNAL, "refinement cut is not symmetric");
+        cut = ctx.host_scalars[0] / 2;
     }
     LevelResult res;
     stats.initial_cut = cut;
@@ -3955,6 +3946,7 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known) {
     else if (max_load_host > C) res.repair_failed = !repair();
     if (res.repair_failed) {
         res.cut = cut;
+        res.max_load = max_load_host;
         stats.repair_failed = true;
         stats.final_cut = cut;
         stats.final_max_load = max_load_host;
@@ -3981,6 +3973,7 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known) {
     stats.final_cut = cut;
     stats.final_max_load = max_load_host;
     res.cut = cut;
+    res.max_load = max_load_host;
     res.refined = true;
     return res;
 }
@@ -4011,16 +4004,15 @@ RefineOutcome uncoarsen(Context& ctx, Hierarchy& h, const std::vector<int>& coar
     GP_CUDA(cudaMemsetAsync(loads, 0, sizeof(u64) * k, s));
     launch(k_loads, std::min(blocks_for(coarsest.n, 256), 148 * 4), 256, sizeof(u64) * k, s, coarsest.n, k,
            level_labels[L - 1], coarsest.vw, loads);
-    GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, loads, sizeof(u64) * k, cudaMemcpyDeviceToHost, s));
-    GP_CUDA(cudaStreamSynchronize(s));
+    ctx.fetch(loads, k);
     u64 total = 0, maxload = 0;
     for (int p = 0; p < k; ++p) { total += ctx.host_scalars[p]; maxload = std::max<u64>(maxload, ctx.host_scalars[p]); }
-    auto refine = [&](const DGraph& g, int* lab, bool has_known, u64 known) {
+    auto refine = [&](const DGraph& g, int* lab, bool has_known, u64 known, u64 known_load) {
         const auto t_begin = std::chrono::steady_clock::now();
         const LevelResult r =
             g.incident_bound <= 0xffffffffULL
-                ? LevelRefiner<u32>(ctx, g, k, eps, lab, loads, total, log, verify, mapping).run(has_known, known)
-                : LevelRefiner<u64>(ctx, g, k, eps, lab, loads, total, log, verify, mapping).run(has_known, known);
+                ? LevelRefiner<u32>(ctx, g, k, eps, lab, loads, total, log, verify, mapping).run(has_known, known, known_load)
+                : LevelRefiner<u64>(ctx, g, k, eps, lab, loads, total, log, verify, mapping).run(has_known, known, known_load);
         if (log) {  // host time of the level; the stream is drained first
             GP_CUDA(cudaStreamSynchronize(s));
             std::printf("refine_level_time vertices=%lld ms=%.3f\n", static_cast<long long>(g.n),
@@ -4028,7 +4020,8 @@ RefineOutcome uncoarsen(Context& ctx, Hierarchy& h, const std::vector<int>& coar
         }
         return r;
     };
-    LevelResult res = refine(coarsest, level_labels[L - 1], false, 0);
+    LevelResult res = refine(coarsest, level_labels[L - 1], false, 0, maxload);
+    maxload = res.max_load;
     u64 last_cut = res.cut;
     i64 last_refined = coarsest.n;
     RefineOutcome out;
@@ -4054,14 +4047,11 @@ RefineOutcome uncoarsen(Context& ctx, Hierarchy& h, const std::vector<int>& coar
             if (fine_cut != coarse_cut || fine_cut != last_cut || a != b)
                 fail(GP_INTERNAL, "GPU projection failed cut or part-weight preservation");
         }
-        GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, loads, sizeof(u64) * k, cudaMemcpyDeviceToHost, s));
-        GP_CUDA(cudaStreamSynchronize(s));
-        maxload = 0;
-        for (int p = 0; p < k; ++p) maxload = std::max<u64>(maxload, ctx.host_scalars[p]);
         const bool refine_here = f == 0 || maxload > cap || static_cast<double>(fg.n) >= 2.0 * static_cast<double>(last_refined);
         LevelResult lr;
         if (refine_here) {
-            lr = refine(fg, level_labels[f], true, last_cut);
+            lr = refine(fg, level_labels[f], true, last_cut, maxload);
+            maxload = lr.max_load;
             if (!lr.repair_failed) last_refined = fg.n;
             out.levels_refined += lr.refined;
         } else {
@@ -4069,10 +4059,6 @@ RefineOutcome uncoarsen(Context& ctx, Hierarchy& h, const std::vector<int>& coar
         }
         last_cut = lr.cut;
     }
-    GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, loads, sizeof(u64) * k, cudaMemcpyDeviceToHost, s));
-    GP_CUDA(cudaStreamSynchronize(s));
-    maxload = 0;
-    for (int p = 0; p < k; ++p) maxload = std::max<u64>(maxload, ctx.host_scalars[p]);
     if (maxload > cap) fail(GP_INTERNAL, "final original partition violates capacity");
     if (verify && device_cut(ctx, h.levels[0], labels) != last_cut) fail(GP_INTERNAL, "final cut differs from CSR scan");
     out.cut = last_cut;
@@ -4089,17 +4075,19 @@ LevelStats refine_single(Context& ctx, const DGraph& g, int* labels, int k, doub
     GP_CUDA(cudaMemsetAsync(loads, 0, sizeof(u64) * k, s));
     launch(k_loads, std::min(blocks_for(g.n, 256), 148 * 4), 256, sizeof(u64) * k, s, g.n, k,
            static_cast<const int*>(labels), g.vw, loads);
-    GP_CUDA(cudaMemcpyAsync(ctx.host_scalars, loads, sizeof(u64) * k, cudaMemcpyDeviceToHost, s));
-    GP_CUDA(cudaStreamSynchronize(s));
-    u64 total = 0;
-    for (int p = 0; p < k; ++p) total += ctx.host_scalars[p];
+    ctx.fetch(loads, k);
+    u64 total = 0, maxload = 0;
+    for (int p = 0; p < k; ++p) {
+        total += ctx.host_scalars[p];
+        maxload = std::max<u64>(maxload, ctx.host_scalars[p]);
+    }
     if (g.incident_bound <= 0xffffffffULL) {
         LevelRefiner<u32> r(ctx, g, k, eps, labels, loads, total, log, verify, mapping, budget);
-        r.run(false, 0);
+        r.run(false, 0, maxload);
         return r.stats;
     }
     LevelRefiner<u64> r(ctx, g, k, eps, labels, loads, total, log, verify, mapping, budget);
-    r.run(false, 0);
+    r.run(false, 0, maxload);
     return r.stats;
 }
 
