@@ -2267,162 +2267,148 @@ struct MoveOrder {  // JointOrder (exchange.cuh:29-36)
         return r;
     }
 };
-// Device counts of one exchange pass.  k_match_parts clears them; the lists
+// Device counts of one exchange pass, cleared by k_match_parts.  The lists
 // grow by atomic appends (their order does not matter: the sorts' comparators
-// end with the move's unique id).
+// end with the move's unique id) and are sorted a block per part, as both
+// orders begin with the part a.
 struct JointCounts {
-    u64 fragments;  // appended by k_grow
-    u64 moves;      // appended by k_grow and k_combine
-    u32 unique;     // distinct fragments
-    u32 active;     // ordered moves; 0 when a list is longer than one block sorts
+    u64 fragments, moves;  // appended by k_grow; by k_grow and k_combine
+    u64 work;              // row chunks of the settled moves
 };
-template <class Cmp>
-__global__ void k_move_keys(int count, const JointMove* moves, MoveKey* keys) {
-    after_previous();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count) keys[i] = Cmp::key(moves[i]);
+// Only a part and its partner seed moves of a part, two policies a seed: what
+// a part's lists can hold, and so what a block has to sort.
+constexpr int kPartFragments = 2 * kJointSeeds * 2 * kJointArchive;
+constexpr int kPartMoves = 2 * kJointSeeds * 2 + 2 * kPartFragments;
+struct JointParts {
+    u32 fragments[kMaxParts], unique[kMaxParts], moves[kMaxParts];
+};
+// offset[p]: entries of the parts before p, offset[k]: of all.  Every thread
+// of the block.
+__device__ __forceinline__ void part_offsets(int k, const u32* counts, int* offset) {
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int carry = 0;
+        for (int base = 0; base < k; base += 32) {
+            const int c = base + lane < k ? static_cast<int>(counts[base + lane]) : 0;
+            int inc = c;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int o = __shfl_up_sync(0xffffffffu, inc, d);
+                if (lane >= d) inc += o;
+            }
+            if (base + lane < k) offset[base + lane] = carry + inc - c;
+            carry += __shfl_sync(0xffffffffu, inc, 31);
+        }
+        if (lane == 0) offset[k] = carry;
+    }
+    __syncthreads();
 }
-// Whether move b sorts before move a (both real entries).
-template <class Cmp>
-__device__ __forceinline__ bool move_before(const MoveKey& kb, const MoveKey& ka, const JointMove* moves, int b, int a,
-                                            Cmp cmp) {
-    if (kb.k1 != ka.k1) return kb.k1 < ka.k1;
-    if (kb.k2 != ka.k2) return kb.k2 < ka.k2;
-    if (kb.k3 != ka.k3) return kb.k3 < ka.k3;
-    if (kb.k4 != ka.k4) return kb.k4 < ka.k4;
-    return cmp(moves[b], moves[a]);
-}
-
-// One bitonic stage over an index permutation padded to a power of two.
-template <class Cmp>
-__global__ void k_bitonic(int size, int count, const JointMove* moves, const MoveKey* keys, int* idx, int kk, int jj,
-                          Cmp cmp) {
-    after_previous();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= size) return;
-    const int x = i ^ jj;
-    if (x <= i) return;
-    const int a = idx[i], b = idx[x];
-    // Padding (index >= count) sorts after every real entry.
-    bool greater;
-    if (a >= count) greater = b < count;
-    else if (b >= count) greater = false;
-    else greater = move_before(keys[b], keys[a], moves, b, a, cmp);
-    const bool up = (i & kk) == 0;
-    if (greater == up) { idx[i] = b; idx[x] = a; }
-}
-// One compare-exchange step (partner distance jj, direction block kk) over
-// the shared-memory segment that starts at permutation position `base`.
-template <class Cmp>
-__device__ __forceinline__ void bitonic_step_smem(int seg, int base, int count, int kk, int jj, const JointMove* moves,
-                                                  MoveKey* s_key, int* s_idx, Cmp cmp) {
-    for (int p = threadIdx.x; p < seg / 2; p += blockDim.x) {
-        const int i = (p / jj) * 2 * jj + p % jj;
-        const int x = i + jj;
-        const int a = s_idx[i], b = s_idx[x];
-        bool greater;
-        if (a >= count) greater = b < count;
-        else if (b >= count) greater = false;
-        else greater = move_before(s_key[x], s_key[i], moves, b, a, cmp);
-        const bool up = ((base + i) & kk) == 0;
-        if (greater == up) {
-            s_idx[i] = b;
-            s_idx[x] = a;
-            const MoveKey t = s_key[i];
-            s_key[i] = s_key[x];
-            s_key[x] = t;
+// Shared memory of a part's sort: the first Words key words of each entry, the
+// permutation (a power of two of places) and each entry's place in the list.
+template <int Words, int Capacity>
+struct PartSort {
+    static constexpr int places() {
+        int p = 1;
+        while (p < Capacity) p <<= 1;
+        return p;
+    }
+    u64 key[Words][Capacity];
+    int idx[places()];
+    int item[Capacity];
+    u32 count;
+};
+// The entries of part p gathered from a list and sorted by a bitonic network
+// over the permutation (sm.idx); their number.  A comparison reads key words,
+// and the moves themselves only when all words are equal.  The keys stay in
+// place, so an exchange writes two indices.
+constexpr int kPartSortThreads = 512;
+template <int Words, int Capacity, class Cmp>
+__device__ __forceinline__ int sort_part(PartSort<Words, Capacity>& sm, int p, int total, const JointMove* list,
+                                         const unsigned char* list_part, Cmp cmp) {
+    if (threadIdx.x == 0) sm.count = 0;
+    __syncthreads();
+    // Four parts to a load (the lists are padded to whole words), four loads
+    // in flight.
+    const u32* words = reinterpret_cast<const u32*>(list_part);
+    for (int i0 = threadIdx.x; 4 * i0 < total; i0 += 4 * kPartSortThreads) {
+        u32 w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = 4 * (i0 + j * kPartSortThreads) < total ? words[i0 + j * kPartSortThreads] : 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int i = 4 * (i0 + j * kPartSortThreads) + b;
+                if (i < total && static_cast<int>((w[j] >> (8 * b)) & 0xffu) == p) sm.item[atomicAdd(&sm.count, 1u)] = i;
+            }
+    }
+    __syncthreads();
+    const int count = static_cast<int>(sm.count);
+    int size = 1;
+    while (size < count) size <<= 1;
+    for (int i = threadIdx.x; i < size; i += kPartSortThreads) {
+        sm.idx[i] = i;
+        if (i < count) {
+            const MoveKey key = Cmp::key(list[sm.item[i]]);
+            const u64 word[4] = {key.k1, key.k2, key.k3, key.k4};
+#pragma unroll
+            for (int w = 0; w < Words; ++w) sm.key[w][i] = word[w];
         }
     }
     __syncthreads();
-}
-// Bitonic stages on segments of kBitonicSegment indices held in shared
-// memory with their keys: for kk from kk_first to kk_last, every jj below the
-// segment size (the first kk starts at jj_first).  Same compare-exchange as
-// k_bitonic.
-constexpr int kBitonicSegment = 4096;
-constexpr size_t kBitonicEntryBytes = sizeof(MoveKey) + sizeof(int);
-template <class Cmp>
-__global__ void __launch_bounds__(1024) k_bitonic_local(int size, int count, const JointMove* moves, const MoveKey* keys,
-                                                       int* idx, int kk_first, int kk_last, int jj_first, Cmp cmp) {
-    after_previous();
-    extern __shared__ __align__(16) unsigned char bitonic_smem[];
-    MoveKey* s_key = reinterpret_cast<MoveKey*>(bitonic_smem);
-    int* s_idx = reinterpret_cast<int*>(s_key + kBitonicSegment);
-    const int base = blockIdx.x * kBitonicSegment;
-    const int seg = min(kBitonicSegment, size - base);
-    for (int i = threadIdx.x; i < seg; i += blockDim.x) {
-        const int a = idx[base + i];
-        s_idx[i] = a;
-        if (a < count) s_key[i] = keys[a];
-    }
-    __syncthreads();
-    for (int kk = kk_first; kk <= kk_last; kk <<= 1)
-        for (int jj = kk == kk_first ? jj_first : kk >> 1; jj; jj >>= 1)
-            bitonic_step_smem(seg, base, count, kk, jj, moves, s_key, s_idx, cmp);
-    for (int i = threadIdx.x; i < seg; i += blockDim.x) idx[base + i] = s_idx[i];
-}
-// A whole sort of up to kBitonicSegment moves in one block: the full network
-// over indices in shared memory (the same compare-exchange steps as
-// k_bitonic_local over one segment).  The keys stay in place, indexed by move,
-// so an exchange writes two indices and no keys.  Leaves the order in s_idx.
-template <class Cmp>
-__device__ __forceinline__ void sort_moves_smem(int size, int count, const JointMove* in, MoveKey* s_key, int* s_idx,
-                                                Cmp cmp) {
-    for (int i = threadIdx.x; i < size; i += blockDim.x) {
-        s_idx[i] = i;
-        if (i < count) s_key[i] = Cmp::key(in[i]);
-    }
-    __syncthreads();
+    auto before = [&](int b, int a) {
+#pragma unroll
+        for (int w = 0; w < Words; ++w) {
+            const u64 kb = sm.key[w][b], ka = sm.key[w][a];
+            if (kb != ka) return kb < ka;
+        }
+        return static_cast<bool>(cmp(list[sm.item[b]], list[sm.item[a]]));
+    };
     for (int kk = 2; kk <= size; kk <<= 1)
         for (int jj = kk >> 1; jj; jj >>= 1) {
-            for (int p = threadIdx.x; p < size / 2; p += blockDim.x) {
-                const int i = 2 * p - (p & (jj - 1));
+            for (int q = threadIdx.x; q < size / 2; q += kPartSortThreads) {
+                const int i = 2 * q - (q & (jj - 1));
                 const int x = i + jj;
-                const int a = s_idx[i], b = s_idx[x];
-                bool greater;
+                const int a = sm.idx[i], b = sm.idx[x];
+                bool greater;  // padding sorts after every entry
                 if (a >= count) greater = b < count;
                 else if (b >= count) greater = false;
-                else greater = move_before(s_key[b], s_key[a], in, b, a, cmp);
+                else greater = before(b, a);
                 if (greater == ((i & kk) == 0)) {
-                    s_idx[i] = b;
-                    s_idx[x] = a;
+                    sm.idx[i] = b;
+                    sm.idx[x] = a;
                 }
             }
             __syncthreads();
         }
+    return count;
 }
-// The fragments sorted and without duplicates, when one block takes them.
-__global__ void __launch_bounds__(1024) k_sort_fragments(const JointMove* in, JointMove* out, JointCounts* counts) {
-    after_previous();
-    extern __shared__ __align__(16) unsigned char bitonic_smem[];
+using FragmentSort = PartSort<4, kPartFragments>;
+using MoveSort = PartSort<2, kPartMoves>;  // MoveOrder's other words are zero
+// A part's fragments sorted and without duplicates, behind those of the parts
+// before it (by their counts with duplicates).  (One block for all parts took
+// 100 us for 4096 fragments; the parts in parallel sort a few hundred each.)
+__global__ void __launch_bounds__(kPartSortThreads) k_sort_fragments(int k, const JointMove* in,
+                                                                    const unsigned char* in_part, JointMove* out,
+                                                                    JointParts* parts) {
+    extern __shared__ __align__(16) unsigned char part_smem[];
+    __shared__ int s_offset[kMaxParts + 1];
     __shared__ u32 s_scan[33];
-    if (counts->fragments > kBitonicSegment) return;
-    const int count = static_cast<int>(counts->fragments);
-    int size = 1;
-    while (size < count) size <<= 1;
-    MoveKey* s_key = reinterpret_cast<MoveKey*>(bitonic_smem);
-    int* s_idx = reinterpret_cast<int*>(s_key + size);
-    sort_moves_smem(size, count, in, s_key, s_idx, NetOrder{});
+    FragmentSort& sm = *reinterpret_cast<FragmentSort*>(part_smem);
+    const int p = blockIdx.x;
+    part_offsets(k, parts->fragments, s_offset);
+    if (!parts->fragments[p]) return;
+    const int count = sort_part(sm, p, s_offset[k], in, in_part, NetOrder{});
     u32 kept = 0;
-    for (int base = 0; base < count; base += blockDim.x) {
+    for (int base = 0; base < count; base += kPartSortThreads) {
         const int i = base + static_cast<int>(threadIdx.x);
-        const bool head = i < count && (i == 0 || !joint_same(in[s_idx[i - 1]], in[s_idx[i]]));
+        const bool head = i < count && (i == 0 || !joint_same(in[sm.item[sm.idx[i - 1]]], in[sm.item[sm.idx[i]]]));
         u32 total;
         const u32 slot = kept + block_exclusive_scan_wide<u32>(head ? 1u : 0u, total, s_scan);
-        if (head) out[slot] = in[s_idx[i]];
+        if (head) out[s_offset[p] + slot] = in[sm.item[sm.idx[i]]];
         kept += total;
     }
-    if (threadIdx.x == 0) counts->unique = kept;
-}
-__global__ void k_iota(int n, int* idx) {
-    after_previous();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) idx[i] = i;
-}
-__global__ void k_gather_moves(int count, const int* idx, const JointMove* in, JointMove* out) {
-    after_previous();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count) out[i] = in[idx[i]];
+    if (threadIdx.x == 0) parts->unique[p] = kept;
 }
 
 // joint_quotient (exchange.cuh:41-54).
@@ -2446,11 +2432,12 @@ constexpr int kMatchThreads = 1024;
 // Also clears the pass's seeds and counts.
 __global__ void __launch_bounds__(kMatchThreads) k_match_parts(int k, const u64* quotient, int* partner, int* visits,
                                                                u64* seeds, int seed_count, JointCounts* counts,
-                                                               u64* movers) {
+                                                               JointParts* parts, u64* movers) {
     after_previous();
     for (int x = threadIdx.x; x < seed_count; x += blockDim.x) seeds[x] = ~0ULL;
+    for (int x = threadIdx.x; x < kMaxParts; x += blockDim.x) parts->fragments[x] = parts->unique[x] = parts->moves[x] = 0;
     if (threadIdx.x == 0) {
-        *counts = JointCounts{0, 0, 0, 0};
+        *counts = JointCounts{0, 0, 0};
         *movers = 0;
     }
     extern __shared__ double s_score[];  // k * k, pair (a, b) with a < b at a * k + b; -1 = no edge
@@ -2505,13 +2492,13 @@ __global__ void __launch_bounds__(kMatchThreads) k_match_parts(int k, const u64*
     }
     for (int p = threadIdx.x; p < k; p += blockDim.x) partner[p] = s_partner[p];
 }
-// joint_seeds (exchange.cuh:83-93).  Also frees every vertex of an owner.
+// joint_seeds (exchange.cuh:83-93).  Also frees every vertex of claims and owner.
 template <class C>
 __global__ void k_seeds(i64 n, const int* labels, const C* A, int k, const int* partner, u64* seeds, int sw, int pass,
-                        int* owners) {
+                        int* claims, int* owners) {
     after_previous();
     for (i64 v = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += static_cast<i64>(gridDim.x) * blockDim.x) {
-        owners[v] = INT_MAX;
+        claims[v] = owners[v] = INT_MAX;
         const int p = labels[v], q = partner[p];
         if (q < 0 || !A[v * k + q]) continue;
         const u32 h = mix32(static_cast<u32>(v) ^ mix32(static_cast<u32>(pass + 17)));
@@ -2519,12 +2506,21 @@ __global__ void k_seeds(i64 n, const int* labels, const C* A, int k, const int* 
     }
 }
 
+__device__ __forceinline__ void append_move(const JointMove& m, JointMove* moves, unsigned char* move_part,
+                                            JointCounts* counts, JointParts* parts) {
+    const u64 at = atomicAdd(&counts->moves, 1ULL);
+    moves[at] = m;
+    move_part[at] = static_cast<unsigned char>(m.a);
+    atomicAdd(parts->moves + m.a, 1u);
+}
+
 // joint_grow (exchange.cuh:95-204): one warp per (seed, policy) slot.  Its
 // partial moves are appended to the fragments, its best one to the moves.
 template <class C>
 __global__ void k_grow(int slots, int sw, const u64* seeds, const int* partner, const int* off, const int* nbr,
                        const u32* ew, const u32* masses, const int* labels, const C* A, int k, const u64* loads,
-                       u64 capacity, JointMove* moves, JointMove* fragments, JointCounts* joint) {
+                       u64 capacity, JointMove* moves, unsigned char* move_part, JointMove* fragments,
+                       unsigned char* fragment_part, JointCounts* joint, JointParts* parts) {
     after_previous();
     const int lane = threadIdx.x & 31;
     const int slot = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -2553,7 +2549,10 @@ __global__ void k_grow(int slots, int sw, const u64* seeds, const int* partner, 
                 while (pos && st.vertices[pos - 1] > members[j]) { st.vertices[pos] = st.vertices[pos - 1]; --pos; }
                 st.vertices[pos] = members[j];
             }
-            fragments[atomicAdd(&joint->fragments, 1ULL)] = st;
+            const u64 at = atomicAdd(&joint->fragments, 1ULL);
+            fragments[at] = st;
+            fragment_part[at] = static_cast<unsigned char>(st.a);
+            atomicAdd(parts->fragments + st.a, 1u);
         }
         if (gain > best.gain && !joint_gap(net, lo, hi)) {
             best.size = size; best.a = min(source, target); best.b = max(source, target);
@@ -2619,34 +2618,25 @@ __global__ void k_grow(int slots, int sw, const u64* seeds, const int* partner, 
         gain += cgain;
         net += side ? -static_cast<long long>(masses[chosen]) : static_cast<long long>(masses[chosen]);
     }
-    if (!lane && best.size) moves[atomicAdd(&joint->moves, 1ULL)] = best;
+    if (!lane && best.size) append_move(best, moves, move_part, joint, parts);
 }
 
-struct CopyMove {
-    const JointMove* in;
-    JointMove* out;
-    __device__ void operator()(u32 slot, i64 i) const { out[slot] = in[i]; }
-};
-struct UniqueHead {
-    const JointMove* moves;
-    __device__ bool operator()(i64 i) const { return i == 0 || !joint_same(moves[i - 1], moves[i]); }
-};
 
 // joint_combine (complementary_moves.cuh:31-75): one warp per fragment of the
-// distinct sorted ones; appends to the moves.
-__global__ void k_combine(JointCounts* counts, const JointMove* archive, const int* off, const int* nbr, const u32* ew,
-                          const int* labels, const u64* loads, u64 capacity, int id_base, JointMove* out) {
-    after_previous();
-    const int lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5);
-    const int count = static_cast<int>(counts->unique);
-    if (i >= count) return;
+// distinct sorted ones; appends to the moves.  A fragment's partners are of its
+// own part, so it looks for them in its part's run of `archive`.
+__device__ void combine_fragment(int i, int count, int unique_before, int unique_total, const JointMove* archive,
+                                 const int* off, const int* nbr, const u32* ew, const int* labels, const u64* loads,
+                                 u64 capacity, int id_base, JointMove* out, unsigned char* out_part, JointCounts* counts,
+                                 JointParts* parts) {
+    const int lane = threadIdx.x & 31;
     const JointMove x = archive[i];
     const long long lo = static_cast<long long>(loads[x.a]) - static_cast<long long>(capacity);
     const long long hi = static_cast<long long>(capacity) - static_cast<long long>(loads[x.b]);
     if (!lane && !joint_gap(x.net, lo, hi)) {
         JointMove y = x;
-        y.id = id_base + i;
-        out[atomicAdd(&counts->moves, 1ULL)] = y;
+        y.id = id_base + unique_before + i;
+        append_move(y, out, out_part, counts, parts);
     }
     // First position whose move does not come before (x.a, net) (after it,
     // with upper).  The warp probes 32 evenly spaced positions at once, so
@@ -2740,141 +2730,93 @@ __global__ void k_combine(JointCounts* counts, const JointMove* archive, const i
         for (int j = 0; j < y.size; ++j) r.vertices[r.size++] = y.vertices[j];
         r.gain = best_gain;
         r.net += y.net;
-        r.id = id_base + count + i;
-        out[atomicAdd(&counts->moves, 1ULL)] = r;
+        r.id = id_base + unique_total + unique_before + i;
+        append_move(r, out, out_part, counts, parts);
     }
 }
-__global__ void k_claim(int count, const JointMove* moves, int* owners) {
+__global__ void __launch_bounds__(kThreads) k_combine(int k, JointCounts* counts, JointParts* parts,
+                                                      const JointMove* archive, const int* off, const int* nbr,
+                                                      const u32* ew, const int* labels, const u64* loads, u64 capacity,
+                                                      int id_base, JointMove* out, unsigned char* out_part) {
     after_previous();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count && moves[i].size)
-        for (int j = 0; j < moves[i].size; ++j) atomicMin(owners + moves[i].vertices[j], i);
+    __shared__ int s_offset[kMaxParts + 1], s_unique[kMaxParts + 1];
+    part_offsets(k, parts->fragments, s_offset);
+    part_offsets(k, parts->unique, s_unique);
+    const int total = s_unique[k];
+    for (int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < total; g += (gridDim.x * blockDim.x) >> 5) {
+        int lo = 0, hi = k;  // the part of distinct fragment g: the last with s_unique[p] <= g
+        while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s_unique[mid] <= g) lo = mid; else hi = mid; }
+        combine_fragment(g - s_unique[lo], s_unique[lo + 1] - s_unique[lo], s_unique[lo], total, archive + s_offset[lo],
+                         off, nbr, ew, labels, loads, capacity, id_base, out, out_part, counts, parts);
+    }
 }
-__global__ void k_resolve(int count, JointMove* moves, const int* owners) {
-    after_previous();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    for (int j = 0; j < moves[i].size; ++j)
-        if (owners[moves[i].vertices[j]] != i) { moves[i].size = 0; break; }
+// A part's moves sorted, behind those of the parts before it; each claims its
+// vertices for its place in the order.
+__global__ void __launch_bounds__(kPartSortThreads) k_sort_moves(int k, const JointMove* in, const unsigned char* in_part,
+                                                                JointMove* out, const JointParts* parts, int* claims) {
+    extern __shared__ __align__(16) unsigned char part_smem[];
+    __shared__ int s_offset[kMaxParts + 1];
+    MoveSort& sm = *reinterpret_cast<MoveSort*>(part_smem);
+    const int p = blockIdx.x;
+    part_offsets(k, parts->moves, s_offset);
+    if (!parts->moves[p]) return;
+    const int count = sort_part(sm, p, s_offset[k], in, in_part, MoveOrder{});
+    for (int i = threadIdx.x; i < count; i += kPartSortThreads) {
+        const JointMove m = in[sm.item[sm.idx[i]]];
+        out[s_offset[p] + i] = m;
+        for (int j = 0; j < m.size; ++j) atomicMin(claims + m.vertices[j], s_offset[p] + i);
+    }
 }
-__global__ void k_mark(int count, const JointMove* moves, const int* labels, int* owners, int* targets) {
-    after_previous();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count)
-        for (int j = 0; j < moves[i].size; ++j) {
-            const int v = moves[i].vertices[j];
-            owners[v] = i;
-            targets[v] = labels[v] == moves[i].a ? moves[i].b : moves[i].a;
-        }
-}
-// joint_events (exchange.cuh:227-262).  The rows of the moves' vertices
-// are cut into chunks of kEventChunk entries, a warp per chunk, so that a
-// hub among a move's vertices does not leave one warp with the whole row.
-// chunk_off[x] (x = move * 8 + vertex slot) is the exclusive prefix of the
-// chunk counts (EventChunks) and *total_chunks their sum.
+// joint_events (exchange.cuh:227-262) cuts the rows of the moves' vertices into
+// chunks of kEventChunk entries, a warp per chunk, so that a hub among a move's
+// vertices does not leave one warp with the whole row.  A chunk of the work
+// list: move << 32 | vertex slot << 28 | chunk.
 constexpr int kEventChunk = 256;
-struct EventChunks {
-    const JointMove* moves;
-    const int* off;
-    __device__ u32 operator()(i64 x) const {
-        const JointMove& m = moves[x >> 3];
-        const int j = static_cast<int>(x & 7);
-        if (j >= m.size) return 0;
-        const int v = m.vertices[j];
-        return static_cast<u32>((off[v + 1] - off[v] + kEventChunk - 1) / kEventChunk);
-    }
-};
-// The moves sorted, their claims settled (k_claim, k_resolve, k_mark) and the
-// chunks of their rows counted, by one block when neither list of the pass is
-// longer than it sorts; otherwise leaves no active move.
-__global__ void __launch_bounds__(1024) k_rank_moves(const JointMove* in, JointMove* out, JointCounts* counts,
-                                                     const int* off, const int* labels, int* owners, int* targets,
-                                                     u64* events, u32* chunk_off, u32* total_chunks) {
+// A move keeps its vertices only if every claim is its own; then it owns them
+// (k_resolve, k_mark), its events start at 0 and its rows' chunks join the
+// work list.  A block per part.
+__global__ void __launch_bounds__(kThreads) k_settle(int k, JointMove* moves, JointCounts* counts,
+                                                     const JointParts* parts, const int* off, const int* labels,
+                                                     const int* claims, int* owners, int* targets, u64* events,
+                                                     u64* work) {
     after_previous();
-    extern __shared__ __align__(16) unsigned char bitonic_smem[];
-    __shared__ u32 s_scan[33];
-    constexpr int kPer = kBitonicSegment / 1024;  // consecutive moves per thread
-    if (counts->fragments > kBitonicSegment || counts->moves > kBitonicSegment) return;
-    const int count = static_cast<int>(counts->moves);
-    int size = 1;
-    while (size < count) size <<= 1;
-    MoveKey* s_key = reinterpret_cast<MoveKey*>(bitonic_smem);
-    int* s_idx = reinterpret_cast<int*>(s_key + size);
-    sort_moves_smem(size, count, in, s_key, s_idx, MoveOrder{});
-    // Every vertex goes to the first move that wants it; a move keeps its
-    // vertices only if it gets them all.
-    const int first = static_cast<int>(threadIdx.x) * kPer;
-    for (int i = first; i < first + kPer && i < count; ++i) {
-        const JointMove& m = in[s_idx[i]];
-        for (int j = 0; j < m.size; ++j) atomicMin(owners + m.vertices[j], i);
-    }
-    __syncthreads();
-    unsigned wins = 0;
-    for (int i = first; i < first + kPer && i < count; ++i) {
-        const JointMove& m = in[s_idx[i]];
-        bool all = true;
-        for (int j = 0; j < m.size; ++j) all &= __ldcg(owners + m.vertices[j]) == i;
-        wins |= all ? 1u << (i - first) : 0u;
-    }
-    __syncthreads();
-    for (int i = first; i < first + kPer && i < count; ++i) {
-        const JointMove& m = in[s_idx[i]];
-        for (int j = 0; j < m.size; ++j) owners[m.vertices[j]] = INT_MAX;
-    }
-    __syncthreads();
-    u32 chunks[kPer][2 * kJointSide], local = 0;
-#pragma unroll
-    for (int q = 0; q < kPer; ++q)
-#pragma unroll
-        for (int j = 0; j < 2 * kJointSide; ++j) chunks[q][j] = 0;
-#pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-        const int i = first + q;
-        if (i >= count) continue;
-        JointMove m = in[s_idx[i]];
-        if (!(wins & (1u << q))) m.size = 0;
-#pragma unroll
-        for (int j = 0; j < 2 * kJointSide; ++j)
-            if (j < m.size) {
-                const int v = m.vertices[j];
-                owners[v] = i;
-                targets[v] = labels[v] == m.a ? m.b : m.a;
-                chunks[q][j] = static_cast<u32>((off[v + 1] - off[v] + kEventChunk - 1) / kEventChunk);
-                local += chunks[q][j];
-            }
-        out[i] = m;
+    __shared__ int s_offset[kMaxParts + 1];
+    part_offsets(k, parts->moves, s_offset);
+    for (int i = s_offset[blockIdx.x] + static_cast<int>(threadIdx.x); i < s_offset[blockIdx.x + 1]; i += kThreads) {
+        const JointMove m = moves[i];
         events[i] = 0;
-    }
-    u32 total;
-    u32 run = block_exclusive_scan_wide<u32>(local, total, s_scan);
-#pragma unroll
-    for (int q = 0; q < kPer; ++q)
-#pragma unroll
-        for (int j = 0; j < 2 * kJointSide; ++j) {
-            if (first + q < count) chunk_off[(first + q) * 2 * kJointSide + j] = run;
-            run += chunks[q][j];
+        bool all = true;
+        for (int j = 0; j < m.size; ++j) all &= claims[m.vertices[j]] == i;
+        if (!all) {
+            moves[i].size = 0;
+            continue;
         }
-    if (threadIdx.x == 0) {
-        *total_chunks = total;
-        counts->active = static_cast<u32>(count);
+        int chunks = 0;
+        for (int j = 0; j < m.size; ++j) {
+            const int v = m.vertices[j];
+            owners[v] = i;
+            targets[v] = labels[v] == m.a ? m.b : m.a;
+            chunks += (off[v + 1] - off[v] + kEventChunk - 1) / kEventChunk;
+        }
+        u64 at = atomicAdd(&counts->work, static_cast<u64>(chunks));
+        for (int j = 0; j < m.size; ++j) {
+            const int v = m.vertices[j], own = (off[v + 1] - off[v] + kEventChunk - 1) / kEventChunk;
+            for (int c = 0; c < own; ++c)
+                work[at++] = (static_cast<u64>(i) << 32) | (static_cast<u64>(j) << 28) | static_cast<u64>(c);
+        }
     }
 }
-__global__ void k_events(const u32* count_ptr, const JointMove* moves, const u32* chunk_off, const u32* total_chunks,
-                         const int* owners, const int* targets, const int* labels, const int* off, const int* nbr,
-                         const u32* ew, u64* events) {
+__global__ void k_events(const JointCounts* counts, const u64* work, const JointMove* moves, const int* owners,
+                         const int* targets, const int* labels, const int* off, const int* nbr, const u32* ew,
+                         u64* events) {
     after_previous();
     const int lane = threadIdx.x & 31;
-    const int items = static_cast<int>(*count_ptr) * 8;
-    const u32 total = items ? *total_chunks : 0;
-    for (u32 w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < total; w += (gridDim.x * blockDim.x) >> 5) {
-        int lo = 0, hi = items - 1;  // the last item whose chunks start at or before w
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (chunk_off[mid] <= w) lo = mid; else hi = mid - 1;
-        }
-        const int i = lo >> 3;
-        const int ma = moves[i].a, mb = moves[i].b, v = moves[i].vertices[lo & 7];
-        const int begin = off[v] + static_cast<int>(w - chunk_off[lo]) * kEventChunk;
+    const u64 total = counts->work;
+    for (u64 w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < total; w += (gridDim.x * blockDim.x) >> 5) {
+        const u64 item = work[w];
+        const int i = static_cast<int>(item >> 32);
+        const int ma = moves[i].a, mb = moves[i].b, v = moves[i].vertices[(item >> 28) & 7];
+        const int begin = off[v] + static_cast<int>(item & 0xfffffffULL) * kEventChunk;
         const int end = min(off[v + 1], begin + kEventChunk);
         u64 own = 0;
         for (int e = begin + lane; e < end; e += 32) {
@@ -2904,24 +2846,17 @@ __global__ void k_events(const u32* count_ptr, const JointMove* moves, const u32
 // largest one above zero, the move at which the serial scan last improved.
 // Then appends the vertices of the moves up to it to the movers.
 constexpr int kPrefixThreads = kScanThreads;
-__global__ void __launch_bounds__(kPrefixThreads) k_prefix(const u32* count_ptr, const JointMove* moves,
+__global__ void __launch_bounds__(kPrefixThreads) k_prefix(int k, const JointParts* parts, const JointMove* moves,
                                                            const u64* events, const u64* loads, u64 capacity,
                                                            int* movers, u64* mover_count) {
     after_previous();
-    const int count = static_cast<int>(*count_ptr);
+    __shared__ int s_offset[kMaxParts + 1];
+    part_offsets(k, parts->moves, s_offset);
     __shared__ long long s_scan[9];
-    __shared__ int s_range[2];
     __shared__ long long s_best_gain[kPrefixThreads / 32];
     __shared__ int s_best_index[kPrefixThreads / 32];
     const int a = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x < 2) {
-        const int key = a + static_cast<int>(threadIdx.x);  // first move of part a, first after it
-        int low = 0, high = count;
-        while (low < high) { const int mid = (low + high) / 2; if (moves[mid].a < key) low = mid + 1; else high = mid; }
-        s_range[threadIdx.x] = low;
-    }
-    __syncthreads();
-    const int first = s_range[0], last = s_range[1];
+    const int first = s_offset[a], last = s_offset[a + 1];
     const long long lo = static_cast<long long>(loads[a]) - static_cast<long long>(capacity);
     long long gain_carry = 0, net_carry = 0, best = 0;
     int stop = -1;
@@ -3633,8 +3568,7 @@ void LevelRefiner<T>::restore_best(bool moved) {
 }
 
 // The exchange passes.  A pass runs on device counts from the matching to the
-// applied batch, so the host reads back once per pass; only when it finds a
-// list longer than one block sorts does it finish the pass step by step.
+// applied batch, so the host reads back once per pass.
 template <class T>
 void LevelRefiner<T>::exchange(u64& best_cut) {
     Arena& A_ = ctx.scratch;
@@ -3651,21 +3585,19 @@ void LevelRefiner<T>::exchange(u64& best_cut) {
     JointMove* frag_sorted = A_.alloc<JointMove>(frag_cap);
     JointMove* act = A_.alloc<JointMove>(move_cap);
     JointMove* act_sorted = A_.alloc<JointMove>(move_cap);
+    unsigned char* frag_part = A_.alloc<unsigned char>(frag_cap);
+    unsigned char* act_part = A_.alloc<unsigned char>(move_cap);
+    int* claims = A_.alloc<int>(n);
     int* owners = A_.alloc<int>(n);
     u64* events = A_.alloc<u64>(move_cap);
-    u32* chunk_off = A_.alloc<u32>(move_cap * 8);
-    u32* total_chunks = A_.alloc<u32>(1);
-    // Behind the batch's counters, so that one fetch brings both.
-    constexpr int kJointWords = sizeof(JointCounts) / sizeof(u64);
-    JointCounts* counts = reinterpret_cast<JointCounts*>(counters + 10);
+    // Every vertex is in one settled move at most.
+    u64* work = A_.alloc<u64>(static_cast<size_t>(n) + static_cast<size_t>(g.m) / kEventChunk);
+    JointParts* parts = A_.alloc<JointParts>(1);
+    JointCounts* counts = A_.alloc<JointCounts>(1);
     u64* mover_count = counters + 9;
     GP_CUDA(cudaMemsetAsync(quotient, 0, sizeof(u64) * k * k, s()));
     GP_CUDA(cudaMemsetAsync(visits, 0, sizeof(int) * k * k, s()));
     launch(k_quotient<T>, grid_for(n, kThreads), kThreads, 0, s(), n, labels, static_cast<const T*>(A), k, quotient);
-    auto read_counts = [&]() {
-        ctx.fetch(counters + 2, 8 + kJointWords);
-        return *reinterpret_cast<const JointCounts*>(ctx.host_scalars + 8);
-    };
     // (Shared-memory limits are set to one value for every size, on every
     // call: the limit belongs to the kernel for the whole process, on
     // whichever device is current, and concurrent worker contexts must not
@@ -3673,97 +3605,35 @@ void LevelRefiner<T>::exchange(u64& best_cut) {
     auto allow = [](auto kernel, size_t smem) {
         GP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
     };
-    constexpr size_t sort_smem = kBitonicEntryBytes * kBitonicSegment;
-    // Events, prefixes and the batch of the ordered moves.
-    auto settle = [&]() {
-        launch(k_events, 148 * 8, kThreads, 0, s(), static_cast<const u32*>(&counts->active),
-               static_cast<const JointMove*>(act_sorted), static_cast<const u32*>(chunk_off),
-               static_cast<const u32*>(total_chunks), static_cast<const int*>(owners), static_cast<const int*>(targets),
-               static_cast<const int*>(labels), g.off, g.nbr, g.ew, events);
-        launch(k_prefix, k, kPrefixThreads, 0, s(), static_cast<const u32*>(&counts->active),
-               static_cast<const JointMove*>(act_sorted), static_cast<const u64*>(events),
-               static_cast<const u64*>(loads), C, movers, mover_count);
-        apply(movers, mover_count, n, false, false);
-    };
-    auto sort_long = [&](JointMove* in, JointMove* out, int count, auto cmp) {
-        using Cmp = decltype(cmp);
-        ArenaScope ss(A_);
-        int size = kBitonicSegment;
-        while (size < count) size <<= 1;
-        int* idx = A_.alloc<int>(size);
-        MoveKey* move_keys = A_.alloc<MoveKey>(count);
-        launch(k_iota, blocks_for(size, kThreads), kThreads, 0, s(), size, idx);
-        launch(k_move_keys<Cmp>, blocks_for(count, kThreads), kThreads, 0, s(), count,
-               static_cast<const JointMove*>(in), move_keys);
-        // Stages whose partner distance stays inside a segment run in shared
-        // memory, the rest one launch per stage.
-        allow(k_bitonic_local<Cmp>, sort_smem);
-        const int segments = size / kBitonicSegment;
-        const JointMove* m = in;
-        const MoveKey* mk = move_keys;
-        launch(k_bitonic_local<Cmp>, segments, 1024, sort_smem, s(), size, count, m, mk, idx, 2, kBitonicSegment, 1, cmp);
-        for (int kk = 2 * kBitonicSegment; kk <= size; kk <<= 1) {
-            for (int jj = kk >> 1; jj >= kBitonicSegment; jj >>= 1)
-                launch(k_bitonic<Cmp>, blocks_for(size, kThreads), kThreads, 0, s(), size, count, m, mk, idx, kk, jj,
-                       cmp);
-            launch(k_bitonic_local<Cmp>, segments, 1024, sort_smem, s(), size, count, m, mk, idx, kk, kk,
-                   kBitonicSegment / 2, cmp);
-        }
-        launch(k_gather_moves, blocks_for(count, kThreads), kThreads, 0, s(), count, static_cast<const int*>(idx),
-               static_cast<const JointMove*>(in), out);
-    };
-    auto combine = [&](int most) {
-        launch(k_combine, blocks_for(most, 8), kThreads, 0, s(), counts, static_cast<const JointMove*>(frag_sorted),
-               g.off, g.nbr, g.ew, labels, loads, C, slots, act);
-    };
-    // A pass with a long list, from the lists on the device.
-    auto finish_long = [&](JointCounts found) {
-        if (found.fragments > kBitonicSegment) {  // no fragment was combined yet
-            const int fragments = static_cast<int>(found.fragments);
-            ArenaScope fs(A_);
-            JointMove* ordered = A_.alloc<JointMove>(fragments);
-            sort_long(frag, ordered, fragments, NetOrder{});
-            select_if(A_, s(), fragments, UniqueHead{ordered}, CopyMove{ordered, frag_sorted}, &counts->unique);
-            combine(fragments);
-            found = read_counts();
-        }
-        const int active = static_cast<int>(found.moves);
-        if (!active) return;
-        sort_long(act, act_sorted, active, MoveOrder{});
-        const u32 length = static_cast<u32>(active);
-        ctx.host_scalars[24] = length;
-        GP_CUDA(cudaMemcpyAsync(&counts->active, ctx.host_scalars + 24, sizeof(u32), cudaMemcpyHostToDevice, s()));
-        fill<int>(s(), owners, n, INT_MAX);
-        launch(k_claim, blocks_for(active, kThreads), kThreads, 0, s(), active, static_cast<const JointMove*>(act_sorted), owners);
-        launch(k_resolve, blocks_for(active, kThreads), kThreads, 0, s(), active, act_sorted, static_cast<const int*>(owners));
-        fill<int>(s(), owners, n, INT_MAX);
-        launch(k_mark, blocks_for(active, kThreads), kThreads, 0, s(), active, static_cast<const JointMove*>(act_sorted),
-               static_cast<const int*>(labels), owners, targets);
-        GP_CUDA(cudaMemsetAsync(events, 0, sizeof(u64) * active, s()));
-        exclusive_scan<u32>(A_, s(), static_cast<i64>(active) * 8,
-                            EventChunks{static_cast<const JointMove*>(act_sorted), g.off}, chunk_off, total_chunks);
-        settle();
-        read_counts();
-    };
     int empty = 0;
     for (int pass = 0; pass < budget.exchange_rounds; ++pass) {
         // One value for every k (see `allow`).
         allow(k_match_parts, sizeof(double) * kMaxParts * kMaxParts);
         launch(k_match_parts, 1, kMatchThreads, sizeof(double) * k * k, s(), k, quotient, partner, visits, seeds, k * sw,
-               counts, mover_count);
+               counts, parts, mover_count);
         launch(k_seeds<T>, grid_for(n, kThreads), kThreads, 0, s(), n, labels, static_cast<const T*>(A), k, partner,
-               seeds, sw, pass, owners);
+               seeds, sw, pass, claims, owners);
         launch(k_grow<T>, blocks_for(slots, 8), kThreads, 0, s(), slots, sw, seeds, partner, g.off, g.nbr, g.ew, g.vw,
-               labels, static_cast<const T*>(A), k, loads, C, act, frag, counts);
-        allow(k_sort_fragments, sort_smem);
-        launch(k_sort_fragments, 1, 1024, sort_smem, s(), static_cast<const JointMove*>(frag), frag_sorted, counts);
-        combine(kBitonicSegment);
-        allow(k_rank_moves, sort_smem);
-        launch(k_rank_moves, 1, 1024, sort_smem, s(), static_cast<const JointMove*>(act), act_sorted, counts, g.off,
-               static_cast<const int*>(labels), owners, targets, events, chunk_off, total_chunks);
-        settle();
-        const JointCounts found = read_counts();
-        if (found.fragments > kBitonicSegment || found.moves > kBitonicSegment) finish_long(found);
+               labels, static_cast<const T*>(A), k, loads, C, act, act_part, frag, frag_part, counts, parts);
+        allow(k_sort_fragments, sizeof(FragmentSort));
+        launch(k_sort_fragments, k, kPartSortThreads, sizeof(FragmentSort), s(), k, static_cast<const JointMove*>(frag),
+               static_cast<const unsigned char*>(frag_part), frag_sorted, parts);
+        launch(k_combine, 148 * 8, kThreads, 0, s(), k, counts, parts, static_cast<const JointMove*>(frag_sorted), g.off,
+               g.nbr, g.ew, static_cast<const int*>(labels), static_cast<const u64*>(loads), C, slots, act, act_part);
+        allow(k_sort_moves, sizeof(MoveSort));
+        launch(k_sort_moves, k, kPartSortThreads, sizeof(MoveSort), s(), k, static_cast<const JointMove*>(act),
+               static_cast<const unsigned char*>(act_part), act_sorted, static_cast<const JointParts*>(parts), claims);
+        launch(k_settle, k, kThreads, 0, s(), k, act_sorted, counts, static_cast<const JointParts*>(parts), g.off,
+               static_cast<const int*>(labels), static_cast<const int*>(claims), owners, targets, events, work);
+        launch(k_events, 148 * 8, kThreads, 0, s(), static_cast<const JointCounts*>(counts),
+               static_cast<const u64*>(work), static_cast<const JointMove*>(act_sorted),
+               static_cast<const int*>(owners), static_cast<const int*>(targets), static_cast<const int*>(labels), g.off,
+               g.nbr, g.ew, events);
+        launch(k_prefix, k, kPrefixThreads, 0, s(), k, static_cast<const JointParts*>(parts),
+               static_cast<const JointMove*>(act_sorted), static_cast<const u64*>(events),
+               static_cast<const u64*>(loads), C, movers, mover_count);
+        apply(movers, mover_count, n, false, false);
+        ctx.fetch(counters + 2, 8);
         const i64 count = static_cast<i64>(ctx.host_scalars[7] & 0xffffffffULL);
         if (!count) { if (++empty >= 2) break; continue; }
         empty = 0;
@@ -3882,10 +3752,9 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known, u64 known_load) {
     movers = A_.alloc<int>(n);
     // [8]: k_commit's finished-block count, zero between launches; [9]: the
     // movers of a repair or exchange (a 32-bit count in a zeroed word); [10],
-    // [11]: the repair's donors and listed donors; [10] to [12]: the exchange's
-    // JointCounts.
-    counters = A_.alloc<u64>(13);
-    GP_CUDA(cudaMemsetAsync(counters + 8, 0, 5 * sizeof(u64), s()));
+    // [11]: the repair's donors and listed donors.
+    counters = A_.alloc<u64>(12);
+    GP_CUDA(cudaMemsetAsync(counters + 8, 0, 4 * sizeof(u64), s()));
     corr_acc = A_.alloc<long long>(g.heavy_count + 1);
     if (g.chunks) {
         chunk_work = A_.alloc<int>(g.chunks);
