@@ -22,21 +22,23 @@ constexpr int kEvalWarps = kEvalThreads / 32;
 constexpr int kEvalStride = kMaxParts + 2;
 constexpr int kEvalWindow = 256;  // entries a warp reads per step, eight per lane
 
-// Number of row ends before item d of the merged sequence of rows and entries
-// (row i's end comes before entry j when off[i + 1] - first <= j): the
-// merge-path split of Merrill and Garland ("Merge-based Parallel Sparse
-// Matrix-Vector Multiplication", 2016), found by the whole warp with 31 probes
-// a step.  Always in [max(0, d - entries), min(d, n)], whatever the offsets.
-__device__ __forceinline__ i64 merge_split(const int* off, i64 n, i64 first, i64 entries, i64 d) {
+constexpr int kEvalRowCost = kEvalWindow / 32;  // a step reads 256 entries or ends 32 rows
+
+// Rows finished within the first d units of the work, a row costing
+// kEvalRowCost units and an entry one: a merge-path split (Merrill and Garland,
+// "Merge-based Parallel Sparse Matrix-Vector Multiplication", 2016) whose row
+// ends weigh what they cost here, found by the whole warp with 32 probes a
+// step.  Always in [0, n], whatever the offsets.
+__device__ __forceinline__ i64 work_split(const int* off, i64 n, i64 first, i64 d) {
     const int lane = threadIdx.x & 31;
-    i64 lo = d > entries ? d - entries : 0, hi = d < n ? d : n;
+    i64 lo = 0, hi = min(n, d / kEvalRowCost);
     while (lo < hi) {
         const i64 step = (hi - lo + 31) >> 5;
         const i64 at = lo + lane * step;
-        const bool before = at < hi && off[at + 1] - first <= d - 1 - at;
+        const bool within = at < hi && (at + 1) * kEvalRowCost + (off[at + 1] - first) <= d;
         // The probes that hold are a prefix for monotone offsets; only that
         // prefix is used.
-        const unsigned fails = ~__ballot_sync(0xffffffffu, before);
+        const unsigned fails = ~__ballot_sync(0xffffffffu, within);
         const int holds = fails ? __ffs(fails) - 1 : 32;
         if (holds == 0) {
             hi = lo;
@@ -48,16 +50,24 @@ __device__ __forceinline__ i64 merge_split(const int* off, i64 n, i64 first, i64
     }
     return lo;
 }
+// Entries read within the first d units, `row` rows being finished: all of the
+// open row's at most.
+__device__ __forceinline__ i64 entries_within(const int* off, i64 n, i64 first, i64 entries, i64 d, i64 row) {
+    const i64 row_end = row < n ? min(max(off[row + 1] - first, 0LL), entries) : entries;
+    return min(max(d - row * kEvalRowCost, 0LL), row_end);
+}
 
 // Pass 1.  Loads: every thread takes four vertices at a time, 32 apart, and
 // adds neighbouring ones of equal labels once, a warp of one label once.  Cut: every warp
-// takes an equal share of the merged sequence of rows and entries, so neither a
-// hub row nor a stretch of empty rows falls to one warp; it reads 256 entries
+// takes an equal share of the work over rows and entries, so neither a
+// hub row nor a stretch of short rows falls to one warp; it reads 256 entries
 // a step, eight gathers per lane in flight, next to the ends and labels of the
 // next 32 rows, and finds each entry's row from the marks that non-empty rows
 // leave at their first entry.  Bound by the label gathers, served by L2.
-// R-MAT scale 22, k = 64 (124 M entries): 1.12 ms with the reduction; a warp per
-// row took 6.58 ms, its longest row alone setting the time.
+// R-MAT scale 22, k = 64 (124 M entries): 0.59 ms with the reduction; a warp per
+// row took 6.60 ms, its longest row alone setting the time, and shares of equal
+// rows plus entries 1.14, half of the SMs' time idle at the end.  (Labels packed
+// into bytes first gained nothing.)
 // Every access is range-checked, so a malformed labelling or CSR cannot reach
 // memory outside the caller's arrays or the block's shared tables.
 __global__ void __launch_bounds__(kEvalThreads, 5) k_eval_partials(i64 n, i64 m, const int* off, const int* nbr,
@@ -113,16 +123,16 @@ __global__ void __launch_bounds__(kEvalThreads, 5) k_eval_partials(i64 n, i64 m,
     u64 cut = 0;
     const i64 first = min(max(static_cast<i64>(off[0]), 0LL), m);
     const i64 entries = min(max(static_cast<i64>(off[n]), first), m) - first;
-    const i64 items = n + entries;
+    const i64 units = n * kEvalRowCost + entries;
     const i64 warps = static_cast<i64>(gridDim.x) * kEvalWarps;
-    const i64 share = max((items + warps - 1) / warps, static_cast<i64>(kEvalWindow));
+    const i64 share = max((units + warps - 1) / warps, static_cast<i64>(kEvalWindow));
     const i64 d0 = (static_cast<i64>(blockIdx.x) * kEvalWarps + warp) * share;
-    if (d0 < items) {
-        const i64 d1 = min(items, d0 + share);
-        int row = static_cast<int>(merge_split(off, n, first, entries, d0));
-        const int last_row = static_cast<int>(merge_split(off, n, first, entries, d1));
-        i64 e = first + d0 - row;
-        const i64 last = first + d1 - last_row;
+    if (d0 < units) {
+        const i64 d1 = min(units, d0 + share);
+        int row = static_cast<int>(work_split(off, n, first, d0));
+        const int last_row = static_cast<int>(work_split(off, n, first, d1));
+        i64 e = first + entries_within(off, n, first, entries, d0, row);
+        const i64 last = first + entries_within(off, n, first, entries, d1, last_row);
         const int rows = static_cast<int>(n);
         signed char* mark = marks[warp];
         while (e < last && row <= last_row && row < rows) {
@@ -242,7 +252,7 @@ void check_evaluate_args(const gp_csr* g, const int32_t* labels, int32_t k, cons
 void launch_evaluate(const gp_csr* g, const int32_t* labels, int32_t k, uint64_t* cut_out, uint64_t* loads_out,
                      u64* partial, u64* invalid, cudaStream_t s) {
     // No more blocks than give every warp one window of entries.
-    const int blocks = std::min(blocks_for(g->n + g->m, kEvalWarps * kEvalWindow), kEvalBlocks);
+    const int blocks = std::min(blocks_for(g->n * kEvalRowCost + g->m, kEvalWarps * kEvalWindow), kEvalBlocks);
     launch_ordinary(k_eval_partials, blocks, kEvalThreads, 0, s, static_cast<i64>(g->n), static_cast<i64>(g->m),
            g->offsets, g->neighbors, g->edge_weights, g->vertex_weights, labels, static_cast<int>(k), partial);
     launch_ordinary(k_eval_reduce, 1, 1024, 0, s, blocks, static_cast<int>(k), static_cast<const u64*>(partial),
