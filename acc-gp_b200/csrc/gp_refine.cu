@@ -1145,41 +1145,74 @@ __device__ int gain_bucket(u64 best, u64 current, u64 relief) {
     return max(2, min(49, 25 + lo));
 }
 
-// initialize_receiver_slack (rebalance_select.cuh:79-104) by one thread.
-// One thread per part; the CDF is a saturating prefix sum over the parts.
 __device__ __forceinline__ u64 saturating_add(u64 a, u64 b) { return ~0ULL - a < b ? ~0ULL : a + b; }
-// Also clears the iteration's three counts (placed donors, donors, listed
-// donors).
+
+// initialize_receiver_slack (rebalance_select.cuh:79-104) and the fallback
+// tickets of every donor weight (enumerate_repair_destination,
+// rebalance_select.cuh:9-75): a donor without a connected destination draws a
+// ticket over the free room of the parts that fit its weight, in part order.
+// Which parts fit changes only where the weight passes a part's room, so a
+// block per rank c of the parts by room (descending) writes the prefix sums,
+// in part order, of the rooms of at least the c-th largest (saturating), and
+// rooms[c]; a ticket is then two binary searches (ticket_part) instead of two
+// walks over all parts, which with seven threads in 32 active bounded the
+// destination kernels: a 256^3 mesh at k = 128 went from 147-154 to 126 ms
+// (device time 139 to 113 ms, k_repair_dest_od to 6.4 ms of it).
+// Block 0 also clears the iteration's three counts (placed donors, donors,
+// listed donors).
 __global__ void __launch_bounds__(kMaxParts) k_slack(int k, const u64* loads, u64 capacity, u64* slack, u64* requests,
-                                                     u64* cdf, u64* counts) {
+                                                     u64* rooms, u64* tickets, u64* counts) {
     after_previous();
-    __shared__ u64 warp_total[kMaxParts / 32], warp_min[kMaxParts / 32];
-    const int p = threadIdx.x, lane = p & 31, warp = p >> 5;
+    __shared__ u64 s_room[kMaxParts], s_total[kMaxParts / 32], s_least;
+    const int p = threadIdx.x, lane = p & 31, warp = p >> 5, c = blockIdx.x;
     const u64 room = p < k ? (loads[p] < capacity ? capacity - loads[p] : 0) : 0;
-    u64 inc = room, least = room ? room : ~0ULL;
+    s_room[p] = room;
+    __syncthreads();
+    int rank = 0;
+    for (int q = 0; q < k; ++q) rank += s_room[q] > room || (s_room[q] == room && q < p);
+    if (p < k && rank == c) s_least = room;
+    __syncthreads();
+    const u64 least = s_least;
+    u64 inc = least && room >= least ? room : 0;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
         const u64 o = __shfl_up_sync(0xffffffffu, inc, d);
         if (lane >= d) inc = saturating_add(inc, o);
-        const u64 m = __shfl_xor_sync(0xffffffffu, least, d);
-        least = m < least ? m : least;
     }
-    if (lane == 31) warp_total[warp] = inc;
-    if (lane == 0) warp_min[warp] = least;
+    if (lane == 31) s_total[warp] = inc;
     __syncthreads();
     u64 before = 0;
-    for (int w = 0; w < warp; ++w) before = saturating_add(before, warp_total[w]);
-    if (p < k) {
-        slack[p] = room;
-        requests[p] = 0;
-        cdf[p] = saturating_add(before, inc);
+    for (int w = 0; w < warp; ++w) before = saturating_add(before, s_total[w]);
+    if (p < k) tickets[static_cast<i64>(c) * k + p] = saturating_add(before, inc);
+    if (p == 0) rooms[c] = least;
+    if (c == 0) {
+        if (p < k) {
+            slack[p] = room;
+            requests[p] = 0;
+        }
+        if (p < 3) counts[p] = 0;
     }
-    if (p < 3) counts[p] = 0;
-    if (p == 0) {
-        u64 m = ~0ULL;
-        for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) m = warp_min[w] < m ? warp_min[w] : m;
-        cdf[k] = m;
+}
+// The part that a donor of weight w draws with `hash`: -1 when no part fits it.
+// rooms: in shared memory, descending.
+__device__ __forceinline__ int ticket_part(int k, u64 w, u32 hash, const u64* rooms, const u64* tickets) {
+    int lo = 0, hi = k;  // parts that fit w
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (rooms[mid] >= w) lo = mid + 1;
+        else hi = mid;
     }
+    if (!lo) return -1;
+    const u64* upto = tickets + static_cast<i64>(lo - 1) * k;
+    const u64 t = static_cast<u64>(hash) % upto[k - 1];
+    lo = 0;
+    hi = k - 1;  // the first part whose prefix exceeds the ticket
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (upto[mid] <= t) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
 }
 
 // A donor's plan of one repair iteration, one word per vertex: its order
@@ -1227,18 +1260,19 @@ __device__ __forceinline__ void load_affinities(const C* p, C (&val)[N]) {
 template <class C, int W, bool Vectorized>
 __global__ void __launch_bounds__(kThreads) k_repair_dest(i64 n, const C* A, const C* totals, const int* labels,
                                                           const u32* vw, int k, const u64* loads, u64 capacity,
-                                                          const u64* cdf, u32* plan, u64* hist, u64* donor_count) {
+                                                          const u64* rooms, const u64* tickets, u32* plan,
+                                                          u64* hist, u64* donor_count) {
     after_previous();
     constexpr int N = Vectorized ? AffinityVec<C>::N : 1;
     constexpr int G = 32 / W;
-    __shared__ u64 s_room[kMaxParts], s_excess[kMaxParts];
+    __shared__ u64 s_room[kMaxParts], s_excess[kMaxParts], s_rooms[kMaxParts];
     for (int p = threadIdx.x; p < k; p += blockDim.x) {
         s_room[p] = loads[p] < capacity ? capacity - loads[p] : 0;
         s_excess[p] = loads[p] > capacity ? loads[p] - capacity : 0;
+        s_rooms[p] = rooms[p];
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, gid = lane / W, sub = lane % W;
-    const int span = (k + W - 1) / W;  // contiguous parts per lane for the fallback ticket
     u64 donors = 0;
     for (i64 base = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) & ~31LL; base < n;
          base += static_cast<i64>(gridDim.x) * blockDim.x) {
@@ -1283,57 +1317,11 @@ __global__ void __launch_bounds__(kThreads) k_repair_dest(i64 n, const C* A, con
                 }
             }
             if (!conn) part = -1;
-            // Fallback ticket over the parts' room when no connected destination
-            // fits: from the slack CDF when the source is at capacity, else over
-            // the parts that fit w, in part order (saturating sums).
-            // (A donor's part is over capacity.)
-            const bool ticket = valid && part < 0 && w > cdf[k];
-            const u32 hash = mix32(static_cast<u32>(v));
-            if (__any_sync(0xffffffffu, ticket)) {
-                const int lo = sub * span, hi = min(k, lo + span);
-                u64 mine = 0;
-                if (ticket)
-                    for (int p = lo; p < hi; ++p)
-                        if (p != src && w <= s_room[p]) mine = ~0ULL - mine < s_room[p] ? ~0ULL : mine + s_room[p];
-                u64 upto = mine;  // inclusive scan over the group, saturating
-#pragma unroll
-                for (int d = 1; d < W; d <<= 1) {
-                    const u64 o = __shfl_up_sync(0xffffffffu, upto, d, W);
-                    if (sub >= d) upto = ~0ULL - upto < o ? ~0ULL : upto + o;
-                }
-                const u64 total = __shfl_sync(0xffffffffu, upto, W - 1, W);
-                // Exclusive prefix, saturated: exact for the lane holding the
-                // ticket (ticket < total), above the ticket for every later lane.
-                const u64 prev = __shfl_up_sync(0xffffffffu, upto, 1, W);
-                const u64 before = sub == 0 ? 0 : prev;
-                int found = -1;
-                if (ticket && total) {
-                    u64 t = static_cast<u64>(hash) % total;
-                    if (t >= before && (t - before) < mine) {
-                        t -= before;
-                        for (int p = lo; p < hi; ++p)
-                            if (p != src && w <= s_room[p]) {
-                                if (t < s_room[p]) { found = p; break; }
-                                t -= s_room[p];
-                            }
-                    }
-                }
-#pragma unroll
-                for (int d = W / 2; d; d >>= 1) found = max(found, __shfl_xor_sync(0xffffffffu, found, d, W));
-                if (ticket) part = found;
-            }
             if (valid && sub == 0) {
-                if (part < 0 && !ticket) {
+                if (part < 0) {
                     conn = 0;
-                    const u64 sum = cdf[k - 1];
-                    if (sum) {
-                        const u64 t = static_cast<u64>(hash) % sum;
-                        int lo = 0, hi = k;
-                        while (lo < hi) { const int mid = (lo + hi) / 2; if (cdf[mid] <= t) lo = mid + 1; else hi = mid; }
-                        part = lo;
-                    }
+                    part = ticket_part(k, w, mix32(static_cast<u32>(v)), s_rooms, tickets);
                 }
-                if (ticket) conn = 0;
                 const u32 word = make_plan(v, part, conn, current, w, s_excess[src]);
                 plan[v] = word;
                 if (part >= 0) atomicAdd(hist + src * kBalanceWidth + plan_class(word), w);
@@ -1343,74 +1331,80 @@ __global__ void __launch_bounds__(kThreads) k_repair_dest(i64 n, const C* A, con
     block_atomic_add(donor_count, donors);
 }
 
-// k_repair_dest with on-demand affinities, one thread per vertex: the best
+// k_repair_dest with on-demand affinities, one thread per donor: the best
 // connected destination with room (largest affinity, then room, then lowest
-// part), else the same fallback tickets.
+// part), else the same fallback ticket.  A block takes the donors among 1024
+// consecutive vertices at a time off a list in shared memory, so that its
+// warps are full where parts overlap.
 template <int D>
 __global__ void __launch_bounds__(kThreads) k_repair_dest_od(i64 n, const int* off, const int* nbr, const u32* ew,
                                                              const int* labels, const u32* vw, int k, const u64* loads,
-                                                             u64 capacity, const u64* cdf, u32* plan, u64* hist,
-                                                             u64* donor_count) {
+                                                             u64 capacity, const u64* rooms, const u64* tickets,
+                                                             u32* plan, u64* hist, u64* donor_count) {
     after_previous();
-    __shared__ u64 s_room[kMaxParts], s_excess[kMaxParts];
+    constexpr int U = 4;
+    __shared__ u64 s_room[kMaxParts], s_excess[kMaxParts], s_rooms[kMaxParts];
+    __shared__ int s_donor[U * kThreads];
+    __shared__ u32 s_count;
     for (int p = threadIdx.x; p < k; p += blockDim.x) {
         s_room[p] = loads[p] < capacity ? capacity - loads[p] : 0;
         s_excess[p] = loads[p] > capacity ? loads[p] - capacity : 0;
+        s_rooms[p] = rooms[p];
     }
-    __syncthreads();
+    const int lane = threadIdx.x & 31;
     u64 donors = 0;
-    for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += static_cast<i64>(gridDim.x) * blockDim.x) {
-        const int v = static_cast<int>(i);
-        const int src = labels[v];
-        if (!s_excess[src]) continue;
-        ++donors;
-        const u64 w = vw[v];
-        RowRegs<D> r;
-        r.load(v, off, nbr, ew, labels);
-        const u64 current = r.of(src);
-        int part = -1;
-        u64 conn = 0, best_room = 0;
-        if (current != r.total)
+    for (i64 base = static_cast<i64>(blockIdx.x) * U * kThreads; base < n;
+         base += static_cast<i64>(gridDim.x) * U * kThreads) {
+        __syncthreads();
+        if (threadIdx.x == 0) s_count = 0;
+        __syncthreads();
+        int label[U];
 #pragma unroll
-            for (int j = 0; j < D; ++j) {
-                const int p = r.part[j];
-                if (p < 0 || p == src || !r.first(j)) continue;
-                const u64 room = s_room[p];
-                if (w > room) continue;
-                const u64 value = r.of(p);
-                if (part < 0 || value > conn || (value == conn && (room > best_room || (room == best_room && p < part)))) {
-                    part = p; conn = value; best_room = room;
-                }
-            }
-        if (!conn) part = -1;
-        if (part < 0) {
-            conn = 0;
-            const u32 hash = mix32(static_cast<u32>(v));
-            if (w <= cdf[k]) {  // a donor's part is over capacity
-                const u64 sum = cdf[k - 1];
-                if (sum) {
-                    const u64 t = static_cast<u64>(hash) % sum;
-                    int lo = 0, hi = k;
-                    while (lo < hi) { const int mid = (lo + hi) / 2; if (cdf[mid] <= t) lo = mid + 1; else hi = mid; }
-                    part = lo;
-                }
-            } else {
-                u64 total = 0;
-                for (int p = 0; p < k; ++p)
-                    if (p != src && w <= s_room[p]) total = ~0ULL - total < s_room[p] ? ~0ULL : total + s_room[p];
-                if (total) {
-                    u64 t = static_cast<u64>(hash) % total;
-                    for (int p = 0; p < k; ++p)
-                        if (p != src && w <= s_room[p]) {
-                            if (t < s_room[p]) { part = p; break; }
-                            t -= s_room[p];
-                        }
-                }
-            }
+        for (int j = 0; j < U; ++j) {
+            const i64 v = base + j * kThreads + threadIdx.x;
+            label[j] = v < n ? labels[v] : -1;
         }
-        const u32 word = make_plan(v, part, conn, current, w, s_excess[src]);
-        plan[v] = word;
-        if (part >= 0) atomicAdd(hist + src * kBalanceWidth + plan_class(word), w);
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const bool donor = label[j] >= 0 && s_excess[label[j] < 0 ? 0 : label[j]] != 0;
+            const unsigned mask = __ballot_sync(0xffffffffu, donor);
+            u32 at = 0;
+            if (mask && lane == 0) at = atomicAdd(&s_count, static_cast<u32>(__popc(mask)));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(mask & ((1u << lane) - 1u));
+            if (donor) s_donor[at] = static_cast<int>(base) + j * kThreads + static_cast<int>(threadIdx.x);
+        }
+        __syncthreads();
+        const int count = static_cast<int>(s_count);
+        if (threadIdx.x == 0) donors += static_cast<u64>(count);
+        for (int i = threadIdx.x; i < count; i += kThreads) {
+            const int v = s_donor[i];
+            const int src = labels[v];
+            const u64 w = vw[v];
+            RowRegs<D> r;
+            r.load(v, off, nbr, ew, labels);
+            const u64 current = r.of(src);
+            int part = -1;
+            u64 conn = 0, best_room = 0;
+            if (current != r.total)
+#pragma unroll
+                for (int j = 0; j < D; ++j) {
+                    const int p = r.part[j];
+                    if (p < 0 || p == src || !r.first(j)) continue;
+                    const u64 room = s_room[p];
+                    if (w > room) continue;
+                    const u64 value = r.of(p);
+                    if (part < 0 || value > conn || (value == conn && (room > best_room || (room == best_room && p < part)))) {
+                        part = p; conn = value; best_room = room;
+                    }
+                }
+            if (!conn) {
+                part = ticket_part(k, w, mix32(static_cast<u32>(v)), s_rooms, tickets);
+                conn = 0;
+            }
+            const u32 word = make_plan(v, part, conn, current, w, s_excess[src]);
+            plan[v] = word;
+            if (part >= 0) atomicAdd(hist + src * kBalanceWidth + plan_class(word), w);
+        }
     }
     block_atomic_add(donor_count, donors);
 }
@@ -2968,10 +2962,11 @@ private:
     Sample* samples = nullptr;
     // Repair: donor weight per part and class (zero between iterations), each
     // part's bounding class and the weight before it, free room, requests,
-    // prefix sums of the room, and the donors' plans and list.
+    // and the donors' plans and list.
     u64* class_weights = nullptr;
     int* bound = nullptr;
-    u64 *start = nullptr, *slack = nullptr, *requests = nullptr, *cdf = nullptr, *list = nullptr;
+    u64 *start = nullptr, *slack = nullptr, *requests = nullptr, *list = nullptr;
+    u64 *rooms = nullptr, *tickets = nullptr;  // the parts' rooms in order, and the ticket sums of each (k_slack)
     u32* plan = nullptr;
     bool in_cluster = false;  // the rounds run in one launch (k_refine_cluster)
     int* saved_labels = nullptr;
@@ -3253,14 +3248,15 @@ bool LevelRefiner<T>::repair(i64 interrupted, int iterations) {
         if (listed) {
             GP_CUDA(cudaMemsetAsync(counters + 2, 0, 10 * sizeof(u64), s()));
         } else {
-            launch(k_slack, 1, kMaxParts, 0, s(), k, loads, C, slack, requests, cdf, counters + 9);
+            launch(k_slack, k, kMaxParts, 0, s(), k, static_cast<const u64*>(loads), C, slack, requests, rooms, tickets,
+                   counters + 9);
             if (on_demand)
                 with_row_size([&](auto d) {
                     launch(k_repair_dest_od<decltype(d)::value>, grid_for(n, kThreads), kThreads, 0, s(), n,
                            static_cast<const int*>(g.off), static_cast<const int*>(g.nbr), static_cast<const u32*>(g.ew),
                            static_cast<const int*>(labels), static_cast<const u32*>(g.vw), k,
-                           static_cast<const u64*>(loads), C, static_cast<const u64*>(cdf), plan, class_weights,
-                           donor_count);
+                           static_cast<const u64*>(loads), C, static_cast<const u64*>(rooms),
+                           static_cast<const u64*>(tickets), plan, class_weights, donor_count);
                 });
             else
                 with_groups([&](auto width, auto vec) {
@@ -3268,7 +3264,7 @@ bool LevelRefiner<T>::repair(i64 interrupted, int iterations) {
                     launch(k_repair_dest<T, W, decltype(vec)::value>, grid_for(n, kThreads), kThreads, 0, s(), n,
                            static_cast<const T*>(A), static_cast<const T*>(totals), static_cast<const int*>(labels),
                            static_cast<const u32*>(g.vw), k, static_cast<const u64*>(loads), C,
-                           static_cast<const u64*>(cdf), plan, class_weights, donor_count);
+                           static_cast<const u64*>(rooms), static_cast<const u64*>(tickets), plan, class_weights, donor_count);
                 });
             launch(k_repair_bounds, k, kScanThreads, 0, s(), static_cast<const u64*>(loads), C, class_weights, bound,
                    start);
@@ -3773,7 +3769,8 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known, u64 known_load) {
     }
     slack = A_.alloc<u64>(k);
     requests = A_.alloc<u64>(k);
-    cdf = A_.alloc<u64>(k + 1);
+    rooms = A_.alloc<u64>(k);
+    tickets = A_.alloc<u64>(static_cast<size_t>(k) * k);
     bound = A_.alloc<int>(k);
     start = A_.alloc<u64>(k);
     plan = A_.alloc<u32>(n);

@@ -1,7 +1,8 @@
 """Coarsening and contraction at the sizes where another kernel takes over, against the oracle.
 
 Coarse rows of up to 16 raw entries are sorted two to a warp; levels of 65,536 vertices and more are matched with 1, 8 or
-32 lanes a row by their average row; up to 2048 requests of a round are ordered by one block.
+32 lanes a row by their average row; up to 2048 requests of a round are ordered by one block; long rows are counted by
+one block up to 49,152 targets, a segment of targets at a time above.
 """
 import numpy as np
 import pytest
@@ -40,6 +41,11 @@ def test_regular_rows(gp, ctx, oracle, degree):
 def test_ordered_requests(gp, ctx, oracle, n, hubs, weight):
     """Leaves that ask for few receivers: from a handful to far more than one block orders."""
     check(gp, ctx, oracle, hubs_and_leaves(gp, n, hubs, n, weight), 8, 3)
+
+
+@pytest.mark.parametrize("n,hubs", [(60000, 5), (110000, 5), (150000, 6), (450000, 9)])
+def test_long_coarse_rows(gp, ctx, oracle, n, hubs):
+    check(gp, ctx, oracle, hubs_and_leaves(gp, n, hubs, n, 3), 4, 2)
 
 
 @pytest.mark.parametrize("n,degree", [(65535, 12), (65536, 6), (65536, 12), (70001, 40)])
