@@ -153,6 +153,31 @@ inline void launch_cluster(void (*kernel)(Params...), int blocks, int threads, s
     if (timed) g_profiler->after(stream);
 }
 
+// Whether the current device has room for a cluster of `blocks` such blocks (a
+// slice of a GPU may not).
+template <class K>
+inline bool cluster_fits(K kernel, int blocks, int threads, size_t smem) {
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(static_cast<unsigned>(blocks));
+    config.blockDim = dim3(static_cast<unsigned>(threads));
+    config.dynamicSmemBytes = smem;
+    cudaLaunchAttribute shape{};
+    shape.id = cudaLaunchAttributeClusterDimension;
+    shape.val.clusterDim.x = static_cast<unsigned>(blocks);
+    shape.val.clusterDim.y = 1;
+    shape.val.clusterDim.z = 1;
+    config.attrs = &shape;
+    config.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return clusters > 0;
+}
+
 inline int blocks_for(i64 items, int per_block) {
     const i64 b = (items + per_block - 1) / per_block;
     return static_cast<int>(b < 1 ? 1 : b);

@@ -103,6 +103,9 @@ struct Context {
     u64* dev_scalars = nullptr;
     u64* host_scalars = nullptr;  // pinned: kScalars words and the number of the last fetch
     u64 fetched = 0;
+    // Whether the device has room for the refinement's cluster; asked once per
+    // context (-1: not yet).
+    int refine_clusters = -1;
     cudaEvent_t ev[8] = {};
     // Kept host copies (GP_FLAG_KEEP_HIERARCHY).
     struct HostLevel {

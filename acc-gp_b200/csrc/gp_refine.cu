@@ -3711,6 +3711,11 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known, u64 known_load) {
     // (No level this small goes without a cache.)
     in_cluster = std::is_same_v<T, u32> && !verify && n <= kClusterVertices && n * k <= kClusterCells &&
                  g.m <= kClusterEntries && g.m <= kClusterRow * n;
+    if (in_cluster) {
+        if (ctx.refine_clusters < 0)
+            ctx.refine_clusters = cluster_fits(k_refine_cluster<u32>, kClusterBlocks, kClusterThreads, cluster_smem<u32>());
+        in_cluster = ctx.refine_clusters == 1;
+    }
     const int heavy_min = n <= 65536 ? mapping.refine_heavy_small
                           : n <= (1 << 20) ? mapping.refine_heavy_mid : mapping.refine_heavy_large;
     if (!in_cluster && heavy_min != g.heavy_min && (g.maximum_degree > static_cast<u64>(std::min(heavy_min, g.heavy_min)) || g.heavy_count))
