@@ -2385,6 +2385,7 @@ using MoveSort = PartSort<2, kPartMoves>;  // MoveOrder's other words are zero
 __global__ void __launch_bounds__(kPartSortThreads) k_sort_fragments(int k, const JointMove* in,
                                                                     const unsigned char* in_part, JointMove* out,
                                                                     JointParts* parts) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char part_smem[];
     __shared__ int s_offset[kMaxParts + 1];
     __shared__ u32 s_scan[33];
@@ -2748,6 +2749,7 @@ __global__ void __launch_bounds__(kThreads) k_combine(int k, JointCounts* counts
 // vertices for its place in the order.
 __global__ void __launch_bounds__(kPartSortThreads) k_sort_moves(int k, const JointMove* in, const unsigned char* in_part,
                                                                 JointMove* out, const JointParts* parts, int* claims) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char part_smem[];
     __shared__ int s_offset[kMaxParts + 1];
     MoveSort& sm = *reinterpret_cast<MoveSort*>(part_smem);
