@@ -47,3 +47,12 @@ def test_repair_without_a_cache(gp, ctx, oracle):
     g = gp.mesh3d(50, 45, 41, weighted=True, seed=3)
     for extra in (300, 20000):
         check(gp, ctx, oracle, g, overloaded(g.n, 100, extra, 1), 100, 1.05, 4)
+
+
+@pytest.mark.parametrize("n,degree,k,vw_max,eps", [
+    (3000, 0, 3, 200, 1.03), (3000, 0, 33, 200, 1.05), (3000, 2, 128, 12, 1.20), (40000, 1, 128, 200, 1.03),
+    (70000, 0, 128, 3000, 1.01), (70000, 2, 32, 3000, 1.002)])
+def test_tickets_over_parts_that_fit(gp, ctx, oracle, n, degree, k, vw_max, eps):
+    """Donors without a neighbour elsewhere, many heavier than the room of some or of all parts."""
+    g = random_graph(gp, n, degree, n + k, 3, vw_max)
+    check(gp, ctx, oracle, g, overloaded(n, k, n // 5, k), k, eps, 6)
