@@ -1464,8 +1464,8 @@ __global__ void __launch_bounds__(Threads, 1024 / Threads) k_sort_rows_big(const
 // bits (a counter is then zero exactly when its target is absent).  The row is
 // read once per segment, mostly from L2, so this pays while there are few
 // segments: 4 bytes an entry and segment against 96 for the global sort's four
-// passes.  R-MAT scale 22 at k = 64 went from 124.3 to about 118 ms (1.11x to
-// 1.18x of one start).
+// passes.  R-MAT scale 22 at k = 64 went from 124.3 to
+// 118 ms.
 constexpr int kDenseThreads = 1024;
 constexpr int kDenseSegment = 49152;      // u32 counters: 192 KB
 constexpr int kDenseSegments = 16;        // more: the global sort
