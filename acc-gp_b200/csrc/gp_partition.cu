@@ -1,6 +1,6 @@
 // C ABI and pipeline driver: upload -> coarsen -> METIS -> uncoarsen -> labels
 // (the sequence app/partition_main.cu:99-137 runs), on one CUDA stream.
-#include "gp_graph.h"
+#include "gp_hierarchy_cache.h"
 #include "gp_metis.h"
 #include "gp_primitives.cuh"
 
@@ -12,12 +12,10 @@
 #include <cstdio>
 #include <cstring>
 #include <limits>
-#include <map>
 #include <memory>
 #include <mutex>
 #include <numeric>
 #include <string>
-#include <tuple>
 
 struct gp_context {
     gp::Context ctx;
@@ -284,83 +282,6 @@ void publish(cudaStream_t stream, const u64* from, u64* to, int words, u64* flag
     launch(k_publish, 1, 128, 0, stream, from, to, words, flag, sequence);
 }
 
-// Kept hierarchies of resident graphs (see gp_internal.h).  An entry owns the
-// arena its levels live in; entries in use by a call are never dropped.
-struct HierarchyCache {
-    struct Key {
-        uint64_t graph;
-        int k;
-        uint32_t seed, flags;
-        bool operator<(const Key& o) const {
-            return std::tie(graph, k, seed, flags) < std::tie(o.graph, o.k, o.seed, o.flags);
-        }
-    };
-    struct Entry {
-        Arena storage;
-        Hierarchy h;
-        u64 total = 0, directed = 0;
-        int users = 0;
-        u64 last_use = 0;
-    };
-    int device = 0;
-    uint64_t budget = 0;
-    std::mutex mu;
-    std::map<Key, std::unique_ptr<Entry>> entries;
-    u64 clock = 0;
-
-    Entry* find(const Key& key) {
-        std::lock_guard<std::mutex> lock(mu);
-        auto it = entries.find(key);
-        if (it == entries.end()) return nullptr;
-        ++it->second->users;
-        it->second->last_use = ++clock;
-        return it->second.get();
-    }
-    // Keeps a complete `fresh` entry, in use by the caller, and drops least
-    // recently used idle entries while the total exceeds the budget.  When
-    // another call kept the same key first, `fresh` is still the caller's
-    // and is freed at its release.  Returns the caller's entry.
-    Entry* insert(const Key& key, std::unique_ptr<Entry> fresh) {
-        std::lock_guard<std::mutex> lock(mu);
-        fresh->users = 1;
-        fresh->last_use = ++clock;
-        Entry* out = fresh.get();
-        if (entries.count(key)) retired.push_back(std::move(fresh));
-        else entries.emplace(key, std::move(fresh));
-        evict();
-        return out;
-    }
-    void release(Entry* e) {
-        std::lock_guard<std::mutex> lock(mu);
-        --e->users;
-        evict();
-        free_retired();
-    }
-    uint64_t bytes() const {
-        uint64_t b = 0;
-        for (auto& kv : entries) b += kv.second->storage.reserved();
-        return b;
-    }
-
-private:
-    std::vector<std::unique_ptr<Entry>> retired;  // duplicates, freed once idle
-    void evict() {
-        while (bytes() > budget) {
-            auto victim = entries.end();
-            for (auto it = entries.begin(); it != entries.end(); ++it)
-                if (!it->second->users && (victim == entries.end() || it->second->last_use < victim->second->last_use))
-                    victim = it;
-            if (victim == entries.end()) break;  // everything is in use
-            cudaSetDevice(device);
-            entries.erase(victim);
-        }
-    }
-    void free_retired() {
-        for (auto& e : retired) if (e && !e->users) { cudaSetDevice(device); e.reset(); }
-        retired.erase(std::remove(retired.begin(), retired.end(), nullptr), retired.end());
-    }
-};
-
 namespace {
 
 gp_status run(gp_context* handle, const gp_csr* in, bool device_input, int k, double eps, uint32_t seed,
@@ -391,7 +312,7 @@ gp_status run(gp_context* handle, const gp_csr* in, bool device_input, int k, do
         ~Release() { if (cache && entry) cache->release(entry); }
     } release{cache, kept};
     const HierarchyCache::Key key{graph_key, k, seed, flags & GP_FLAG_NO_SEED_MATCHING};
-    if (cache) kept = cache->find(key);
+    if (cache) kept = cache->find(key, s);
     Input input;
     const bool reused = kept != nullptr;
     // On a miss with a cache, the input's own arrays (unit vertex weights) and
@@ -448,7 +369,7 @@ gp_status run(gp_context* handle, const gp_csr* in, bool device_input, int k, do
         fresh->h = h;
         fresh->total = total;
         fresh->directed = directed;
-        kept = cache->insert(key, std::move(fresh));
+        kept = cache->insert(key, std::move(fresh), s);
     }
     GP_CUDA(cudaEventRecord(ctx.ev[2], s));
     if (flags & GP_FLAG_KEEP_HIERARCHY) keep_levels(ctx, h);

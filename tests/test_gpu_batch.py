@@ -160,3 +160,22 @@ def test_server_keeps_hierarchies(gp, ctx):
             labels, st, _, _ = server.wait(server.submit(gid, 32, eps, 5))
             assert st.hierarchy_reused == 0
         assert server.kept_bytes() == 0
+
+
+def test_server_shares_a_fresh_hierarchy(gp, ctx):
+    """Identical requests that arrive together at a fresh cache: whichever
+    finds the hierarchy that another one has just published refines the same
+    levels.  Long coarse rows leave the most work behind the last read-back."""
+    g = gp.rmat(17, 16, 0.57, 0.19, 0.19, 12)
+    with gp.Server(0, workers=8) as server:
+        server.keep_hierarchies(16 << 30)
+        gid = server.add_graph(g)
+        for seed in range(4):
+            alone = ctx.partition(g, 64, 1.03, seed)[0]
+            tickets = [server.submit(gid, 64, 1.03, seed) for _ in range(16)]
+            reused = 0
+            for ticket in tickets:
+                labels, st, _, _ = server.wait(ticket)
+                np.testing.assert_array_equal(labels, alone)
+                reused += st.hierarchy_reused
+            assert reused >= 8  # eight workers make their own at most
