@@ -93,10 +93,10 @@ __global__ void __launch_bounds__(256) k_level0_meta(i64 n, const int* off, cons
 __global__ void k_level0_meta_chunks(DGraph g, u64* bounds, u64* sc) {
     after_previous();
     const int c = blockIdx.x, v = g.chunk_row[c];
-    const int begin = g.off[v];
+    const EntryPos begin = g.off[v];
     u64 d = 0;
     u32 flags = 0;
-    for (int e = g.chunk_begin[c] + threadIdx.x; e < chunk_end(g, c, v); e += blockDim.x) {
+    for (EntryPos e = g.chunk_begin[c] + threadIdx.x; e < chunk_end(g, c, v); e += blockDim.x) {
         const u64 w = edge_w(g.ew, e);
         d += w;
         if (e > begin && g.nbr[e] <= g.nbr[e - 1]) flags |= 1u;
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(256) k_affinity_heavy_insert(DGraph g, const u
     if (!is_mover(p, v, src)) return;
     const int h = g.chunk_hidx[c];
     const u64 size = heavy_slots(g.off[v + 1] - g.off[v]);
-    hash_row(p, v, g.chunk_begin[c] + static_cast<int>(threadIdx.x), chunk_end(g, c, v), static_cast<int>(blockDim.x),
+    hash_row<Table, EntryPos>(p, v, g.chunk_begin[c] + threadIdx.x, chunk_end(g, c, v), static_cast<int>(blockDim.x),
              Table{keys + table_off[h], vals + table_off[h]}, size - 1);
 }
 // Also empties the slots it read, so the tables start the next round clean
@@ -1046,11 +1046,11 @@ __global__ void k_scatter(i64 n, const int* off, const int* nbr, const u32* ew, 
     const i64 v = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) / W;
     const int lane = threadIdx.x % W;
     if (v >= n) return;
-    const int begin = off[v], end = off[v + 1];
+    const EntryPos begin = off[v], end = off[v + 1];
     if (end - begin > kHeavyRow) return;
     const int c = map[v];
-    const int out = base[v] - begin;
-    for (int e0 = begin + lane; e0 < end; e0 += U * W) {
+    const EntryPos out = base[v] - begin;  // wraps; out + e does not
+    for (EntryPos e0 = begin + lane; e0 < end; e0 += U * W) {
         int u[U], t[U];
         u32 w[U];
 #pragma unroll
@@ -1076,9 +1076,9 @@ __global__ void k_scatter_chunks(DGraph g, const int* map, const int* base, int*
     constexpr int U = 8;
     const int ch = blockIdx.x, v = g.chunk_row[ch];
     const int c = map[v];
-    const int out = base[v] - g.off[v];
-    const int end = chunk_end(g, ch, v), stride = static_cast<int>(blockDim.x);
-    for (int e0 = g.chunk_begin[ch] + static_cast<int>(threadIdx.x); e0 < end; e0 += U * stride) {
+    const EntryPos out = base[v] - g.off[v];  // wraps; out + e does not
+    const EntryPos end = chunk_end(g, ch, v), stride = blockDim.x;
+    for (EntryPos e0 = g.chunk_begin[ch] + threadIdx.x; e0 < end; e0 += U * stride) {
         int u[U], t[U];
 #pragma unroll
         for (int j = 0; j < U; ++j) u[j] = e0 + j * stride < end ? g.nbr[e0 + j * stride] : 0;
@@ -1473,15 +1473,16 @@ constexpr size_t dense_smem(int targets) { return sizeof(u32) * static_cast<size
 // Zeroes the counters and adds the row's entries with targets in
 // [lo, lo + targets); every thread of the block.
 __device__ __forceinline__ void dense_count(u32* count, int targets, int lo, const int* raw_t, const u32* raw_w,
-                                            int begin, int degree) {
+                                            EntryPos begin, EntryPos degree) {
     constexpr int U = 4;
+    static_assert(U * kDenseThreads <= kEntryStep, "the step of the loop below");
     for (int i = threadIdx.x; i < targets; i += kDenseThreads) count[i] = 0;
     __syncthreads();
-    for (int e0 = threadIdx.x; e0 < degree; e0 += U * kDenseThreads) {
+    for (EntryPos e0 = threadIdx.x; e0 < degree; e0 += U * kDenseThreads) {
         int t[U];
 #pragma unroll
         for (int j = 0; j < U; ++j) {
-            const int e = e0 + j * kDenseThreads;
+            const EntryPos e = e0 + j * kDenseThreads;
             t[j] = e < degree ? raw_t[begin + e] - lo : -1;  // dropped entries (INT_MAX) lie past every segment
         }
 #pragma unroll
@@ -1676,9 +1677,10 @@ __global__ void k_copy_rows(i64 nc, const int* raw_off, const int* raw_t, const 
     const i64 c = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) / W;
     const int lane = threadIdx.x % W;
     if (c >= nc) return;
-    const int begin = off[c], end = off[c + 1], raw = raw_off[c];
+    const EntryPos begin = off[c], end = off[c + 1];
+    const int raw = raw_off[c];
     if (end - begin > kHeavyRow || raw_off[c + 1] - raw > raw_max) return;
-    for (int e0 = begin + lane; e0 < end; e0 += U * W) {
+    for (EntryPos e0 = begin + lane; e0 < end; e0 += U * W) {
         int t[U];
         u32 w[U];
 #pragma unroll
@@ -1700,9 +1702,9 @@ __global__ void k_copy_chunks(DGraph g, const int* raw_off, const int* raw_t, co
     constexpr int U = 8;
     const int ch = blockIdx.x, c = g.chunk_row[ch];
     if (raw_off[c + 1] - raw_off[c] > raw_max) return;
-    const int shift = raw_off[c] - g.off[c];
-    const int end = chunk_end(g, ch, c), stride = static_cast<int>(blockDim.x);
-    for (int e0 = g.chunk_begin[ch] + static_cast<int>(threadIdx.x); e0 < end; e0 += U * stride) {
+    const EntryPos shift = raw_off[c] - g.off[c];  // not negative: a row keeps at most its raw entries
+    const EntryPos end = chunk_end(g, ch, c), stride = blockDim.x;
+    for (EntryPos e0 = g.chunk_begin[ch] + threadIdx.x; e0 < end; e0 += U * stride) {
         int t[U];
         u32 w[U];
 #pragma unroll
@@ -1728,7 +1730,7 @@ __global__ void k_heavy_counts(i64 n, const int* off, int heavy_min, u64* sc) {
     u64 rows = 0, chunks = 0, entries = 0;
     if (v < n) {
         const int d = off[v + 1] - off[v];
-        if (d > heavy_min) { rows = 1; chunks = (d + kChunk - 1) / kChunk; entries = d; }
+        if (d > heavy_min) { rows = 1; chunks = row_pieces(d, kChunk); entries = d; }
     }
     block_atomic_add(sc, rows);
     block_atomic_add(sc + 1, chunks);
@@ -1742,7 +1744,7 @@ struct IsHeavyRow {
 struct ChunkCount {
     const int* heavy;
     const int* off;
-    __device__ int operator()(i64 h) const { return (off[heavy[h] + 1] - off[heavy[h]] + kChunk - 1) / kChunk; }
+    __device__ int operator()(i64 h) const { return row_pieces(off[heavy[h] + 1] - off[heavy[h]], kChunk); }
 };
 __global__ void k_emit_chunks(i64 count, const int* heavy, const int* off, const int* chunk_off, int* chunk_row,
                               int* chunk_hidx, int* chunk_begin) {
@@ -1750,7 +1752,7 @@ __global__ void k_emit_chunks(i64 count, const int* heavy, const int* off, const
     const i64 h = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (h >= count) return;
     const int v = heavy[h], d = off[v + 1] - off[v];
-    const int chunks = (d + kChunk - 1) / kChunk;
+    const int chunks = row_pieces(d, kChunk);
     for (int i = 0; i < chunks; ++i) {
         chunk_row[chunk_off[h] + i] = v;
         chunk_hidx[chunk_off[h] + i] = static_cast<int>(h);

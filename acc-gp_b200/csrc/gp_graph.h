@@ -10,6 +10,18 @@ namespace gp {
 
 constexpr int kInvalid = 0x7fffffff;  // SCLP_INVALID (src/coarsen.cu:292)
 
+// A position among a level's entries.  A level holds up to 2^31 - 1 of them and
+// a loop over a row's entries steps up to kEntryStep past the row's end, so
+// such a loop's index and bounds are unsigned: as int, the last steps of a row
+// that ends there would wrap to negative positions and read before the arrays.
+using EntryPos = u32;
+constexpr u32 kEntryStep = 4096;
+static_assert(0x7fffffffu + 2 * kEntryStep < 0xffffffffu, "a step past the last row does not wrap");
+// Pieces of `size` entries that a row of `degree` entries is cut into.
+__host__ __device__ __forceinline__ int row_pieces(int degree, int size) {
+    return static_cast<int>((static_cast<u32>(degree) + static_cast<u32>(size) - 1) / static_cast<u32>(size));
+}
+
 // A CSR level on the device (DeviceWeightedGraph, include/graph.hpp:148-171).
 // ew == nullptr means unit edge weights.  The three metadata fields follow
 // the reference's meaning exactly: maximum_degree is a bound (exact after an
@@ -43,9 +55,9 @@ struct DGraph {
 };
 
 // Chunk-parallel loop body helpers: the chunk's edge range.
-__device__ __forceinline__ int chunk_end(const DGraph& g, int chunk, int row) {
-    const int end = g.chunk_begin[chunk] + kChunk;
-    const int row_end = g.off[row + 1];
+__host__ __device__ __forceinline__ EntryPos chunk_end(const DGraph& g, int chunk, int row) {
+    const EntryPos end = static_cast<EntryPos>(g.chunk_begin[chunk]) + kChunk;
+    const EntryPos row_end = g.off[row + 1];
     return end < row_end ? end : row_end;
 }
 

@@ -33,7 +33,7 @@ __global__ void k_cut_chunks(DGraph g, const int* labels, u64* out) {
     const int c = blockIdx.x, v = g.chunk_row[c];
     const int p = labels[v];
     u64 local = 0;
-    for (int e = g.chunk_begin[c] + threadIdx.x; e < chunk_end(g, c, v); e += blockDim.x)
+    for (EntryPos e = g.chunk_begin[c] + threadIdx.x; e < chunk_end(g, c, v); e += blockDim.x)
         if (labels[g.nbr[e]] != p) local += edge_w(g.ew, e);
     block_atomic_add(out, local);
 }
@@ -47,7 +47,8 @@ __global__ void k_cut(i64 n, const int* off, const int* nbr, const u32* ew, cons
          v += (static_cast<i64>(gridDim.x) * blockDim.x) >> 5) {
         const int p = labels[v];
         if (off[v + 1] - off[v] > heavy_min) continue;  // k_cut_chunks
-        for (int e = off[v] + lane; e < off[v + 1]; e += 32)
+        const EntryPos end = off[v + 1];
+        for (EntryPos e = static_cast<EntryPos>(off[v]) + lane; e < end; e += 32)
             if (labels[nbr[e]] != p) local += edge_w(ew, e);
     }
     cut_sum.finish(warp_sum(local), out);
@@ -113,14 +114,14 @@ template <> struct AffinityVec<u64> { using V = ulonglong2; static constexpr int
 // `stride` lanes apart starting at `first`, four entries per lane at a time
 // so that four neighbour and four label loads are in flight together.
 template <class C>
-__device__ __forceinline__ void accumulate_row(const int* nbr, const u32* ew, const int* labels, int v, int first,
-                                               int end, int stride, C* hist) {
+__device__ __forceinline__ void accumulate_row(const int* nbr, const u32* ew, const int* labels, int v,
+                                               EntryPos first, EntryPos end, int stride, C* hist) {
     constexpr int kUnroll = 4;
-    for (int e0 = first; e0 < end; e0 += kUnroll * stride) {
+    for (EntryPos e0 = first; e0 < end; e0 += kUnroll * stride) {
         int u[kUnroll];
 #pragma unroll
         for (int j = 0; j < kUnroll; ++j) {
-            const int e = e0 + j * stride;
+            const EntryPos e = e0 + j * stride;
             u[j] = e < end ? nbr[e] : v;
         }
         int part[kUnroll];
@@ -164,8 +165,8 @@ __global__ void __launch_bounds__(kThreads) k_build(i64 n, const int* off, const
     for (i64 base = ((static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * G; base < n; base += warps * G) {
         const i64 v = base + gid;
         const bool valid = v < n;
-        const int begin = valid ? off[v] : 0, end = valid ? off[v + 1] : 0;
-        const int deg = end - begin;
+        const EntryPos begin = valid ? off[v] : 0, end = valid ? off[v + 1] : 0;
+        const int deg = static_cast<int>(end - begin);
         if constexpr (Vectorized) {
             for (int p0 = sub * N; p0 < k; p0 += W * N) *reinterpret_cast<typename AffinityVec<C>::V*>(hist + p0) = {};
         } else {
@@ -181,7 +182,7 @@ __global__ void __launch_bounds__(kThreads) k_build(i64 n, const int* off, const
              rest &= rest - 1) {
             const int leader = __ffs(rest) - 1;
             const int vv = static_cast<int>(base) + leader / W;
-            const int b = __shfl_sync(0xffffffffu, begin, leader), e_end = __shfl_sync(0xffffffffu, end, leader);
+            const EntryPos b = __shfl_sync(0xffffffffu, begin, leader), e_end = __shfl_sync(0xffffffffu, end, leader);
             C* h = warp_hist + (leader / W) * k;
             accumulate_row(nbr, ew, labels, vv, b + lane, e_end, 32, h);
         }
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(kThreads) k_build_long(i64 count, const int* r
         const int v = rows[i];
         for (int p = lane; p < k; p += 32) hist[p] = 0;
         __syncwarp();
-        accumulate_row(nbr, ew, labels, v, off[v] + lane, off[v + 1], 32, hist);
+        accumulate_row(nbr, ew, labels, v, static_cast<EntryPos>(off[v]) + lane, off[v + 1], 32, hist);
         __syncwarp();
         C total = 0;
         C* row = A + static_cast<i64>(v) * k;
@@ -306,7 +307,7 @@ __global__ void k_build_chunks(DGraph g, const int* labels, int k, C* A, C* tota
     const int c = blockIdx.x, v = g.chunk_row[c];
     for (int p = threadIdx.x; p < k; p += blockDim.x) hist[p] = 0;
     __syncthreads();
-    accumulate_row(g.nbr, g.ew, labels, v, g.chunk_begin[c] + static_cast<int>(threadIdx.x), chunk_end(g, c, v),
+    accumulate_row(g.nbr, g.ew, labels, v, g.chunk_begin[c] + threadIdx.x, chunk_end(g, c, v),
                    static_cast<int>(blockDim.x), hist);
     __syncthreads();
     C total = 0;
@@ -498,10 +499,10 @@ struct RowRegs {
     u64 w[D];
     u64 total;
     __device__ __forceinline__ void load(int v, const int* off, const int* nbr, const u32* ew, const int* labels) {
-        const int b = off[v], end = off[v + 1];
+        const int b = off[v], degree = off[v + 1] - b;
         int u[D];
 #pragma unroll
-        for (int j = 0; j < D; ++j) u[j] = b + j < end ? nbr[b + j] : v;
+        for (int j = 0; j < D; ++j) u[j] = j < degree ? nbr[b + j] : v;
         total = 0;
 #pragma unroll
         for (int j = 0; j < D; ++j) {
@@ -595,11 +596,11 @@ __global__ void __launch_bounds__(kThreads) k_proposals_od(LpParams q, const int
 // first, first + stride, ... < end: the moves of its higher-priority
 // neighbours.  Four entries per lane at a time: their neighbour ids first,
 // then every neighbour's target, gain and label, all in flight together.
-__device__ __forceinline__ long long filter_entries(const LpParams& q, int v, int s, int t, long long gain, int first,
-                                                    int end, int stride) {
+__device__ __forceinline__ long long filter_entries(const LpParams& q, int v, int s, int t, long long gain,
+                                                    EntryPos first, EntryPos end, int stride) {
     constexpr int U = 4;
     long long corr = 0;
-    for (int e0 = first; e0 < end; e0 += U * stride) {
+    for (EntryPos e0 = first; e0 < end; e0 += U * stride) {
         int u[U];
         u64 w[U];
 #pragma unroll
@@ -637,8 +638,8 @@ __global__ void __launch_bounds__(kThreads, 6) k_filter(LpParams q) {
          base += warps * G) {
         const i64 i = base + gid;
         const int v = i < count ? q.cand[i] : -1;
-        const int begin = v >= 0 ? q.off[v] : 0, end = v >= 0 ? q.off[v + 1] : 0;
-        const bool light = v >= 0 && end - begin <= q.heavy_min;  // heavier rows: k_filter_chunks / k_filter_finish
+        const EntryPos begin = v >= 0 ? q.off[v] : 0, end = v >= 0 ? q.off[v + 1] : 0;
+        const bool light = v >= 0 && static_cast<int>(end - begin) <= q.heavy_min;  // heavier rows: k_filter_chunks / k_filter_finish
         const int s = light ? q.labels[v] : 0, t = light ? q.targets[v] : 0;
         const long long gain = light ? q.gains[v] : 0;
         long long corr = light && end - begin <= kFilterShort ? filter_entries(q, v, s, t, gain, begin + sub, end, W) : 0;
@@ -646,8 +647,8 @@ __global__ void __launch_bounds__(kThreads, 6) k_filter(LpParams q) {
              rest &= rest - 1) {
             const int leader = __ffs(rest) - 1;
             const int vv = __shfl_sync(0xffffffffu, v, leader), ss = __shfl_sync(0xffffffffu, s, leader),
-                      tt = __shfl_sync(0xffffffffu, t, leader), b = __shfl_sync(0xffffffffu, begin, leader),
-                      e = __shfl_sync(0xffffffffu, end, leader);
+                      tt = __shfl_sync(0xffffffffu, t, leader);
+            const EntryPos b = __shfl_sync(0xffffffffu, begin, leader), e = __shfl_sync(0xffffffffu, end, leader);
             const long long gg = __shfl_sync(0xffffffffu, gain, leader);
             const long long c = warp_sum(filter_entries(q, vv, ss, tt, gg, b + lane, e, 32));
             if (lane == leader) corr += c;
@@ -677,10 +678,10 @@ __global__ void __launch_bounds__(kThreads) k_filter_od(LpParams q) {
         const int v = q.cand[i];
         const int s = q.labels[v], t = q.targets[v];
         const long long gain = q.gains[v];
-        const int b = q.off[v], end = q.off[v + 1];
+        const int b = q.off[v], degree = q.off[v + 1] - b;
         int u[D];
 #pragma unroll
-        for (int j = 0; j < D; ++j) u[j] = b + j < end ? q.nbr[b + j] : v;
+        for (int j = 0; j < D; ++j) u[j] = j < degree ? q.nbr[b + j] : v;
         long long corr = 0;
 #pragma unroll
         for (int j = 0; j < D; ++j) {
@@ -718,10 +719,10 @@ __global__ void __launch_bounds__(kThreads) k_update_od(i64 count, const int* mo
     for (i64 i = static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += static_cast<i64>(gridDim.x) * blockDim.x) {
         const int v = movers[i];
         const int s = labels[v], t = targets[v];
-        const int b = off[v], end = off[v + 1];
+        const int b = off[v], degree = off[v + 1] - b;
         int u[D];
 #pragma unroll
-        for (int j = 0; j < D; ++j) u[j] = b + j < end ? nbr[b + j] : v;
+        for (int j = 0; j < D; ++j) u[j] = j < degree ? nbr[b + j] : v;
         long long gain = 0;
 #pragma unroll
         for (int j = 0; j < D; ++j) {
@@ -766,7 +767,8 @@ __global__ void k_touch_rows(i64 count, const int* movers, const u64* live_count
         const int v = movers[i];
         if (lane == 0) touch(f, v);
         if (off[v + 1] - off[v] > heavy_min) continue;
-        for (int e = off[v] + lane; e < off[v + 1]; e += 32) touch(f, nbr[e]);
+        const EntryPos end = off[v + 1];
+        for (EntryPos e = static_cast<EntryPos>(off[v]) + lane; e < end; e += 32) touch(f, nbr[e]);
     }
 }
 // The chunks of heavy rows of a list (k_heavy_chunk_list) of movers, a block
@@ -776,7 +778,7 @@ __global__ void k_touch_chunks(DGraph g, const int* work, const u64* work_count,
     const i64 count = static_cast<i64>(*work_count);
     for (i64 w = blockIdx.x; w < count; w += gridDim.x) {
         const int c = work[w], v = g.chunk_row[c];
-        for (int e = g.chunk_begin[c] + threadIdx.x; e < chunk_end(g, c, v); e += blockDim.x) touch(f, g.nbr[e]);
+        for (EntryPos e = g.chunk_begin[c] + threadIdx.x; e < chunk_end(g, c, v); e += blockDim.x) touch(f, g.nbr[e]);
     }
 }
 
@@ -800,7 +802,7 @@ __global__ void k_heavy_chunk_list(i64 count, const int* list, const u64* live_c
             if (g.heavy[mid] < v) lo = mid + 1;
             else hi = mid;
         }
-        const int c0 = g.heavy_chunk0[lo], chunks = (d + kChunk - 1) / kChunk;
+        const int c0 = g.heavy_chunk0[lo], chunks = row_pieces(d, kChunk);
         const u64 base = atomicAdd(reinterpret_cast<unsigned long long*>(work_count), static_cast<unsigned long long>(chunks));
         for (int j = 0; j < chunks; ++j) work[base + static_cast<u64>(j)] = c0 + j;
     }
@@ -857,7 +859,7 @@ __global__ void k_filter_chunks(DGraph g, LpParams q, long long* corr_acc, const
         const int s = q.labels[v];
         const long long gain = q.gains[v];
         // q.nbr and q.ew are g's arrays: four entries per thread in flight.
-        long long corr = filter_entries(q, v, s, t, gain, g.chunk_begin[c] + static_cast<int>(threadIdx.x),
+        long long corr = filter_entries(q, v, s, t, gain, g.chunk_begin[c] + threadIdx.x,
                                         chunk_end(g, c, v), static_cast<int>(blockDim.x));
         corr = warp_sum(corr);
         if ((threadIdx.x & 31) == 0 && corr)
@@ -905,16 +907,16 @@ __global__ void k_state_init(i64 n, const int* labels, u32* state) {
 // neighbour, weight and state loads all issued before any is used.  An edge
 // whose both ends move is counted by its larger endpoint's partner rule.
 template <class C>
-__device__ __forceinline__ long long update_entries(int v, int s, int t, int first, int end, int stride, const int* nbr,
-                                                    const u32* ew, const u32* state, int k, C* A) {
+__device__ __forceinline__ long long update_entries(int v, int s, int t, EntryPos first, EntryPos end, int stride,
+                                                    const int* nbr, const u32* ew, const u32* state, int k, C* A) {
     constexpr int U = 4;
     long long gain = 0;
-    for (int e0 = first; e0 < end; e0 += U * stride) {
+    for (EntryPos e0 = first; e0 < end; e0 += U * stride) {
         int u[U];
         u32 w[U], st[U];
 #pragma unroll
         for (int j = 0; j < U; ++j) {
-            const int e = e0 + j * stride;
+            const EntryPos e = e0 + j * stride;
             u[j] = e < end ? nbr[e] : v;
             w[j] = e < end ? edge_w(ew, e) : 0u;
         }
@@ -972,8 +974,8 @@ __global__ void __launch_bounds__(kThreads, 6) k_update(i64 count, const int* mo
          base += warps * G) {
         const i64 i = base + gid;
         const int v = i < count ? movers[i] : -1;
-        const int begin = v >= 0 ? off[v] : 0, end = v >= 0 ? off[v + 1] : 0;
-        const bool light = v >= 0 && end - begin <= heavy_min;  // heavier rows: k_update_chunks
+        const EntryPos begin = v >= 0 ? off[v] : 0, end = v >= 0 ? off[v + 1] : 0;
+        const bool light = v >= 0 && static_cast<int>(end - begin) <= heavy_min;  // heavier rows: k_update_chunks
         if (work && sub == 0 && light) bytes += update_row_bytes<C>(end - begin, ew != nullptr, A != nullptr);
         const u32 sv = light ? state[v] : 0u;
         const int s = state_label(sv), t = static_cast<int>((sv >> 8) & 0xffu);
@@ -984,8 +986,8 @@ __global__ void __launch_bounds__(kThreads, 6) k_update(i64 count, const int* mo
              rest &= rest - 1) {
             const int leader = __ffs(rest) - 1;
             const int vv = __shfl_sync(0xffffffffu, v, leader), ss = __shfl_sync(0xffffffffu, s, leader),
-                      tt = __shfl_sync(0xffffffffu, t, leader), b = __shfl_sync(0xffffffffu, begin, leader),
-                      e = __shfl_sync(0xffffffffu, end, leader);
+                      tt = __shfl_sync(0xffffffffu, t, leader);
+            const EntryPos b = __shfl_sync(0xffffffffu, begin, leader), e = __shfl_sync(0xffffffffu, end, leader);
             const long long g = warp_sum(update_entries(vv, ss, tt, b + lane, e, 32, nbr, ew, state, k, A));
             if (lane == leader) gain += g;
         }
@@ -1022,7 +1024,7 @@ __global__ void k_update_chunks(DGraph g, const int* chunk_list, const u64* chun
             atomicAdd(reinterpret_cast<unsigned long long*>(work),
                       update_row_bytes<C>(chunk_end(g, c, v) - g.chunk_begin[c], g.ew != nullptr, true) - 8ULL);
         const int s = state_label(sv), t = static_cast<int>((sv >> 8) & 0xffu);
-        long long gain = update_entries(v, s, t, g.chunk_begin[c] + static_cast<int>(threadIdx.x), chunk_end(g, c, v),
+        long long gain = update_entries(v, s, t, g.chunk_begin[c] + threadIdx.x, chunk_end(g, c, v),
                                         static_cast<int>(blockDim.x), g.nbr, g.ew, state, k, A);
         gain = block_sum(gain);
         if (threadIdx.x == 0 && gain) {
@@ -2611,9 +2613,9 @@ __global__ void k_grow(int slots, int sw, const u64* seeds, const int* partner, 
             const bool reverse = origin < 0;
             if (reverse && counts[1]) continue;
             const int m = reverse ? -1 : members[origin];
-            const int begin = reverse ? 0 : off[m];
-            const int end = reverse ? sw : min(off[m + 1], begin + 128);
-            for (int e = begin + lane; e < end; e += 32) {
+            const EntryPos begin = reverse ? 0 : off[m];
+            const EntryPos end = reverse ? sw : min(static_cast<EntryPos>(off[m + 1]), begin + 128);
+            for (EntryPos e = begin + lane; e < end; e += 32) {
                 int u;
                 if (reverse) {
                     const u64 value = seeds[static_cast<i64>(target) * sw + e];
@@ -2652,7 +2654,8 @@ __global__ void k_grow(int slots, int sw, const u64* seeds, const int* partner, 
         if (chosen == INT_MAX) break;
         const int side = labels[chosen] == source ? 0 : 1;
         long long correction = 0;
-        for (int e = off[chosen] + lane; e < off[chosen + 1]; e += 32)
+        const EntryPos row_end = off[chosen + 1];
+        for (EntryPos e = static_cast<EntryPos>(off[chosen]) + lane; e < row_end; e += 32)
             for (int j = 0; j < size; ++j)
                 if (nbr[e] == members[j]) correction += (labels[members[j]] == labels[chosen] ? 2LL : -2LL) * edge_w(ew, e);
         correction = warp_sum(correction);
@@ -2739,9 +2742,9 @@ __device__ void combine_fragment(int i, int count, int unique_before, int unique
         for (int u = 0; u < x.size; ++u) {
             const int v = x.vertices[u];
             const int lv = labels[v];
-            const int end = off[v + 1];
+            const EntryPos end = off[v + 1];
             // Four entries per lane in flight.
-            for (int e0 = off[v] + lane; e0 < end; e0 += 4 * 32) {
+            for (EntryPos e0 = static_cast<EntryPos>(off[v]) + lane; e0 < end; e0 += 4 * 32) {
                 int w4[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) w4[j] = e0 + 32 * j < end ? nbr[e0 + 32 * j] : -1;
@@ -2841,11 +2844,11 @@ __global__ void __launch_bounds__(kThreads) k_settle(int k, JointMove* moves, Jo
             const int v = m.vertices[j];
             owners[v] = i;
             targets[v] = labels[v] == m.a ? m.b : m.a;
-            chunks += (off[v + 1] - off[v] + kEventChunk - 1) / kEventChunk;
+            chunks += row_pieces(off[v + 1] - off[v], kEventChunk);
         }
         u64 at = atomicAdd(&counts->work, static_cast<u64>(chunks));
         for (int j = 0; j < m.size; ++j) {
-            const int v = m.vertices[j], own = (off[v + 1] - off[v] + kEventChunk - 1) / kEventChunk;
+            const int v = m.vertices[j], own = row_pieces(off[v + 1] - off[v], kEventChunk);
             for (int c = 0; c < own; ++c)
                 work[at++] = (static_cast<u64>(i) << 32) | (static_cast<u64>(j) << 28) | static_cast<u64>(c);
         }
@@ -2861,10 +2864,10 @@ __global__ void k_events(const JointCounts* counts, const u64* work, const Joint
         const u64 item = work[w];
         const int i = static_cast<int>(item >> 32);
         const int ma = moves[i].a, mb = moves[i].b, v = moves[i].vertices[(item >> 28) & 7];
-        const int begin = off[v] + static_cast<int>(item & 0xfffffffULL) * kEventChunk;
-        const int end = min(off[v + 1], begin + kEventChunk);
+        const EntryPos begin = off[v] + static_cast<EntryPos>(item & 0xfffffffULL) * kEventChunk;
+        const EntryPos end = min(static_cast<EntryPos>(off[v + 1]), begin + kEventChunk);
         u64 own = 0;
-        for (int e = begin + lane; e < end; e += 32) {
+        for (EntryPos e = begin + lane; e < end; e += 32) {
             const int u = nbr[e], other = owners[u];
             if (u == v || (other != INT_MAX && v > u)) continue;
             if (other != INT_MAX && labels[u] != ma && labels[u] != mb) continue;

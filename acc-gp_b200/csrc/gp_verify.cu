@@ -19,7 +19,8 @@ __global__ void k_verify_csr(i64 n, const int* off, const int* nbr, const u32* e
     u64 bad = 0;
     for (i64 v = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; v < n;
          v += (static_cast<i64>(gridDim.x) * blockDim.x) >> 5) {
-        for (int e = off[v] + lane; e < off[v + 1]; e += 32) {
+        const EntryPos end = off[v + 1];
+        for (EntryPos e = static_cast<EntryPos>(off[v]) + lane; e < end; e += 32) {
             const int u = nbr[e];
             if (u == v && !allow_self_loops) bad |= 4;
             int lo = off[u], hi = off[u + 1];  // lower_bound of v in row u
@@ -66,7 +67,8 @@ __global__ void k_probe_cut(i64 n, const int* off, const int* nbr, const u32* ew
     for (i64 v = (static_cast<i64>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; v < n;
          v += (static_cast<i64>(gridDim.x) * blockDim.x) >> 5) {
         const int p = probe_label(map, static_cast<int>(v));
-        for (int e = off[v] + lane; e < off[v + 1]; e += 32)
+        const EntryPos end = off[v + 1];
+        for (EntryPos e = static_cast<EntryPos>(off[v]) + lane; e < end; e += 32)
             if (probe_label(map, nbr[e]) != p) cut += edge_w(ew, e);
     }
     block_atomic_add(out, cut);
