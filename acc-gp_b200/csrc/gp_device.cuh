@@ -73,6 +73,18 @@ inline unsigned long long* work_counter(K kernel) {
                ? g_profiler->device_bytes : nullptr;
 }
 
+// A launch that did not start (bad configuration, missing shared-memory
+// opt-in) must fail the call, not leave its results silently unwritten.
+// `started` is what the launch returned.  This library clears the error of
+// every failure it has handled where it handles it (GP_CUDA, the read-back's
+// query, the server's own allocations), so what is pending here belongs to this
+// launch or to an unhandled fault.
+inline void check_launch(cudaError_t started) {
+    const cudaError_t pending = cudaGetLastError();
+    if (started == cudaSuccess) started = pending;
+    if (started != cudaSuccess) ::gp::fail(GP_CUDA_ERROR, std::string("kernel launch: ") + cudaGetErrorString(started));
+}
+
 // Waits until the kernel before this one in the stream is complete and its
 // writes are visible.  The first statement of every kernel that launch()
 // starts: launch() lets a kernel's blocks be set up while the previous kernel
@@ -102,14 +114,7 @@ inline void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem
     dependent.val.programmaticStreamSerializationAllowed = 1;
     config.attrs = &dependent;
     config.numAttrs = 1;
-    // A launch that did not start (bad configuration, missing shared-memory
-    // opt-in) must fail the call, not leave its results silently unwritten.
-    // This library clears the error of every failure it has handled where it
-    // handles it (GP_CUDA, the server's own allocations), so what is pending
-    // here belongs to this launch or to an unhandled fault.
-    cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
-    if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess)
-        ::gp::fail(GP_CUDA_ERROR, std::string("kernel launch: ") + cudaGetErrorString(e));
+    check_launch(cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...));
     if (timed) g_profiler->after(stream);
 }
 
@@ -123,8 +128,7 @@ inline void launch_ordinary(void (*kernel)(Params...), dim3 grid, dim3 block, si
     if (g_profiler) g_profiler->last_timed = timed;
     if (timed) g_profiler->before(stream);
     kernel<<<grid, block, smem, stream>>>(static_cast<Params>(args)...);
-    if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess)
-        ::gp::fail(GP_CUDA_ERROR, std::string("kernel launch: ") + cudaGetErrorString(e));
+    check_launch(cudaSuccess);
     if (timed) g_profiler->after(stream);
 }
 

@@ -142,6 +142,7 @@ struct Context {
             const cudaError_t e = cudaStreamQuery(stream);
             if (e == cudaSuccess) break;  // complete: the words are there
             if (e != cudaErrorNotReady) GP_CUDA(e);
+            cudaGetLastError();  // an answer, not a failure: a launch check must not report it
             std::this_thread::yield();
         }
         std::atomic_thread_fence(std::memory_order_acquire);

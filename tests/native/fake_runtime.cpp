@@ -1,12 +1,17 @@
 #include "fake_runtime.h"
 
 std::vector<Call> calls;
+Runtime runtime;
 
 extern "C" {
 cudaError_t cudaMalloc(void** p, size_t bytes) { *p = std::malloc(bytes); return cudaSuccess; }
 cudaError_t cudaFree(void* p) { std::free(p); return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+    const cudaError_t e = runtime.last;
+    runtime.last = cudaSuccess;
+    return e;
+}
 const char* cudaGetErrorString(cudaError_t) { return "error"; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
     *e = static_cast<cudaEvent_t>(std::malloc(1));
@@ -17,6 +22,14 @@ cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { calls.push_back({"r
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) {
     calls.push_back({"wait", s, e});
     return cudaSuccess;
+}
+cudaError_t cudaStreamQuery(cudaStream_t s) {
+    calls.push_back({"query", s, nullptr});
+    return runtime.last = runtime.query();
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* kernel, void**) {
+    calls.push_back({"launch", c->stream, kernel});
+    return runtime.launch;
 }
 }
 

@@ -6,6 +6,7 @@
 
 #include <cstdio>
 #include <cstdlib>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -15,6 +16,14 @@ struct Call {
     const void* object;
 };
 extern std::vector<Call> calls;
+
+// What the calls return.
+struct Runtime {
+    cudaError_t last = cudaSuccess;         // the thread's last error
+    cudaError_t launch = cudaSuccess;       // of a kernel launch (not noted as the last error)
+    std::function<cudaError_t()> query;     // of cudaStreamQuery (noted as the last error)
+};
+extern Runtime runtime;
 
 #define EXPECT(x)                                                              \
     do {                                                                       \
