@@ -133,20 +133,42 @@ struct Context {
     // a kernel writes them to the pinned memory, then the call's number behind
     // them, for which the host polls (11 us a round trip against 15 us of a
     // copy and a stream synchronisation, and a V-cycle makes 100-500 of them).
-    // The stream is asked now and then, so a failed kernel ends the wait.
     const u64* fetch(const u64* from, int words, int at = 0) {
         publish(stream, from, host_scalars + at, words, host_scalars + kScalars, ++fetched);
+        wait_fetched();
+        std::atomic_thread_fence(std::memory_order_acquire);
+        return host_scalars + at;
+    }
+    // Waits the way the program chose for this device (cudaSetDeviceFlags), as
+    // a stream synchronisation does: a program that blocks gets its core back.
+    // Polling gives the core to another thread that wants it every microsecond
+    // or two (batch workers share the cores with each other's METIS steps),
+    // and asks the stream now and then, so a failed kernel ends the wait.
+    void wait_fetched() {
+        unsigned how = 0;
+        GP_CUDA(cudaGetDeviceFlags(&how));
+        how &= cudaDeviceScheduleMask;
+        if (how == cudaDeviceScheduleBlockingSync) {
+            GP_CUDA(cudaStreamSynchronize(stream));
+            return;
+        }
+        const unsigned pauses = how == cudaDeviceScheduleYield ? 1 : how == cudaDeviceScheduleSpin ? kQueryPolls : 32;
         const volatile u64* flag = host_scalars + kScalars;
-        for (unsigned spins = 1; *flag != fetched; ++spins) {
-            if (spins % 4096) continue;
+        for (unsigned polls = 1; *flag != fetched; ++polls) {
+            cpu_pause();
+            if (polls % pauses == 0) std::this_thread::yield();
+            if (polls % kQueryPolls) continue;
             const cudaError_t e = cudaStreamQuery(stream);
             if (e == cudaSuccess) break;  // complete: the words are there
             if (e != cudaErrorNotReady) GP_CUDA(e);
             cudaGetLastError();  // an answer, not a failure: a launch check must not report it
-            std::this_thread::yield();
         }
-        std::atomic_thread_fence(std::memory_order_acquire);
-        return host_scalars + at;
+    }
+    static constexpr unsigned kQueryPolls = 2048;
+    static void cpu_pause() {
+#if defined(__x86_64__)
+        __builtin_ia32_pause();
+#endif
     }
     const u64* read_scalars(int count) { return fetch(dev_scalars, count); }
     void clear_scalars(int count) {

@@ -27,6 +27,11 @@ cudaError_t cudaStreamQuery(cudaStream_t s) {
     calls.push_back({"query", s, nullptr});
     return runtime.last = runtime.query();
 }
+cudaError_t cudaGetDeviceFlags(unsigned* flags) { *flags = runtime.flags; return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+    calls.push_back({"synchronize", s, nullptr});
+    return runtime.synchronize;
+}
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* kernel, void**) {
     calls.push_back({"launch", c->stream, kernel});
     return runtime.launch;

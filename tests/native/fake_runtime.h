@@ -21,6 +21,8 @@ extern std::vector<Call> calls;
 struct Runtime {
     cudaError_t last = cudaSuccess;         // the thread's last error
     cudaError_t launch = cudaSuccess;       // of a kernel launch (not noted as the last error)
+    cudaError_t synchronize = cudaSuccess;  // of cudaStreamSynchronize
+    unsigned flags = cudaDeviceScheduleAuto | cudaDeviceMapHost;
     std::function<cudaError_t()> query;     // of cudaStreamQuery (noted as the last error)
 };
 extern Runtime runtime;

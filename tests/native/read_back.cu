@@ -1,5 +1,6 @@
 // A read-back that has to wait leaves no error behind, a failed stream ends
-// it, and a kernel that did not start fails its launch.
+// it, it blocks where the program chose so, and a kernel that did not start
+// fails its launch.
 #include "../../acc-gp_b200/csrc/gp_graph.h"
 #include "fake_runtime.h"
 
@@ -50,6 +51,19 @@ int main() {
     // A failed stream ends the wait.
     runtime.query = [] { return cudaErrorLaunchFailure; };
     EXPECT(throws([&] { ctx.fetch(nullptr, 1); }) && runtime.last == cudaSuccess);
+
+    // A program that chose to block: no polling, and errors as before.
+    for (unsigned how : {cudaDeviceScheduleSpin, cudaDeviceScheduleYield, cudaDeviceScheduleBlockingSync}) {
+        runtime.flags = how | cudaDeviceMapHost;
+        runtime.query = [&] { arrive(); return cudaErrorNotReady; };
+        calls.clear();
+        EXPECT(!throws([&] { ctx.fetch(nullptr, 1); }));
+        EXPECT(calls.size() == 2 && calls[0].name == "publish" && calls[1].stream == stream(3));
+        EXPECT(calls[1].name == (how == cudaDeviceScheduleBlockingSync ? "synchronize" : "query"));
+    }
+    runtime.synchronize = cudaErrorLaunchFailure;
+    EXPECT(throws([&] { ctx.fetch(nullptr, 1); }));
+    runtime.flags = cudaDeviceScheduleAuto;
 
     // A launch that returns an error fails, whether or not the runtime keeps it as the last one.
     runtime.launch = cudaErrorInvalidConfiguration;
