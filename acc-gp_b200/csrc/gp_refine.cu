@@ -3498,7 +3498,8 @@ void LevelRefiner<T>::reserve_long(i64 listed, u64* list, const u32* plan, const
 
 // The initial repair and the label-propagation rounds by k_refine_cluster.
 // The host only steps in where a repair lists more donors than one block
-// orders, and starts the kernel again after it.
+// orders (and, with GP_FLAG_VERIFY, to check every batch), and starts the
+// kernel again after it.
 template <class T>
 void LevelRefiner<T>::refine_in_cluster(double filter, LevelResult& res, int& rounds, bool& restored) {
     if constexpr (std::is_same_v<T, u32>) {
@@ -3513,6 +3514,7 @@ void LevelRefiner<T>::refine_in_cluster(double filter, LevelResult& res, int& ro
         L.max_rounds = budget.rounds;
         L.heavy_min = mapping.refine_heavy_small;
         L.region = region;
+        L.check = verify;
         L.capacity = C;
         L.filter = filter;
         L.off = g.off;
@@ -3565,6 +3567,10 @@ void LevelRefiner<T>::refine_in_cluster(double filter, LevelResult& res, int& ro
             cut = st.loop.cut;
             const int status = st.loop.status;
             if (status == kClusterCutUnderflow) fail(GP_INTERNAL, "incremental cut underflow");
+            if (status == kClusterCheck) {
+                check_state("incremental cut differs from CSR scan");
+                continue;
+            }
             if (status != kClusterHostInitialRepair && status != kClusterHostRoundRepair) break;
             // A long repair, completed step by step.  Its statistics go to
             // `stats`, the kernel's own are added at the end.
@@ -3763,7 +3769,7 @@ LevelResult LevelRefiner<T>::run(bool has_known, u64 known, u64 known_load) {
     // the block-per-chunk kernels instead of one warp each, which otherwise
     // set the time of every row-parallel pass of the level.
     // (No level this small goes without a cache.)
-    in_cluster = std::is_same_v<T, u32> && !verify && n <= kClusterVertices && n * k <= kClusterCells &&
+    in_cluster = std::is_same_v<T, u32> && n <= kClusterVertices && n * k <= kClusterCells &&
                  g.m <= kClusterEntries && g.m <= kClusterRow * n;
     if (in_cluster) {
         if (ctx.refine_clusters < 0)

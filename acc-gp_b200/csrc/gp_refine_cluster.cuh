@@ -21,13 +21,21 @@ constexpr int kClusterHeavyCap = 512;  // rows a block sets aside for all its th
 
 // Loop state of a level, in global memory: where the kernel starts, and what
 // it found.
-enum ClusterStart : int { kStartLevel = 0, kStartAfterInitialRepair = 1, kStartAfterRoundRepair = 2 };
+enum ClusterStart : int {
+    kStartLevel = 0,
+    kStartAfterInitialRepair = 1,
+    kStartAfterRoundRepair = 2,
+    kStartInInitialRepair = 3,  // its next iteration
+    kStartAfterPropagation = 4, // a round's label propagation is applied
+    kStartInRoundRepair = 5,
+};
 enum ClusterStatus : int {
     kClusterDone = 0,
     kClusterInitialRepairFailed = 1,
     kClusterHostInitialRepair = 2,  // more listed donors than one block takes: the host
     kClusterHostRoundRepair = 3,    // completes this repair and starts the kernel again
     kClusterCutUnderflow = 4,
+    kClusterCheck = 5,  // GP_FLAG_VERIFY: the host checks the batch just applied and starts the kernel again
 };
 struct ClusterLoop {
     u64 cut, best, feasible_start;
@@ -42,13 +50,14 @@ struct ClusterState {
     ClusterLoop loop;
     ClusterTotals totals;
     u64 max_load;
-    u64 listed, iterations;  // of an interrupted repair
+    u64 listed, iterations;  // of a repair that the host completes or checks
 };
 
 template <class C>
 struct ClusterLevel {
     i64 n;
     int k, max_rounds, heavy_min, region;  // region: list entries of one block
+    bool check;  // stop after every batch (kClusterCheck)
     u64 capacity;
     double filter;
     const int* off;
@@ -125,31 +134,32 @@ public:
         if (threadIdx.x == 0) sm.totals = L.io->totals;
         st = L.io->loop;
         const int begin = st.start;
+        iterations = static_cast<int>(L.io->iterations);
         refresh_loads();
-        bool feasible = true;
+        bool feasible = max_load <= L.capacity;
         st.status = kClusterDone;
-        if (begin == kStartLevel) {
-            if (max_load > L.capacity) {
-                feasible = repair();
-                if (st.status == kClusterHostRoundRepair) {
-                    st.status = kClusterHostInitialRepair;
-                    return finish();
-                }
+        // Steps of the first round that are done already: none, the
+        // propagation, some of the repair, the repair.
+        const int done = begin == kStartAfterPropagation ? 1 : begin == kStartInRoundRepair ? 2
+                         : begin == kStartAfterRoundRepair ? 3 : 0;
+        if (!done) {
+            if (begin != kStartAfterInitialRepair && !feasible) {
+                feasible = repair(begin == kStartInInitialRepair);
+                if (st.status == kClusterHostRoundRepair) st.status = kClusterHostInitialRepair;
+                if (st.status == kClusterCheck) return stop(kStartInInitialRepair);
                 if (st.status != kClusterDone) return finish();
-                if (!feasible) {
-                    st.status = kClusterInitialRepairFailed;
-                    return finish();
-                }
+                if (L.check) return stop(kStartAfterInitialRepair);
             }
-        }
-        if (begin != kStartAfterRoundRepair) {
+            if (!feasible) {
+                st.status = kClusterInitialRepairFailed;
+                return finish();
+            }
             st.feasible_start = st.best = st.cut;
             st.moved = 0;
             save();
         }
-        bool resumed = begin == kStartAfterRoundRepair;
-        while (resumed || (st.rounds < L.max_rounds && st.stale < 3)) {
-            if (!resumed) {
+        for (int skip = done; skip || (st.rounds < L.max_rounds && st.stale < 3); skip = 0) {
+            if (skip < 1) {
                 ++st.rounds;
                 const u64 count = lp_round();
                 if (st.status != kClusterDone) return finish();
@@ -159,10 +169,15 @@ public:
                     continue;
                 }
                 st.empty = 0;
-                feasible = max_load <= L.capacity || repair();
-                if (st.status != kClusterDone) return finish();
+                feasible = max_load <= L.capacity;
+                if (L.check) return stop(kStartAfterPropagation);
             }
-            resumed = false;
+            if (skip < 3 && !feasible) {
+                feasible = repair(skip == 2);
+                if (st.status == kClusterCheck) return stop(kStartInRoundRepair);
+                if (st.status != kClusterDone) return finish();
+                if (L.check) return stop(kStartAfterRoundRepair);
+            }
             if (!feasible) break;
             if (L.samples) {
                 for (int p = threadIdx.x; p < L.k; p += kClusterThreads) {
@@ -201,6 +216,11 @@ private:
         // Set batch + 2 was last used two batches ago, before at least two
         // barriers that every block has passed.
         if (rank == 0 && threadIdx.x < kCtlWords) counters(batch + 2)[threadIdx.x] = 0;
+    }
+    __device__ void stop(int start) {
+        st.status = kClusterCheck;
+        st.start = start;
+        finish();
     }
     // Ends the launch: a finished level goes back to its best labels (the
     // cache does not), and the state to global memory.
@@ -557,9 +577,10 @@ private:
 
     // One capacity repair (the iterations of LevelRefiner::repair); whether
     // the parts fit at its end.  With more listed donors than one block
-    // orders, leaves st.status at kClusterHostRoundRepair.
-    __device__ bool repair() {
-        iterations = 0;
+    // orders, leaves st.status at kClusterHostRoundRepair; between checked
+    // iterations, at kClusterCheck.
+    __device__ bool repair(bool resumed) {
+        if (!resumed) iterations = 0;
         while (true) {
             next_batch();
             u64* ctl = counters(batch);
@@ -598,6 +619,10 @@ private:
             ++iterations;
             const bool feasible = max_load <= L.capacity;
             if (feasible || placed == 0 || iterations >= 2 * L.k + 4) return feasible;
+            if (L.check) {
+                st.status = kClusterCheck;
+                return false;
+            }
         }
     }
     // k_slack: free room per part, its saturating prefix sums and the least

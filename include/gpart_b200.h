@@ -83,7 +83,7 @@ typedef struct gp_stats {
 } gp_stats;
 
 /* Flags for gp_partition / gp_partition_device. */
-#define GP_FLAG_VERIFY           0x1u /* the reference's --verify invariants, on host copies */
+#define GP_FLAG_VERIFY           0x1u /* the reference's --verify invariants, checked on the device */
 #define GP_FLAG_KEEP_HIERARCHY   0x2u /* keep host copies of every level for gp_level_*     */
 #define GP_FLAG_NO_SEED_MATCHING 0x4u /* GPART_HEM_COARSEN=0 (app/partition_main.cu:57)    */
 #define GP_FLAG_QUIET            0x8u /* no per-level key=value log lines on stdout        */

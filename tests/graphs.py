@@ -1,4 +1,6 @@
 """Small symmetric graphs for the size tests, from edge lists."""
+import contextlib
+
 import numpy as np
 
 
@@ -33,3 +35,14 @@ def hubs_and_leaves(gp, n, hubs, seed, max_weight=0):
     u = np.concatenate([leaf, leaf, rng.integers(0, n, n)])
     v = np.concatenate([rng.integers(0, hubs, n), rng.integers(0, hubs, n), rng.integers(0, n, n)])
     return symmetric(gp, n, u, v, None, seed, max_weight)
+
+
+@contextlib.contextmanager
+def launches_of(ctx, kernel):
+    """A list that holds, after the block, how often kernels of this name were started by the context's calls in it."""
+    count = []
+    ctx.profile_begin(kernel)
+    try:
+        yield count
+    finally:
+        count.append(ctx.profile_end()[0])
