@@ -384,7 +384,11 @@ extern "C" gp_status gp_server_add_graph(gp_server* server, const gp_csr* graph,
              upload(reinterpret_cast<void**>(&a.off), graph->offsets, sizeof(int32_t) * (g.n + 1)) &&
              upload(reinterpret_cast<void**>(&a.nbr), graph->neighbors, sizeof(int32_t) * g.m) &&
              upload(reinterpret_cast<void**>(&a.vw), graph->vertex_weights, sizeof(uint32_t) * g.n) &&
-             upload(reinterpret_cast<void**>(&a.ew), graph->edge_weights, sizeof(uint32_t) * g.m);
+             upload(reinterpret_cast<void**>(&a.ew), graph->edge_weights, sizeof(uint32_t) * g.m) &&
+             // A copy from pageable memory returns once the data is staged; the
+             // workers' streams do not wait for the default stream.
+             cudaStreamSynchronize(nullptr) == cudaSuccess;
+        if (!ok) cudaGetLastError();
         g.on.push_back(a);
         if (!ok) break;
     }

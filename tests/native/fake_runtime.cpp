@@ -27,6 +27,11 @@ cudaError_t cudaStreamQuery(cudaStream_t s) {
     calls.push_back({"query", s, nullptr});
     return runtime.last = runtime.query();
 }
+cudaError_t cudaGetDeviceCount(int* count) { *count = 2; return cudaSuccess; }
+cudaError_t cudaMemcpy(void* to, const void*, size_t, cudaMemcpyKind) {
+    calls.push_back({"copy", nullptr, to});
+    return cudaSuccess;
+}
 cudaError_t cudaGetDeviceFlags(unsigned* flags) { *flags = runtime.flags; return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) {
     calls.push_back({"synchronize", s, nullptr});

@@ -13,7 +13,7 @@ NVCC = os.path.join(CUDA, "bin", "nvcc")
 
 
 @pytest.mark.skipif(not os.path.exists(NVCC) or not shutil.which("g++"), reason="needs nvcc and g++")
-@pytest.mark.parametrize("program", ["hierarchy_cache", "entry_positions", "read_back"])
+@pytest.mark.parametrize("program", ["hierarchy_cache", "entry_positions", "read_back", "resident_graph"])
 def test_host_side(program, tmp_path):
     fake, out = str(tmp_path / "fake_runtime.o"), str(tmp_path / program)
     subprocess.run(["g++", "-std=c++17", "-I", os.path.join(CUDA, "include"), "-c",
