@@ -2463,6 +2463,7 @@ Hierarchy coarsen(Context& ctx, const DGraph& input, const CoarsenOptions& o) {
     return h;
 }
 
+// On the context's stream: the last level's kernels may still run on it.
 void keep_levels(Context& ctx, const Hierarchy& h) {
     ctx.kept.clear();
     for (size_t i = 0; i < h.levels.size(); ++i) {
@@ -2474,15 +2475,16 @@ void keep_levels(Context& ctx, const Hierarchy& h) {
         lv.nbr.resize(g.m);
         lv.ew.resize(g.m);
         lv.vw.resize(g.n);
-        GP_CUDA(cudaMemcpy(lv.off.data(), g.off, sizeof(int) * (g.n + 1), cudaMemcpyDeviceToHost));
-        if (g.m) GP_CUDA(cudaMemcpy(lv.nbr.data(), g.nbr, sizeof(int) * g.m, cudaMemcpyDeviceToHost));
-        if (g.ew) { if (g.m) GP_CUDA(cudaMemcpy(lv.ew.data(), g.ew, sizeof(u32) * g.m, cudaMemcpyDeviceToHost)); }
+        GP_CUDA(cudaMemcpyAsync(lv.off.data(), g.off, sizeof(int) * (g.n + 1), cudaMemcpyDeviceToHost, ctx.stream));
+        if (g.m) GP_CUDA(cudaMemcpyAsync(lv.nbr.data(), g.nbr, sizeof(int) * g.m, cudaMemcpyDeviceToHost, ctx.stream));
+        if (g.ew) { if (g.m) GP_CUDA(cudaMemcpyAsync(lv.ew.data(), g.ew, sizeof(u32) * g.m, cudaMemcpyDeviceToHost, ctx.stream)); }
         else std::fill(lv.ew.begin(), lv.ew.end(), 1u);
-        GP_CUDA(cudaMemcpy(lv.vw.data(), g.vw, sizeof(u32) * g.n, cudaMemcpyDeviceToHost));
+        GP_CUDA(cudaMemcpyAsync(lv.vw.data(), g.vw, sizeof(u32) * g.n, cudaMemcpyDeviceToHost, ctx.stream));
         if (i < h.maps.size()) {
             lv.map.resize(g.n);
-            GP_CUDA(cudaMemcpy(lv.map.data(), h.maps[i], sizeof(int) * g.n, cudaMemcpyDeviceToHost));
+            GP_CUDA(cudaMemcpyAsync(lv.map.data(), h.maps[i], sizeof(int) * g.n, cudaMemcpyDeviceToHost, ctx.stream));
         }
+        GP_CUDA(cudaStreamSynchronize(ctx.stream));
         lv.meta[0] = g.maximum_degree;
         lv.meta[1] = g.has_heavy_rows;
         lv.meta[2] = g.incident_bound;

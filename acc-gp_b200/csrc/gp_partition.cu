@@ -739,15 +739,15 @@ gp_status gp_autotune(gp_context* ctx, const gp_csr* graph, int32_t k, double ep
         GP_CUDA(cudaMalloc(&buf.p[0], sizeof(int) * (n + 1)));
         GP_CUDA(cudaMalloc(&buf.p[1], sizeof(int) * std::max<i64>(m, 1)));
         GP_CUDA(cudaMalloc(&buf.p[4], sizeof(int) * n));
-        GP_CUDA(cudaMemcpy(buf.p[0], graph->offsets, sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
-        if (m) GP_CUDA(cudaMemcpy(buf.p[1], graph->neighbors, sizeof(int) * m, cudaMemcpyHostToDevice));
+        GP_CUDA(cudaMemcpyAsync(buf.p[0], graph->offsets, sizeof(int) * (n + 1), cudaMemcpyHostToDevice, c.stream));
+        if (m) GP_CUDA(cudaMemcpyAsync(buf.p[1], graph->neighbors, sizeof(int) * m, cudaMemcpyHostToDevice, c.stream));
         if (graph->vertex_weights) {
             GP_CUDA(cudaMalloc(&buf.p[2], sizeof(u32) * n));
-            GP_CUDA(cudaMemcpy(buf.p[2], graph->vertex_weights, sizeof(u32) * n, cudaMemcpyHostToDevice));
+            GP_CUDA(cudaMemcpyAsync(buf.p[2], graph->vertex_weights, sizeof(u32) * n, cudaMemcpyHostToDevice, c.stream));
         }
         if (graph->edge_weights && m) {
             GP_CUDA(cudaMalloc(&buf.p[3], sizeof(u32) * m));
-            GP_CUDA(cudaMemcpy(buf.p[3], graph->edge_weights, sizeof(u32) * m, cudaMemcpyHostToDevice));
+            GP_CUDA(cudaMemcpyAsync(buf.p[3], graph->edge_weights, sizeof(u32) * m, cudaMemcpyHostToDevice, c.stream));
         }
         const gp_csr dg{n, m, static_cast<int*>(buf.p[0]), static_cast<int*>(buf.p[1]), static_cast<u32*>(buf.p[2]),
                         static_cast<u32*>(buf.p[3])};
@@ -761,7 +761,8 @@ gp_status gp_autotune(gp_context* ctx, const gp_csr* graph, int32_t k, double ep
                 gp_stats st{};
                 if (gp_status s = run(ctx, &dg, true, k, epsilon, seed, GP_FLAG_QUIET, labels_dev, nullptr, &st); s != GP_OK)
                     fail(s, last_error());
-                GP_CUDA(cudaMemcpy(labels.data(), labels_dev, sizeof(int) * n, cudaMemcpyDeviceToHost));
+                GP_CUDA(cudaMemcpyAsync(labels.data(), labels_dev, sizeof(int) * n, cudaMemcpyDeviceToHost, c.stream));
+                GP_CUDA(cudaStreamSynchronize(c.stream));
                 if (first && r == 0) { reference = labels; continue; }
                 if (labels != reference) fail(GP_INTERNAL, "mapping thresholds changed the partition");
                 best = std::min(best, st.algorithm_seconds * 1e3);
@@ -844,7 +845,7 @@ gp_status gp_profile_begin(gp_context* ctx, const char* kernel_substring) {
     return guarded([&]() -> gp_status {
         GP_CUDA(cudaSetDevice(ctx->ctx.device));
         if (!ctx->profiler.device_bytes) GP_CUDA(cudaMalloc(&ctx->profiler.device_bytes, sizeof(unsigned long long)));
-        GP_CUDA(cudaMemset(ctx->profiler.device_bytes, 0, sizeof(unsigned long long)));
+        GP_CUDA(cudaMemsetAsync(ctx->profiler.device_bytes, 0, sizeof(unsigned long long), ctx->ctx.stream));
         g_profiler = &ctx->profiler;
         return GP_OK;
     });
@@ -865,8 +866,10 @@ gp_status gp_profile_end(gp_context* ctx, uint64_t* launches, double* total_ms, 
         if (launches) *launches = p.used;
         if (total_ms) *total_ms = ms;
         unsigned long long device_bytes = 0;
-        if (p.device_bytes)
-            GP_CUDA(cudaMemcpy(&device_bytes, p.device_bytes, sizeof(device_bytes), cudaMemcpyDeviceToHost));
+        if (p.device_bytes) {
+            GP_CUDA(cudaMemcpyAsync(&device_bytes, p.device_bytes, sizeof(device_bytes), cudaMemcpyDeviceToHost, ctx->ctx.stream));
+            GP_CUDA(cudaStreamSynchronize(ctx->ctx.stream));
+        }
         if (algorithmic_bytes) *algorithmic_bytes = p.bytes + static_cast<double>(device_bytes);
         p.used = 0;
         p.bytes = 0;

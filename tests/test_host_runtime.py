@@ -1,5 +1,6 @@
 """What the library's host code asks of the CUDA runtime: programs of tests/native, linked with a recording stand-in."""
 import os
+import re
 import shutil
 import subprocess
 
@@ -22,3 +23,13 @@ def test_host_side(program, tmp_path):
                     "-cudart", "none", "-w", os.path.join(NATIVE, program + ".cu"), fake, "-o", out], check=True)
     done = subprocess.run([out], capture_output=True, text=True, timeout=60)
     assert done.returncode == 0, done.stdout + done.stderr
+
+
+def test_copies_are_ordered_with_the_contexts_stream():
+    """A context's stream does not wait for the default stream, nor the other way round, so copies and fills of a
+    context's data name its stream.  (The server's own copies wait for what they need, see resident_graph.cu.)"""
+    csrc = os.path.join(ROOT, "acc-gp_b200", "csrc")
+    for name in sorted(os.listdir(csrc)):
+        if name != "gp_batch.cpp":
+            text = open(os.path.join(csrc, name)).read()
+            assert not re.search(r"\bcuda(Memcpy|Memset)\(", text), name
