@@ -610,6 +610,11 @@ int gain_bucket(u64 best_conn, u64 current, u64 relief) {
 // Order key of the deterministic repair (bucket ranks and receiver tickets).
 inline u32 repair_hash(int32_t v) { return mix32(static_cast<u32>(v) ^ 0x85ebca6bU); }
 
+// What the exchange of the last refinement on this thread had to sort: the most
+// fragments (duplicates included) and moves of one part.
+struct ExchangeLists { u64 fragments = 0, moves = 0; };
+thread_local ExchangeLists g_lists;
+
 struct JointMove {  // exchange.cuh:9-13
     int vertices[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
     int size = 0, a = -1, b = -1, id = 0;
@@ -979,6 +984,7 @@ struct Refiner {
             // remove_if empty, sort by JointNetOrder, unique by canonical set
             std::vector<JointMove> frag;
             for (const auto& x : archive) if (x.size) frag.push_back(x);
+            note_lists(frag, g_lists.fragments);
             std::sort(frag.begin(), frag.end(), [](const JointMove& x, const JointMove& y) {
                 if (x.a != y.a) return x.a < y.a;
                 if (x.net != y.net) return x.net < y.net;
@@ -999,6 +1005,7 @@ struct Refiner {
             for (int i = 0; i < fragments; ++i) combine(frag, i, slots, &pool[static_cast<size_t>(slots)], gap);
             std::vector<JointMove> act;
             for (const auto& x : pool) if (x.size) act.push_back(x);
+            note_lists(act, g_lists.moves);
             if (act.empty()) { if (++empty >= 2) break; continue; }
             std::sort(act.begin(), act.end(), [](const JointMove& x, const JointMove& y) {
                 if (x.a != y.a) return x.a < y.a;
@@ -1083,6 +1090,11 @@ struct Refiner {
         return true;
     }
 
+    // The largest number of a part's moves in a list, kept in `most`.
+    void note_lists(const std::vector<JointMove>& list, u64& most) const {
+        std::vector<u64> count(static_cast<size_t>(k), 0);
+        for (const auto& x : list) most = std::max(most, ++count[static_cast<size_t>(x.a)]);
+    }
     // joint_grow (exchange.cuh:95-204), one slot.
     template <class Gap>
     void grow(int slot, int sw, const std::vector<u64>& seeds, const std::vector<int>& partner, JointMove& out,
@@ -1446,6 +1458,7 @@ int orc_refine(const orc_csr* in, int32_t k, double epsilon, int32_t max_rounds,
             if (lab[v] < 0 || lab[v] >= k) fail(1, "refinement partition has an invalid part id");
             loads[lab[v]] += g.vw[v];
         }
+        g_lists = ExchangeLists{};
         const LevelResult r = refine_level(g, k, epsilon, lab, loads, false, 0, max_rounds, exchange_rounds);
         if (stats) *stats = r.stats;
         if (r.repair_failed) fail(2, "initial refinement capacity repair failed");
@@ -1458,6 +1471,11 @@ int orc_refine(const orc_csr* in, int32_t k, double epsilon, int32_t max_rounds,
         g_error = e.what();
         return 5;
     }
+}
+
+void orc_exchange_lists(uint64_t* fragments, uint64_t* moves) {
+    *fragments = g_lists.fragments;
+    *moves = g_lists.moves;
 }
 
 const char* orc_last_error(void) { return g_error.c_str(); }

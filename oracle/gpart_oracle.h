@@ -56,6 +56,10 @@ typedef struct orc_refine_stats {
 int orc_refine(const orc_csr* graph, int32_t k, double epsilon, int32_t max_rounds,
                int32_t exchange_rounds, int32_t* labels, orc_refine_stats* stats);
 
+/* The most fragments (duplicates included) and moves of one part that an
+ * exchange pass of the last orc_refine on this thread had to sort. */
+void orc_exchange_lists(uint64_t* fragments, uint64_t* moves);
+
 /* Refined labels of every level (level order as in the hierarchy). */
 int orc_level_labels(int32_t level, int32_t* labels);
 /* Cut after refinement of a level, and whether that level was refined. */

@@ -83,6 +83,13 @@ def refine(graph, labels, k, epsilon=1.03, max_rounds=32, exchange_rounds=2):
     return out, {name: getattr(st, name) for name, _ in _RefineStats._fields_ if name != "reserved"}
 
 
+def exchange_lists():
+    """(fragments, moves): the most of one part in an exchange pass of the last refine()."""
+    fragments, moves = C.c_uint64(), C.c_uint64()
+    lib().orc_exchange_lists(C.byref(fragments), C.byref(moves))
+    return fragments.value, moves.value
+
+
 def levels():
     L = lib()
     out = []

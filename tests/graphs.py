@@ -37,6 +37,32 @@ def hubs_and_leaves(gp, n, hubs, seed, max_weight=0):
     return symmetric(gp, n, u, v, None, seed, max_weight)
 
 
+def stuck_pairs(gp, n, k, light_max, seed):
+    """A graph and labels whose first round cannot be repaired, which leaves everything to the exchange: every light
+    vertex (weight 1..light_max) is drawn to the other part of its pair (p, p ^ 1), and each part holds a heavy vertex
+    that is drawn there as well and does not fit.  Two strong edges a vertex across, three weak ones within the part."""
+    rng = np.random.default_rng(seed)
+    vertex = np.arange(n)
+    across, within = np.repeat(vertex, 2), np.repeat(vertex, 3)
+    there = rng.integers(0, n // k, len(across)) * k + (across % k ^ 1)
+    here = rng.integers(0, n // k, len(within)) * k + within % k
+    heavy = n + np.arange(k)
+    u, v = np.concatenate([across, within, heavy[0::2]]), np.concatenate([there, here, heavy[1::2]])
+    weight = np.concatenate([np.full(len(across), 9), np.full(len(within), 1), np.full(k // 2, 10**6)])
+    labels = np.concatenate([vertex % k, np.arange(k)]).astype(np.int32)
+    total = n + k
+    keep = u != v
+    key, first = np.unique(np.minimum(u, v)[keep] * total + np.maximum(u, v)[keep], return_index=True)
+    weight = weight[keep][first]
+    src, dst = np.concatenate([key // total, key % total]), np.concatenate([key % total, key // total])
+    order = np.argsort(src * total + dst, kind="stable")
+    off = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=total))]).astype(np.int32)
+    vw = np.concatenate([rng.integers(1, light_max + 1, n), np.zeros(k)]).astype(np.uint32)
+    loads = np.bincount(labels, weights=vw, minlength=k).astype(np.uint32)
+    vw[n:] = loads.max() * 5 // 2 - loads
+    return gp.Graph(off, dst[order].astype(np.int32), vw, np.concatenate([weight, weight])[order].astype(np.uint32)), labels
+
+
 @contextlib.contextmanager
 def launches_of(ctx, kernel):
     """A list that holds, after the block, how often kernels of this name were started by the context's calls in it."""

@@ -7,7 +7,7 @@ one block up to 49,152 targets, a segment of targets at a time above.
 import numpy as np
 import pytest
 
-from graphs import hubs_and_leaves, random_graph, symmetric
+from graphs import hubs_and_leaves, launches_of, random_graph, symmetric
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +57,33 @@ def test_isolated_and_empty(gp, ctx, oracle):
     rng = np.random.default_rng(5)
     u, v = rng.integers(0, 700, 1500), rng.integers(0, 700, 1500)
     check(gp, ctx, oracle, symmetric(gp, 6000, u, v), 4)
+
+
+@pytest.mark.parametrize("build,taken,absent", [
+    (lambda gp: random_graph(gp, 65536, 6, 6, 4, 3), ["k_match_choose<1>", "k_sort_rows_short"], ["k_dense_rows"]),
+    (lambda gp: random_graph(gp, 65536, 12, 12, 4, 3), ["k_match_choose<8>"], ["k_match_choose<32>"]),
+    (lambda gp: random_graph(gp, 70001, 40, 40, 4, 3), ["k_match_choose<32>"], ["k_match_choose<8>"]),
+    (lambda gp: hubs_and_leaves(gp, 2600, 3, 2600), ["k_order_block<false>", "k_order_block<true>"],
+     ["k_ordered_accept", "k_pair_flags"]),
+    (lambda gp: hubs_and_leaves(gp, 40000, 300, 40000), ["k_order_block<false>", "k_ordered_accept", "k_pair_flags"], []),
+    (lambda gp: hubs_and_leaves(gp, 60000, 5, 60000, 3), ["k_dense_rows"], ["k_dense_pieces", "k_large_records"]),
+    (lambda gp: hubs_and_leaves(gp, 450000, 9, 450000, 3), ["k_dense_rows", "k_dense_pieces", "k_dense_copy"],
+     ["k_large_records"])])
+def test_the_named_kernels_run(gp, ctx, build, taken, absent):
+    g = build(gp)
+    for kernel in taken + absent:
+        with launches_of(ctx, kernel) as started:
+            ctx.partition(g, 6, 1.05, 1)
+        assert (started[0] > 0) == (kernel in taken), kernel
+
+
+def test_long_rows_with_zero_weights_are_sorted(gp, ctx, oracle):
+    """A counter cannot tell a target of weight zero from an absent one: the sorts take such levels' long rows."""
+    g = hubs_and_leaves(gp, 60000, 5, 60000, 3)
+    g = gp.Graph(g.offsets, g.neighbors, g.vertex_weights, g.edge_weights - 1)
+    assert (g.edge_weights == 0).any()
+    check(gp, ctx, oracle, g, 4, 2)
+    for kernel in ("k_large_records", "k_dense_rows"):
+        with launches_of(ctx, kernel) as started:
+            ctx.partition(g, 4, 1.05, 2)
+        assert (started[0] > 0) == (kernel == "k_large_records")

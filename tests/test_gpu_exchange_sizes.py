@@ -1,8 +1,11 @@
-"""The capacity exchange with lists on both sides of what one block sorts (4096), against the oracle."""
+"""The capacity exchange, whose lists one block per part sorts, against the oracle.
+
+A part's lists hold at most 2048 fragments and 4608 moves; the oracle says how long the longest were.
+"""
 import numpy as np
 import pytest
 
-from graphs import hubs_and_leaves, random_graph
+from graphs import hubs_and_leaves, random_graph, stuck_pairs
 from test_gpu_cluster_levels import mixed
 from test_gpu_repair_sizes import check
 
@@ -20,3 +23,11 @@ def test_exchange(gp, ctx, oracle, n, degree, k, weighted):
 def test_exchange_with_hubs(gp, ctx, oracle):
     g = hubs_and_leaves(gp, 30000, 60, 2, 4)
     check(gp, ctx, oracle, g, mixed(g.n, 24, 0.1, 5), 24, 1.05, 2)
+
+
+@pytest.mark.parametrize("n,k,lights,slack", [(20000, 2, 1, 2), (20000, 2, 5, 0), (40000, 32, 1, 3), (40000, 32, 50, 8)])
+def test_lists_at_their_bounds(gp, ctx, oracle, n, k, lights, slack):
+    g, start = stuck_pairs(gp, n, k, lights, 1)
+    check(gp, ctx, oracle, g, start, k, 1 + slack * k / int(g.vertex_weights.sum()) + 1e-9, 1)
+    fragments, moves = oracle.exchange_lists()
+    assert fragments == 2048 and moves > 2048

@@ -7,7 +7,7 @@ in few gain classes, make lists on both sides; the oracle says what the labels a
 import numpy as np
 import pytest
 
-from graphs import random_graph
+from graphs import launches_of, random_graph
 
 pytestmark = pytest.mark.gpu
 FIELDS = ("rounds", "admission_iterations", "checkpoint_updates", "proposals", "accepted", "initial_cut", "final_cut",
@@ -56,3 +56,30 @@ def test_tickets_over_parts_that_fit(gp, ctx, oracle, n, degree, k, vw_max, eps)
     """Donors without a neighbour elsewhere, many heavier than the room of some or of all parts."""
     g = random_graph(gp, n, degree, n + k, 3, vw_max)
     check(gp, ctx, oracle, g, overloaded(n, k, n // 5, k), k, eps, 6)
+
+
+@pytest.mark.parametrize("n,degree,k,extra,weighted,short,long", [
+    (90000, 5, 40, 700, False, True, True), (90000, 5, 40, 700, True, True, False),
+    (40000, 8, 128, 12000, False, False, True), (40000, 0, 16, 9000, False, False, True)])
+def test_both_paths_are_taken(gp, ctx, n, degree, k, extra, weighted, short, long):
+    """Iterations whose list one block places and iterations whose list goes through the device-wide path."""
+    g = random_graph(gp, n, degree, n + extra, 9 if weighted else 0, 5 if weighted else 0)
+    start = overloaded(n, k, extra, k)
+    took = {}
+    for kernel in ("k_repair_block", "k_repair_active", "k_repair_bounds"):
+        with launches_of(ctx, kernel) as started:
+            ctx.refine(g, start, k, 1.10 if weighted else 1.05, 6, 2)
+        took[kernel] = started[0]
+    assert (took["k_repair_active"] > 0) == long
+    assert (took["k_repair_bounds"] > took["k_repair_active"]) == short  # one launch an iteration
+    assert took["k_repair_block"] > 0  # offered the first list whatever its length
+
+
+def test_both_paths_without_a_cache(gp, ctx):
+    g = gp.mesh3d(50, 45, 41, weighted=True, seed=3)
+    for extra, long in ((300, False), (20000, True)):
+        with launches_of(ctx, "k_repair_dest_od") as iterations:
+            ctx.refine(g, overloaded(g.n, 100, extra, 1), 100, 1.05, 4, 2)
+        with launches_of(ctx, "k_repair_active") as long_lists:
+            ctx.refine(g, overloaded(g.n, 100, extra, 1), 100, 1.05, 4, 2)
+        assert (long_lists[0] > 0) == long and iterations[0] > long_lists[0]
