@@ -1265,8 +1265,8 @@ __device__ void warp_radix_row(int begin, int degree, int* keys_io, u32* w_io, i
 // Rows of up to kShortRow raw entries, one entry per lane of a group of that
 // many, two rows to a warp: the same network and run reduction as the warp's,
 // ten steps instead of fifteen and no idle half.  Mesh levels consist of such
-// rows: sorted by a warp each they took 10.1 ms of the 189 ms partition of the
-// 256^3 mesh at k = 128; with this and the matching's lanes it takes 172-181.
+// rows: over a partition of the 256^3 mesh at k = 128 all rows of up to 128
+// entries took 10.1 ms a warp each; now these take 2.8 and the longer ones 3.7.
 __global__ void __launch_bounds__(256) k_sort_rows_short(i64 count, const int* rows, const int* raw_off, int* raw_t,
                                                          u32* raw_w, int* ucount) {
     after_previous();
@@ -1464,8 +1464,9 @@ __global__ void __launch_bounds__(Threads, 1024 / Threads) k_sort_rows_big(const
 // bits (a counter is then zero exactly when its target is absent).  The row is
 // read once per segment, mostly from L2, so this pays while there are few
 // segments: 4 bytes an entry and segment against 96 for the global sort's four
-// passes.  R-MAT scale 22 at k = 64 went from 124.3 to
-// 118 ms.
+// passes.  A partition of R-MAT scale 22 at k = 64 takes 6 ms less than with
+// the sorts.  Half of the issue slots and 3% of the memory rate are used (R-MAT
+// scale 20): a block counts, then scans, its counters with half of the SM's warps.
 constexpr int kDenseThreads = 1024;
 constexpr int kDenseSegment = 49152;      // u32 counters: 192 KB
 constexpr int kDenseSegments = 16;        // more: the global sort

@@ -58,16 +58,17 @@ __device__ __forceinline__ i64 entries_within(const int* off, i64 n, i64 first, 
 }
 
 // Pass 1.  Loads: every thread takes four vertices at a time, 32 apart, and
-// adds neighbouring ones of equal labels once, a warp of one label once.  Cut: every warp
-// takes an equal share of the work over rows and entries, so neither a
-// hub row nor a stretch of short rows falls to one warp; it reads 256 entries
+// adds neighbouring ones of equal labels once, a warp of one label once.  Cut:
+// every warp takes an equal share of the work over rows and entries, so neither
+// a hub row nor a stretch of short rows falls to one warp; it reads 256 entries
 // a step, eight gathers per lane in flight, next to the ends and labels of the
 // next 32 rows, and finds each entry's row from the marks that non-empty rows
-// leave at their first entry.  Bound by the label gathers, served by L2.
-// R-MAT scale 22, k = 64 (124 M entries): 0.59 ms with the reduction; a warp per
-// row took 6.60 ms, its longest row alone setting the time, and shares of equal
-// rows plus entries 1.14, half of the SMs' time idle at the end.  (Labels packed
-// into bytes first gained nothing.)
+// leave at their first entry.  Bound by the label gathers: L1 works at 77% of
+// its rate, L2 at 48%, DRAM at 12% (R-MAT scale 21).  R-MAT scale 22, k = 64
+// (124 M entries): 0.59 ms with the reduction; a warp per row took 6.60 ms, its
+// longest row alone setting the time, and shares of equal rows plus entries
+// 1.14, half of the SMs' time idle at the end.  (Labels packed into bytes first
+// gained nothing.)
 // Every access is range-checked, so a malformed labelling or CSR cannot reach
 // memory outside the caller's arrays or the block's shared tables.
 __global__ void __launch_bounds__(kEvalThreads, 5) k_eval_partials(i64 n, i64 m, const int* off, const int* nbr,
@@ -216,8 +217,8 @@ __global__ void __launch_bounds__(kEvalThreads, 5) k_eval_partials(i64 n, i64 m,
 }
 
 // Pass 2: sums the partials of all blocks, a warp per value.  (One thread per
-// value walked the 592 blocks' partials one after another: most of the 61 us
-// that judging a 256x256 grid took; 23 us now.)  With any invalid
+// value walked the 592 blocks' partials one after another: most of the 61 us that
+// judging a 256x256 grid took; it takes 22.)  With any invalid
 // entry the cut output is UINT64_MAX (no real cut reaches it) and, when
 // `invalid` is given, the count is stored there.
 __global__ void __launch_bounds__(1024) k_eval_reduce(int blocks, int k, const u64* partial, u64* cut_out,

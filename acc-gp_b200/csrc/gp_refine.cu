@@ -1,10 +1,12 @@
 // Projection and refinement on the B200 (Acc-GPart src/refine.cu,
 // src/refinement/*.cuh): dense affinity cache, label propagation with the
 // priority filter, exact cut/cache updates, capacity repair and the
-// capacity-complementary exchange.  One host loop per level with one small
-// read-back per LP round; every decision is a pure function of the state, so
-// the result does not depend on thread scheduling.  The repair ranks donors
-// and receiver tickets in the deterministic (bucket, repair hash, id) order.
+// capacity-complementary exchange.  A host loop per level reads back once per
+// LP round and repair iteration; small levels of short rows run theirs in one
+// launch of a thread-block cluster (gp_refine_cluster.cuh).  Every decision is
+// a pure function of the state, so the result does not depend on thread
+// scheduling.  The repair ranks donors and receiver tickets in the
+// deterministic (bucket, repair hash, id) order.
 #include "gp_graph.h"
 #include "gp_primitives.cuh"
 
@@ -1157,9 +1159,9 @@ __device__ __forceinline__ u64 saturating_add(u64 a, u64 b) { return ~0ULL - a <
 // block per rank c of the parts by room (descending) writes the prefix sums,
 // in part order, of the rooms of at least the c-th largest (saturating), and
 // rooms[c]; a ticket is then two binary searches (ticket_part) instead of two
-// walks over all parts, which with seven threads in 32 active bounded the
-// destination kernels: a 256^3 mesh at k = 128 went from 147-154 to 126 ms
-// (device time 139 to 113 ms, k_repair_dest_od to 6.4 ms of it).
+// walks over all parts, in which seven threads of 32 were active and which
+// bounded the destination kernels (26 ms of a partition of the 256^3 mesh at
+// k = 128, whose k_repair_dest_od takes 6.4 ms since).
 // Block 0 also clears the iteration's three counts (placed donors, donors,
 // listed donors).
 __global__ void __launch_bounds__(kMaxParts) k_slack(int k, const u64* loads, u64 capacity, u64* slack, u64* requests,
@@ -1247,9 +1249,9 @@ __device__ __forceinline__ void load_affinities(const C* p, C (&val)[N]) {
 // A warp takes 32 consecutive vertices: its lanes find the donors among them
 // (vertices of overloaded parts), W lanes scan the row of each donor that has a
 // connection elsewhere, and the lanes finish their own donors (the rest is
-// 64-bit arithmetic, which W - 1 lanes would wait for: a 256^3 mesh at k = 128
-// went from 126 to 118.6 ms without their waiting).  The parts' free room is
-// staged per block.  A part p is a feasible destination for
+// 64-bit arithmetic, which W - 1 lanes would wait for: 7 ms of a partition of
+// the 256^3 mesh at k = 128).  The parts' free room is staged per block.  Half
+// of the issue slots are used and a tenth of the memory rate (128^3 mesh).  A part p is a feasible destination for
 // weight w when w <= room[p] (room = C - load for parts under capacity, else
 // 0; vertex weights are positive).  Every donor's weight is added to its
 // class of its part in `hist` (kBalanceWidth per part), from which
@@ -1260,8 +1262,7 @@ __device__ __forceinline__ void load_affinities(const C* p, C (&val)[N]) {
 // in sequence, and no array in repair order has to exist.  On the 256^3 mesh
 // at k = 128 (100 M donors over 32 iterations at the finest level) reading the
 // destinations in hashed order took 37 ms and ordering the donors by class
-// with a radix sort about 20 ms more; a partition went from 202 to 189 ms, one
-// of a 256x256 grid at k = 8 from 20.1 to 16.0 ms.
+// with a radix sort about 20 ms more.
 template <class C, int W, bool Vectorized>
 __global__ void __launch_bounds__(kThreads) k_repair_dest(i64 n, const C* A, const C* totals, const int* labels,
                                                           const u32* vw, int k, const u64* loads, u64 capacity,
@@ -1761,7 +1762,7 @@ __global__ void k_repair_active(i64 count, const int* want, const u32* items, co
 }
 
 // The remaining attempts of a receiver reservation by one block, for a small
-// set of open donors: the choice of k_choose and the ticket rule of k_admit,
+// set of open donors: the choice of k_choose and the ticket rule of k_admit_tiles,
 // attempt after attempt, without a round trip to the host.  open[j] (j <
 // *count, ascending) indexes the active donors, so the requests of one target
 // are admitted in repair order exactly as the device-wide path does.
@@ -2088,10 +2089,10 @@ __global__ void __launch_bounds__(kAttemptThreads) k_attempts(const u32* open, c
 // the donor test; the active donors are left in `donor`, their number returned.
 // The order: a word's leading bits, the hash's, name one of kAttemptCap buckets,
 // so a bucket holds about one word, and a word's place is its bucket's start
-// and the smaller words of the bucket.  That takes seven barriers, where a
-// bitonic network takes 66 for 2048 words (a 256^3 mesh at k = 128 with 143
-// such lists went from 118.6 to 115.1 ms).  sm.slack, sm.requests and, as each
-// part's weight before its bounding class, sm.base are set by the caller.
+// and the smaller words of the bucket.  That takes nine barriers (three of them
+// in the scan), where a bitonic network takes 66 for 2048 words: 24 us less a
+// list (143 lists of a 256^3 mesh at k = 128).  sm.slack, sm.requests and, as
+// each part's weight before its bounding class, sm.base are set by the caller.
 constexpr int kBucketShift = 53;
 static_assert(kAttemptCap == 1 << (64 - kBucketShift), "a bucket per leading value");
 template <class C, int Threads>
@@ -2820,9 +2821,9 @@ __global__ void __launch_bounds__(kPartSortThreads) k_sort_moves(int k, const Jo
 // vertices does not leave one warp with the whole row.  A chunk of the work
 // list: move << 32 | vertex slot << 28 | chunk.
 constexpr int kEventChunk = 256;
-// A move keeps its vertices only if every claim is its own; then it owns them
-// (k_resolve, k_mark), its events start at 0 and its rows' chunks join the
-// work list.  A block per part.
+// A move keeps its vertices only if every claim is its own; then it owns them,
+// its events start at 0 and its rows' chunks join the work list.  A block per
+// part.
 __global__ void __launch_bounds__(kThreads) k_settle(int k, JointMove* moves, JointCounts* counts,
                                                      const JointParts* parts, const int* off, const int* labels,
                                                      const int* claims, int* owners, int* targets, u64* events,
